@@ -50,7 +50,7 @@ class GemmArgs(C.Structure):
 
 
 EPI_BIAS, EPI_GELU, EPI_STORE_PRE, EPI_RESIDUAL, EPI_DGELU_MUL = 1, 2, 4, 8, 16
-EPI_ACCUM, EPI_OUT_FP32, EPI_SWIGLU, EPI_DSWIGLU = 32, 64, 128, 256
+EPI_ACCUM, EPI_OUT_FP32, EPI_SWIGLU, EPI_DSWIGLU, EPI_B_STATIC = 32, 64, 128, 256, 512
 
 STATUS_NAMES = {
     1: "wait for a free shared-memory stage expired",

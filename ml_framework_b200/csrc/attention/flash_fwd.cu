@@ -109,6 +109,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_trigger();
+  pdl_wait();
   const uint32_t tS = tmem_base;         // + 64 * buffer
   const uint32_t tPV = tmem_base + 128;
 
@@ -351,8 +353,7 @@ MLF_API int mlf_flash_fwd(const void* q, const void* k, const void* v, void* out
     attr_set[dev & 63] = true;
   }
   dim3 grid((S + FA_BQ - 1) / FA_BQ, Hq, B);
-  flash_fwd_kernel<<<grid, FA_THREADS, FA_SMEM, st>>>(tq, tk, tv, p);
+  MLF_CHECK_CUDA(launch_pdl(flash_fwd_kernel, grid, dim3(FA_THREADS), FA_SMEM, st, tq, tk, tv, p));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

@@ -130,6 +130,8 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_trigger();
+  pdl_wait();
   auto tS = [&](int t) { return tmem_base + 128u * t; };
   auto tO = [&](int t) { return tmem_base + 256u + 128u * t; };
 
@@ -426,9 +428,8 @@ MLF_API int mlf_flash_fwd_prefix(const void* q, const void* k, const void* v, vo
     attr_set[dev & 63] = true;
   }
   dim3 grid(((S + 2 * W_BQ - 1) / (2 * W_BQ)) * Hq * B);
-  flash_fwd_ws_kernel<<<grid, W_THREADS, W_SMEM, st>>>(tq, tk, tv, p);
+  MLF_CHECK_CUDA(launch_pdl(flash_fwd_ws_kernel, grid, dim3(W_THREADS), W_SMEM, st, tq, tk, tv, p));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -473,9 +474,8 @@ MLF_API int mlf_flash_fwd_paged(const void* q, const void* cache, const int* blo
     attr_set[dev & 63] = true;
   }
   dim3 grid(((Sq + 2 * W_BQ - 1) / (2 * W_BQ)) * Hq * B);
-  flash_fwd_ws_kernel<<<grid, W_THREADS, W_SMEM, st>>>(tq, tkv, tkv, p);
+  MLF_CHECK_CUDA(launch_pdl(flash_fwd_ws_kernel, grid, dim3(W_THREADS), W_SMEM, st, tq, tkv, tkv, p));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 

@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(P_THREADS)
 paged_decode_kernel(const PagedDecodeParams p) {
   extern __shared__ __align__(128) uint8_t p_dsm[];
   const int b = blockIdx.x, hkv = blockIdx.y, sp = blockIdx.z;
+  pdl_trigger();
+  pdl_wait();
   // A length beyond what the row of the block table can describe would index past the table: it is
   // clamped to the table's capacity and reported, like every other rejected index in this file.
   int len = p.seq_lens[b];
@@ -297,6 +299,8 @@ paged_decode_kernel(const PagedDecodeParams p) {
 // Merge the per-split partial results: out = sum_s exp2(m_s - M) o_s / sum_s exp2(m_s - M) l_s.
 __global__ void __launch_bounds__(128)
 paged_decode_merge_kernel(const float* ws, __nv_bfloat16* out, int B, int Hq, int Hkv, int G, int splits) {
+  pdl_trigger();
+  pdl_wait();
   const int bh = blockIdx.x;      // b * Hq + h
   const int b = bh / Hq, h = bh % Hq;
   const int hkv = h / G, g = h % G;
@@ -346,6 +350,8 @@ rope_kv_write_kernel(__nv_bfloat16* qkv, long long ld, const long long* pos, con
   const int heads = Hq + 2 * Hkv;
   const long long total = T * heads * 16;                    // 16 threads per head: 4 + 4 elements each
   const float log_theta = __logf(theta);
+  pdl_trigger();
+  pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int d = (int)(i & 15) * 4;                         // 0..60: pairs (d, d + 64)
     const long long th = i >> 4;
@@ -410,6 +416,8 @@ kv_gather_kernel(const __nv_bfloat16* cache, const int* block_table, int len, in
 constexpr int AM_THREADS = 1024;
 __global__ void __launch_bounds__(AM_THREADS)
 argmax_rows_kernel(const __nv_bfloat16* logits, long long ld, int vocab, long long* out, int vec) {
+  pdl_trigger();
+  pdl_wait();
   const long long r = blockIdx.x;
   const __nv_bfloat16* row = logits + r * ld;
   float best = -INFINITY;
@@ -506,18 +514,13 @@ MLF_API int mlf_paged_decode_ld(const void* q, long long ldq, const void* cache,
     MLF_CHECK_CUDA(cudaFuncSetAttribute(paged_decode_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
     attr_set[dev & 63] = true;
   }
-  switch (G) {
-    case 1: paged_decode_kernel<1><<<grid, P_THREADS, P_SMEM, st>>>(p); break;
-    case 2: paged_decode_kernel<2><<<grid, P_THREADS, P_SMEM, st>>>(p); break;
-    case 4: paged_decode_kernel<4><<<grid, P_THREADS, P_SMEM, st>>>(p); break;
-    default: paged_decode_kernel<8><<<grid, P_THREADS, P_SMEM, st>>>(p); break;
-  }
+  const auto kernel = G == 1 ? paged_decode_kernel<1> : G == 2 ? paged_decode_kernel<2> : G == 4 ? paged_decode_kernel<4> : paged_decode_kernel<8>;
+  MLF_CHECK_CUDA(launch_pdl(kernel, grid, dim3(P_THREADS), P_SMEM, st, p));
   count_launch();
   if (splits > 1 && p.counters == nullptr) {
-    paged_decode_merge_kernel<<<B * Hq, 128, 0, st>>>(ws, p.out, B, Hq, Hkv, G, splits);
+    MLF_CHECK_CUDA(launch_pdl(paged_decode_merge_kernel, dim3(B * Hq), dim3(128), 0, st, (const float*)ws, p.out, B, Hq, Hkv, G, splits));
     count_launch();
   }
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -542,11 +545,10 @@ MLF_API int mlf_rope_kv_write(void* qkv, long long ld, const long long* pos, con
   long long g = (T * (Hq + 2 * Hkv) * 16 + 255) / 256;
   const long long cap = (long long)sm_count() * 8;
   if (g > cap) g = cap;
-  rope_kv_write_kernel<<<(int)g, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(qkv), ld, pos, slots, static_cast<__nv_bfloat16*>(cache), T, Hq, Hkv, block_size, num_blocks, theta,
-      device_status_word());
+  MLF_CHECK_CUDA(launch_pdl(rope_kv_write_kernel, dim3((unsigned)g), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
+                            static_cast<__nv_bfloat16*>(qkv), ld, pos, slots, static_cast<__nv_bfloat16*>(cache), T, Hq, Hkv, block_size,
+                            num_blocks, theta, device_status_word()));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -569,9 +571,8 @@ MLF_API int mlf_kv_gather(const void* cache, const int* block_table, int table_l
 MLF_API int mlf_argmax_rows(const void* logits, long long rows, long long ld, int vocab, long long* out, uint64_t stream) {
   if (rows <= 0) return 0;
   const int vec = (ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) ? 1 : 0;
-  argmax_rows_kernel<<<(int)rows, AM_THREADS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(logits), ld,
-                                                                                          vocab, out, vec);
+  MLF_CHECK_CUDA(launch_pdl(argmax_rows_kernel, dim3((unsigned)rows), dim3(AM_THREADS), 0, reinterpret_cast<cudaStream_t>(stream),
+                            static_cast<const __nv_bfloat16*>(logits), ld, vocab, out, vec));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

@@ -199,6 +199,18 @@ __device__ __forceinline__ void tma_store_wait_all() {
 }
 
 // ---------------------------------------------------------------------------------
+// programmatic dependent launch
+// ---------------------------------------------------------------------------------
+// A kernel started with launch_pdl() may become resident while the kernel before it on the stream is still running.
+// pdl_wait() returns once every earlier kernel has completed and its writes are visible: no thread touches global
+// memory that an earlier kernel writes, or that one still reads, before it, and nothing that an earlier kernel may
+// write is read through the non-coherent path (no const __restrict__, no __ldg). pdl_trigger() lets the next kernel of the
+// stream become resident; a kernel that allocates tensor memory calls it only AFTER its allocation (the next kernel
+// could otherwise take the tensor memory this one still needs and wait for this one's end).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------
 // tcgen05: TMEM management
 // ---------------------------------------------------------------------------------
 // One full warp calls these. ncols is a power of two in [32, 512].

@@ -24,6 +24,7 @@ struct GemmKernelParams {
   long long ldo, ld_aux_in, ld_aux_out;
   int tiles_m, tiles_n;
   int rot_m, rot_n;  // tile-order rotation (tiles), so locally owned rows come first
+  int b_static;      // operand B may be read before the kernels ahead on the stream have finished
   int* err;
   // gather
   int gather_operand, world, rank, n_copy_ctas, rows_per_rank, flag_rows, row_bytes, total_rows;

@@ -18,6 +18,11 @@
 // Warp roles as in the other tcgen05 GEMMs: warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2..5
 // epilogue; two accumulators so that a run's epilogue overlaps the next run's products. Every wait is bounded.
 //
+// In a decode step the products alternate with kernels of 2 - 5 us, so the launch, the set-up and the first loads of a
+// product count: it is launched with programmatic overlap and starts on its weight early (kPace below). Together with
+// the clearing of the outputs inside the normalisation's launch (six-layer decode step of the Llama-8B shape, CUDA-graph
+// replay): 1 row 692 -> 615 us, 13 rows 841 -> 755 us, 64 rows 878 -> 794 us.
+//
 // Reference behaviour covered: the per-token projections of the decode phase
 // (src/MLFramework/Inference/PagedAttention/Phases/DecodeOrchestrator.cs:28-66 drives one token per sequence through
 // the model's linear layers, Linear.Forward src/MLFramework/Modules/Linear.cs:81).
@@ -30,6 +35,12 @@ int cached_tmap_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_
 
 constexpr int FR_WT = 128;                         // weight rows per tile (MMA M)
 constexpr int FR_STAGE_W = FR_WT * BK * 2;         // 16 KB
+// Clocks between the weight tiles that a CTA requests while the kernels ahead still run: 16 KB x 148 SMs per 700 clocks
+// is the rate HBM delivers. Requested in one burst, the ring's 19 MB queue up in front of the few loads of the short
+// kernel that is running (RMSNorm, SwiGLU, ...) and delay it by what they gain: a six-layer decode step of one row took
+// 666 us with the burst, 652 us without any early load, 615 us with this pace (400 - 1000 clocks: 616 - 627 us). Bringing
+// further tiles into L2 was slower at every pace (627 - 692 us).
+constexpr int kPace = 700;
 
 template <int BT>
 struct FewRowCfg {
@@ -45,6 +56,7 @@ struct FewRowParams {
   int M, N, K;
   int num_kb;            // k blocks per weight tile
   long long units;       // weight tiles x k blocks
+  int w_static;          // the weight may be read before the kernels ahead on the stream have finished
   int* err;
 };
 
@@ -107,13 +119,29 @@ gemm_fewrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   // this CTA's run of (tile, k block) units
   const long long u_begin = p.units * (long long)blockIdx.x / gridDim.x;
   const long long u_end = p.units * (long long)(blockIdx.x + 1) / gridDim.x;
+  pdl_trigger();                                 // tensor memory is allocated: the next kernel may become resident
 
   if (warp == 0) {
     // ===================== TMA producer =====================
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 0;
-      for (long long u = u_begin; u < u_end; ++u) {
+      // A weight that nobody writes starts streaming while the kernels ahead are still running: the ring is filled
+      // with weight tiles here, the MMA thread adds the token rows of these stages once the kernels ahead are done.
+      long long u_first = u_begin;
+      if (p.w_static) {
+        const long long t0 = clock64();
+        int n = 0;
+        for (; u_first < u_end && n < kStages; ++u_first, ++n) {
+          const int tile = (int)(u_first / p.num_kb);
+          while (clock64() - t0 < (long long)n * kPace) {}
+          mbar_expect_tx(full_bar(n), Cfg::kStage);
+          tma_load_2d(smem_base + n * Cfg::kStage, &tmW, (int)(u_first - (long long)tile * p.num_kb) * BK, tile * FR_WT, full_bar(n));
+        }
+        if (n == kStages) ph = 1u;               // a run shorter than the ring leaves nothing for the loop below
+      }
+      pdl_wait();
+      for (long long u = u_first; u < u_end; ++u) {
         const int tile = (int)(u / p.num_kb);
         const int kb = (int)(u - (long long)tile * p.num_kb);
         if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.err, ERR_WAIT_SMEM_EMPTY)) break;
@@ -131,6 +159,13 @@ gemm_fewrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     // ===================== MMA issuer =====================
     if (lane == 0) {
       const uint32_t idesc = make_idesc_bf16(FR_WT, BT, 0, 0);
+      pdl_wait();
+      if (p.w_static) {
+        for (long long u = u_begin; u < u_end && u - u_begin < kStages; ++u) {
+          const int i = (int)(u - u_begin);
+          tma_load_2d(smem_base + i * Cfg::kStage + FR_STAGE_W, &tmX, (int)(u % p.num_kb) * BK, 0, full_bar(i));
+        }
+      }
       int s = 0;
       uint32_t ph = 0;
       int it = 0;
@@ -172,6 +207,7 @@ gemm_fewrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
   } else {
     // ===================== epilogue (warps 2..5) =====================
+    pdl_wait();                                   // `out` may be in use by earlier kernels until here
     const int q = warp & 3;                       // TMEM lane quarter this warp may read
     const int n_loc = q * 32 + lane;              // weight row of this thread inside the tile
     const int half = n_loc >> 6;                  // staging box (64 output columns each)
@@ -254,19 +290,14 @@ static int launch_fewrow(const CUtensorMap& tmW, const CUtensorMap& tmX, const C
     MLF_CHECK_CUDA(cudaFuncSetAttribute(gemm_fewrow_kernel<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
     attr_set[dev & 63] = true;
   }
-  gemm_fewrow_kernel<BT><<<ctas, kGemmThreads, Cfg::kSmemBytes, st>>>(tmW, tmX, tmOut, p);
+  MLF_CHECK_CUDA(launch_pdl(gemm_fewrow_kernel<BT>, dim3(ctas), dim3(kGemmThreads), Cfg::kSmemBytes, st, tmW, tmX, tmOut, p));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
-}  // namespace mlf
-
-using namespace mlf;
-
 // Returns -4 when the shape or the alignment is not one this route handles (the caller falls back).
-MLF_API int mlf_gemm_fewrow(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo,
-                            int accumulate, int max_ctas, uint64_t stream) {
+int gemm_fewrow(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo,
+                int accumulate, int max_ctas, int w_static, uint64_t stream) {
   if (M < 1 || M > 128 || N < 128 || K < 64) return -4;
   if (ldx % 8 || ldw % 8 || ldo % 8 || K % 8) return -4;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15) return -4;
@@ -275,6 +306,7 @@ MLF_API int mlf_gemm_fewrow(const void* x, const void* w, void* out, int M, int 
   FewRowParams p;
   p.M = M; p.N = N; p.K = K;
   p.num_kb = (K + BK - 1) / BK;
+  p.w_static = w_static;
   const int tiles = (N + FR_WT - 1) / FR_WT;
   p.units = (long long)tiles * p.num_kb;
   p.err = device_status_word();
@@ -295,4 +327,13 @@ MLF_API int mlf_gemm_fewrow(const void* x, const void* w, void* out, int M, int 
   if (BT == 32) return launch_fewrow<32>(tmW, tmX, tmOut, p, ctas, st);
   if (BT == 64) return launch_fewrow<64>(tmW, tmX, tmOut, p, ctas, st);
   return launch_fewrow<128>(tmW, tmX, tmOut, p, ctas, st);
+}
+
+}  // namespace mlf
+
+using namespace mlf;
+
+MLF_API int mlf_gemm_fewrow(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo,
+                            int accumulate, int max_ctas, uint64_t stream) {
+  return gemm_fewrow(x, w, out, M, N, K, ldx, ldw, ldo, accumulate, max_ctas, 0, stream);
 }

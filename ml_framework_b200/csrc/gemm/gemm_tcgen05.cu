@@ -105,6 +105,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_trigger();
+  pdl_wait();
 
   const int num_tiles = p.tiles_m * p.tiles_n;
   const int num_kb = (p.K + BK - 1) / BK;
@@ -313,9 +315,13 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
                                         Cfg::kSmemBytes));
     attr_set[dev & 63] = true;
   }
-  gemm_tcgen05_kernel<BN><<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(tmA, tmB, p);
+  if (p.n_copy_ctas == 0 && !p.scatter_out) {
+    MLF_CHECK_CUDA(launch_pdl(gemm_tcgen05_kernel<BN>, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, st, tmA, tmB, p));
+  } else {                                       // copy CTAs and routed rows touch peers' memory: after everything ahead
+    gemm_tcgen05_kernel<BN><<<grid, kGemmThreads, Cfg::kSmemBytes, st>>>(tmA, tmB, p);
+    MLF_CHECK_CUDA(cudaGetLastError());
+  }
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -333,24 +339,26 @@ static int g_small_m_split = 1;
 // Routes plain GEMMs with M <= 256 and a large weight to the split-K CTA-pair kernel.
 MLF_API void mlf_set_gemm_small_m_split(int on) { g_small_m_split = on; }
 
-MLF_API int mlf_gemm_fewrow(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo,
-                            int accumulate, int max_ctas, uint64_t stream);
+namespace mlf {
+int gemm_fewrow(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo,
+                int accumulate, int max_ctas, int w_static, uint64_t stream);
+}
 static int g_fewrow = 1;
 // Routes plain products with at most 128 rows against a K-major weight to the weight-as-M stream-K kernel.
 MLF_API void mlf_set_gemm_fewrow(int on) { g_fewrow = on; }
 
 MLF_API int mlf_gemm_bf16(const MlfGemmArgs* a, uint64_t stream) {
   MLF_REQUIRE(a != nullptr, "null args");
-  if (g_fewrow && a->tile_n == 0 && a->comm == nullptr && (a->flags & ~MLF_EPI_ACCUM) == 0 && !a->a_mn && !a->b_mn && a->M <= 128 &&
+  if (g_fewrow && a->tile_n == 0 && a->comm == nullptr && (a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) == 0 && !a->a_mn && !a->b_mn && a->M <= 128 &&
       a->N >= 1024 && a->K >= 512 && a->alpha == 1.0f) {
-    const int rcf = mlf_gemm_fewrow(a->a, a->b, a->out, a->M, a->N, a->K, a->lda, a->ldb, a->ldo, (a->flags & MLF_EPI_ACCUM) ? 1 : 0,
-                                    a->max_ctas, stream);
+    const int rcf = gemm_fewrow(a->a, a->b, a->out, a->M, a->N, a->K, a->lda, a->ldb, a->ldo, (a->flags & MLF_EPI_ACCUM) ? 1 : 0,
+                                a->max_ctas, (a->flags & MLF_EPI_B_STATIC) ? 1 : 0, stream);
     if (rcf != -4) return rcf;
   }
   // CTA pairs for everything with at least 16 pair tiles (split-K fills the GPU when tiles alone cannot).
   // Few rows against a large weight (a decode step: M <= 256) is a weight-streaming problem: one row of
   // tiles cannot occupy the GPU, so the pair kernel splits K and every SM streams a slice of the weight.
-  const bool plain_out = (a->flags & ~MLF_EPI_ACCUM) == 0 && a->comm == nullptr;
+  const bool plain_out = (a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) == 0 && a->comm == nullptr;
   const bool small_m = g_small_m_split && a->tile_n == 0 && plain_out && a->M <= 256 && a->N >= 1024 && a->K >= 1024;
   if (a->tile_n == 512 || small_m ||
       (g_use_2cta && a->tile_n == 0 && a->M >= 512 && a->N >= 512 && (long long)((a->M + 255) / 256) * ((a->N + 255) / 256) >= 16)) {

@@ -158,6 +158,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   cluster_sync_all();                          // both CTAs' barriers are initialised before any remote arrive
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_trigger();                               // tensor memory is allocated: the next kernel may become resident
 
   const int pair = ((int)blockIdx.x - p.n_copy_ctas) >> 1;
   const int n_pairs = ((int)gridDim.x - p.n_copy_ctas) >> 1;
@@ -172,6 +173,27 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 0;
+      // A weight that nobody writes starts streaming while the kernels ahead are still running: the first pass over
+      // the ring gets its B halves here, its A halves after the wait.
+      int pre = 0;
+      if (p.b_static && pair < num_tiles) {
+        int tm, tn;
+        tile_coords(pair / k_splits, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);
+        const int kb0 = (pair % k_splits) * kb_per, kb1 = min(num_kb_all, kb0 + kb_per);
+        const int n0 = tn * T2_BN + (int)rank * T2_BNH;
+        for (; pre < T2_STAGES && kb0 + pre < kb1; ++pre) {
+          const uint32_t sb = smem_base + pre * T2_STAGE + T2_STAGE_A;
+          const uint32_t lead_full = mapa_u32(full_bar(pre), 0);
+          if (rank == 0) mbar_expect_tx(full_bar(pre), 2 * T2_STAGE);
+          if (!p.b_mn) {
+            tma_load_2d_pair(sb, &tmB, (kb0 + pre) * BK, n0, lead_full);
+          } else {
+#pragma unroll
+            for (int j = 0; j < T2_BNH / 64; ++j) tma_load_2d_pair(sb + j * (BK * 128), &tmB, n0 + 64 * j, (kb0 + pre) * BK, lead_full);
+          }
+        }
+      }
+      pdl_wait();
       for (int t = pair; t < num_tiles; t += n_pairs) {
         int tm, tn;
         tile_coords(t / k_splits, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);
@@ -190,11 +212,13 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           fence_proxy_async_all();
         }
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.err, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
+          const bool b_loaded = pre > 0;
+          if (b_loaded) --pre;
+          else if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.err, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
           const uint32_t sa = smem_base + s * T2_STAGE;
           const uint32_t sb = sa + T2_STAGE_A;
           const uint32_t lead_full = mapa_u32(full_bar(s), 0);
-          if (rank == 0) mbar_expect_tx(full_bar(s), 2 * T2_STAGE);
+          if (rank == 0 && !b_loaded) mbar_expect_tx(full_bar(s), 2 * T2_STAGE);
           const int k0 = kb * BK;
           if (!p.a_mn) {
             tma_load_2d_pair(sa, &tmA, k0, m0, lead_full);
@@ -202,7 +226,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * (BK * 128), &tmA, m0 + 64 * j, k0, lead_full);
           }
-          if (!p.b_mn) {
+          if (b_loaded) {
+          } else if (!p.b_mn) {
             tma_load_2d_pair(sb, &tmB, k0, n0, lead_full);
           } else {
 #pragma unroll
@@ -255,6 +280,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     }
   } else {
     // ===================== epilogue (warps 2..5 of both CTAs) =====================
+    pdl_wait();                                // `out` and aux_in may be in use by earlier kernels until here
     const int q = warp & 3;
     const bool out_fp32 = (p.flags & MLF_EPI_OUT_FP32) != 0;
     const bool swiglu = (p.flags & MLF_EPI_SWIGLU) != 0;
@@ -358,7 +384,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             if (nvalid == 64 && ((reinterpret_cast<uintptr_t>(p.bias + nb) & 15) == 0)) {
 #pragma unroll
               for (int c = 0; c < 8; ++c) {
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(p.bias + nb) + c);
+                const uint4 w = reinterpret_cast<const uint4*>(p.bias + nb)[c];
                 const float2 f0 = unpack_bf16x2(w.x), f1 = unpack_bf16x2(w.y), f2 = unpack_bf16x2(w.z), f3 = unpack_bf16x2(w.w);
                 v[8 * c + 0] += f0.x; v[8 * c + 1] += f0.y; v[8 * c + 2] += f1.x; v[8 * c + 3] += f1.y;
                 v[8 * c + 4] += f2.x; v[8 * c + 5] += f2.y; v[8 * c + 6] += f3.x; v[8 * c + 7] += f3.y;
@@ -459,7 +485,7 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   MLF_REQUIRE(a != nullptr, "null args");
   const MlfGemmComm* cm = a->comm;
   // fewer than 256 rows only as a plain product (optionally accumulated), where K is split over the pairs
-  if (a->N < 256 || (a->M < 256 && ((a->flags & ~MLF_EPI_ACCUM) != 0 || cm != nullptr))) return -4;
+  if (a->N < 256 || (a->M < 256 && ((a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) != 0 || cm != nullptr))) return -4;
   const bool gatherA = cm && cm->gather_operand == 1;
   const bool gatherB = cm && cm->gather_operand == 2;
   if (cm && cm->gather_operand && (cm->flag_rows <= 0 || cm->flag_rows % 128 != 0)) return -4;
@@ -470,6 +496,7 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   p.M = a->M; p.N = a->N; p.K = a->K;
   p.a_mn = a->a_mn ? 1 : 0; p.b_mn = a->b_mn ? 1 : 0;
   p.flags = a->flags; p.alpha = a->alpha;
+  p.b_static = (a->flags & MLF_EPI_B_STATIC) != 0 && cm == nullptr ? 1 : 0;
   p.out = a->out;
   p.bias = static_cast<const __nv_bfloat16*>(a->bias);
   p.aux_in = static_cast<const __nv_bfloat16*>(a->aux_in);
@@ -535,7 +562,7 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   memset(&peer_maps, 0, sizeof(peer_maps));
   int tma_epi = 0, tma_aux = 0;
   const bool scatter = cm && cm->scatter_out;
-  const bool plain = (a->flags & ~MLF_EPI_ACCUM) == 0 && cm == nullptr;      // nothing but (optionally) out += product
+  const bool plain = (a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) == 0 && cm == nullptr;      // nothing but (optionally) out += product
   if (!(a->flags & (MLF_EPI_OUT_FP32 | MLF_EPI_SWIGLU | MLF_EPI_DSWIGLU)) && (!(a->flags & MLF_EPI_ACCUM) || plain) && a->ldo % 8 == 0 &&
       (scatter || (reinterpret_cast<uintptr_t>(a->out) & 15) == 0) &&
       (!(a->flags & MLF_EPI_STORE_PRE) || (a->ld_aux_out % 8 == 0 && (reinterpret_cast<uintptr_t>(a->aux_out) & 15) == 0))) {
@@ -610,9 +637,14 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   if (pairs > max_clusters[dev & 63]) pairs = max_clusters[dev & 63];
   if (pairs > num_tiles * k_splits) pairs = num_tiles * k_splits;
   if (pairs < 1) pairs = 1;
-  gemm_tcgen05_2cta_kernel<<<n_copy + 2 * pairs, kGemmThreads, T2_SMEM, st>>>(tmA, tmB, tmOut, tmPre, tmAux, peer_maps, p, tma_epi, tma_aux,
-                                                                              k_splits, reduce_out);
+  if (cm == nullptr) {
+    MLF_CHECK_CUDA(launch_pdl(gemm_tcgen05_2cta_kernel, dim3(2 * pairs), dim3(kGemmThreads), T2_SMEM, st, tmA, tmB, tmOut, tmPre, tmAux,
+                              peer_maps, p, tma_epi, tma_aux, k_splits, reduce_out));
+  } else {                                       // copy CTAs and routed rows touch peers' memory: after everything ahead
+    gemm_tcgen05_2cta_kernel<<<n_copy + 2 * pairs, kGemmThreads, T2_SMEM, st>>>(tmA, tmB, tmOut, tmPre, tmAux, peer_maps, p, tma_epi, tma_aux,
+                                                                                k_splits, reduce_out);
+    MLF_CHECK_CUDA(cudaGetLastError());
+  }
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

@@ -178,6 +178,8 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(__nv_bfloat16* dx, const 
 // or interleaved (gate, up) pairs when `interleaved` != 0. out[r, F] = silu(gate) * up.
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(__nv_bfloat16* out, const __nv_bfloat16* gu, long long rows, int F, int interleaved) {
   const long long total = rows * F / 8;
+  pdl_trigger();
+  pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / (F / 8);
     const int c = (int)(i % (F / 8)) * 8;
@@ -305,6 +307,7 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(__nv_bfloat16* out, 
                                                             long long T, int D, int vocab, int max_pos, int* err) {
   const int vec_per_row = D / 8;
   const long long total = T * vec_per_row;
+  pdl_trigger();       // launched without programmatic overlap itself: everything ahead of it on the stream is complete
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long t = i / vec_per_row;
     const int c = (int)(i % vec_per_row) * 8;
@@ -427,9 +430,9 @@ MLF_API int mlf_gelu_bwd(void* dx, const void* dy, const void* x, long long n, u
 }
 MLF_API int mlf_swiglu_fwd(void* out, const void* gu, long long rows, int F, int interleaved, uint64_t stream) {
   MLF_REQUIRE(F % 8 == 0, "swiglu: F must be a multiple of 8");
-  swiglu_fwd_kernel<<<ew_grid(rows * F / 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)gu, rows, F, interleaved);
+  MLF_CHECK_CUDA(launch_pdl(swiglu_fwd_kernel, dim3(ew_grid(rows * F / 8)), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
+                            (__nv_bfloat16*)out, (const __nv_bfloat16*)gu, rows, F, interleaved));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 MLF_API int mlf_swiglu_bwd(void* dgu, const void* dout, const void* gu, long long rows, int F, int interleaved, uint64_t stream) {

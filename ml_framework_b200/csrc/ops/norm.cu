@@ -32,16 +32,30 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return u;
 }
 
+// CTAs past the first `norm_ctas` of a forward launch clear a buffer for a later kernel (the output that the next
+// product adds its partial tiles into): a clearing launch of its own would stand in the chain of kernels.
+__device__ __forceinline__ void zero_role(uint4* z, long long n, int norm_ctas) {
+  const long long stride = (long long)(gridDim.x - norm_ctas) * blockDim.x;
+  for (long long i = (long long)(blockIdx.x - norm_ctas) * blockDim.x + threadIdx.x; i < n; i += stride) z[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // D = NV * 256. rms != 0 selects RMSNorm (no mean subtraction, no beta).
 template <int NV>
 __global__ void __launch_bounds__(256)
-norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
-                const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
-                float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, int rms) {
+norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
+                const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* y,
+                float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, int rms, int norm_ctas,
+                uint4* zero, long long n_zero) {
   constexpr int D = NV * 256;
+  pdl_trigger();
+  pdl_wait();
+  if ((int)blockIdx.x >= norm_ctas) {
+    zero_role(zero, n_zero, norm_ctas);
+    return;
+  }
   const int lane = threadIdx.x & 31;
   const int warps_per_cta = blockDim.x >> 5;
-  for (int row = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps_per_cta) {
+  for (int row = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); row < rows; row += norm_ctas * warps_per_cta) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * D);
     uint4 xv[NV];
 #pragma unroll
@@ -95,10 +109,17 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // Few rows (a decode step: 64 x 4096) then still occupy one CTA per row group instead of one warp per row.
 template <int NVT, int R>
 __global__ void __launch_bounds__(256, 3)
-norm_fwd_cta_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
-                    const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
-                    float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, int rms) {
+norm_fwd_cta_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
+                    const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* y,
+                    float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, int rms, int norm_ctas,
+                    uint4* zero, long long n_zero) {
   constexpr int D = NVT * 2048;
+  pdl_trigger();
+  pdl_wait();
+  if ((int)blockIdx.x >= norm_ctas) {
+    zero_role(zero, n_zero, norm_ctas);
+    return;
+  }
   __shared__ float red[2][2][8][R];          // [iteration parity][sum | centred squares][warp][row]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float g[NVT][8], bt[NVT][8];
@@ -113,7 +134,7 @@ norm_fwd_cta_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
   }
   const float inv_d = 1.f / D;
   int par = 0;
-  for (int row0 = blockIdx.x * R; row0 < rows; row0 += gridDim.x * R, par ^= 1) {
+  for (int row0 = blockIdx.x * R; row0 < rows; row0 += norm_ctas * R, par ^= 1) {
     uint4 xv[R][NVT];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -445,13 +466,12 @@ norm_bwd_finalize_kernel(const float* __restrict__ partials, int nparts, int D, 
 
 template <int NV>
 static int launch_fwd(const void* x, const void* g, const void* b, void* y, float* mean, float* rstd, int rows,
-                      float eps, int rms, cudaStream_t st) {
+                      float eps, int rms, uint4* zero, long long n_zero, int zero_ctas, cudaStream_t st) {
   const int grid = min((rows + 7) / 8, sm_count() * 8);
-  norm_fwd_kernel<NV><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(g),
-                                            static_cast<const __nv_bfloat16*>(b), static_cast<__nv_bfloat16*>(y), mean,
-                                            rstd, rows, eps, rms);
-                                            count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
+  MLF_CHECK_CUDA(launch_pdl(norm_fwd_kernel<NV>, dim3(grid + zero_ctas), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(x),
+                            static_cast<const __nv_bfloat16*>(g), static_cast<const __nv_bfloat16*>(b), static_cast<__nv_bfloat16*>(y), mean,
+                            rstd, rows, eps, rms, grid, zero, n_zero));
+  count_launch();
   return 0;
 }
 
@@ -490,10 +510,16 @@ using namespace mlf;
   }
 
 // y = norm(x) * gamma (+ beta). D must be a multiple of 256 from {256..1024, 1536, 2048, 3072,
-// 4096, 5120, 6144, 8192}. mean/rstd (fp32 [rows]) may be null for inference.
-MLF_API int mlf_norm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
-                         int rows, int D, float eps, int rms, uint64_t stream) {
+// 4096, 5120, 6144, 8192}. mean/rstd (fp32 [rows]) may be null for inference. `zero` (optional, 16-byte aligned,
+// zero_bytes a multiple of 16) is cleared by additional CTAs of the same launch.
+MLF_API int mlf_norm_fwd_zero(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
+                              int rows, int D, float eps, int rms, void* zero, long long zero_bytes, uint64_t stream) {
   MLF_REQUIRE(D % 256 == 0, "norm: D=%d must be a multiple of 256", D);
+  MLF_REQUIRE(zero_bytes >= 0 && zero_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(zero) & 15) == 0, "norm: the buffer to clear must be 16-byte aligned");
+  uint4* zp = static_cast<uint4*>(zero);
+  const long long nz = zero != nullptr ? zero_bytes / 16 : 0;
+  // 32 KB per CTA: eight 16-byte stores per thread
+  const int zc = (int)(nz == 0 ? 0 : (nz + 2047) / 2048 < sm_count() ? (nz + 2047) / 2048 : sm_count());
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (D == 2048 || D == 4096) {
     const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
@@ -504,24 +530,27 @@ MLF_API int mlf_norm_fwd(const void* x, const void* gamma, const void* beta, voi
     if (D == 2048) {
       const int r = rows >= 4 * cap ? 4 : (rows >= 2 * cap ? 2 : 1);      // few rows: one row per CTA, more CTAs
       const int grid = min((rows + r - 1) / r, cap);
-      if (r == 4) norm_fwd_cta_kernel<1, 4><<<grid, 256, 0, st>>>(xp, gp, bp, yp, mean, rstd, rows, eps, rms);
-      else if (r == 2) norm_fwd_cta_kernel<1, 2><<<grid, 256, 0, st>>>(xp, gp, bp, yp, mean, rstd, rows, eps, rms);
-      else norm_fwd_cta_kernel<1, 1><<<grid, 256, 0, st>>>(xp, gp, bp, yp, mean, rstd, rows, eps, rms);
+      const auto kernel = r == 4 ? norm_fwd_cta_kernel<1, 4> : r == 2 ? norm_fwd_cta_kernel<1, 2> : norm_fwd_cta_kernel<1, 1>;
+      MLF_CHECK_CUDA(launch_pdl(kernel, dim3(grid + zc), dim3(256), 0, st, xp, gp, bp, yp, mean, rstd, rows, eps, rms, grid, zp, nz));
     } else {
       const int r = rows >= 2 * cap ? 2 : 1;
       const int grid = min((rows + r - 1) / r, cap);
-      if (r == 2) norm_fwd_cta_kernel<2, 2><<<grid, 256, 0, st>>>(xp, gp, bp, yp, mean, rstd, rows, eps, rms);
-      else norm_fwd_cta_kernel<2, 1><<<grid, 256, 0, st>>>(xp, gp, bp, yp, mean, rstd, rows, eps, rms);
+      const auto kernel = r == 2 ? norm_fwd_cta_kernel<2, 2> : norm_fwd_cta_kernel<2, 1>;
+      MLF_CHECK_CUDA(launch_pdl(kernel, dim3(grid + zc), dim3(256), 0, st, xp, gp, bp, yp, mean, rstd, rows, eps, rms, grid, zp, nz));
     }
     count_launch();
-    MLF_CHECK_CUDA(cudaGetLastError());
     return 0;
   }
-#define CALL(NV) launch_fwd<NV>(x, gamma, beta, y, mean, rstd, rows, eps, rms, st)
+#define CALL(NV) launch_fwd<NV>(x, gamma, beta, y, mean, rstd, rows, eps, rms, zp, nz, zc, st)
   MLF_NORM_DISPATCH(D / 256, CALL)
 #undef CALL
   set_error("norm: unsupported D=%d", D);
   return -2;
+}
+
+MLF_API int mlf_norm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
+                         int rows, int D, float eps, int rms, uint64_t stream) {
+  return mlf_norm_fwd_zero(x, gamma, beta, y, mean, rstd, rows, D, eps, rms, nullptr, 0, stream);
 }
 
 // CTAs of the backward kernel: whole-CTA rows for the wide model dimensions, warp rows otherwise.

@@ -89,7 +89,8 @@ def reduce_all(op: str, a: torch.Tensor) -> torch.Tensor:
 
 # ------------------------------------------------------------------ norms
 def norm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor], eps: float, rms: bool,
-             want_stats: bool = True):
+             want_stats: bool = True, zero: Optional[torch.Tensor] = None):
+    """``zero``: a contiguous buffer that the same launch clears (the output a following product accumulates into)."""
     D = x.shape[-1]
     x2 = x.reshape(-1, D)
     assert x2.is_contiguous() and x2.dtype == torch.bfloat16
@@ -97,7 +98,12 @@ def norm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor],
     y = torch.empty_like(x2)
     mean = torch.empty(rows, dtype=torch.float32, device=x.device) if want_stats and not rms else None
     rstd = torch.empty(rows, dtype=torch.float32, device=x.device) if want_stats else None
-    rc = _L().mlf_norm_fwd(_p(x2), _p(gamma), _p(beta), _p(y), _p(mean), _p(rstd), rows, D, C.c_float(eps), int(rms), _st())
+    zbytes = 0
+    if zero is not None:
+        assert zero.is_contiguous() and zero.device == x.device
+        zbytes = zero.numel() * zero.element_size()
+    rc = _L().mlf_norm_fwd_zero(_p(x2), _p(gamma), _p(beta), _p(y), _p(mean), _p(rstd), rows, D, C.c_float(eps), int(rms),
+                                _p(zero), C.c_longlong(zbytes), _st())
     _lib.check(rc, "mlf_norm_fwd")
     return y.view(x.shape), mean, rstd
 

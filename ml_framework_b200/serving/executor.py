@@ -100,6 +100,16 @@ class PagedLlamaExecutor:
         tp.pg.all_reduce(partial, ReduceOp.SUM)
         return partial + residual if residual is not None else partial
 
+    def _norm_product(self, x: torch.Tensor, gamma: torch.Tensor, w: torch.Tensor, few_rows: bool):
+        """(rms_norm(x), rms_norm(x) @ w^T). The first kernel of a step is the embedding lookup, which starts after all
+        earlier work of the stream; nothing in the step writes a weight, so the products may read theirs early."""
+        if not few_rows:
+            h, _, _ = native.norm_fwd(x, gamma, None, self.mc.norm_eps, True, want_stats=False)
+            return h, gemm(h, w, flags=_lib.EPI_B_STATIC)
+        out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
+        h, _, _ = native.norm_fwd(x, gamma, None, self.mc.norm_eps, True, want_stats=False, zero=out)
+        return h, gemm(h, w, out=out, flags=_lib.EPI_ACCUM | _lib.EPI_B_STATIC)
+
     # ---- one transformer block over T tokens
     def _block(self, li: int, blk, x: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, attend):
         mc = self.mc
@@ -112,35 +122,38 @@ class PagedLlamaExecutor:
         cache = self.kv.caches[li]
         T = x.shape[0]
         if self.native:
-            h, _, _ = native.norm_fwd(x, blk.norm1.weight, None, mc.norm_eps, True, want_stats=False)
-            qkv = gemm(h, qkv_w)
+            # A decode step (few rows, whole weights) streams weights: plain products let the GEMM split K over all SMs
+            # and accumulate, into a buffer that the normalisation's launch clears; the weights are read ahead.
+            few_rows = T <= 256
+            h, qkv = self._norm_product(x, blk.norm1.weight, qkv_w, few_rows)
             q = qkv[:, :self.hq * D].view(T, self.hq, D)
             k = qkv[:, self.hq * D:(self.hq + self.hkv) * D].view(T, self.hkv, D)
             v = qkv[:, (self.hq + self.hkv) * D:].view(T, self.hkv, D)
             native.rope_kv_write_(qkv, positions, slots, cache, self.hq, self.hkv, mc.rope_theta)
             a = attend(li, q, k, v)
             multi = self.tp is not None and self.tp.world > 1
-            # A decode step (few rows, whole weights) streams weights: plain products let the GEMM split K over
-            # all SMs, the residual stream takes the product as an accumulation, SwiGLU runs as its own pass.
-            few_rows = T <= 256
+            # few rows: the residual stream takes the product as an accumulation, SwiGLU runs as its own pass
             sync_ar = multi and self.tp.fused
             if sync_ar:
                 x = self._row_parallel(a.reshape(T, self.hq * D), o_w, x)
             elif multi:
                 x = self._reduce(gemm(a.reshape(T, self.hq * D), o_w), x)
             elif few_rows:
-                gemm(a.reshape(T, self.hq * D), o_w, out=x, flags=_lib.EPI_ACCUM)
+                gemm(a.reshape(T, self.hq * D), o_w, out=x, flags=_lib.EPI_ACCUM | _lib.EPI_B_STATIC)
             else:
-                x = gemm(a.reshape(T, self.hq * D), o_w, aux_in=x, flags=_lib.EPI_RESIDUAL)
-            h, _, _ = native.norm_fwd(x, blk.norm2.weight, None, mc.norm_eps, True, want_stats=False)
-            hid = native.swiglu_fwd(gemm(h, gu_w), interleaved=True) if few_rows else gemm(h, gu_w, flags=_lib.EPI_SWIGLU)
+                x = gemm(a.reshape(T, self.hq * D), o_w, aux_in=x, flags=_lib.EPI_RESIDUAL | _lib.EPI_B_STATIC)
+            if few_rows:
+                hid = native.swiglu_fwd(self._norm_product(x, blk.norm2.weight, gu_w, True)[1], interleaved=True)
+            else:
+                h, _, _ = native.norm_fwd(x, blk.norm2.weight, None, mc.norm_eps, True, want_stats=False)
+                hid = gemm(h, gu_w, flags=_lib.EPI_SWIGLU | _lib.EPI_B_STATIC)
             if sync_ar:
                 return self._row_parallel(hid, dn_w, x)
             if multi:
                 return self._reduce(gemm(hid, dn_w), x)
             if few_rows:
-                return gemm(hid, dn_w, out=x, flags=_lib.EPI_ACCUM)
-            return gemm(hid, dn_w, aux_in=x, flags=_lib.EPI_RESIDUAL)
+                return gemm(hid, dn_w, out=x, flags=_lib.EPI_ACCUM | _lib.EPI_B_STATIC)
+            return gemm(hid, dn_w, aux_in=x, flags=_lib.EPI_RESIDUAL | _lib.EPI_B_STATIC)
         if self.cfg.torch_ops:
             return self._block_torch(x, blk, qkv_w, o_w, gu_w, dn_w, cache, positions, slots, attend, li)
         # ---- PyTorch statement of the same block (CPU / fp32)
@@ -238,8 +251,7 @@ class PagedLlamaExecutor:
     def _logits_argmax(self, x_last: torch.Tensor) -> torch.Tensor:
         mc = self.mc
         if self.native:
-            h, _, _ = native.norm_fwd(x_last.contiguous(), self.m.norm_f.weight, None, mc.norm_eps, True, want_stats=False)
-            logits = gemm(h, self.m.lm_head)
+            _, logits = self._norm_product(x_last.contiguous(), self.m.norm_f.weight, self.m.lm_head, x_last.shape[0] <= 256)
             if self.tp is not None and self.tp.world > 1 and self.tp.fused:
                 cand = self.tp.symm_buffer("serve.argmax", max(self.cfg.max_batch, 1) * 8)
                 return self.tp.symm.tp_argmax(logits, self.tp.rank * logits.shape[1], mc.vocab_size, cand)

@@ -1,0 +1,53 @@
+"""Kernels launched with programmatic overlap: a chain of dependent launches gives what the operators give one by one,
+at the sizes where the early weight loads end (runs shorter than the ring, remainders, each token-tile width)."""
+import pytest
+import torch
+
+from ml_framework_b200 import _lib
+from ml_framework_b200.ops import native
+from ml_framework_b200.ops.gemm import gemm
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 32, 33, 64, 128, 129, 256])
+@pytest.mark.parametrize("N,K", [(1024, 512), (1096, 2048), (4096, 5120)])
+def test_chain_with_static_weights(M, N, K):
+    torch.manual_seed(M + N)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    g = torch.rand(K, device="cuda").to(torch.bfloat16)
+    w1 = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    w2 = (torch.randn(K, N, device="cuda") * N ** -0.5).to(torch.bfloat16)
+    flags = _lib.EPI_ACCUM | _lib.EPI_B_STATIC
+    mid = torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    res = x.clone()
+    for _ in range(3):                       # each round overlaps the end of the one before it
+        h, _, _ = native.norm_fwd(x, g, None, 1e-5, True, want_stats=False, zero=mid)
+        gemm(h, w1, out=mid, flags=flags)
+        res.copy_(x)
+        gemm(mid, w2, out=res, flags=flags)
+    torch.cuda.synchronize()
+    xf = x.float()
+    hf = (xf * torch.rsqrt((xf * xf).mean(-1, keepdim=True) + 1e-5) * g.float()).to(torch.bfloat16).float()
+    mf = hf @ w1.float().t()
+    # every partial tile is added in bf16: at most one rounding (2^-9 of the running value) per SM that shares the tile,
+    # and a value at a rounding boundary of h may round the other way; 4 sigma of that in the root mean square
+    rms = lambda t: t.pow(2).mean().sqrt().item()
+    assert rms(mid.float() - mf) <= 2 ** -7 * rms(mf)
+    rf = x.float() + mid.float() @ w2.float().t()
+    assert rms(res.float() - rf) <= 2 ** -7 * rms(rf)
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("rows,D", [(1, 256), (5, 1024), (3, 2048), (300, 4096), (2, 5120)])
+@pytest.mark.parametrize("zero_elems", [8, 16384 + 8, 5_000_000])
+def test_norm_clears_a_buffer(rows, D, zero_elems):
+    torch.manual_seed(0)
+    x = torch.randn(rows, D, device="cuda").to(torch.bfloat16)
+    g = torch.rand(D, device="cuda").to(torch.bfloat16)
+    guard = torch.ones(zero_elems + 64, device="cuda", dtype=torch.bfloat16)
+    y0, _, _ = native.norm_fwd(x, g, None, 1e-5, True, want_stats=False)
+    y1, _, _ = native.norm_fwd(x, g, None, 1e-5, True, want_stats=False, zero=guard[:zero_elems])
+    assert torch.equal(y0, y1)
+    assert not guard[:zero_elems].any() and bool((guard[zero_elems:] == 1).all())
+    assert _lib.read_status() == 0
