@@ -168,7 +168,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  t_dQ = tmem_base + 384;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int krow = (int)(row_base + k0);
       mbar_expect_tx(kv_full, 2 * FB_KV_BYTES);
       tma_load_2d(sK, &tmK, hkv * FB_D, krow, kv_full);
@@ -190,7 +190,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(128, FB_BQ, 0, 0);    // S^T, dP^T
       const uint32_t idesc_g = make_idesc_bf16(128, FB_D, 0, 1);     // dV, dK: B = dO / Q MN-major
       const uint32_t idesc_q = make_idesc_bf16(128, FB_BQ, 1, 1);    // dQ^T: A = K MN-major, B = dS^T MN-major

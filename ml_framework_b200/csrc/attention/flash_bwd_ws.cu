@@ -134,7 +134,7 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 0) {
       // ===================== TMA producer =====================
-      if (lane == 0) {
+      if (elect_one()) {
         const int krow = (int)(row_base + k0);
         mbar_expect_tx(kv_full, 2 * G_TILE);
         tma_load_2d(sK, &tmK, hkv * G_D, krow, kv_full);
@@ -161,7 +161,7 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     } else if (warp == 1) {
       // ===================== MMA issuer =====================
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t idesc_kk = make_idesc_bf16(128, 128, 0, 0);   // S^T, dP^T: both operands K-major
         const uint32_t idesc_kn = make_idesc_bf16(128, 128, 0, 1);   // dV, dK: B (dO / Q) MN-major
         const uint32_t idesc_nn = make_idesc_bf16(128, 128, 1, 1);   // dQ: A (dS) and B (K) MN-major

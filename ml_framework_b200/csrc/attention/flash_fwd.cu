@@ -115,7 +115,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t tPV = tmem_base + 128;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, FA_Q_BYTES);
       tma_load_2d(sQ, &tmQ, h * FA_D, (int)(row_base + q0), q_full);
       tma_load_2d(sQ + FA_Q_BYTES / 2, &tmQ, h * FA_D + 64, (int)(row_base + q0), q_full);
@@ -135,7 +135,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(128, FA_BKV, 0, 0);
       const uint32_t idesc_pv = make_idesc_bf16(128, FA_D, 0, 1);
       auto issue_s = [&](int j) -> bool {

@@ -139,7 +139,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
     // ===================== TMA producer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       for (int t = 0; t < 2; ++t) {
         mbar_expect_tx(q_full(t), W_TILE_BYTES);
         const int qrow = (int)(row_base + q0 + t * W_BQ);
@@ -195,7 +195,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(128, W_BKV, 0, 0);
       const uint32_t idesc_pv = make_idesc_bf16(128, W_D, 0, 1);
       auto issue_s = [&](int t, int j) {

@@ -47,6 +47,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
+// One thread of a converged warp. The roles that issue TMA and tcgen05 instructions are entered through it and not
+// through a test of the lane number: those instructions take their descriptors and addresses in uniform registers, and
+// only behind elect.sync does the compiler know that one thread executes them (behind `lane == 0` every MMA paid for
+// making its operands uniform). bf16 products 8192 x 8192 x 2048 193 -> 175 us, 8192 x 2048 x 8192 201 -> 188 us,
+// 4096 x 28672 x 4096 656 -> 601 us; attention backward of 4 x 2048, 16 heads, 382 -> 339 us, forward 113 -> 105 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(

@@ -123,7 +123,7 @@ gemm_fewrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     // ===================== TMA producer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       // A weight that nobody writes starts streaming while the kernels ahead are still running: the ring is filled
@@ -157,7 +157,7 @@ gemm_fewrow_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(FR_WT, BT, 0, 0);
       pdl_wait();
       if (p.w_static) {

@@ -113,7 +113,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   if (warp == 0) {
     // ===================== TMA producer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -161,7 +161,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(BM, BN, p.a_mn, p.b_mn);
       // K-major: 8-row groups 1024 B apart, K advance = 32 B inside the swizzle atom.
       // MN-major: 8-k-row groups 1024 B apart, 64-column blocks BK*128 B apart, K advance = 2048 B.
