@@ -55,6 +55,40 @@ struct BlockManager {
   }
 };
 
+// Room for `new_tokens` more tokens of `seq` (the caller holds the lock); see mlf_bm_append_tokens.
+static int append_locked(BlockManager* m, long long seq, int new_tokens, long long* slots, int* cow_src, int* cow_dst) {
+  auto& s = m->seqs[seq];
+  const int bs = m->block_size;
+  if (cow_src) *cow_src = -1;
+  if (cow_dst) *cow_dst = -1;
+  const int used_in_last = s.blocks.empty() ? 0 : s.tokens - ((int)s.blocks.size() - 1) * bs;
+  const int room = s.blocks.empty() ? 0 : bs - used_in_last;
+  const bool last_shared = !s.blocks.empty() && room > 0 && m->refcount[s.blocks.back()] > 1;
+  int need = new_tokens > room ? (new_tokens - room + bs - 1) / bs : 0;
+  if (last_shared && new_tokens > 0) need += 1;
+  if ((int)m->free_list.size() < need) {
+    ++m->failed_allocs;
+    return -1;
+  }
+  if (last_shared && new_tokens > 0) {
+    const int old = s.blocks.back();
+    const int nb = m->take();
+    s.blocks.back() = nb;
+    m->release(old);
+    ++m->cow_copies;
+    if (cow_src) *cow_src = old;
+    if (cow_dst) *cow_dst = nb;
+  }
+  for (int i = 0; i < new_tokens; ++i) {
+    const int pos = s.tokens + i;
+    const int bi = pos / bs;
+    while ((int)s.blocks.size() <= bi) s.blocks.push_back(m->take());
+    if (slots) slots[i] = (long long)s.blocks[bi] * bs + pos % bs;
+  }
+  s.tokens += new_tokens;
+  return 0;
+}
+
 }  // namespace mlf
 
 using namespace mlf;
@@ -111,35 +145,49 @@ MLF_API int mlf_bm_allocate_blocks(void* h, long long seq, int count, int* out) 
 MLF_API int mlf_bm_append_tokens(void* h, long long seq, int new_tokens, long long* slots, int* cow_src, int* cow_dst) {
   auto* m = static_cast<BlockManager*>(h);
   std::lock_guard<std::mutex> lk(m->mu);
-  auto& s = m->seqs[seq];
-  const int bs = m->block_size;
-  if (cow_src) *cow_src = -1;
-  if (cow_dst) *cow_dst = -1;
-  const int used_in_last = s.blocks.empty() ? 0 : s.tokens - ((int)s.blocks.size() - 1) * bs;
-  const int room = s.blocks.empty() ? 0 : bs - used_in_last;
-  const bool last_shared = !s.blocks.empty() && room > 0 && m->refcount[s.blocks.back()] > 1;
-  int need = new_tokens > room ? (new_tokens - room + bs - 1) / bs : 0;
-  if (last_shared && new_tokens > 0) need += 1;
-  if ((int)m->free_list.size() < need) {
-    ++m->failed_allocs;
-    return -1;
+  return append_locked(m, seq, new_tokens, slots, cow_src, cow_dst);
+}
+
+// Everything a decode step of `n` sequences needs from the pool, in one call: the tokens each sequence holds (pos[i],
+// the position of its new token), one more slot for each (slots[i]), the lengths afterwards (lens[i]) and `width`
+// entries of each block table (-1 past its blocks). Rows n .. rows - 1 are padding: position 0, slot -1, length 1,
+// table 0. cow[2 i], cow[2 i + 1]: the (source, destination) block copy of sequence i or -1. *max_pos: the largest
+// pos[i]. Returns 0; -1 when the pool is exhausted (*n_done sequences have got their slot, as after as many calls of
+// mlf_bm_append_tokens); -2 when a sequence holds more than max_blocks blocks.
+MLF_API int mlf_bm_append_decode(void* h, const long long* seqs, int n, int rows, int max_blocks, int width, long long* pos, long long* slots,
+                                 int* lens, int* table, int* cow, int* n_done, int* max_pos) {
+  auto* m = static_cast<BlockManager*>(h);
+  std::lock_guard<std::mutex> lk(m->mu);
+  *n_done = 0;
+  *max_pos = 0;
+  for (int i = 0; i < n; ++i) {
+    auto it = m->seqs.find(seqs[i]);
+    pos[i] = it == m->seqs.end() ? 0 : it->second.tokens;
+    if (pos[i] > *max_pos) *max_pos = (int)pos[i];
   }
-  if (last_shared && new_tokens > 0) {
-    const int old = s.blocks.back();
-    const int nb = m->take();
-    s.blocks.back() = nb;
-    m->release(old);
-    ++m->cow_copies;
-    if (cow_src) *cow_src = old;
-    if (cow_dst) *cow_dst = nb;
+  for (int i = 0; i < n; ++i) {
+    if (append_locked(m, seqs[i], 1, slots + i, cow + 2 * i, cow + 2 * i + 1) != 0) return -1;
+    *n_done = i + 1;
   }
-  for (int i = 0; i < new_tokens; ++i) {
-    const int pos = s.tokens + i;
-    const int bi = pos / bs;
-    while ((int)s.blocks.size() <= bi) s.blocks.push_back(m->take());
-    if (slots) slots[i] = (long long)s.blocks[bi] * bs + pos % bs;
+  for (int i = 0; i < n; ++i) {
+    const auto& s = m->seqs[seqs[i]];
+    const int nb = (int)s.blocks.size();
+    if (nb > max_blocks) {
+      set_error("sequence %lld has %d blocks, table holds %d", seqs[i], nb, max_blocks);
+      return -2;
+    }
+    int* row = table + (long long)i * width;
+    const int k = nb < width ? nb : width;
+    memcpy(row, s.blocks.data(), (size_t)k * sizeof(int));
+    for (int j = k; j < width; ++j) row[j] = -1;
+    lens[i] = s.tokens;
   }
-  s.tokens += new_tokens;
+  for (int i = n; i < rows; ++i) {
+    pos[i] = 0;
+    slots[i] = -1;
+    lens[i] = 1;
+    memset(table + (long long)i * width, 0, (size_t)width * sizeof(int));
+  }
   return 0;
 }
 

@@ -16,8 +16,9 @@ or a process-group all-reduce. Rank 0 runs the scheduler and broadcasts each ite
 """
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass
-from typing import Dict, List, Optional
+from typing import Dict, List, Optional, Sequence
 
 import torch
 import torch.nn.functional as F
@@ -265,6 +266,16 @@ class PagedLlamaExecutor:
             logits = self.tp.pg.all_gather(logits, dim=-1)
         return logits[:, :mc.vocab_size].float().argmax(-1)
 
+    # ---- host side of a step: everything the kernels need goes up in one copy
+    def _host_rows(self, rows: int, n: int) -> torch.Tensor:
+        return torch.empty(rows, n, dtype=torch.int64, pin_memory=self.device.type == "cuda")
+
+    @staticmethod
+    def _put_ids(dst: torch.Tensor, ids: Sequence[int]):
+        """``dst[:] = ids`` through a typed array (torch.tensor inspects every element of a list twice)."""
+        if len(ids):
+            dst.copy_(torch.frombuffer(array("q", ids), dtype=torch.int64))
+
     # ---- prefill of one request chunk
     @torch.no_grad()
     def _prefill(self, r: Request) -> Optional[int]:
@@ -275,10 +286,13 @@ class PagedLlamaExecutor:
         if slots is None:
             raise MemoryError(f"KV cache exhausted while prefilling request {r.id}")
         dev = self.device
-        ids = torch.tensor(chunk, dtype=torch.int64, device=dev)
-        pos = torch.arange(start, start + n, dtype=torch.int64, device=dev)
-        slots = slots.to(dev)
-        table, _ = self.kv.build_tables([r.id], self.max_blocks, dev)
+        host = self._host_rows(3, n)
+        self._put_ids(host[0], chunk)
+        torch.arange(start, start + n, out=host[1])
+        host[2].copy_(slots)
+        ids, pos, slots = host.to(dev, non_blocking=True)
+        # the first chunk attends to its own rows only
+        table = self.kv.build_tables([r.id], self.max_blocks, dev)[0] if start > 0 or not self.native else None
         total = start + n
 
         paged_prefill = self.native and start > 0 and self.kv.block_size == 16
@@ -325,9 +339,13 @@ class PagedLlamaExecutor:
             if s is None:
                 raise MemoryError(f"KV cache exhausted while prefilling request {r.id}")
             slot_list.append(s)
-        ids = torch.tensor([r.prompt_tokens[:n] for r in reqs], dtype=torch.int64, device=dev)
-        pos = torch.arange(n, dtype=torch.int64, device=dev).repeat(B)
-        slots = torch.cat(slot_list).to(dev)
+        host = self._host_rows(3, B * n)
+        host[1].view(B, n).copy_(torch.arange(n))
+        for i, (r, s) in enumerate(zip(reqs, slot_list)):
+            self._put_ids(host[0, i * n:(i + 1) * n], r.prompt_tokens[:n])
+            host[2, i * n:(i + 1) * n].copy_(s)
+        ids, pos, slots = host.to(dev, non_blocking=True)
+        ids = ids.view(B, n)
 
         def attend(li, q, k, v):
             out, _ = native.flash_fwd(q, k, v, B, n, causal=True, want_lse=False)
@@ -373,40 +391,33 @@ class PagedLlamaExecutor:
         dev = self.device
         B = len(reqs)
         last_l = [r.generated[-1] if r.generated else r.prompt_tokens[-1] for r in reqs]
-        lens_before = [self.kv.get_sequence_length(r.id) for r in reqs]
-        slot_list = []
-        for r in reqs:
-            s, _ = self.kv.append_tokens(r.id, 1)
-            if s is None:
-                raise MemoryError(f"KV cache exhausted while decoding request {r.id}")
-            slot_list.append(s)
-        table, lens = self.kv.build_tables([r.id for r in reqs], self.max_blocks, dev)
-        max_len = max(lens_before) + 1
-        if self._graphs is None:
-            last = torch.tensor(last_l, dtype=torch.int64, device=dev)
-            slots = torch.cat(slot_list).to(dev)
-            pos = torch.tensor(lens_before, dtype=torch.int64, device=dev)
-            return self._decode_core(last, pos, slots, table, lens, max_len).tolist()
-        # Graph path: pad the batch to a power of two and the length bound to a multiple of 512 so that a
+        # Graph path: pad the batch to a power of two and the length bound to a power of two from 512 so that a
         # handful of captured graphs covers every step. Padding rows write nowhere (slot -1) and attend to
         # one token of block 0; their outputs are dropped.
-        Bp = self._bucket(B)
+        Bp = self._bucket(B) if self._graphs is not None else B
+        # one buffer, one copy: token ids, positions, slots (int64 [3, Bp]), then lengths and block tables (int32)
+        head = 3 * Bp
+        host = torch.empty(head + (Bp * (1 + self.max_blocks) + 1) // 2, dtype=torch.int64, pin_memory=dev.type == "cuda")
+        host32 = host[head:].view(torch.int32)
+        self._put_ids(host[:B], last_l)
+        host[B:Bp] = 0
+        ids = [r.id for r in reqs]
+        width = self.max_blocks
+        done, top = self.kv.append_decode(ids, self.max_blocks, Bp, width, host[Bp:2 * Bp], host[2 * Bp:head], host32[:Bp],
+                                          host32[Bp:Bp * (1 + width)])
+        if done < B:
+            raise MemoryError(f"KV cache exhausted while decoding request {ids[done]}")
+        max_len = top + 1
+        packed = host.to(dev, non_blocking=True)
+
+        def step(buf, length):
+            b32 = buf[head:].view(torch.int32)
+            return self._decode_core(buf[:Bp], buf[Bp:2 * Bp], buf[2 * Bp:head], b32[Bp:Bp * (1 + width)].view(Bp, width), b32[:Bp], length)
+
+        if self._graphs is None:
+            return step(packed, max_len).tolist()
         Lp = min(self._bucket(max_len, 512), max(self.cfg.max_seq_len, 512))
-        pad = Bp - B
-        host = torch.empty(3, Bp, dtype=torch.int64, pin_memory=True)
-        host[0, :B] = torch.tensor(last_l, dtype=torch.int64)
-        host[1, :B] = torch.tensor(lens_before, dtype=torch.int64)
-        host[2, :B] = torch.cat(slot_list).to(torch.int64).cpu()
-        if pad:
-            host[0, B:] = 0
-            host[1, B:] = 0
-            host[2, B:] = -1
-        devt = host.to(dev, non_blocking=True)
-        if pad:
-            table = torch.cat([table, table.new_zeros(pad, table.shape[1])], 0)
-            lens = torch.cat([lens, lens.new_ones(pad)], 0)
-        fn = lambda a, b_, c, t, l: self._decode_core(a, b_, c, t, l, Lp)
-        out = self._graphs.run(f"decode_L{Lp}", fn, devt[0], devt[1], devt[2], table.contiguous(), lens.contiguous())
+        out = self._graphs.run(f"decode_B{Bp}_L{Lp}", lambda buf: step(buf, Lp), packed)
         return out[:B].tolist()
 
     # ---- scheduler entry point

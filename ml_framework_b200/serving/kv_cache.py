@@ -11,6 +11,7 @@ copy-on-divergence, speculative decoding with verify / reject).
 from __future__ import annotations
 
 import ctypes as C
+from array import array
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -83,16 +84,41 @@ class KVCacheBlockManager:
     def append_tokens(self, seq_id: int, n: int) -> Tuple[Optional[torch.Tensor], Optional[Tuple[int, int]]]:
         """Reserve cache slots for ``n`` more tokens. Returns (slots int64 [n] or None when the pool
         is exhausted, (src, dst) block copy to perform on the device for copy-on-write or None)."""
-        slots = (C.c_longlong * max(n, 1))()
+        slots = torch.empty(max(n, 1), dtype=torch.int64)
         cs, cd = C.c_int(-1), C.c_int(-1)
-        rc = self._L.mlf_bm_append_tokens(self._h, C.c_longlong(seq_id), n, slots, C.byref(cs), C.byref(cd))
+        rc = self._L.mlf_bm_append_tokens(self._h, C.c_longlong(seq_id), n, C.c_void_p(slots.data_ptr()), C.byref(cs), C.byref(cd))
         if rc != 0:
             return None, None
         cow = (cs.value, cd.value) if cs.value >= 0 else None
         if cow is not None:
-            for cache in self.caches:
-                cache[cow[1]].copy_(cache[cow[0]])
-        return torch.tensor(list(slots[:n]), dtype=torch.int64), cow
+            self._copy_block(*cow)
+        return slots[:n], cow
+
+    def _copy_block(self, src: int, dst: int):
+        for cache in self.caches:
+            cache[dst].copy_(cache[src])
+
+    def append_decode(self, seq_ids: Sequence[int], max_blocks: int, rows: int, width: int, pos: torch.Tensor, slots: torch.Tensor,
+                      lens: torch.Tensor, table: torch.Tensor) -> Tuple[int, int]:
+        """One more cache slot for each sequence and what a decode step needs to know, in one native call. Fills the
+        contiguous host tensors ``pos`` and ``slots`` (int64 [rows]), ``lens`` (int32 [rows]) and ``table`` (int32
+        [rows, width]); rows past the sequences become padding (slot -1, length 1, block 0). Returns (sequences that got
+        a slot, largest position): fewer than asked for when the pool is exhausted, with those before it kept, like as
+        many calls of :meth:`append_tokens`."""
+        n = len(seq_ids)
+        ids = array("q", seq_ids)
+        cow = (C.c_int * (2 * max(n, 1)))()
+        done, top = C.c_int(0), C.c_int(0)
+        p = C.c_void_p
+        rc = self._L.mlf_bm_append_decode(self._h, p(ids.buffer_info()[0]), n, rows, max_blocks, width, p(pos.data_ptr()),
+                                          p(slots.data_ptr()), p(lens.data_ptr()), p(table.data_ptr()), cow, C.byref(done), C.byref(top))
+        if self.caches:
+            for i in range(done.value):
+                if cow[2 * i] >= 0:
+                    self._copy_block(cow[2 * i], cow[2 * i + 1])
+        if rc != -1:
+            _lib.check(rc, "mlf_bm_append_decode")
+        return done.value, top.value
 
     def free_sequence_blocks(self, seq_id: int) -> int:
         return self._L.mlf_bm_free_sequence(self._h, C.c_longlong(seq_id))
