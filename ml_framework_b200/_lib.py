@@ -124,6 +124,11 @@ def raise_on_status() -> None:
 
 
 def stream_handle(stream=None) -> int:
+    """Raw handle of ``stream`` or of the current device's current stream. Every launch asks for it: building the stream
+    object that ``torch.cuda.current_stream()`` returns costs 5 us, the raw handle 0.2 us."""
+    if stream is not None:
+        return int(stream.cuda_stream)
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return int(s.cuda_stream)
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
