@@ -26,7 +26,7 @@
 namespace mlf {
 
 int cached_tmap_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
-                     uint32_t bi, uint32_t bo);
+                     uint32_t bi, uint32_t bo, bool swizzle = true);
 
 constexpr int FB_BKV = 128;
 constexpr int FB_BQ = 64;

@@ -31,7 +31,7 @@
 namespace mlf {
 
 int cached_tmap_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
-                     uint32_t bi, uint32_t bo);
+                     uint32_t bi, uint32_t bo, bool swizzle = true);
 
 constexpr int FR_WT = 128;                         // weight rows per tile (MMA M)
 constexpr int FR_STAGE_W = FR_WT * BK * 2;         // 16 KB

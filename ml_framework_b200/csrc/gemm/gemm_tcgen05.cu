@@ -285,8 +285,8 @@ static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> g_tmaps;
 static std::mutex g_tmap_mu;
 
 int cached_tmap_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
-                     uint32_t bi, uint32_t bo) {
-  TmapKey k{base, inner, outer, ld, bi, bo};
+                     uint32_t bi, uint32_t bo, bool swizzle = true) {
+  TmapKey k{base, inner, outer, ld, bi, swizzle ? bo : bo | 0x80000000u};
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
     auto it = g_tmaps.find(k);
@@ -295,7 +295,7 @@ int cached_tmap_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_
       return 0;
     }
   }
-  int rc = make_tmap_2d(out, base, 2, inner, outer, ld, bi, bo, true);
+  int rc = make_tmap_2d(out, base, 2, inner, outer, ld, bi, bo, swizzle);
   if (rc) return rc;
   std::lock_guard<std::mutex> lk(g_tmap_mu);
   if (g_tmaps.size() > 8192) g_tmaps.clear();

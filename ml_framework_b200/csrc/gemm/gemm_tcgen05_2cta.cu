@@ -15,7 +15,7 @@
 //             an earlier phase: the peer refills a stage only after the MMAs that read it are done.
 //   empty[s]  in each CTA: the leader commits twice after the k-block's MMAs, once to its own and
 //             once to the peer's barrier (address translated with mapa).
-//   tfull[a]  in each CTA (same double commit), tempty[a] in the leader, count 8: the four
+//   tfull[a]  in each CTA (same double commit), tempty[a] in the leader, count 8 or 16: the
 //             epilogue warps of each CTA arrive (the peer's through a cluster-scope arrive).
 // Every wait is bounded; a cluster barrier at the end keeps either CTA from exiting while the
 // other may still touch its shared memory.
@@ -26,7 +26,7 @@
 namespace mlf {
 
 int cached_tmap_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
-                     uint32_t bi, uint32_t bo);
+                     uint32_t bi, uint32_t bo, bool swizzle = true);
 
 constexpr int T2_BN = 256;                       // tile columns (both CTAs)
 constexpr int T2_BNH = 128;                      // columns of B staged per CTA
@@ -34,8 +34,10 @@ constexpr int T2_STAGE_A = BM * BK * 2;          // 16 KB
 constexpr int T2_STAGE_B = T2_BNH * BK * 2;      // 16 KB
 constexpr int T2_STAGE = T2_STAGE_A + T2_STAGE_B;
 constexpr int T2_STAGES = 6;
-constexpr int T2_STG_BYTES = 128 * 64 * 2;     // epilogue staging: 128 rows x 64 bf16 columns, 128B-swizzled
-constexpr int T2_SMEM = T2_STAGES * T2_STAGE + 1024 /*barriers*/ + 2 * T2_STG_BYTES + 1024 /*align*/;
+constexpr int T2_EPI_WARPS = 8;
+constexpr int T2_THREADS = 64 + 32 * T2_EPI_WARPS;
+constexpr int T2_STG_BYTES = 32 * 64 * 2;      // staging tile of one epilogue warp: 32 rows x 64 bf16 columns, 128B-swizzled
+constexpr int T2_SMEM = T2_STAGES * T2_STAGE + 1024 /*barriers*/ + T2_EPI_WARPS * T2_STG_BYTES + 1024 /*align*/;
 constexpr int T2_TMEM_COLS = 512;
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -101,12 +103,12 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* tm, uint32_
                : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ CUtensorMap tmPre,
                          const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ PeerMaps peer_maps,
                          const GemmKernelParams p, const int tma_epilogue, const int tma_aux, const int k_splits,
-                         const int reduce_out) {
+                         const int reduce_out, const int epi_halves) {
   // Copy CTAs come in whole clusters (their count is even) and never touch the cluster barrier.
   if ((int)blockIdx.x < p.n_copy_ctas) {
     gather_copy_role(p);
@@ -120,10 +122,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   auto empty_bar = [&](int s) { return bar_base + 8u * (T2_STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * T2_STAGES + a); };
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * T2_STAGES + 2 + a); };
-  const uint32_t epi_bar = bar_base + 8u * (2 * T2_STAGES + 4);      // the four epilogue warps meet here (128 arrivals)
-  const uint32_t aux_bar = bar_base + 8u * (2 * T2_STAGES + 5);      // aux_in tile landed in the staging buffer
-  const uint32_t stg_base = bar_base + 1024u;                        // two staging buffers
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem_al + T2_STAGES * T2_STAGE + 8 * (2 * T2_STAGES + 6));
+  auto aux_bar = [&](int w) { return bar_base + 8u * (2 * T2_STAGES + 4 + w); };   // aux_in tile of epilogue warp w landed
+  const uint32_t stg_base = bar_base + 1024u;                        // staging tiles of the epilogue warps
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem_al + T2_STAGES * T2_STAGE + 8 * (2 * T2_STAGES + 4 + T2_EPI_WARPS));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -138,10 +139,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 8);
+      mbar_init(tempty_bar(a), 8 * epi_halves);
     }
-    mbar_init(epi_bar, 128);
-    mbar_init(aux_bar, 1);
+    for (int w = 0; w < T2_EPI_WARPS; ++w) mbar_init(aux_bar(w), 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -278,14 +278,43 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         ++it;
       }
     }
-  } else {
-    // ===================== epilogue (warps 2..5 of both CTAs) =====================
+  } else if (warp < 2 + 4 * epi_halves) {
+    // ===================== epilogue (warps 2..5 or 2..9 of both CTAs) =====================
+    // One warp per 32-lane quarter of the accumulator, or two with half of the columns each (epi_halves). A warp stages
+    // its own 32 rows x 64 columns and hands them to the copy engine by itself, so that no warp waits for another one.
     pdl_wait();                                // `out` and aux_in may be in use by earlier kernels until here
     const int q = warp & 3;
+    const int ew = warp - 2;
+    const int half = ew >> 2;                  // which half of the tile's columns (0 when there is one warp per quarter)
+    const int my_cols = T2_BN / epi_halves;
+    const bool two_bufs = epi_halves == 1;     // the staging tiles of the absent warps are the second ones
     const bool out_fp32 = (p.flags & MLF_EPI_OUT_FP32) != 0;
     const bool swiglu = (p.flags & MLF_EPI_SWIGLU) != 0;
     const bool dswiglu = (p.flags & MLF_EPI_DSWIGLU) != 0;
-    uint32_t epi_units = 0;
+    // Column units of this warp: 64 accumulator columns, or 32 where (gate, up) pairs make 64 output columns of them.
+    const int unit_cols = dswiglu ? 32 : 64;
+    const int n_units = my_cols / unit_cols;
+    const uint32_t stg0 = stg_base + (uint32_t)ew * T2_STG_BYTES;
+    uint32_t emits = 0;                        // staging tiles handed out by this warp
+    uint32_t aux_units = 0;                    // aux tiles consumed by this warp
+    // aux_in (residual, dGELU or dSwiGLU input) comes in through the staging tile, one unit ahead
+    int ax_t = pair, ax_u = -1;                // unit whose aux tile was requested last
+    uint32_t ax_n = 0;                         // aux tiles requested
+    auto request_aux = [&]() {                 // lane 0; the staging tile it goes to is free
+      while (true) {
+        if (++ax_u >= n_units) { ax_u = 0; ax_t += n_pairs; }
+        if (ax_t >= num_tiles) return;
+        int tm, tn;
+        tile_coords(ax_t, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);     // k_splits is 1 whenever there is an aux_in
+        const int nb = tn * T2_BN + half * my_cols + ax_u * unit_cols;
+        if (nb >= p.N) continue;
+        mbar_expect_tx(aux_bar(ew), T2_STG_BYTES);
+        tma_load_2d(stg0 + (two_bufs ? (ax_n & 1u) * 4u * T2_STG_BYTES : 0u), &tmAux, dswiglu ? 2 * nb : nb, tm * 256 + (int)rank * BM + q * 32, aux_bar(ew));
+        ++ax_n;
+        return;
+      }
+    };
+    if (tma_aux && lane == 0) request_aux();
     int it = 0;
     for (int t = pair; t < num_tiles; t += n_pairs) {
       if ((t % k_splits) * kb_per >= min(num_kb_all, (t % k_splits) * kb_per + kb_per)) continue;
@@ -293,169 +322,183 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       const uint32_t acc_ph = (it >> 1) & 1;
       int tm, tn;
       tile_coords(t / k_splits, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);
-      const int m = tm * 256 + (int)rank * BM + q * 32 + lane;
-      const int n0 = tn * T2_BN;
+      const int m0 = tm * 256 + (int)rank * BM;
+      const int m = m0 + q * 32 + lane;
+      const int nh = tn * T2_BN + half * my_cols;                       // first column of this warp
+      const uint32_t t_acc = tmem_base + acc * T2_BN + half * my_cols + ((uint32_t)(q * 32) << 16);
       if (!mbar_wait_warp(tfull_bar(acc), acc_ph, abort_flag, p.err, ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after_sync();
       const bool row_ok = m < p.M;
-      char* out_row = nullptr;
-      if (row_ok) {
-        const int esz = out_fp32 ? 4 : 2;
-        if (p.scatter_out) {               // rows routed to their owner's partial buffer (possibly on a peer)
-          const int owner = min(m / p.rows_per_owner, p.world - 1);
-          const long long lr = (long long)p.rank * p.rows_per_owner + (m - owner * p.rows_per_owner);
-          out_row = static_cast<char*>(p.out_peer[owner]) + lr * p.ldo * esz;
-        } else {
-          out_row = static_cast<char*>(p.out) + (long long)m * p.ldo * esz;
-        }
-      }
       if (tma_epilogue) {
-        // Outputs leave through shared memory and TMA stores: each thread writes its row's 64
-        // columns (128 bytes) into a swizzled staging tile, the four warps meet, one thread hands
-        // the tile to the copy engine. Two staging tiles alternate; the elected thread makes sure
-        // the previous store has finished reading before the meeting point that releases its tile.
-        const int r = q * 32 + lane;
-        const bool elected = warp == 2 && lane == 0;
-        const int m_tile = tm * 256 + (int)rank * BM;
-        bool ok = true;
-        // aux_in (residual / dGELU input) comes in through the same staging tile, fetched by the copy
-        // engine one unit ahead: unit u's tile may be overwritten once the store of unit u-2 has
-        // finished reading, which the meeting point of unit u-1 guarantees.
-        auto prefetch_aux = [&](uint32_t unit, int x, int y) {
-          mbar_expect_tx(aux_bar, T2_STG_BYTES);
-          tma_load_2d(stg_base + (unit & 1u) * T2_STG_BYTES, &tmAux, x, y, aux_bar);
-        };
-        if (tma_aux && elected && epi_units == 0) prefetch_aux(0, n0, m_tile);
-        auto emit = [&](const float (&v)[64], const CUtensorMap* tmap, int x) -> bool {
-          const uint32_t buf = stg_base + (epi_units & 1u) * T2_STG_BYTES;
-          const uint32_t rowaddr = buf + r * 128;
+        // a staged row: 64 columns (128 bytes) at x of tmap, or 32 columns (64 bytes, not swizzled) when narrow
+        auto emit = [&](const float* v, const CUtensorMap* tmap, int x, bool narrow) {
+          const uint32_t buf = stg0 + (two_bufs ? (emits & 1u) * 4u * T2_STG_BYTES : 0u);
+          if (!tma_aux) {                      // with an aux tile the buffer is free: its store was waited for before the request
+            if (lane == 0) {
+              if (two_bufs) tma_store_wait_read<1>();
+              else tma_store_wait_read<0>();
+            }
+            __syncwarp();
+          }
+          if (!narrow) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const uint32_t addr = rowaddr + (((uint32_t)c ^ (uint32_t)(r & 7)) << 4);
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pack_bf16x2(v[8 * c], v[8 * c + 1])),
-                         "r"(pack_bf16x2(v[8 * c + 2], v[8 * c + 3])), "r"(pack_bf16x2(v[8 * c + 4], v[8 * c + 5])),
-                         "r"(pack_bf16x2(v[8 * c + 6], v[8 * c + 7])) : "memory");
+            for (int c = 0; c < 8; ++c) {
+              const uint32_t addr = buf + lane * 128 + (((uint32_t)c ^ (uint32_t)(lane & 7)) << 4);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pack_bf16x2(v[8 * c], v[8 * c + 1])),
+                           "r"(pack_bf16x2(v[8 * c + 2], v[8 * c + 3])), "r"(pack_bf16x2(v[8 * c + 4], v[8 * c + 5])),
+                           "r"(pack_bf16x2(v[8 * c + 6], v[8 * c + 7])) : "memory");
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + lane * 64 + c * 16), "r"(pack_bf16x2(v[8 * c], v[8 * c + 1])),
+                           "r"(pack_bf16x2(v[8 * c + 2], v[8 * c + 3])), "r"(pack_bf16x2(v[8 * c + 4], v[8 * c + 5])),
+                           "r"(pack_bf16x2(v[8 * c + 6], v[8 * c + 7])) : "memory");
           }
           fence_proxy_async_smem();
-          if (elected) tma_store_wait_read<0>();
-          mbar_arrive(epi_bar);
-          if (!mbar_wait_warp(epi_bar, epi_units & 1u, abort_flag, p.err, ERR_WAIT_TMEM_FULL)) return false;
-          if (elected) {
+          __syncwarp();
+          if (lane == 0) {
+            const int y = m0 + q * 32;
             if (p.scatter_out) {                 // the whole 128-row block belongs to one owner (possibly a peer)
-              const int owner = min(m_tile / p.rows_per_owner, p.world - 1);
-              tma_store_2d(&peer_maps.m[owner], buf, x, p.rank * p.rows_per_owner + (m_tile - owner * p.rows_per_owner));
+              const int owner = min(m0 / p.rows_per_owner, p.world - 1);
+              tma_store_2d(&peer_maps.m[owner], buf, x, p.rank * p.rows_per_owner + (y - owner * p.rows_per_owner));
             } else if (reduce_out) {
-              tma_reduce_add_2d(tmap, buf, x, m_tile);
+              tma_reduce_add_2d(tmap, buf, x, y);
             } else {
-              tma_store_2d(tmap, buf, x, m_tile);
+              tma_store_2d(tmap, buf, x, y);
             }
             tma_store_commit();
-            if (tma_aux) {                       // next unit: next column group of this tile, or the first of the next tile
-              int nx = x + 64, ny = m_tile;
-              bool have = nx < n0 + T2_BN && nx < p.N;
-              if (!have && t + n_pairs < num_tiles) {
-                int tm2, tn2;
-                tile_coords((t + n_pairs) / k_splits, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm2, tn2);
-                nx = tn2 * T2_BN;
-                ny = tm2 * 256 + (int)rank * BM;
-                have = true;
-              }
-              if (have) prefetch_aux(epi_units + 1, nx, ny);
-            }
           }
-          ++epi_units;
+          ++emits;
+        };
+        // this warp's aux row of the current unit, 64 bf16 in the staging tile
+        auto aux_row = [&](float (&a)[64]) -> bool {
+          if (!mbar_wait_warp(aux_bar(ew), aux_units & 1u, abort_flag, p.err, ERR_WAIT_TMEM_FULL)) return false;
+          const uint32_t src = stg0 + (two_bufs ? (aux_units & 1u) * 4u * T2_STG_BYTES : 0u);
+          ++aux_units;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            uint4 w;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
+                         : "r"(src + lane * 128 + (((uint32_t)c ^ (uint32_t)(lane & 7)) << 4)));
+            const float2 f0 = unpack_bf16x2(w.x), f1 = unpack_bf16x2(w.y), f2 = unpack_bf16x2(w.z), f3 = unpack_bf16x2(w.w);
+            a[8 * c + 0] = f0.x; a[8 * c + 1] = f0.y; a[8 * c + 2] = f1.x; a[8 * c + 3] = f1.y;
+            a[8 * c + 4] = f2.x; a[8 * c + 5] = f2.y; a[8 * c + 6] = f3.x; a[8 * c + 7] = f3.y;
+          }
           return true;
         };
+        bool ok = true;
 #pragma unroll 1
-        for (int g = 0; g < T2_BN / 64 && ok; ++g) {
-          const int nb = n0 + 64 * g;
+        for (int u = 0; u < n_units && ok; ++u) {
+          const int nb = nh + u * unit_cols;
           if (nb >= p.N) break;
-          float v[64];
-#pragma unroll
-          for (int h2 = 0; h2 < 2; ++h2) {
+          if (dswiglu) {
+            // v = dL/dh of 32 hidden columns; aux holds their (gate, up) pairs, out gets (dgate, dup)
             uint32_t t32[32];
-            tmem_ld_32x32b_x32(tmem_base + acc * T2_BN + g * 64 + h2 * 32 + ((uint32_t)(q * 32) << 16), t32);
+            tmem_ld_32x32b_x32(t_acc + u * 32, t32);
+            float gu[64];
+            ok = aux_row(gu);
+            if (!ok) break;
             tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[32 * h2 + j] = __uint_as_float(t32[j]) * p.alpha;
-          }
-          const int nvalid = min(64, p.N - nb);
-          if (p.flags & MLF_EPI_BIAS) {
-            if (nvalid == 64 && ((reinterpret_cast<uintptr_t>(p.bias + nb) & 15) == 0)) {
-#pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                const uint4 w = reinterpret_cast<const uint4*>(p.bias + nb)[c];
-                const float2 f0 = unpack_bf16x2(w.x), f1 = unpack_bf16x2(w.y), f2 = unpack_bf16x2(w.z), f3 = unpack_bf16x2(w.w);
-                v[8 * c + 0] += f0.x; v[8 * c + 1] += f0.y; v[8 * c + 2] += f1.x; v[8 * c + 3] += f1.y;
-                v[8 * c + 4] += f2.x; v[8 * c + 5] += f2.y; v[8 * c + 6] += f3.x; v[8 * c + 7] += f3.y;
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 64; ++j)
-                if (j < nvalid) v[j] += __bfloat162float(p.bias[nb + j]);
+            for (int j = 0; j < 32; ++j) {
+              const float gate = gu[2 * j], up = gu[2 * j + 1], dh = __uint_as_float(t32[j]) * p.alpha;
+              const float sg = 1.f / (1.f + __expf(-gate));
+              gu[2 * j] = dh * up * sg * (1.f + gate * (1.f - sg));
+              gu[2 * j + 1] = dh * gate * sg;
             }
-          }
-          if (p.flags & MLF_EPI_STORE_PRE) {
-            ok = emit(v, &tmPre, nb);
-            if (!ok) break;
-          }
-          if (p.flags & MLF_EPI_GELU) {
+            emit(gu, &tmOut, 2 * nb, false);
+          } else {
+            float v[64];
 #pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = gelu_tanh(v[j]);
-          }
-          if (p.flags & (MLF_EPI_RESIDUAL | MLF_EPI_DGELU_MUL)) {
-            const bool resid = (p.flags & MLF_EPI_RESIDUAL) != 0;
-            const __nv_bfloat16* ar = p.aux_in + (long long)m * p.ld_aux_in + nb;
-            if (tma_aux) {
-              if (!mbar_wait_warp(aux_bar, epi_units & 1u, abort_flag, p.err, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-              const uint32_t rowaddr = stg_base + (epi_units & 1u) * T2_STG_BYTES + r * 128;
+            for (int h2 = 0; h2 < 2; ++h2) {
+              uint32_t t32[32];
+              tmem_ld_32x32b_x32(t_acc + u * 64 + h2 * 32, t32);
+              tmem_wait_ld();
 #pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                uint4 w;
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
-                             : "r"(rowaddr + (((uint32_t)c ^ (uint32_t)(r & 7)) << 4)));
-                const float2 f0 = unpack_bf16x2(w.x), f1 = unpack_bf16x2(w.y), f2 = unpack_bf16x2(w.z), f3 = unpack_bf16x2(w.w);
-                const float a8[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
+              for (int j = 0; j < 32; ++j) v[32 * h2 + j] = __uint_as_float(t32[j]) * p.alpha;
+            }
+            const int nvalid = min(64, p.N - nb);
+            if (p.flags & MLF_EPI_BIAS) {
+              if (nvalid == 64 && ((reinterpret_cast<uintptr_t>(p.bias + nb) & 15) == 0)) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[8 * c + j] = resid ? v[8 * c + j] + a8[j] : v[8 * c + j] * dgelu_tanh(a8[j]);
-              }
-            } else if (row_ok && nvalid == 64 && ((reinterpret_cast<uintptr_t>(ar) & 15) == 0)) {
+                for (int c = 0; c < 8; ++c) {
+                  const uint4 w = reinterpret_cast<const uint4*>(p.bias + nb)[c];
+                  const float2 f0 = unpack_bf16x2(w.x), f1 = unpack_bf16x2(w.y), f2 = unpack_bf16x2(w.z), f3 = unpack_bf16x2(w.w);
+                  v[8 * c + 0] += f0.x; v[8 * c + 1] += f0.y; v[8 * c + 2] += f1.x; v[8 * c + 3] += f1.y;
+                  v[8 * c + 4] += f2.x; v[8 * c + 5] += f2.y; v[8 * c + 6] += f3.x; v[8 * c + 7] += f3.y;
+                }
+              } else {
 #pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                const uint4 w = reinterpret_cast<const uint4*>(ar)[c];
-                const float2 f0 = unpack_bf16x2(w.x), f1 = unpack_bf16x2(w.y), f2 = unpack_bf16x2(w.z), f3 = unpack_bf16x2(w.w);
-                const float a8[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[8 * c + j] = resid ? v[8 * c + j] + a8[j] : v[8 * c + j] * dgelu_tanh(a8[j]);
-              }
-            } else if (row_ok) {
-#pragma unroll
-              for (int j = 0; j < 64; ++j) {
-                const float a1 = j < nvalid ? __bfloat162float(ar[j]) : 0.f;
-                v[j] = resid ? v[j] + a1 : v[j] * dgelu_tanh(a1);
+                for (int j = 0; j < 64; ++j)
+                  if (j < nvalid) v[j] += __bfloat162float(p.bias[nb + j]);
               }
             }
+            if (p.flags & MLF_EPI_STORE_PRE) emit(v, &tmPre, nb, false);
+            if (swiglu) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = silu(v[2 * j]) * v[2 * j + 1];
+              emit(v, &tmOut, nb / 2, true);
+              continue;
+            }
+            if (p.flags & MLF_EPI_GELU) {
+#pragma unroll
+              for (int j = 0; j < 64; ++j) v[j] = gelu_tanh(v[j]);
+            }
+            if (p.flags & (MLF_EPI_RESIDUAL | MLF_EPI_DGELU_MUL)) {
+              const bool resid = (p.flags & MLF_EPI_RESIDUAL) != 0;
+              if (tma_aux) {
+                float a[64];
+                ok = aux_row(a);
+                if (!ok) break;
+#pragma unroll
+                for (int j = 0; j < 64; ++j) v[j] = resid ? v[j] + a[j] : v[j] * dgelu_tanh(a[j]);
+              } else if (row_ok) {
+                const __nv_bfloat16* ar = p.aux_in + (long long)m * p.ld_aux_in + nb;
+#pragma unroll
+                for (int j = 0; j < 64; ++j) {
+                  const float a1 = j < nvalid ? __bfloat162float(ar[j]) : 0.f;
+                  v[j] = resid ? v[j] + a1 : v[j] * dgelu_tanh(a1);
+                }
+              }
+            }
+            emit(v, &tmOut, nb, false);
           }
-          ok = emit(v, &tmOut, nb);
+          if (tma_aux && lane == 0) {          // the next unit's aux tile, once the store that read its buffer is through
+            if (two_bufs) tma_store_wait_read<1>();
+            else tma_store_wait_read<0>();
+            request_aux();
+          }
         }
         if (!ok) break;
       } else {
+        char* out_row = nullptr;
+        if (row_ok) {
+          const int esz = out_fp32 ? 4 : 2;
+          if (p.scatter_out) {               // rows routed to their owner's partial buffer (possibly on a peer)
+            const int owner = min(m / p.rows_per_owner, p.world - 1);
+            const long long lr = (long long)p.rank * p.rows_per_owner + (m - owner * p.rows_per_owner);
+            out_row = static_cast<char*>(p.out_peer[owner]) + lr * p.ldo * esz;
+          } else {
+            out_row = static_cast<char*>(p.out) + (long long)m * p.ldo * esz;
+          }
+        }
 #pragma unroll 1
-      for (int c = 0; c < T2_BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(tmem_base + acc * T2_BN + c * 32 + ((uint32_t)(q * 32) << 16), r);
-        tmem_wait_ld();
-        const int nb = n0 + c * 32;
-        if (!row_ok || nb >= p.N) continue;
-        gemm_epilogue_chunk(p, m, nb, r, out_row, out_fp32, swiglu, dswiglu);
-      }
+        for (int c = 0; c < my_cols / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(t_acc + c * 32, r);
+          tmem_wait_ld();
+          const int nb = nh + c * 32;
+          if (!row_ok || nb >= p.N) continue;
+          gemm_epilogue_chunk(p, m, nb, r, out_row, out_fp32, swiglu, dswiglu);
+        }
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
       ++it;
     }
-    if (tma_epilogue && warp == 2 && lane == 0) tma_store_wait_all<0>();   // shared memory stays valid until the copies have read it
+    if (tma_epilogue && lane == 0) tma_store_wait_all<0>();   // shared memory stays valid until the copies have read it
   }
 
   // ===================== teardown =====================
@@ -556,34 +599,42 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   if (!a->b_mn) rc = cached_tmap_bf16(&tmB, b_base, a->K, a->N, a->ldb, BK, T2_BNH);
   else rc = cached_tmap_bf16(&tmB, b_base, a->N, a->K, a->ldb, 64, BK);
   if (rc) return rc;
-  // Outputs go through TMA stores when they are plain bf16 rows this GPU owns.
+  // Outputs go through TMA stores when they are bf16 rows with aligned pitches.
   CUtensorMap tmOut = tmA, tmPre = tmA, tmAux = tmA;
   PeerMaps peer_maps;                        // only read by the kernel when rows are routed
   memset(&peer_maps, 0, sizeof(peer_maps));
   int tma_epi = 0, tma_aux = 0;
   const bool scatter = cm && cm->scatter_out;
   const bool plain = (a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) == 0 && cm == nullptr;      // nothing but (optionally) out += product
-  if (!(a->flags & (MLF_EPI_OUT_FP32 | MLF_EPI_SWIGLU | MLF_EPI_DSWIGLU)) && (!(a->flags & MLF_EPI_ACCUM) || plain) && a->ldo % 8 == 0 &&
+  const bool sw = (a->flags & MLF_EPI_SWIGLU) != 0, dsw = (a->flags & MLF_EPI_DSWIGLU) != 0;
+  const bool aux_aligned = a->ld_aux_in % 8 == 0 && (reinterpret_cast<uintptr_t>(a->aux_in) & 15) == 0;
+  // (gate, up) forms: no other operation beside theirs, whole pairs, and the aux tile through the copy engine
+  const bool gated_ok = !(sw || dsw) || (!scatter && !(sw && dsw) && a->N % 2 == 0 &&
+                                         !(a->flags & (MLF_EPI_GELU | MLF_EPI_RESIDUAL | MLF_EPI_DGELU_MUL)) &&
+                                         (!dsw || (aux_aligned && !(a->flags & (MLF_EPI_STORE_PRE | MLF_EPI_BIAS)))));
+  if (!(a->flags & MLF_EPI_OUT_FP32) && gated_ok && (!(a->flags & MLF_EPI_ACCUM) || plain) && a->ldo % 8 == 0 &&
       (scatter || (reinterpret_cast<uintptr_t>(a->out) & 15) == 0) &&
       (!(a->flags & MLF_EPI_STORE_PRE) || (a->ld_aux_out % 8 == 0 && (reinterpret_cast<uintptr_t>(a->aux_out) & 15) == 0))) {
     if (scatter) {
       for (int r = 0; r < cm->world; ++r) {
         MLF_REQUIRE((reinterpret_cast<uintptr_t>(cm->out_peer[r]) & 15) == 0, "partial buffers must be 16-byte aligned");
-        rc = cached_tmap_bf16(&peer_maps.m[r], cm->out_peer[r], a->N, (uint64_t)cm->world * cm->rows_per_owner, a->ldo, 64, 128);
+        rc = cached_tmap_bf16(&peer_maps.m[r], cm->out_peer[r], a->N, (uint64_t)cm->world * cm->rows_per_owner, a->ldo, 64, 32);
         if (rc) return rc;
       }
+    } else if (sw) {
+      rc = cached_tmap_bf16(&tmOut, a->out, a->N / 2, a->M, a->ldo, 32, 32, false);
+      if (rc) return rc;
     } else {
-      rc = cached_tmap_bf16(&tmOut, a->out, a->N, a->M, a->ldo, 64, 128);
+      rc = cached_tmap_bf16(&tmOut, a->out, dsw ? 2 * (uint64_t)a->N : a->N, a->M, a->ldo, 64, 32);
       if (rc) return rc;
     }
     if (a->flags & MLF_EPI_STORE_PRE) {
-      rc = cached_tmap_bf16(&tmPre, a->aux_out, a->N, a->M, a->ld_aux_out, 64, 128);
+      rc = cached_tmap_bf16(&tmPre, a->aux_out, a->N, a->M, a->ld_aux_out, 64, 32);
       if (rc) return rc;
     }
     tma_epi = 1;
-    if ((a->flags & (MLF_EPI_RESIDUAL | MLF_EPI_DGELU_MUL)) && !(a->flags & MLF_EPI_STORE_PRE) && a->ld_aux_in % 8 == 0 &&
-        (reinterpret_cast<uintptr_t>(a->aux_in) & 15) == 0) {
-      rc = cached_tmap_bf16(&tmAux, a->aux_in, a->N, a->M, a->ld_aux_in, 64, 128);
+    if ((a->flags & (MLF_EPI_RESIDUAL | MLF_EPI_DGELU_MUL | MLF_EPI_DSWIGLU)) && !(a->flags & MLF_EPI_STORE_PRE) && aux_aligned) {
+      rc = cached_tmap_bf16(&tmAux, a->aux_in, dsw ? 2 * (uint64_t)a->N : a->N, a->M, a->ld_aux_in, 64, 32);
       if (rc) return rc;
       tma_aux = 1;
     }
@@ -601,7 +652,7 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   if (!max_clusters[dev & 63]) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (sm_count() / 2));
-    cfg.blockDim = dim3(kGemmThreads);
+    cfg.blockDim = dim3(T2_THREADS);
     cfg.dynamicSmemBytes = T2_SMEM;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -630,6 +681,13 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
       if (cost < best * 0.9) { best = cost; k_splits = ks; }
     }
   }
+  // Two epilogue warps per quarter where the work of one does not fit behind the next tile's products: gated and
+  // derivative epilogues (8192 x 14336 x 4096 with dSwiGLU 960 -> 691 us, 4096 x 28672 x 4096 with SwiGLU 686 -> 612 us,
+  // 8192 x 8192 x 2048 with dGELU 225 -> 211 us), a residual (its tile has to arrive first), and any short K (2331 x 4096
+  // x 1024 with GELU 33.5 -> 28.1 us). Elsewhere the second warp only takes power from the products: 8192 x 8192 x 2048
+  // plain 182 us with one, 186 us with two.
+  const bool heavy = (a->flags & (MLF_EPI_DGELU_MUL | MLF_EPI_SWIGLU | MLF_EPI_DSWIGLU | MLF_EPI_RESIDUAL)) != 0;
+  const int epi_halves = heavy || a->K <= 1024 * k_splits ? 2 : 1;
   const int reduce_out = (k_splits > 1 || (a->flags & MLF_EPI_ACCUM)) ? 1 : 0;
   if (k_splits > 1 && !(a->flags & MLF_EPI_ACCUM))
     MLF_CHECK_CUDA(cudaMemset2DAsync(a->out, (size_t)a->ldo * 2, 0, (size_t)a->N * 2, (size_t)a->M, st));
@@ -638,11 +696,11 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   if (pairs > num_tiles * k_splits) pairs = num_tiles * k_splits;
   if (pairs < 1) pairs = 1;
   if (cm == nullptr) {
-    MLF_CHECK_CUDA(launch_pdl(gemm_tcgen05_2cta_kernel, dim3(2 * pairs), dim3(kGemmThreads), T2_SMEM, st, tmA, tmB, tmOut, tmPre, tmAux,
-                              peer_maps, p, tma_epi, tma_aux, k_splits, reduce_out));
+    MLF_CHECK_CUDA(launch_pdl(gemm_tcgen05_2cta_kernel, dim3(2 * pairs), dim3(T2_THREADS), T2_SMEM, st, tmA, tmB, tmOut, tmPre, tmAux,
+                              peer_maps, p, tma_epi, tma_aux, k_splits, reduce_out, epi_halves));
   } else {                                       // copy CTAs and routed rows touch peers' memory: after everything ahead
-    gemm_tcgen05_2cta_kernel<<<n_copy + 2 * pairs, kGemmThreads, T2_SMEM, st>>>(tmA, tmB, tmOut, tmPre, tmAux, peer_maps, p, tma_epi, tma_aux,
-                                                                                k_splits, reduce_out);
+    gemm_tcgen05_2cta_kernel<<<n_copy + 2 * pairs, T2_THREADS, T2_SMEM, st>>>(tmA, tmB, tmOut, tmPre, tmAux, peer_maps, p, tma_epi, tma_aux,
+                                                                                k_splits, reduce_out, epi_halves);
     MLF_CHECK_CUDA(cudaGetLastError());
   }
   count_launch();
