@@ -46,7 +46,23 @@ struct PagedDecodeParams {
   int B, Hq, Hkv, G, block_size, bs_shift, max_blocks, num_blocks, split_tokens, splits;   // bs_shift: log2(block_size) or -1
   float scale_log2;
   int* err;
+  // packed form (mlf_paged_decode_rope): q, k_new and v_new are unrotated heads of packed QKV rows of pitch ldq, the new
+  // token of a sequence is its last one (position seq_lens - 1) and its key and value go to cache slot slots[b]
+  const __nv_bfloat16* k_new;
+  const __nv_bfloat16* v_new;
+  const long long* slots;
+  float theta;
 };
+
+// Rotary embedding of a pair (d, d + 64) at position pos, as rope_kv_write_kernel computes it.
+__device__ __forceinline__ void rope_pair(float& a, float& b, int d, float pos, float log_theta) {
+  const float inv_freq = __expf(-log_theta * (2.f * d / PD));
+  float sn, cs;
+  sincosf(pos * inv_freq, &sn, &cs);
+  const float x = a, y = b;
+  a = x * cs - y * sn;
+  b = y * cs + x * sn;
+}
 
 // 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros (rows past the sequence end)
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int src_bytes) {
@@ -113,7 +129,11 @@ __device__ __forceinline__ void finish_split(const PagedDecodeParams& p, int b, 
 // of the tcgen05 path, and this way a chunk costs a warp ~100 instructions instead of ~1000 scalar
 // ones. Each warp owns 16 tokens of every chunk with its own running (max, sum, output); the four
 // warps merge at the end. Each sequence divides its own length evenly over the launch's splits.
-template <int G>
+//
+// ROPE: the rotary embedding of the query heads and of the new key, and the write of the new key and value to the cache,
+// happen here: the CTA whose split holds the last token puts its row into the staged chunk from registers. A launch of
+// its own for that stood between the QKV product and this kernel in every layer of a decode step.
+template <int G, bool ROPE>
 __global__ void __launch_bounds__(P_THREADS)
 paged_decode_kernel(const PagedDecodeParams p) {
   extern __shared__ __align__(128) uint8_t p_dsm[];
@@ -170,7 +190,7 @@ paged_decode_kernel(const PagedDecodeParams p) {
 #pragma unroll
       for (int e = 0; e < P_CH / 8; ++e) {
         const int i = tg + 8 * e;
-        const int sz = tbase + i < t_hi ? 16 : 0;
+        const int sz = tbase + i < t_hi && !(ROPE && tbase + i == len - 1) ? 16 : 0;   // the new row comes from registers
         if (blk[e] < 0 || blk[e] >= p.num_blocks) { atomicCAS(p.err, 0, ERR_BAD_INDEX); blk[e] = 0; }
         const __nv_bfloat16* src = p.cache + blk[e] * blk_stride + ((long long)(tt[e] - lb[e] * p.block_size) * p.Hkv + hkv) * PD + dl * 8;
         const uint32_t off = stage + chunk_off(i, dl);
@@ -182,6 +202,40 @@ paged_decode_kernel(const PagedDecodeParams p) {
   };
   issue(0);
   issue(1);
+
+  const float log_theta = ROPE ? __logf(p.theta) : 0.f;
+  // the new token's key (rotated) and value, 16 bytes of each in the 16 threads that stage its row
+  uint4 nk = make_uint4(0u, 0u, 0u, 0u), nv = nk;
+  const bool has_new = ROPE && t_hi == len;
+  const int new_i = (len - 1 - t_lo) % P_CH, new_c = (len - 1 - t_lo) / P_CH;
+  if (has_new && tg == (new_i & 7)) {
+    const __nv_bfloat16* kr = p.k_new + (long long)b * p.ldq + (long long)hkv * PD;
+    const uint4 own = *reinterpret_cast<const uint4*>(kr + dl * 8), other = *reinterpret_cast<const uint4*>(kr + (dl ^ 8) * 8);
+    nv = *reinterpret_cast<const uint4*>(p.v_new + (long long)b * p.ldq + (long long)hkv * PD + dl * 8);
+    const uint32_t* ow = reinterpret_cast<const uint32_t*>(&own);
+    const uint32_t* tw = reinterpret_cast<const uint32_t*>(&other);
+    uint32_t rw[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 a = unpack_bf16x2(dl < 8 ? ow[j] : tw[j]), c = unpack_bf16x2(dl < 8 ? tw[j] : ow[j]);
+      float2 lo = a, hi = c;
+      rope_pair(lo.x, hi.x, (dl & 7) * 8 + 2 * j, (float)(len - 1), log_theta);
+      rope_pair(lo.y, hi.y, (dl & 7) * 8 + 2 * j + 1, (float)(len - 1), log_theta);
+      rw[j] = dl < 8 ? pack_bf16x2(lo.x, lo.y) : pack_bf16x2(hi.x, hi.y);
+    }
+    nk = make_uint4(rw[0], rw[1], rw[2], rw[3]);
+    const long long slot = p.slots[b];
+    if (slot >= 0) {
+      const long long blk = slot / p.block_size;
+      if (blk >= p.num_blocks) {
+        atomicCAS(p.err, 0, ERR_BAD_INDEX);
+      } else {
+        __nv_bfloat16* kd = const_cast<__nv_bfloat16*>(p.cache) + blk * blk_stride + ((slot % p.block_size) * p.Hkv + hkv) * PD + dl * 8;
+        *reinterpret_cast<uint4*>(kd) = nk;
+        *reinterpret_cast<uint4*>(kd + v_off) = nv;
+      }
+    }
+  }
 
   // Q as the A operand: row = lane / 4 is the head of the group (rows >= G and rows 8..15 are zero)
   const int qrow = lane >> 2, qcol = (lane & 3) * 2;
@@ -195,6 +249,18 @@ paged_decode_kernel(const PagedDecodeParams p) {
       qa[ks][1] = *reinterpret_cast<const uint32_t*>(qp + 8);
     }
   }
+  if (ROPE && qrow < G) {
+#pragma unroll
+    for (int ks = 0; ks < PD / 32; ++ks)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float2 lo = unpack_bf16x2(qa[ks][h]), hi = unpack_bf16x2(qa[ks + PD / 32][h]);
+        rope_pair(lo.x, hi.x, ks * 16 + h * 8 + qcol, (float)(len - 1), log_theta);
+        rope_pair(lo.y, hi.y, ks * 16 + h * 8 + qcol + 1, (float)(len - 1), log_theta);
+        qa[ks][h] = pack_bf16x2(lo.x, lo.y);
+        qa[ks + PD / 32][h] = pack_bf16x2(hi.x, hi.y);
+      }
+  }
   float o[PD / 8][4];
 #pragma unroll
   for (int nt = 0; nt < PD / 8; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
@@ -206,6 +272,10 @@ paged_decode_kernel(const PagedDecodeParams p) {
     const int tok0 = warp * 16;              // this warp's 16 tokens of the chunk
     const bool active = tok0 < cn;           // warp-uniform
     cp_async_wait<1>();                      // chunk c: one younger group may still be in flight
+    if (has_new && c == new_c && tg == (new_i & 7)) {      // over this thread's own zero-filled copy, which has landed
+      *reinterpret_cast<uint4*>(p_dsm + (kst - sK) + chunk_off(new_i, dl)) = nk;
+      *reinterpret_cast<uint4*>(p_dsm + (vst - sK) + chunk_off(new_i, dl)) = nv;
+    }
     __syncthreads();
     float sacc[2][4];
     if (active) {
@@ -473,12 +543,11 @@ MLF_API int mlf_paged_decode(const void* q, const void* cache, const int* block_
                              num_blocks, max_seq_len, split_tokens, scale, stream);
 }
 
-// q rows may sit inside a wider packed buffer: ldq = elements between consecutive sequences' query rows.
-// counters (optional, B * Hkv zeroed uint32 that the kernel leaves zero): the last split of each (sequence, kv head)
-// merges the splits inside the same launch; without it a second small kernel does.
-MLF_API int mlf_paged_decode_ld(const void* q, long long ldq, const void* cache, const int* block_table, const int* seq_lens, void* out,
-                                float* ws, void* counters, int B, int Hq, int Hkv, int block_size, int max_blocks, int num_blocks,
-                                int max_seq_len, int split_tokens, float scale, uint64_t stream) {
+namespace mlf {
+// slots != null: the packed form (theta)
+static int launch_paged_decode(const void* q, long long ldq, const void* cache, const int* block_table, const int* seq_lens,
+                               const long long* slots, void* out, float* ws, void* counters, int B, int Hq, int Hkv, int block_size,
+                               int max_blocks, int num_blocks, int max_seq_len, int split_tokens, float scale, float theta, uint64_t stream) {
   MLF_REQUIRE(ldq % 2 == 0 && (reinterpret_cast<uintptr_t>(q) & 3) == 0, "paged_decode: query rows must be 4-byte aligned");
   MLF_REQUIRE(B > 0 && Hq % Hkv == 0, "paged_decode: bad head counts");
   const int G = Hq / Hkv;
@@ -502,19 +571,25 @@ MLF_API int mlf_paged_decode_ld(const void* q, long long ldq, const void* cache,
   for (int sh = 0; sh < 16; ++sh) if ((1 << sh) == block_size) p.bs_shift = sh;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.err = device_status_word();
+  const bool rope = slots != nullptr;
+  p.k_new = rope ? p.q + (long long)Hq * PD : nullptr;
+  p.v_new = rope ? p.k_new + (long long)Hkv * PD : nullptr;
+  p.slots = slots;
+  p.theta = theta;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   dim3 grid(B, Hkv, splits);
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
+  void (*const kernels[2][4])(PagedDecodeParams) = {
+      {paged_decode_kernel<1, false>, paged_decode_kernel<2, false>, paged_decode_kernel<4, false>, paged_decode_kernel<8, false>},
+      {paged_decode_kernel<1, true>, paged_decode_kernel<2, true>, paged_decode_kernel<4, true>, paged_decode_kernel<8, true>}};
   if (!attr_set[dev & 63]) {
-    MLF_CHECK_CUDA(cudaFuncSetAttribute(paged_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
-    MLF_CHECK_CUDA(cudaFuncSetAttribute(paged_decode_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
-    MLF_CHECK_CUDA(cudaFuncSetAttribute(paged_decode_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
-    MLF_CHECK_CUDA(cudaFuncSetAttribute(paged_decode_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
+    for (int i = 0; i < 8; ++i)
+      MLF_CHECK_CUDA(cudaFuncSetAttribute(kernels[i / 4][i % 4], cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
     attr_set[dev & 63] = true;
   }
-  const auto kernel = G == 1 ? paged_decode_kernel<1> : G == 2 ? paged_decode_kernel<2> : G == 4 ? paged_decode_kernel<4> : paged_decode_kernel<8>;
+  const auto kernel = kernels[rope ? 1 : 0][G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : 3];
   MLF_CHECK_CUDA(launch_pdl(kernel, grid, dim3(P_THREADS), P_SMEM, st, p));
   count_launch();
   if (splits > 1 && p.counters == nullptr) {
@@ -522,6 +597,30 @@ MLF_API int mlf_paged_decode_ld(const void* q, long long ldq, const void* cache,
     count_launch();
   }
   return 0;
+}
+}  // namespace mlf
+
+// q rows may sit inside a wider packed buffer: ldq = elements between consecutive sequences' query rows.
+// counters (optional, B * Hkv zeroed uint32 that the kernel leaves zero): the last split of each (sequence, kv head)
+// merges the splits inside the same launch; without it a second small kernel does.
+MLF_API int mlf_paged_decode_ld(const void* q, long long ldq, const void* cache, const int* block_table, const int* seq_lens, void* out,
+                                float* ws, void* counters, int B, int Hq, int Hkv, int block_size, int max_blocks, int num_blocks,
+                                int max_seq_len, int split_tokens, float scale, uint64_t stream) {
+  return launch_paged_decode(q, ldq, cache, block_table, seq_lens, nullptr, out, ws, counters, B, Hq, Hkv, block_size, max_blocks,
+                             num_blocks, max_seq_len, split_tokens, scale, 0.f, stream);
+}
+
+// Decode attention straight from the QKV product: qkv [B, (Hq + 2 Hkv) * 128] (pitch ld, 16-byte aligned rows), not yet
+// rotated. The new token of sequence b is the last of its seq_lens[b] tokens; its rotated key and its value are written
+// to cache slot slots[b] (< 0: not written) and attended to like the cached ones. Same results as mlf_rope_kv_write with
+// positions seq_lens - 1 followed by mlf_paged_decode_ld.
+MLF_API int mlf_paged_decode_rope(const void* qkv, long long ld, void* cache, const int* block_table, const int* seq_lens,
+                                  const long long* slots, void* out, float* ws, int B, int Hq, int Hkv, int block_size, int max_blocks,
+                                  int num_blocks, int max_seq_len, int split_tokens, float scale, float theta, uint64_t stream) {
+  MLF_REQUIRE(slots != nullptr && theta > 0.f, "paged_decode_rope: slots and a positive theta are needed");
+  MLF_REQUIRE(ld % 8 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 15) == 0, "paged_decode_rope: rows must be 16-byte aligned");
+  return launch_paged_decode(qkv, ld, cache, block_table, seq_lens, slots, out, ws, nullptr, B, Hq, Hkv, block_size, max_blocks, num_blocks,
+                             max_seq_len, split_tokens, scale, theta, stream);
 }
 
 MLF_API int mlf_kv_cache_write(void* cache, const void* k, const void* v, const long long* slots, long long T, int Hkv,

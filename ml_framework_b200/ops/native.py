@@ -344,6 +344,16 @@ def flash_bwd(q, k, v, o, dout, lse, B: int, S: int, *, causal: bool = True, sca
 
 
 # ------------------------------------------------------------------ paged attention / KV cache
+def _decode_split(pairs: int, max_seq_len: int) -> int:
+    """Tokens per split of the decode kernel for ``pairs`` (sequence, KV head) pairs: as many splits as keep all CTAs
+    resident at once (three per SM, 444), none when the pairs alone fill the GPU -- CTAs of a second round start when the
+    short sequences of the first end, and a split costs its start and the merge launch. At least 128 tokens per split.
+    13 sequences of up to 2500 tokens x 8 KV heads: 4 splits 26 us (8: 29 us); 64 of up to 576: none 28.6 us (2: 31 us);
+    128 of up to 1024: none 74 us (2: 79 us); 8 of up to 4000: 6 splits 27.5 us (11: 33 us)."""
+    splits = min(max(1, 444 // pairs), max(1, -(-max_seq_len // 128)))
+    return -(-max_seq_len // splits)
+
+
 def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Tensor, seq_lens: torch.Tensor,
                  max_seq_len: int, *, scale: Optional[float] = None, split_tokens: int = 512, fused_merge: bool = False) -> torch.Tensor:
     """One query token per sequence against its paged KV cache.
@@ -363,10 +373,7 @@ def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Ten
     L = _L()
     L.mlf_paged_decode_ws_elems.restype = C.c_longlong
     if split_tokens <= 0:
-        # automatic: about two waves of CTAs (three resident per SM on 148 SMs), at least 128 tokens per split
-        want = max(1, -(-888 // (B * Hkv)))
-        want = min(want, max(1, (max_seq_len + 127) // 128))
-        split_tokens = -(-max_seq_len // want)
+        split_tokens = _decode_split(B * Hkv, max_seq_len)
     st = (max(split_tokens, 128) + 127) // 128 * 128
     splits = max(1, (max_seq_len + st - 1) // st)
     ws = scratch("paged_decode", L.mlf_paged_decode_ws_elems(B, Hq, splits) * 4, q.device) if splits > 1 else None
@@ -381,6 +388,31 @@ def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Ten
     rc = L.mlf_paged_decode_ld(_p(q), C.c_longlong(q.stride(0)), _p(kv_cache), _p(block_table), _p(seq_lens), _p(out), _p(ws), _p(ctr), B, Hq, Hkv,
                                bs, block_table.shape[1], nb, int(max_seq_len), st, C.c_float(scale), _st())
     _lib.check(rc, "mlf_paged_decode_ld")
+    return out
+
+
+def paged_decode_rope(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Tensor, seq_lens: torch.Tensor, slots: torch.Tensor,
+                      Hq: int, Hkv: int, max_seq_len: int, theta: float, *, scale: Optional[float] = None, split_tokens: int = 0) -> torch.Tensor:
+    """:func:`rope_kv_write_` at positions ``seq_lens - 1`` followed by :func:`paged_decode` in one launch: ``qkv``
+    [B, (Hq + 2 Hkv) * 128] holds the unrotated projection of each sequence's newest token, which ``seq_lens`` counts;
+    its key and value go to cache slot ``slots`` (int64, < 0 skips the write). ``qkv`` is left as it is."""
+    B = qkv.shape[0]
+    nb, two, bs, Hc, D = kv_cache.shape
+    assert D == 128 and two == 2 and Hc == Hkv and kv_cache.is_contiguous() and qkv.shape[1] == (Hq + 2 * Hkv) * D
+    assert qkv.stride(1) == 1 and qkv.dtype == torch.bfloat16 and kv_cache.dtype == torch.bfloat16 and slots.dtype == torch.int64
+    assert block_table.dtype == torch.int32 and block_table.is_contiguous() and seq_lens.dtype == torch.int32
+    out = torch.empty(B, Hq, D, dtype=qkv.dtype, device=qkv.device)
+    L = _L()
+    L.mlf_paged_decode_ws_elems.restype = C.c_longlong
+    if split_tokens <= 0:
+        split_tokens = _decode_split(B * Hkv, max_seq_len)
+    st = (max(split_tokens, 128) + 127) // 128 * 128
+    splits = max(1, (max_seq_len + st - 1) // st)
+    ws = torch.empty(int(L.mlf_paged_decode_ws_elems(B, Hq, splits)), dtype=torch.float32, device=qkv.device) if splits > 1 else None
+    rc = L.mlf_paged_decode_rope(_p(qkv), C.c_longlong(qkv.stride(0)), _p(kv_cache), _p(block_table), _p(seq_lens.contiguous()),
+                                 _p(slots.contiguous()), _p(out), _p(ws), B, Hq, Hkv, bs, block_table.shape[1], nb, int(max_seq_len), st,
+                                 C.c_float(scale if scale is not None else D ** -0.5), C.c_float(theta), _st())
+    _lib.check(rc, "mlf_paged_decode_rope")
     return out
 
 

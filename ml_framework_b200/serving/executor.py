@@ -112,7 +112,9 @@ class PagedLlamaExecutor:
         return h, gemm(h, w, out=out, flags=_lib.EPI_ACCUM | _lib.EPI_B_STATIC)
 
     # ---- one transformer block over T tokens
-    def _block(self, li: int, blk, x: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, attend):
+    def _block(self, li: int, blk, x: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, attend, attend_packed=None):
+        """``attend(li, q, k, v)`` gets rotated heads whose keys and values are in the cache; ``attend_packed(li, qkv)``
+        (native path), where given, does the rotation and the cache write itself."""
         mc = self.mc
         D = mc.head_dim
         attn = blk.attn if hasattr(blk, "attn") else None
@@ -127,11 +129,14 @@ class PagedLlamaExecutor:
             # and accumulate, into a buffer that the normalisation's launch clears; the weights are read ahead.
             few_rows = T <= 256
             h, qkv = self._norm_product(x, blk.norm1.weight, qkv_w, few_rows)
-            q = qkv[:, :self.hq * D].view(T, self.hq, D)
-            k = qkv[:, self.hq * D:(self.hq + self.hkv) * D].view(T, self.hkv, D)
-            v = qkv[:, (self.hq + self.hkv) * D:].view(T, self.hkv, D)
-            native.rope_kv_write_(qkv, positions, slots, cache, self.hq, self.hkv, mc.rope_theta)
-            a = attend(li, q, k, v)
+            if attend_packed is not None:
+                a = attend_packed(li, qkv)
+            else:
+                q = qkv[:, :self.hq * D].view(T, self.hq, D)
+                k = qkv[:, self.hq * D:(self.hq + self.hkv) * D].view(T, self.hkv, D)
+                v = qkv[:, (self.hq + self.hkv) * D:].view(T, self.hkv, D)
+                native.rope_kv_write_(qkv, positions, slots, cache, self.hq, self.hkv, mc.rope_theta)
+                a = attend(li, q, k, v)
             multi = self.tp is not None and self.tp.world > 1
             # few rows: the residual stream takes the product as an accumulation, SwiGLU runs as its own pass
             sync_ar = multi and self.tp.fused
@@ -368,15 +373,16 @@ class PagedLlamaExecutor:
     def _decode_core(self, last, pos, slots, table, lens, max_len: int) -> torch.Tensor:
         """Device-only part of a decode step (no host reads): embed, all blocks, head, arg-max."""
         def attend(li, q, k, v):
-            if self.native:
-                return native.paged_decode(q, self.kv.caches[li], table, lens, max_len,
-                                           split_tokens=self.cfg.decode_split_tokens)
             if self.cfg.torch_ops:
                 return self._attend_torch_decode(li, q, table, lens, max_len)
             return reference.paged_attention_ref(q, self.kv.caches[li], table.cpu(), lens.cpu().tolist()).to(q.dtype)
+
+        def attend_packed(li, qkv):
+            return native.paged_decode_rope(qkv, self.kv.caches[li], table, lens, slots, self.hq, self.hkv, max_len, self.mc.rope_theta,
+                                            split_tokens=self.cfg.decode_split_tokens)
         x = self._embed(last[None])[0]
         for li, blk in enumerate(self.m.blocks):
-            x = self._block(li, blk, x, pos, slots, attend)
+            x = self._block(li, blk, x, pos, slots, attend, attend_packed if self.native else None)
         return self._logits_argmax(x)
 
     @staticmethod
