@@ -355,13 +355,18 @@ MLF_API int mlf_gemm_bf16(const MlfGemmArgs* a, uint64_t stream) {
                                 a->max_ctas, (a->flags & MLF_EPI_B_STATIC) ? 1 : 0, stream);
     if (rcf != -4) return rcf;
   }
-  // CTA pairs for everything with at least 16 pair tiles (split-K fills the GPU when tiles alone cannot).
+  // CTA pairs for everything with more than 128 rows and at least 16 pair tiles (split-K fills the GPU when tiles alone
+  // cannot). The line lies at one single-CTA row tile: at 160 / 300 / 400 rows a residual product 4096 x 4096 takes 30 us
+  // on pairs and 38 us on single CTAs, 4096 x 14336 76 against 102 us, SwiGLU 28672 x 4096 54 / 91 / 93 against 66 / 94 / 118.
   // Few rows against a large weight (a decode step: M <= 256) is a weight-streaming problem: one row of
   // tiles cannot occupy the GPU, so the pair kernel splits K and every SM streams a slice of the weight.
   const bool plain_out = (a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) == 0 && a->comm == nullptr;
   const bool small_m = g_small_m_split && a->tile_n == 0 && plain_out && a->M <= 256 && a->N >= 1024 && a->K >= 1024;
+  // An accumulation on pairs is a bf16 addition to the rounded product; below 512 rows it keeps the single-CTA kernel's
+  // fp32 one (a decode step's rows, small_m, aside).
+  const int row_line = a->comm != nullptr || (a->flags & MLF_EPI_ACCUM) ? 511 : 128;
   if (a->tile_n == 512 || small_m ||
-      (g_use_2cta && a->tile_n == 0 && a->M >= 512 && a->N >= 512 && (long long)((a->M + 255) / 256) * ((a->N + 255) / 256) >= 16)) {
+      (g_use_2cta && a->tile_n == 0 && a->M > row_line && a->N >= 512 && (long long)((a->M + 255) / 256) * ((a->N + 255) / 256) >= 16)) {
     const int rc2 = mlf_gemm_bf16_2cta(a, stream);
     if (rc2 != -4) return rc2;
   }

@@ -527,8 +527,9 @@ using namespace mlf;
 MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   MLF_REQUIRE(a != nullptr, "null args");
   const MlfGemmComm* cm = a->comm;
-  // fewer than 256 rows only as a plain product (optionally accumulated), where K is split over the pairs
-  if (a->N < 256 || (a->M < 256 && ((a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) != 0 || cm != nullptr))) return -4;
+  // one row of tiles that is mostly padding only as a plain product (optionally accumulated), where K is split over the pairs
+  if (a->N < 256 || (a->M < 256 && cm != nullptr) ||
+      (a->M <= 128 && (a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) != 0)) return -4;
   const bool gatherA = cm && cm->gather_operand == 1;
   const bool gatherB = cm && cm->gather_operand == 2;
   if (cm && cm->gather_operand && (cm->flag_rows <= 0 || cm->flag_rows % 128 != 0)) return -4;
@@ -670,7 +671,8 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   // Split K when the tiles alone cannot fill the GPU (weight gradients of narrow layers: few tiles, long K).
   // Splits add their partial products into `out` with TMA reduction stores.
   int k_splits = 1;
-  if (plain && tma_epi) {
+  // Between a decode step's rows and 512 a product keeps its single fp32 sum: the partial products meet in bf16.
+  if (plain && tma_epi && (a->M <= 256 || a->M >= 512)) {
     const int kb_all = (a->K + BK - 1) / BK;
     int avail = sms / 2;
     if (avail > max_clusters[dev & 63]) avail = max_clusters[dev & 63];

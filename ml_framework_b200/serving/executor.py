@@ -138,7 +138,8 @@ class PagedLlamaExecutor:
                 native.rope_kv_write_(qkv, positions, slots, cache, self.hq, self.hkv, mc.rope_theta)
                 a = attend(li, q, k, v)
             multi = self.tp is not None and self.tp.world > 1
-            # few rows: the residual stream takes the product as an accumulation, SwiGLU runs as its own pass
+            # few rows: the residual stream takes the product as an accumulation; up to 128 rows (K is split over the SMs
+            # in runs of any length) or for a weight of fewer than 16 pair tiles SwiGLU runs as its own pass
             sync_ar = multi and self.tp.fused
             if sync_ar:
                 x = self._row_parallel(a.reshape(T, self.hq * D), o_w, x)
@@ -148,7 +149,7 @@ class PagedLlamaExecutor:
                 gemm(a.reshape(T, self.hq * D), o_w, out=x, flags=_lib.EPI_ACCUM | _lib.EPI_B_STATIC)
             else:
                 x = gemm(a.reshape(T, self.hq * D), o_w, aux_in=x, flags=_lib.EPI_RESIDUAL | _lib.EPI_B_STATIC)
-            if few_rows:
+            if few_rows and (T <= 128 or gu_w.shape[0] < 4096):
                 hid = native.swiglu_fwd(self._norm_product(x, blk.norm2.weight, gu_w, True)[1], interleaved=True)
             else:
                 h, _, _ = native.norm_fwd(x, blk.norm2.weight, None, mc.norm_eps, True, want_stats=False)
