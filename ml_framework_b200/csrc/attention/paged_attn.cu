@@ -54,14 +54,11 @@ struct PagedDecodeParams {
   float theta;
 };
 
-// Rotary embedding of a pair (d, d + 64) at position pos, as rope_kv_write_kernel computes it.
-__device__ __forceinline__ void rope_pair(float& a, float& b, int d, float pos, float log_theta) {
-  const float inv_freq = __expf(-log_theta * (2.f * d / PD));
-  float sn, cs;
-  sincosf(pos * inv_freq, &sn, &cs);
+// Rotary embedding of a pair (d, d + 64); cs = (cosine, sine) of its angle.
+__device__ __forceinline__ void rope_pair(float& a, float& b, float2 cs) {
   const float x = a, y = b;
-  a = x * cs - y * sn;
-  b = y * cs + x * sn;
+  a = x * cs.x - y * cs.y;
+  b = y * cs.x + x * cs.y;
 }
 
 // 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros (rows past the sequence end)
@@ -203,7 +200,18 @@ paged_decode_kernel(const PagedDecodeParams p) {
   issue(0);
   issue(1);
 
-  const float log_theta = ROPE ? __logf(p.theta) : 0.f;
+  // the 64 angles of the new token's position, shared by the query heads and the key: computed by every thread for its own
+  // elements they took longer than the first chunk's loads
+  __shared__ float2 s_cs[ROPE ? PD / 2 : 1];
+  if (ROPE) {
+    if (tid < PD / 2) {
+      const float inv_freq = __expf(-__logf(p.theta) * (2.f * tid / PD));
+      float sn, cs;
+      sincosf((float)(len - 1) * inv_freq, &sn, &cs);
+      s_cs[tid] = make_float2(cs, sn);
+    }
+    __syncthreads();
+  }
   // the new token's key (rotated) and value, 16 bytes of each in the 16 threads that stage its row
   uint4 nk = make_uint4(0u, 0u, 0u, 0u), nv = nk;
   const bool has_new = ROPE && t_hi == len;
@@ -219,8 +227,8 @@ paged_decode_kernel(const PagedDecodeParams p) {
     for (int j = 0; j < 4; ++j) {
       const float2 a = unpack_bf16x2(dl < 8 ? ow[j] : tw[j]), c = unpack_bf16x2(dl < 8 ? tw[j] : ow[j]);
       float2 lo = a, hi = c;
-      rope_pair(lo.x, hi.x, (dl & 7) * 8 + 2 * j, (float)(len - 1), log_theta);
-      rope_pair(lo.y, hi.y, (dl & 7) * 8 + 2 * j + 1, (float)(len - 1), log_theta);
+      rope_pair(lo.x, hi.x, s_cs[(dl & 7) * 8 + 2 * j]);
+      rope_pair(lo.y, hi.y, s_cs[(dl & 7) * 8 + 2 * j + 1]);
       rw[j] = dl < 8 ? pack_bf16x2(lo.x, lo.y) : pack_bf16x2(hi.x, hi.y);
     }
     nk = make_uint4(rw[0], rw[1], rw[2], rw[3]);
@@ -255,8 +263,8 @@ paged_decode_kernel(const PagedDecodeParams p) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         float2 lo = unpack_bf16x2(qa[ks][h]), hi = unpack_bf16x2(qa[ks + PD / 32][h]);
-        rope_pair(lo.x, hi.x, ks * 16 + h * 8 + qcol, (float)(len - 1), log_theta);
-        rope_pair(lo.y, hi.y, ks * 16 + h * 8 + qcol + 1, (float)(len - 1), log_theta);
+        rope_pair(lo.x, hi.x, s_cs[ks * 16 + h * 8 + qcol]);
+        rope_pair(lo.y, hi.y, s_cs[ks * 16 + h * 8 + qcol + 1]);
         qa[ks][h] = pack_bf16x2(lo.x, lo.y);
         qa[ks + PD / 32][h] = pack_bf16x2(hi.x, hi.y);
       }
