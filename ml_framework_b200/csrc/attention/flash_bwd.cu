@@ -52,10 +52,16 @@ struct FlashBwdParams {
   int* err;
 };
 
-// delta[b, h, s] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (token, head), two such rows per warp in flight.
+// delta[b, h, s] = sum_d dO[t, h, d] * O[t, h, d] (and lse2, the logsumexp in the log2 domain), rows of pitch Sp; one warp per (token, head), two such rows per warp in flight.
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout, float* delta, const float* lse, float* lse2, int B, int S,
+attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout, float* delta, const float* lse, float* lse2, int B, int S, int Sp,
                   int H, long long ldo, long long lddo) {
+  const int pad = Sp - S;                      // statistics past the end of a sequence are zero
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)B * H * pad; i += (long long)gridDim.x * blockDim.x) {
+    const long long at = i / pad * Sp + S + i % pad;
+    delta[at] = 0.f;
+    if (lse2) lse2[at] = 0.f;
+  }
   const long long total = (long long)B * S * H;
   const int lane = threadIdx.x & 31;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -81,8 +87,8 @@ attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout, float* delt
       const long long t = lane ? t1 : t0;
       const int h = lane ? h1 : h0;
       const long long b = t / S, sidx = t % S;
-      delta[(b * H + h) * S + sidx] = lane ? s1 : s0;
-      if (lse2) lse2[(b * H + h) * S + sidx] = lse[(b * H + h) * S + sidx] * 1.4426950408889634f;
+      delta[(b * H + h) * Sp + sidx] = lane ? s1 : s0;
+      if (lse2) lse2[(b * H + h) * Sp + sidx] = lse[(b * H + h) * S + sidx] * 1.4426950408889634f;
     }
   }
 }
@@ -377,19 +383,23 @@ using namespace mlf;
 
 namespace mlf {
 int launch_flash_bwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                        float* dq_accum, void* dk, void* dv, const float* lse2, const float* delta, long long lddk, long long lddv,
+                        float* dq_accum, void* dk, void* dv, const float* lse2, const float* delta, int stat_pitch, long long lddk, long long lddv,
                         int B, int S, int Hq, int Hkv, float scale, int causal, cudaStream_t st);
 }
 
 static int g_flash_bwd_ws = 1;
-// 1 (default): sequences of at least 128 tokens (a multiple of 4) use the 128 x 128 warpgroup kernel; 0: the 128 x 64 kernel.
+// 1 (default): sequences of at least 128 tokens use the 128 x 128 warpgroup kernel; 0: the 128 x 64 kernel.
 MLF_API void mlf_set_flash_bwd_ws(int on) { g_flash_bwd_ws = on; }
 
-// Bytes of fp32 scratch the caller must provide: dq accumulator [B*S, Hq*128] + delta [B, Hq, S] +
-// logsumexp in the log2 domain [B, Hq, S] + 256 floats of slack (the last tile's statistics are
-// fetched as whole 512-byte pieces).
+// The warpgroup kernel fetches a tile's statistics as whole 512-byte pieces: rows of whole tiles, zero past the sequence.
+// With the sequence length itself as the pitch, lengths that are no multiple of four took the 128 x 64 kernel: 3 x 777
+// tokens, 8 heads, 97 us there, 53 us here.
+static int stat_pitch(int S) { return (S + 127) & ~127; }
+
+// Bytes of fp32 scratch the caller must provide: dq accumulator [B*S, Hq*128] + delta [B, Hq, pitch] +
+// logsumexp in the log2 domain [B, Hq, pitch].
 MLF_API long long mlf_flash_bwd_scratch_bytes(int B, int S, int Hq) {
-  return ((long long)B * S * Hq * FB_D + 2 * (long long)B * Hq * S + 256) * 4;
+  return ((long long)B * S * Hq * FB_D + 2 * (long long)B * Hq * stat_pitch(S)) * 4;
 }
 
 // q/k/v/o/dout: bf16 token-major views (row pitches in elements). dq/dk/dv: bf16 outputs with
@@ -404,8 +414,9 @@ MLF_API int mlf_flash_bwd(const void* q, const void* k, const void* v, const voi
   const long long rows = (long long)B * S;
   float* dq_accum = static_cast<float*>(scratch);
   float* delta = dq_accum + rows * Hq * FB_D;
-  float* lse2 = delta + rows * Hq + 128;        // 16-byte aligned when S % 4 == 0; 128 floats of slack after each array
-  const bool use_ws = g_flash_bwd_ws && S >= 128 && S % 4 == 0 && ((reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(lse2)) & 15) == 0;
+  const int Sp = stat_pitch(S);
+  float* lse2 = delta + (long long)B * Hq * Sp;
+  const bool use_ws = g_flash_bwd_ws && S >= 128 && ((reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(lse2)) & 15) == 0;
   MLF_CHECK_CUDA(cudaMemsetAsync(dq_accum, 0, sizeof(float) * rows * Hq * FB_D, st));
   {
     MLF_REQUIRE(((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15) == 0 && ldo % 8 == 0 && lddo % 8 == 0,
@@ -415,7 +426,7 @@ MLF_API int mlf_flash_bwd(const void* q, const void* k, const void* v, const voi
     const long long cap = (long long)sm_count() * 8;
     if (grid > cap) grid = cap;
     attn_delta_kernel<<<(int)grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout),
-                                                 delta, lse, use_ws ? lse2 : nullptr, B, S, Hq, ldo, lddo);
+                                                 delta, lse, use_ws ? lse2 : nullptr, B, S, use_ws ? Sp : S, Hq, ldo, lddo);
                                                  count_launch();
     MLF_CHECK_CUDA(cudaGetLastError());
   }
@@ -426,7 +437,7 @@ MLF_API int mlf_flash_bwd(const void* q, const void* k, const void* v, const voi
     if ((rc = cached_tmap_bf16(&tk, k, (uint64_t)Hkv * FB_D, rows, ldk, 64, 128))) return rc;
     if ((rc = cached_tmap_bf16(&tv, v, (uint64_t)Hkv * FB_D, rows, ldv, 64, 128))) return rc;
     if ((rc = cached_tmap_bf16(&tdo, dout, (uint64_t)Hq * FB_D, rows, lddo, 64, 128))) return rc;
-    if ((rc = launch_flash_bwd_ws(tq, tk, tv, tdo, dq_accum, dk, dv, lse2, delta, lddk, lddv, B, S, Hq, Hkv, scale, causal, st))) return rc;
+    if ((rc = launch_flash_bwd_ws(tq, tk, tv, tdo, dq_accum, dk, dv, lse2, delta, Sp, lddk, lddv, B, S, Hq, Hkv, scale, causal, st))) return rc;
   } else {
   if ((rc = cached_tmap_bf16(&tq, q, (uint64_t)Hq * FB_D, rows, ldq, 64, FB_BQ))) return rc;
   if ((rc = cached_tmap_bf16(&tk, k, (uint64_t)Hkv * FB_D, rows, ldk, 64, FB_BKV))) return rc;

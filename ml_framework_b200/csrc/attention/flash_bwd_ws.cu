@@ -14,9 +14,13 @@
 // The same 128B-swizzled tiles serve as K-major or MN-major operands through their descriptors, so
 // nothing is ever transposed in memory.
 //
-// 384 threads: warps 0..3 control (warp 0 TMA producer, warp 1 MMA issuer), warps 4..7 compute
-// (one key row per thread), warps 8..11 dQ read-out; the control warpgroup hands registers to the
-// other two (setmaxnreg). TMEM (512 columns): dK | dV | S^T (then P^T) | dP^T (then dQ).
+// 512 threads: warps 0..3 control (warp 0 TMA producer, warp 1 MMA issuer), warps 4..11 compute
+// (one key row and half of the tile's queries per thread), warps 12..15 dQ read-out; the control
+// warpgroup hands registers to the others (setmaxnreg 56 / 144 / 144 / 168 of 4 x 128).
+// TMEM (512 columns): dK | dV | S^T (then P^T) | dP^T (then dQ).
+// Bound by the chain dS -> dK, dQ -> dQ read-out -> dP^T -> dS of a tile: without any of the compute
+// warpgroups' arithmetic 4 x 2048, 16 heads takes 268 us. A second compute warpgroup and paired fp32
+// arithmetic shorten their link: 315 -> 300 us; 2 x 4096, 32 / 8 heads 891 -> 862 us.
 // Issue order on the tensor pipe: dV(i), S^T(i+1), dK(i), dQ(i), dP^T(i+1): the next tile's
 // exponentials run while this tile's gradients are multiplied.
 //
@@ -33,7 +37,7 @@ namespace mlf {
 
 constexpr int G_T = 128;                       // tile edge (keys and queries)
 constexpr int G_D = 128;
-constexpr int G_THREADS = 384;
+constexpr int G_THREADS = 512;
 constexpr int G_TILE = G_T * G_D * 2;          // 32 KB: two 64-column blocks of 16 KB
 constexpr int G_HALF = G_TILE / 2;
 constexpr int G_STATS = 2 * G_T * 4;           // lse (log2 domain) | delta, fp32, per stage
@@ -45,8 +49,9 @@ struct FlashBwdWsParams {
   float* dq_accum;          // fp32 [tokens, Hq*128], zeroed by the launcher
   __nv_bfloat16* dk;
   __nv_bfloat16* dv;
-  const float* lse2;        // [B, Hq, S] logsumexp * log2(e)
-  const float* delta;       // [B, Hq, S] rowsum(dO o O)
+  const float* lse2;        // [B, Hq, stat_pitch] logsumexp * log2(e)
+  const float* delta;       // [B, Hq, stat_pitch] rowsum(dO o O)
+  int stat_pitch;           // whole tiles; entries from S on are 0, so that a masked score gives P = 0 and dS = 0
   long long lddk, lddv;
   int B, S, Hq, Hkv, causal;
   float scale, scale_log2;
@@ -109,8 +114,8 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
-    mbar_init(p_full, 128);
-    mbar_init(ds_full, 128);
+    mbar_init(p_full, 256);
+    mbar_init(ds_full, 256);
     mbar_init(dq_full, 1);
     mbar_init(dq_empty, 128);
     mbar_init(do_full, 1);
@@ -145,7 +150,7 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const int h = hkv * group + it / per_head;
           const int q0 = (qt0 + it % per_head) * G_T;
           const int qrow = (int)(row_base + q0);
-          const long long sidx = ((long long)b * p.Hq + h) * p.S + q0;
+          const long long sidx = ((long long)b * p.Hq + h) * p.stat_pitch + q0;
           mbar_expect_tx(q_full(s), G_TILE + G_STATS);
           tma_load_2d(sQ(s), &tmQ, h * G_D, qrow, q_full(s));
           tma_load_2d(sQ(s) + G_HALF, &tmQ, h * G_D + 64, qrow, q_full(s));
@@ -189,7 +194,7 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tc_fence_after_sync();
 #pragma unroll
           for (int k = 0; k < G_T / 16; ++k)     // dV += P^T dO   (A from tensor memory)
-            umma_bf16_ts(t_dV, t_S + 8u * k, make_smem_desc_sw128(sdO + k * 2048, G_HALF, 1024), idesc_kn, (it | k) != 0);
+            umma_bf16_ts(t_dV, t_S + 8u * (k & 3) + 64u * (k >> 2), make_smem_desc_sw128(sdO + k * 2048, G_HALF, 1024), idesc_kn, (it | k) != 0);
           umma_commit(do_empty);                   // dO of this tile has been read (dP^T earlier, dV now)
           const bool more = it + 1 < n_it;
           if (more) {                              // S^T of the next tile goes in behind dV
@@ -224,13 +229,16 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
     }
-  } else if (warp < 8) {
-    // ===================== compute warpgroup: one key row per thread =====================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+  } else if (warp < 12) {
+    // ===================== compute warpgroups: one key row and 64 of the tile's queries per thread =====================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
     const int qd = warp & 3;
+    const int g = (warp - 4) >> 2;             // which 64 query columns
     const int r = qd * 32 + lane;
     const int kv_i = k0 + r;
     const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
+    const uint32_t t_Sg = t_S + 64u * g, t_dPg = t_dP + 64u * g;      // P^T of these columns replaces their own S^T
+    const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2), scale2 = pack_f32x2(p.scale, p.scale);
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
       const int s = it & 1;
@@ -240,74 +248,64 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!mbar_wait_warp(q_full(s), (it >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
       if (!mbar_wait_warp(s_full, it & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
       tc_fence_after_sync();
-      uint32_t pk[64];
-      const uint32_t st_addr = sStats + s * G_STATS;     // shared-window address of this stage's statistics
+      uint32_t pk[32];
+      const uint32_t st_addr = sStats + s * G_STATS + g * 256;     // shared-window address of these columns' statistics
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
-        // 64 columns at a time: S^T from tensor memory and the 64 row statistics from shared memory are
-        // all requested up front (explicit shared-space vector loads, issued back to back) so that
-        // their latencies overlap instead of preceding every group of four exponentials
-        uint32_t sv[64];
-        tmem_ld_32x32b_x32(t_S + 64 * hh + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&sv[0]));
-        tmem_ld_32x32b_x32(t_S + 64 * hh + 32 + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&sv[32]));
-        float4 ls[16];
+        // 32 columns at a time: S^T from tensor memory and the row statistics from shared memory are all requested up
+        // front so that their latencies overlap
+        uint32_t sv[32];
+        tmem_ld_32x32b_x32(t_Sg + 32 * hh + lane_off, sv);
+        uint64_t ls[16];                       // -logsumexp of two queries each
 #pragma unroll
-        for (int c4 = 0; c4 < 16; ++c4)
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(ls[c4].x), "=f"(ls[c4].y), "=f"(ls[c4].z), "=f"(ls[c4].w)
-                       : "r"(st_addr + (64 * hh + 4 * c4) * 4));
+        for (int c4 = 0; c4 < 8; ++c4)
+          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(ls[2 * c4]), "=l"(ls[2 * c4 + 1]) : "r"(st_addr + (32 * hh + 4 * c4) * 4));
         tmem_wait_ld();
-        if (need_mask) {                         // diagonal / ragged tiles only: masked scores become -inf, exp2 gives 0
+        if (need_mask) {                       // diagonal / ragged tiles only: masked scores become -inf, exp2 gives 0
 #pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const int qi = q0 + 64 * hh + i;
+          for (int i = 0; i < 32; ++i) {
+            const int qi = q0 + 64 * g + 32 * hh + i;
             if (qi >= p.S || kv_i >= p.S || (p.causal && qi < kv_i)) sv[i] = __float_as_uint(-INFINITY);
           }
         }
 #pragma unroll
-        for (int c4 = 0; c4 < 16; ++c4) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sv[4 * c4 + 0]), p.scale_log2, -ls[c4].x));
-          const float p1 = exp2f(fmaf(__uint_as_float(sv[4 * c4 + 1]), p.scale_log2, -ls[c4].y));
-          const float p2 = exp2f(fmaf(__uint_as_float(sv[4 * c4 + 2]), p.scale_log2, -ls[c4].z));
-          const float p3 = exp2f(fmaf(__uint_as_float(sv[4 * c4 + 3]), p.scale_log2, -ls[c4].w));
-          pk[32 * hh + 2 * c4] = pack_bf16x2(p0, p1);
-          pk[32 * hh + 2 * c4 + 1] = pack_bf16x2(p2, p3);
+        for (int i = 0; i < 16; ++i) {
+          float e0, e1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), c2, neg_f32x2(ls[i])), e0, e1);
+          pk[16 * hh + i] = pack_bf16x2(exp2f(e0), exp2f(e1));
         }
       }
-      tmem_st_32x32b_x32(t_S + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&pk[0]));
-      tmem_st_32x32b_x32(t_S + 32 + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&pk[32]));
+      tmem_st_32x32b_x32(t_Sg + lane_off, pk);
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive(p_full);
       // dS^T from the rounded P^T (the same values dV is multiplied with)
       if (!mbar_wait_warp(dp_full, it & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
       tc_fence_after_sync();
+      const uint32_t drow = sdS + g * G_HALF + r * 128;
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
-        uint32_t dp[64];
-        tmem_ld_32x32b_x32(t_dP + 64 * hh + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&dp[0]));
-        tmem_ld_32x32b_x32(t_dP + 64 * hh + 32 + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&dp[32]));
-        float4 dls[16];
+        uint32_t dp[32];
+        tmem_ld_32x32b_x32(t_dPg + 32 * hh + lane_off, dp);
+        uint64_t dl[16];
 #pragma unroll
-        for (int c4 = 0; c4 < 16; ++c4)
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(dls[c4].x), "=f"(dls[c4].y), "=f"(dls[c4].z), "=f"(dls[c4].w)
-                       : "r"(st_addr + (G_T + 64 * hh + 4 * c4) * 4));
+        for (int c4 = 0; c4 < 8; ++c4)
+          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(dl[2 * c4]), "=l"(dl[2 * c4 + 1])
+                       : "r"(st_addr + (G_T + 32 * hh + 4 * c4) * 4));
         tmem_wait_ld();
-        uint32_t dsk[32];
+        uint32_t dsk[16];
 #pragma unroll
-        for (int c4 = 0; c4 < 16; ++c4) {
-          const float4 dl = dls[c4];
-          const uint32_t pa = pk[32 * hh + 2 * c4], pb = pk[32 * hh + 2 * c4 + 1];
-          const float d0 = __uint_as_float(pa << 16) * (__uint_as_float(dp[4 * c4 + 0]) - dl.x) * p.scale;
-          const float d1 = __uint_as_float(pa & 0xffff0000u) * (__uint_as_float(dp[4 * c4 + 1]) - dl.y) * p.scale;
-          const float d2 = __uint_as_float(pb << 16) * (__uint_as_float(dp[4 * c4 + 2]) - dl.z) * p.scale;
-          const float d3 = __uint_as_float(pb & 0xffff0000u) * (__uint_as_float(dp[4 * c4 + 3]) - dl.w) * p.scale;
-          dsk[2 * c4] = pack_bf16x2(d0, d1);
-          dsk[2 * c4 + 1] = pack_bf16x2(d2, d3);
+        for (int i = 0; i < 16; ++i) {
+          const uint32_t pa = pk[16 * hh + i];
+          const uint64_t pp = pack_f32x2(__uint_as_float(pa << 16), __uint_as_float(pa & 0xffff0000u));
+          const uint64_t d = add_f32x2(pack_f32x2(__uint_as_float(dp[2 * i]), __uint_as_float(dp[2 * i + 1])), neg_f32x2(dl[i]));
+          float d0, d1;
+          unpack_f32x2(mul_f32x2(mul_f32x2(pp, d), scale2), d0, d1);
+          dsk[i] = pack_bf16x2(d0, d1);
         }
-        const uint32_t drow = sdS + hh * G_HALF + r * 128;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const uint32_t off = ((uint32_t)(c ^ (r & 7))) << 4;
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t off = ((uint32_t)((4 * hh + c) ^ (r & 7))) << 4;
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(drow + off), "r"(dsk[4 * c]), "r"(dsk[4 * c + 1]),
                        "r"(dsk[4 * c + 2]), "r"(dsk[4 * c + 3]) : "memory");
         }
@@ -324,10 +322,10 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       __nv_bfloat16* dk_row = p.dk + (row_base + kv_i) * p.lddk + (long long)hkv * G_D;
       __nv_bfloat16* dv_row = p.dv + (row_base + kv_i) * p.lddv + (long long)hkv * G_D;
 #pragma unroll
-      for (int c = 0; c < G_D / 32; ++c) {
-        uint32_t a[32], g[32];
+      for (int c = 2 * g; c < 2 * g + 2; ++c) {
+        uint32_t a[32], e[32];
         tmem_ld_32x32b_x32(t_dK + 32 * c + lane_off, a);
-        tmem_ld_32x32b_x32(t_dV + 32 * c + lane_off, g);
+        tmem_ld_32x32b_x32(t_dV + 32 * c + lane_off, e);
         tmem_wait_ld();
         if (row_ok) {
 #pragma unroll
@@ -337,10 +335,10 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             w.y = pack_bf16x2(__uint_as_float(a[8 * v + 2]), __uint_as_float(a[8 * v + 3]));
             w.z = pack_bf16x2(__uint_as_float(a[8 * v + 4]), __uint_as_float(a[8 * v + 5]));
             w.w = pack_bf16x2(__uint_as_float(a[8 * v + 6]), __uint_as_float(a[8 * v + 7]));
-            x.x = pack_bf16x2(__uint_as_float(g[8 * v + 0]), __uint_as_float(g[8 * v + 1]));
-            x.y = pack_bf16x2(__uint_as_float(g[8 * v + 2]), __uint_as_float(g[8 * v + 3]));
-            x.z = pack_bf16x2(__uint_as_float(g[8 * v + 4]), __uint_as_float(g[8 * v + 5]));
-            x.w = pack_bf16x2(__uint_as_float(g[8 * v + 6]), __uint_as_float(g[8 * v + 7]));
+            x.x = pack_bf16x2(__uint_as_float(e[8 * v + 0]), __uint_as_float(e[8 * v + 1]));
+            x.y = pack_bf16x2(__uint_as_float(e[8 * v + 2]), __uint_as_float(e[8 * v + 3]));
+            x.z = pack_bf16x2(__uint_as_float(e[8 * v + 4]), __uint_as_float(e[8 * v + 5]));
+            x.w = pack_bf16x2(__uint_as_float(e[8 * v + 6]), __uint_as_float(e[8 * v + 7]));
             reinterpret_cast<uint4*>(dk_row + 32 * c)[v] = w;
             reinterpret_cast<uint4*>(dv_row + 32 * c)[v] = x;
           }
@@ -350,7 +348,7 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tc_fence_before_sync();
   } else {
     // ===================== dQ read-out warpgroup: one query row per thread =====================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
     const int qd = warp & 3;
     const int r = qd * 32 + lane;
     const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
@@ -413,7 +411,7 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
 // Launches the main kernel only; the caller has zeroed dq_accum and filled lse2 / delta.
 int launch_flash_bwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                        float* dq_accum, void* dk, void* dv, const float* lse2, const float* delta, long long lddk, long long lddv,
+                        float* dq_accum, void* dk, void* dv, const float* lse2, const float* delta, int stat_pitch, long long lddk, long long lddv,
                         int B, int S, int Hq, int Hkv, float scale, int causal, cudaStream_t st) {
   FlashBwdWsParams p;
   p.dq_accum = dq_accum;
@@ -421,6 +419,7 @@ int launch_flash_bwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   p.dv = static_cast<__nv_bfloat16*>(dv);
   p.lse2 = lse2;
   p.delta = delta;
+  p.stat_pitch = stat_pitch;
   p.lddk = lddk; p.lddv = lddv;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;
   p.scale = scale;
