@@ -22,7 +22,9 @@
 // warpgroups' arithmetic 4 x 2048, 16 heads takes 268 us. A second compute warpgroup and paired fp32
 // arithmetic shorten their link: 315 -> 300 us; 2 x 4096, 32 / 8 heads 891 -> 862 us.
 // Issue order on the tensor pipe: dV(i), S^T(i+1), dK(i), dQ(i), dP^T(i+1): the next tile's
-// exponentials run while this tile's gradients are multiplied.
+// exponentials run while this tile's gradients are multiplied. The issuing thread polls its barriers:
+// it is on the chain, and a suspended wait wakes late (2 x 4096, 32 / 8 heads: 854 -> 811 us; 4 x 2048,
+// 16 heads: 306 -> 303 us; in the forward kernel, whose chain is in the softmax, polling costs 3 %).
 //
 // The reference has no attention backward (its attention layers are forward-only,
 // src/MLFramework/Inference/PagedAttention/Layers/PagedAttentionLayer.cs:102-144); training the
@@ -175,13 +177,13 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             umma_bf16_ss(d_tmem, make_smem_desc_sw128(a + off, 16, 1024), make_smem_desc_sw128(bm + off, 16, 1024), idesc_kk, k != 0);
           }
         };
-        bool ok = mbar_wait(kv_full, 0, abort_flag, p.err, ERR_WAIT_ATTN);
-        if (ok && n_it > 0) ok = mbar_wait(q_full(0), 0, abort_flag, p.err, ERR_WAIT_ATTN);
+        bool ok = mbar_wait_poll(kv_full, 0, abort_flag, p.err, ERR_WAIT_ATTN);
+        if (ok && n_it > 0) ok = mbar_wait_poll(q_full(0), 0, abort_flag, p.err, ERR_WAIT_ATTN);
         if (ok && n_it > 0) {
           tc_fence_after_sync();
           issue_kk(t_S, sK, sQ(0));
           umma_commit(s_full);
-          ok = mbar_wait(do_full, 0, abort_flag, p.err, ERR_WAIT_ATTN);
+          ok = mbar_wait_poll(do_full, 0, abort_flag, p.err, ERR_WAIT_ATTN);
           if (ok) {
             tc_fence_after_sync();
             issue_kk(t_dP, sV, sdO);
@@ -190,7 +192,7 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         for (int it = 0; it < n_it && ok; ++it) {
           const int s = it & 1;
-          if (!mbar_wait(p_full, it & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
+          if (!mbar_wait_poll(p_full, it & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
           tc_fence_after_sync();
 #pragma unroll
           for (int k = 0; k < G_T / 16; ++k)     // dV += P^T dO   (A from tensor memory)
@@ -198,19 +200,19 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           umma_commit(do_empty);                   // dO of this tile has been read (dP^T earlier, dV now)
           const bool more = it + 1 < n_it;
           if (more) {                              // S^T of the next tile goes in behind dV
-            if (!mbar_wait(q_full(s ^ 1), ((it + 1) >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
+            if (!mbar_wait_poll(q_full(s ^ 1), ((it + 1) >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
             tc_fence_after_sync();
             issue_kk(t_S, sK, sQ(s ^ 1));
             umma_commit(s_full);
           }
-          if (!mbar_wait(ds_full, it & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
+          if (!mbar_wait_poll(ds_full, it & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
           tc_fence_after_sync();
 #pragma unroll
           for (int k = 0; k < G_T / 16; ++k)     // dK += dS^T Q
             umma_bf16_ss(t_dK, make_smem_desc_sw128(sdS + (k >> 2) * G_HALF + (k & 3) * 32, 16, 1024),
                          make_smem_desc_sw128(sQ(s) + k * 2048, G_HALF, 1024), idesc_kn, (it | k) != 0);
           if (it > 0) {                            // dQ lands where the previous dQ was: wait for its read-out
-            if (!mbar_wait(dq_empty, (it - 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
+            if (!mbar_wait_poll(dq_empty, (it - 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
             tc_fence_after_sync();
           }
 #pragma unroll
@@ -220,8 +222,8 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           umma_commit(dq_full);
           umma_commit(q_empty(s));
           if (more) {                              // dP^T of the next tile needs the dQ columns back
-            if (!mbar_wait(dq_empty, it & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
-            if (!mbar_wait(do_full, (it + 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
+            if (!mbar_wait_poll(dq_empty, it & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
+            if (!mbar_wait_poll(do_full, (it + 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
             tc_fence_after_sync();
             issue_kk(t_dP, sV, sdO);
             umma_commit(dp_full);
