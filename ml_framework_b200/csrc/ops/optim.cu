@@ -220,8 +220,19 @@ cross_entropy_kernel(__nv_bfloat16* logits, const long long* targets, float* los
   const float gs = gscale * (gscale_ptr ? *gscale_ptr : 1.f);
   // pass 1: online max / sum-exp
   float mx = -FLT_MAX, se = 0.f;
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    const uint4 u = reinterpret_cast<const uint4*>(row)[i];
+  // four loads in flight per thread: the running maximum chains the iterations, and one load at a time left the few CTAs
+  // that fit beside their cached rows waiting on memory (8192 x 32000: 430 -> 397 us, 8192 x 50304: 652 -> 565 us)
+  constexpr int LD = 4;
+  for (int i0 = threadIdx.x; i0 < nvec; i0 += LD * blockDim.x) {
+    uint4 uu[LD];
+#pragma unroll
+    for (int k = 0; k < LD; ++k)
+      if (i0 + k * (int)blockDim.x < nvec) uu[k] = reinterpret_cast<const uint4*>(row)[i0 + k * blockDim.x];
+#pragma unroll
+    for (int k = 0; k < LD; ++k) {
+    const int i = i0 + k * blockDim.x;
+    if (i >= nvec) break;
+    const uint4 u = uu[k];
     if (cache_row) row_cache[i] = u;
     float f[8];
     float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
@@ -232,6 +243,7 @@ cross_entropy_kernel(__nv_bfloat16* logits, const long long* targets, float* los
     if (lm > mx) { se *= __expf(mx - lm); mx = lm; }
 #pragma unroll
     for (int j = 0; j < 8; ++j) se += __expf(f[j] - mx);
+    }
   }
   for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) {
     const float f = __bfloat162float(row[i]);
