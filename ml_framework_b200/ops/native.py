@@ -214,6 +214,21 @@ def rope_(x: torch.Tensor, pos: torch.Tensor, theta: float, inverse: bool = Fals
     return x
 
 
+def rope_qkv(qkv: torch.Tensor, pos: torch.Tensor, Hq: int, Hkv: int, theta: float, inverse: bool = False,
+             out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Rotary embedding of the query and key heads of packed rows [T, (Hq + 2 Hkv) * 128] into ``out`` (a new tensor by
+    default, ``qkv`` itself for in place); value heads are copied. Rows must be 16-byte aligned."""
+    assert qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.shape[1] == (Hq + 2 * Hkv) * 128 and qkv.dtype == torch.bfloat16
+    assert pos.dtype == torch.int64 and pos.numel() == qkv.shape[0]
+    if out is None:
+        out = torch.empty(qkv.shape, dtype=qkv.dtype, device=qkv.device)
+    assert out.shape == qkv.shape and out.dtype == qkv.dtype and out.stride(1) == 1
+    rc = _L().mlf_rope_qkv(_p(out), _p(qkv), _p(pos.contiguous()), C.c_longlong(qkv.shape[0]), Hq, Hkv, C.c_longlong(out.stride(0)),
+                           C.c_longlong(qkv.stride(0)), C.c_float(theta), int(inverse), _st())
+    _lib.check(rc, "mlf_rope_qkv")
+    return out
+
+
 # ------------------------------------------------------------------ optimizer / AMP / loss
 def adamw_(master, m, v, grad, param_out, *, lr, beta1, beta2, eps, weight_decay, step, grad_scale=1.0,
            inv_scale: Optional[torch.Tensor] = None, found_inf: Optional[torch.Tensor] = None, vmax=None):

@@ -1,0 +1,62 @@
+"""Vectorised element-wise kernels at their edges: remainders of the vector width, unaligned buffers, in place."""
+import pytest
+import torch
+
+from ml_framework_b200 import _lib
+from ml_framework_b200.ops import native
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 4099, 1 << 20])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_cast(n, shift, accumulate):
+    torch.manual_seed(n)
+    src = torch.randn(n + shift, device="cuda")[shift:]
+    buf = torch.randn(n + shift + 8, device="cuda").to(torch.bfloat16)
+    guard = buf.clone()
+    out = buf[shift:shift + n]
+    want = (src + out.float() if accumulate else src).to(torch.bfloat16)
+    native.cast_f32_to_bf16(src, out, accumulate)
+    assert torch.equal(out, want)
+    assert torch.equal(buf[:shift], guard[:shift]) and torch.equal(buf[shift + n:], guard[shift + n:])
+
+
+@pytest.mark.parametrize("T,D", [(1, 8), (37, 264), (513, 1024)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_embedding_gradient(T, D, shift):
+    torch.manual_seed(T)
+    V = 50
+    ids = torch.randint(0, V, (T,), device="cuda")
+    ids[0] = V + 3                                    # outside the table: skipped
+    dout = torch.randn(T, D, device="cuda").to(torch.bfloat16)
+    dw = torch.zeros(V * D + shift, device="cuda")[shift:].view(V, D)
+    native.embedding_bwd(dout, ids, V, dw)
+    want = torch.zeros(V, D, device="cuda", dtype=torch.float64).index_add_(0, ids[1:], dout[1:].double())
+    # fp32 sums of up to T / V + a few terms of order 1 in any order
+    assert ((dw.double() - want).abs() <= 1e-5 * (1 + want.abs())).all()
+
+
+@pytest.mark.parametrize("T", [1, 31, 1000])
+@pytest.mark.parametrize("Hq,Hkv", [(1, 1), (2, 1), (8, 2), (5, 5)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_rope_qkv(T, Hq, Hkv, inverse):
+    torch.manual_seed(T)
+    W = (Hq + 2 * Hkv) * 128
+    wide = torch.randn(T, W + 16, device="cuda").to(torch.bfloat16)
+    src = wide[:, 8:8 + W]
+    pos = torch.randint(0, 5000, (T,), device="cuda")
+    want = src.clone()
+    native.rope_(want[:, :Hq * 128].view(T, Hq, 128), pos, 500000.0, inverse)
+    native.rope_(want[:, Hq * 128:(Hq + Hkv) * 128].view(T, Hkv, 128), pos, 500000.0, inverse)
+    before = wide.clone()
+    got = native.rope_qkv(src, pos, Hq, Hkv, 500000.0, inverse)
+    # the same formula, but the compiler may contract a * c - b * s the other way round: an fp32 rounding (2^-24 of values
+    # below 8) apart before both are rounded to bf16, so neighbours (2^-7 of the value) at most and almost always equal
+    assert ((got.float() - want.float()).abs() <= 2 ** -7 * want.float().abs() + 2 ** -20).all()
+    assert (got != want).float().mean() < 1e-3
+    assert torch.equal(got[:, (Hq + Hkv) * 128:], src[:, (Hq + Hkv) * 128:]) and torch.equal(wide, before)
+    native.rope_qkv(src, pos, Hq, Hkv, 500000.0, inverse, out=src)
+    assert torch.equal(src, got) and torch.equal(wide[:, :8], before[:, :8]) and torch.equal(wide[:, 8 + W:], before[:, 8 + W:])
+    assert _lib.read_status() == 0
