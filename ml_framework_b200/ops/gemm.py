@@ -140,12 +140,10 @@ def gemm_reference(a, b, *, a_mn=False, b_mn=False, bias=None, aux_in=None, flag
     return v, pre
 
 
-def _rows_k(t: torch.Tensor, mn: bool):
-    if t.dim() != 2:
-        raise ValueError("gemm operands must be 2-D")
-    if t.stride(1) != 1:
-        raise ValueError("gemm operands must have a contiguous last dimension")
-    return (t.shape[1], t.shape[0]) if mn else (t.shape[0], t.shape[1])
+def _check_aux(name: str, t: torch.Tensor, M: int, cols: int, dev):
+    if t.dim() != 2 or t.shape[0] != M or t.shape[1] != cols or t.dtype != torch.bfloat16 or t.device != dev or t.stride(-1) != 1:
+        raise ValueError(f"{name} must be a bf16 [{M}, {cols}] tensor on the operands' device with a contiguous last "
+                         f"dimension, got {tuple(t.shape)} {t.dtype}")
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
@@ -159,8 +157,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     ``m_override`` / ``n_override`` give the logical row count of an operand that is gathered
     inside the kernel (``comm.gather_operand``), where ``a`` / ``b`` only hold the local shard.
     """
-    M, K = _rows_k(a, a_mn)
-    N, Kb = _rows_k(b, b_mn)
+    ash, bsh, ast, bst = a.shape, b.shape, a.stride(), b.stride()
+    if len(ash) != 2 or len(bsh) != 2:
+        raise ValueError("gemm operands must be 2-D")
+    if ast[1] != 1 or bst[1] != 1:
+        raise ValueError("gemm operands must have a contiguous last dimension")
+    K, M = ash if a_mn else (ash[1], ash[0])
+    Kb, N = bsh if b_mn else (bsh[1], bsh[0])
     if m_override is not None:
         M = m_override
     if n_override is not None:
@@ -169,7 +172,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         raise ValueError(f"contraction mismatch: {K} vs {Kb}")
     if bias is not None:
         flags |= EPI_BIAS
-    if out_dtype == torch.float32:
+    if out_dtype is torch.float32:
         flags |= EPI_OUT_FP32
     out_cols = N // 2 if flags & EPI_SWIGLU else (2 * N if flags & EPI_DSWIGLU else N)
     if not a.is_cuda:
@@ -182,44 +185,41 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             out.copy_(res)
             return out
         return res
-    if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
+    if a.dtype is not torch.bfloat16 or b.dtype is not torch.bfloat16:
         raise TypeError("gemm expects bf16 operands on the GPU")
+    dev = a.device
     if out is None:
-        out = torch.empty((M, out_cols), dtype=out_dtype, device=a.device)
+        out = torch.empty((M, out_cols), dtype=out_dtype, device=dev)
+        out_ptr, ldo = out.data_ptr(), out_cols
     else:
         # The epilogue's stores are sized from M, N and the pitch: anything else would be written past its end.
         scatter = comm is not None and bool(comm.scatter_out)
         want = (int(comm.rows_per_owner) if scatter else M, out_cols)      # routed rows land in the owners' partial buffers
-        if out.dim() != 2 or out.shape[1] != want[1] or (out.shape[0] < want[0] if scatter else out.shape[0] != want[0]):
-            raise ValueError(f"out has shape {tuple(out.shape)}, the product needs {want}")
-        if out.dtype != out_dtype:
+        osh = out.shape
+        if len(osh) != 2 or osh[1] != want[1] or (osh[0] < want[0] if scatter else osh[0] != want[0]):
+            raise ValueError(f"out has shape {tuple(osh)}, the product needs {want}")
+        if out.dtype is not out_dtype:
             raise ValueError(f"out is {out.dtype}, the epilogue writes {out_dtype}")
-        if out.device != a.device:
+        if out.device != dev:
             raise ValueError("out is on another device than the operands")
-        if out.stride(-1) != 1 or out.data_ptr() % 16 or (out.stride(0) * out.element_size()) % 16:
+        ldo, last = out.stride()
+        out_ptr = out.data_ptr()
+        if last != 1 or out_ptr % 16 or (ldo * out.element_size()) % 16:
             raise ValueError("out needs a contiguous last dimension, a 16-byte aligned base and a 16-byte multiple row pitch")
-    for name, t, cols in (("aux_in", aux_in, 2 * N if flags & EPI_DSWIGLU else N), ("aux_out", aux_out, N)):
-        if t is None:
-            continue
-        if t.dim() != 2 or t.shape[0] != M or t.shape[1] != cols or t.dtype != torch.bfloat16 or t.device != a.device \
-                or t.stride(-1) != 1:
-            raise ValueError(f"{name} must be a bf16 [{M}, {cols}] tensor on the operands' device with a contiguous last "
-                             f"dimension, got {tuple(t.shape)} {t.dtype}")
-    args = GemmArgs()
-    args.a, args.b, args.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.bias = bias.data_ptr() if bias is not None else None
-    args.aux_in = aux_in.data_ptr() if aux_in is not None else None
-    args.aux_out = aux_out.data_ptr() if aux_out is not None else None
-    args.M, args.N, args.K = M, N, K
-    args.lda, args.ldb, args.ldo = a.stride(0), b.stride(0), out.stride(0)
-    args.ld_aux_in = aux_in.stride(0) if aux_in is not None else 0
-    args.ld_aux_out = aux_out.stride(0) if aux_out is not None else 0
-    args.a_mn, args.b_mn = int(a_mn), int(b_mn)
-    args.flags, args.alpha = flags, alpha
-    args.tile_n, args.max_ctas = tile_n, max_ctas
+    if aux_in is not None:
+        _check_aux("aux_in", aux_in, M, 2 * N if flags & EPI_DSWIGLU else N, dev)
+    if aux_out is not None:
+        _check_aux("aux_out", aux_out, M, N, dev)
     if comm is None and _piggyback is not None:
         comm = _take_piggyback(M, N, K, comm)
-    args.comm = C.pointer(comm) if comm is not None else None
+    # fields in the order of the structure: one call instead of an attribute access each
+    args = GemmArgs(a.data_ptr(), b.data_ptr(), out_ptr, bias.data_ptr() if bias is not None else None,
+                    aux_in.data_ptr() if aux_in is not None else None, aux_out.data_ptr() if aux_out is not None else None,
+                    M, N, K, ast[0], bst[0], ldo, aux_in.stride(0) if aux_in is not None else 0,
+                    aux_out.stride(0) if aux_out is not None else 0, a_mn, b_mn, flags, alpha, tile_n, max_ctas)
+    if comm is not None:
+        args.comm = C.pointer(comm)
     rc = _lib.get().mlf_gemm_bf16(C.byref(args), C.c_uint64(_lib.stream_handle()))
-    _lib.check(rc, "mlf_gemm_bf16")
+    if rc:
+        _lib.check(rc, "mlf_gemm_bf16")
     return out
