@@ -52,6 +52,7 @@ struct PagedDecodeParams {
   const __nv_bfloat16* v_new;
   const long long* slots;
   float theta;
+  int early;
 };
 
 // Rotary embedding of a pair (d, d + 64); cs = (cosine, sine) of its angle.
@@ -136,7 +137,10 @@ paged_decode_kernel(const PagedDecodeParams p) {
   extern __shared__ __align__(128) uint8_t p_dsm[];
   const int b = blockIdx.x, hkv = blockIdx.y, sp = blockIdx.z;
   pdl_trigger();
-  pdl_wait();
+  // With step inputs and cached rows that no queued kernel writes (p.early), the lengths, the table and the first chunks
+  // are fetched while the QKV product ahead is still running; what that product writes is touched behind the wait below.
+  const bool early = ROPE && p.early != 0;
+  if (!early) pdl_wait();
   // A length beyond what the row of the block table can describe would index past the table: it is
   // clamped to the table's capacity and reported, like every other rejected index in this file.
   int len = p.seq_lens[b];
@@ -155,6 +159,7 @@ paged_decode_kernel(const PagedDecodeParams p) {
 
   float* ws = p.ws ? p.ws + ((((long long)b * p.Hkv + hkv) * p.splits + sp) * G) * (PD + 2) : nullptr;
   if (t_lo >= t_hi) {
+    if (early) pdl_wait();
     if (ws) {
       for (int i = tid; i < G * (PD + 2); i += P_THREADS) ws[i] = (i % (PD + 2)) == 0 ? -INFINITY : 0.f;
       if (p.counters) finish_split<G>(p, b, hkv);
@@ -212,6 +217,7 @@ paged_decode_kernel(const PagedDecodeParams p) {
     }
     __syncthreads();
   }
+  if (early) pdl_wait();
   // the new token's key (rotated) and value, 16 bytes of each in the 16 threads that stage its row
   uint4 nk = make_uint4(0u, 0u, 0u, 0u), nv = nk;
   const bool has_new = ROPE && t_hi == len;
@@ -555,7 +561,7 @@ namespace mlf {
 // slots != null: the packed form (theta)
 static int launch_paged_decode(const void* q, long long ldq, const void* cache, const int* block_table, const int* seq_lens,
                                const long long* slots, void* out, float* ws, void* counters, int B, int Hq, int Hkv, int block_size,
-                               int max_blocks, int num_blocks, int max_seq_len, int split_tokens, float scale, float theta, uint64_t stream) {
+                               int max_blocks, int num_blocks, int max_seq_len, int split_tokens, float scale, float theta, int early, uint64_t stream) {
   MLF_REQUIRE(ldq % 2 == 0 && (reinterpret_cast<uintptr_t>(q) & 3) == 0, "paged_decode: query rows must be 4-byte aligned");
   MLF_REQUIRE(B > 0 && Hq % Hkv == 0, "paged_decode: bad head counts");
   const int G = Hq / Hkv;
@@ -584,6 +590,7 @@ static int launch_paged_decode(const void* q, long long ldq, const void* cache, 
   p.v_new = rope ? p.k_new + (long long)Hkv * PD : nullptr;
   p.slots = slots;
   p.theta = theta;
+  p.early = early;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   dim3 grid(B, Hkv, splits);
   static bool attr_set[64] = {false};
@@ -615,20 +622,23 @@ MLF_API int mlf_paged_decode_ld(const void* q, long long ldq, const void* cache,
                                 float* ws, void* counters, int B, int Hq, int Hkv, int block_size, int max_blocks, int num_blocks,
                                 int max_seq_len, int split_tokens, float scale, uint64_t stream) {
   return launch_paged_decode(q, ldq, cache, block_table, seq_lens, nullptr, out, ws, counters, B, Hq, Hkv, block_size, max_blocks,
-                             num_blocks, max_seq_len, split_tokens, scale, 0.f, stream);
+                             num_blocks, max_seq_len, split_tokens, scale, 0.f, 0, stream);
 }
 
 // Decode attention straight from the QKV product: qkv [B, (Hq + 2 Hkv) * 128] (pitch ld, 16-byte aligned rows), not yet
 // rotated. The new token of sequence b is the last of its seq_lens[b] tokens; its rotated key and its value are written
 // to cache slot slots[b] (< 0: not written) and attended to like the cached ones. Same results as mlf_rope_kv_write with
-// positions seq_lens - 1 followed by mlf_paged_decode_ld.
+// positions seq_lens - 1 followed by mlf_paged_decode_ld. inputs_static: no kernel queued on the stream since the last
+// launch without programmatic overlap writes block_table, seq_lens or the cached rows of earlier tokens; they may then be
+// read before the kernels ahead have finished.
 MLF_API int mlf_paged_decode_rope(const void* qkv, long long ld, void* cache, const int* block_table, const int* seq_lens,
                                   const long long* slots, void* out, float* ws, int B, int Hq, int Hkv, int block_size, int max_blocks,
-                                  int num_blocks, int max_seq_len, int split_tokens, float scale, float theta, uint64_t stream) {
+                                  int num_blocks, int max_seq_len, int split_tokens, float scale, float theta, int inputs_static,
+                                  uint64_t stream) {
   MLF_REQUIRE(slots != nullptr && theta > 0.f, "paged_decode_rope: slots and a positive theta are needed");
   MLF_REQUIRE(ld % 8 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 15) == 0, "paged_decode_rope: rows must be 16-byte aligned");
   return launch_paged_decode(qkv, ld, cache, block_table, seq_lens, slots, out, ws, nullptr, B, Hq, Hkv, block_size, max_blocks, num_blocks,
-                             max_seq_len, split_tokens, scale, theta, stream);
+                             max_seq_len, split_tokens, scale, theta, inputs_static, stream);
 }
 
 MLF_API int mlf_kv_cache_write(void* cache, const void* k, const void* v, const long long* slots, long long T, int Hkv,

@@ -407,15 +407,18 @@ def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Ten
 
 
 def paged_decode_rope(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Tensor, seq_lens: torch.Tensor, slots: torch.Tensor,
-                      Hq: int, Hkv: int, max_seq_len: int, theta: float, *, scale: Optional[float] = None, split_tokens: int = 0) -> torch.Tensor:
+                      Hq: int, Hkv: int, max_seq_len: int, theta: float, *, scale: Optional[float] = None, split_tokens: int = 0, inputs_static: bool = False) -> torch.Tensor:
     """:func:`rope_kv_write_` at positions ``seq_lens - 1`` followed by :func:`paged_decode` in one launch: ``qkv``
     [B, (Hq + 2 Hkv) * 128] holds the unrotated projection of each sequence's newest token, which ``seq_lens`` counts;
-    its key and value go to cache slot ``slots`` (int64, < 0 skips the write). ``qkv`` is left as it is."""
+    its key and value go to cache slot ``slots`` (int64, < 0 skips the write). ``qkv`` is left as it is. ``inputs_static``: no kernel
+    queued since the last launch without programmatic overlap writes ``block_table``, ``seq_lens`` or the cached rows of
+    earlier tokens, which may then be read ahead of the kernels before this one."""
     B = qkv.shape[0]
     nb, two, bs, Hc, D = kv_cache.shape
     assert D == 128 and two == 2 and Hc == Hkv and kv_cache.is_contiguous() and qkv.shape[1] == (Hq + 2 * Hkv) * D
     assert qkv.stride(1) == 1 and qkv.dtype == torch.bfloat16 and kv_cache.dtype == torch.bfloat16 and slots.dtype == torch.int64
     assert block_table.dtype == torch.int32 and block_table.is_contiguous() and seq_lens.dtype == torch.int32
+    assert not inputs_static or (seq_lens.is_contiguous() and slots.is_contiguous())      # a copy here would write them
     out = torch.empty(B, Hq, D, dtype=qkv.dtype, device=qkv.device)
     L = _L()
     L.mlf_paged_decode_ws_elems.restype = C.c_longlong
@@ -426,7 +429,7 @@ def paged_decode_rope(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: to
     ws = torch.empty(int(L.mlf_paged_decode_ws_elems(B, Hq, splits)), dtype=torch.float32, device=qkv.device) if splits > 1 else None
     rc = L.mlf_paged_decode_rope(_p(qkv), C.c_longlong(qkv.stride(0)), _p(kv_cache), _p(block_table), _p(seq_lens.contiguous()),
                                  _p(slots.contiguous()), _p(out), _p(ws), B, Hq, Hkv, bs, block_table.shape[1], nb, int(max_seq_len), st,
-                                 C.c_float(scale if scale is not None else D ** -0.5), C.c_float(theta), _st())
+                                 C.c_float(scale if scale is not None else D ** -0.5), C.c_float(theta), int(inputs_static), _st())
     _lib.check(rc, "mlf_paged_decode_rope")
     return out
 

@@ -11,8 +11,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("Hq,Hkv", [(4, 4), (4, 2), (16, 4), (8, 1)])
 @pytest.mark.parametrize("split", [0, 128, 384])
-@pytest.mark.parametrize("bs", [16, 24])
-def test_same_as_separate_launches(Hq, Hkv, split, bs):
+@pytest.mark.parametrize("bs,static", [(16, False), (16, True), (24, True)])
+def test_same_as_separate_launches(Hq, Hkv, split, bs, static):
     torch.manual_seed(Hq * 10 + Hkv)
     # chunk and split edges: the newest token alone, first / last of a 64-token chunk, of a split, of a page
     lens = [1, 2, 16, 17, 63, 64, 65, 128, 129, 385, 640, 1, 1000]
@@ -40,7 +40,8 @@ def test_same_as_separate_launches(Hq, Hkv, split, bs):
     probe[pad, 0, 0] = rot[11, Hq * D:(Hq + Hkv) * D].view(Hkv, D)
     probe[pad, 1, 0] = rot[11, (Hq + Hkv) * D:].view(Hkv, D)
     want = native.paged_decode(rot[:, :Hq * D].view(B, Hq, D), probe, table, sl, max(lens), split_tokens=split)
-    got = native.paged_decode_rope(qkv, b_cache, table, sl, slots, Hq, Hkv, max(lens), 500000.0, split_tokens=split)
+    got = native.paged_decode_rope(qkv, b_cache, table, sl, slots, Hq, Hkv, max(lens), 500000.0, split_tokens=split,
+                                   inputs_static=static)
     assert torch.equal(got, want)
     assert torch.equal(a_cache, b_cache)
     assert _lib.read_status() == 0
