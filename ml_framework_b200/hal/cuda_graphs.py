@@ -420,6 +420,18 @@ class CUDAGraphManager:
             self.fallbacks += 1
             return fn(*inputs)
 
+    def run_from_host(self, name: str, fn: Callable, host: torch.Tensor, device: torch.device):
+        """``run(name, fn, host.to(device))`` for one pinned host tensor that goes straight into the captured graph's
+        static input: one copy on the stream instead of an upload into a new buffer and a copy from there."""
+        idx = device.index if device.index is not None else torch.cuda.current_device()
+        cg = self._graphs.get((name, (tuple(host.shape), host.dtype, idx)))
+        if cg is None:
+            return self.run(name, fn, host.to(device, non_blocking=True))
+        cg.static_inputs[0].copy_(host, non_blocking=True)
+        cg.graph.replay()
+        cg.replays += 1
+        return cg.static_outputs
+
     def stats(self) -> Dict[str, int]:
         return {"graphs": len(self._graphs), "fallbacks": self.fallbacks,
                 "replays": sum(g.replays for g in self._graphs.values())}

@@ -380,7 +380,7 @@ class PagedLlamaExecutor:
 
         def attend_packed(li, qkv):
             return native.paged_decode_rope(qkv, self.kv.caches[li], table, lens, slots, self.hq, self.hkv, max_len, self.mc.rope_theta,
-                                            split_tokens=self.cfg.decode_split_tokens)
+                                            split_tokens=self.cfg.decode_split_tokens, inputs_static=True)
         x = self._embed(last[None])[0]
         for li, blk in enumerate(self.m.blocks):
             x = self._block(li, blk, x, pos, slots, attend, attend_packed if self.native else None)
@@ -415,17 +415,16 @@ class PagedLlamaExecutor:
         if done < B:
             raise MemoryError(f"KV cache exhausted while decoding request {ids[done]}")
         max_len = top + 1
-        packed = host.to(dev, non_blocking=True)
 
         def step(buf, length):
             b32 = buf[head:].view(torch.int32)
             return self._decode_core(buf[:Bp], buf[Bp:2 * Bp], buf[2 * Bp:head], b32[Bp:Bp * (1 + width)].view(Bp, width), b32[:Bp], length)
 
         if self._graphs is None:
-            return step(packed, max_len).tolist()
+            return step(host.to(dev, non_blocking=True), max_len).tolist()
         Lp = min(self._bucket(max_len, 512), max(self.cfg.max_seq_len, 512))
-        out = self._graphs.run(f"decode_B{Bp}_L{Lp}", lambda buf: step(buf, Lp), packed)
-        return out[:B].tolist()
+        out = self._graphs.run_from_host(f"decode_B{Bp}_L{Lp}", lambda buf: step(buf, Lp), host, dev)
+        return (out if B == Bp else out[:B]).tolist()
 
     # ---- scheduler entry point
     def execute_batch(self, batch: Batch) -> BatchOutput:
