@@ -17,6 +17,7 @@
 //             once to the peer's barrier (address translated with mapa).
 //   tfull[a]  in each CTA (same double commit), tempty[a] in the leader, count 8 or 16: the
 //             epilogue warps of each CTA arrive (the peer's through a cluster-scope arrive).
+// When the last round of tiles would occupy at most half of the pairs, its tiles run as two items of 128 columns each.
 // Every wait is bounded; a cluster barrier at the end keeps either CTA from exiting while the
 // other may still touch its shared memory.
 #include <cooperative_groups.h>
@@ -108,7 +109,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                          const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ CUtensorMap tmPre,
                          const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ PeerMaps peer_maps,
                          const GemmKernelParams p, const int tma_epilogue, const int tma_aux, const int k_splits,
-                         const int reduce_out, const int epi_halves) {
+                         const int reduce_out, const int epi_halves, const int n_whole) {
   // Copy CTAs come in whole clusters (their count is even) and never touch the cluster barrier.
   if ((int)blockIdx.x < p.n_copy_ctas) {
     gather_copy_role(p);
@@ -164,7 +165,21 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const int n_pairs = ((int)gridDim.x - p.n_copy_ctas) >> 1;
   // Work items: (tile, k-split). Splits of one tile are consecutive items, their partial products meet in
   // global memory through TMA reduction stores (the host cleared or kept `out` accordingly).
-  const int num_tiles = p.tiles_m * p.tiles_n * k_splits;   // tiles of 256 x 256, times splits
+  // Tiles from n_whole on (k_splits is 1 then) are two items each, of 128 columns.
+  const int whole_items = n_whole * k_splits;
+  const int num_items = whole_items + 2 * (p.tiles_m * p.tiles_n - n_whole);
+  auto item_at = [&](int t, int& tm, int& col0, int& cols) {
+    int tile = t / k_splits, tn;
+    cols = T2_BN;
+    col0 = 0;
+    if (t >= whole_items) {
+      tile = n_whole + ((t - whole_items) >> 1);
+      cols = T2_BN / 2;
+      col0 = ((t - whole_items) & 1) * cols;
+    }
+    tile_coords(tile, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);
+    col0 += tn * T2_BN;
+  };
   const int num_kb_all = (p.K + BK - 1) / BK;
   const int kb_per = (num_kb_all + k_splits - 1) / k_splits;
 
@@ -176,31 +191,33 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       // A weight that nobody writes starts streaming while the kernels ahead are still running: the first pass over
       // the ring gets its B halves here, its A halves after the wait.
       int pre = 0;
-      if (p.b_static && pair < num_tiles) {
-        int tm, tn;
-        tile_coords(pair / k_splits, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);
+      // `cols / 2` columns of B per CTA, 64 of them (8 KB) per load
+      auto load_b = [&](uint32_t sb, int k0, int n0, int cols, uint32_t bar) {
+        for (int j = 0; j < cols / 128; ++j) {
+          const int n = n0 + 64 * j;
+          tma_load_2d_pair(sb + j * (BK * 128), &tmB, p.b_mn ? n : k0, p.b_mn ? k0 : n, bar);
+        }
+      };
+      if (p.b_static && pair < num_items) {
+        int tm, col0, cols;
+        item_at(pair, tm, col0, cols);
         const int kb0 = (pair % k_splits) * kb_per, kb1 = min(num_kb_all, kb0 + kb_per);
-        const int n0 = tn * T2_BN + (int)rank * T2_BNH;
+        const int n0 = col0 + (int)rank * (cols / 2);
         for (; pre < T2_STAGES && kb0 + pre < kb1; ++pre) {
           const uint32_t sb = smem_base + pre * T2_STAGE + T2_STAGE_A;
           const uint32_t lead_full = mapa_u32(full_bar(pre), 0);
-          if (rank == 0) mbar_expect_tx(full_bar(pre), 2 * T2_STAGE);
-          if (!p.b_mn) {
-            tma_load_2d_pair(sb, &tmB, (kb0 + pre) * BK, n0, lead_full);
-          } else {
-#pragma unroll
-            for (int j = 0; j < T2_BNH / 64; ++j) tma_load_2d_pair(sb + j * (BK * 128), &tmB, n0 + 64 * j, (kb0 + pre) * BK, lead_full);
-          }
+          if (rank == 0) mbar_expect_tx(full_bar(pre), 2 * T2_STAGE_A + cols * (BK * 2));
+          load_b(sb, (kb0 + pre) * BK, n0, cols, lead_full);
         }
       }
       pdl_wait();
-      for (int t = pair; t < num_tiles; t += n_pairs) {
-        int tm, tn;
-        tile_coords(t / k_splits, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);
+      for (int t = pair; t < num_items; t += n_pairs) {
+        int tm, col0, cols;
+        item_at(t, tm, col0, cols);
         const int kb0 = (t % k_splits) * kb_per, kb1 = min(num_kb_all, kb0 + kb_per);
         if (kb0 >= kb1) continue;
         const int m0 = tm * 256 + (int)rank * BM;
-        const int n0 = tn * T2_BN + (int)rank * T2_BNH;
+        const int n0 = col0 + (int)rank * (cols / 2);
         bool ok = true;
         if (p.gather_operand != 0) {
           // this CTA's 128 rows of the gathered operand must have landed
@@ -218,7 +235,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           const uint32_t sa = smem_base + s * T2_STAGE;
           const uint32_t sb = sa + T2_STAGE_A;
           const uint32_t lead_full = mapa_u32(full_bar(s), 0);
-          if (rank == 0 && !b_loaded) mbar_expect_tx(full_bar(s), 2 * T2_STAGE);
+          if (rank == 0 && !b_loaded) mbar_expect_tx(full_bar(s), 2 * T2_STAGE_A + cols * (BK * 2));
           const int k0 = kb * BK;
           if (!p.a_mn) {
             tma_load_2d_pair(sa, &tmA, k0, m0, lead_full);
@@ -226,13 +243,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * (BK * 128), &tmA, m0 + 64 * j, k0, lead_full);
           }
-          if (b_loaded) {
-          } else if (!p.b_mn) {
-            tma_load_2d_pair(sb, &tmB, k0, n0, lead_full);
-          } else {
-#pragma unroll
-            for (int j = 0; j < T2_BNH / 64; ++j) tma_load_2d_pair(sb + j * (BK * 128), &tmB, n0 + 64 * j, k0, lead_full);
-          }
+          if (!b_loaded) load_b(sb, k0, n0, cols, lead_full);
           if (++s == T2_STAGES) { s = 0; ph ^= 1u; }
         }
         if (!ok) break;
@@ -241,14 +252,16 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   } else if (warp == 1) {
     // ===================== MMA issuer (leader CTA only) =====================
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(256, T2_BN, p.a_mn, p.b_mn);
+      const uint32_t idesc_whole = make_idesc_bf16(256, T2_BN, p.a_mn, p.b_mn);
+      const uint32_t idesc_half = make_idesc_bf16(256, T2_BN / 2, p.a_mn, p.b_mn);
       const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, a_kstep = p.a_mn ? UMMA_K * 128 : UMMA_K * 2;
       const uint32_t b_lbo = p.b_mn ? BK * 128 : 16, b_kstep = p.b_mn ? UMMA_K * 128 : UMMA_K * 2;
       int s = 0;
       uint32_t ph = 0;
       int it = 0;
       bool ok = true;
-      for (int t = pair; t < num_tiles && ok; t += n_pairs) {
+      for (int t = pair; t < num_items && ok; t += n_pairs) {
+        const uint32_t idesc = t < whole_items ? idesc_whole : idesc_half;
         const int kb0 = (t % k_splits) * kb_per, kb1 = min(num_kb_all, kb0 + kb_per);
         if (kb0 >= kb1) continue;
         const int acc = it & 1;
@@ -286,14 +299,12 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     const int q = warp & 3;
     const int ew = warp - 2;
     const int half = ew >> 2;                  // which half of the tile's columns (0 when there is one warp per quarter)
-    const int my_cols = T2_BN / epi_halves;
     const bool two_bufs = epi_halves == 1;     // the staging tiles of the absent warps are the second ones
     const bool out_fp32 = (p.flags & MLF_EPI_OUT_FP32) != 0;
     const bool swiglu = (p.flags & MLF_EPI_SWIGLU) != 0;
     const bool dswiglu = (p.flags & MLF_EPI_DSWIGLU) != 0;
     // Column units of this warp: 64 accumulator columns, or 32 where (gate, up) pairs make 64 output columns of them.
     const int unit_cols = dswiglu ? 32 : 64;
-    const int n_units = my_cols / unit_cols;
     const uint32_t stg0 = stg_base + (uint32_t)ew * T2_STG_BYTES;
     uint32_t emits = 0;                        // staging tiles handed out by this warp
     uint32_t aux_units = 0;                    // aux tiles consumed by this warp
@@ -302,11 +313,13 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     uint32_t ax_n = 0;                         // aux tiles requested
     auto request_aux = [&]() {                 // lane 0; the staging tile it goes to is free
       while (true) {
-        if (++ax_u >= n_units) { ax_u = 0; ax_t += n_pairs; }
-        if (ax_t >= num_tiles) return;
-        int tm, tn;
-        tile_coords(ax_t, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);     // k_splits is 1 whenever there is an aux_in
-        const int nb = tn * T2_BN + half * my_cols + ax_u * unit_cols;
+        ++ax_u;
+        if (ax_t >= num_items) return;
+        int tm, col0, cols;
+        item_at(ax_t, tm, col0, cols);         // k_splits is 1 whenever there is an aux_in
+        const int my_cols = cols / epi_halves;
+        if (ax_u * unit_cols >= my_cols) { ax_u = -1; ax_t += n_pairs; continue; }
+        const int nb = col0 + half * my_cols + ax_u * unit_cols;
         if (nb >= p.N) continue;
         mbar_expect_tx(aux_bar(ew), T2_STG_BYTES);
         tma_load_2d(stg0 + (two_bufs ? (ax_n & 1u) * 4u * T2_STG_BYTES : 0u), &tmAux, dswiglu ? 2 * nb : nb, tm * 256 + (int)rank * BM + q * 32, aux_bar(ew));
@@ -316,15 +329,17 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     };
     if (tma_aux && lane == 0) request_aux();
     int it = 0;
-    for (int t = pair; t < num_tiles; t += n_pairs) {
+    for (int t = pair; t < num_items; t += n_pairs) {
       if ((t % k_splits) * kb_per >= min(num_kb_all, (t % k_splits) * kb_per + kb_per)) continue;
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
-      int tm, tn;
-      tile_coords(t / k_splits, p.tiles_m, p.tiles_n, p.rot_m, p.rot_n, tm, tn);
+      int tm, col0, cols;
+      item_at(t, tm, col0, cols);
+      const int my_cols = cols / epi_halves;
+      const int n_units = my_cols / unit_cols;
       const int m0 = tm * 256 + (int)rank * BM;
       const int m = m0 + q * 32 + lane;
-      const int nh = tn * T2_BN + half * my_cols;                       // first column of this warp
+      const int nh = col0 + half * my_cols;                             // first column of this warp
       const uint32_t t_acc = tmem_base + acc * T2_BN + half * my_cols + ((uint32_t)(q * 32) << 16);
       if (!mbar_wait_warp(tfull_bar(acc), acc_ph, abort_flag, p.err, ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after_sync();
@@ -597,7 +612,7 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   if (!a->a_mn) rc = cached_tmap_bf16(&tmA, a_base, a->K, a->M, a->lda, BK, BM);
   else rc = cached_tmap_bf16(&tmA, a_base, a->M, a->K, a->lda, 64, BK);
   if (rc) return rc;
-  if (!a->b_mn) rc = cached_tmap_bf16(&tmB, b_base, a->K, a->N, a->ldb, BK, T2_BNH);
+  if (!a->b_mn) rc = cached_tmap_bf16(&tmB, b_base, a->K, a->N, a->ldb, BK, 64);
   else rc = cached_tmap_bf16(&tmB, b_base, a->N, a->K, a->ldb, 64, BK);
   if (rc) return rc;
   // Outputs go through TMA stores when they are bf16 rows with aligned pitches.
@@ -664,19 +679,22 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
     if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_2cta_kernel, &cfg) != cudaSuccess || n <= 0) n = sm_count() / 2;
     max_clusters[dev & 63] = n;
   }
-  int pairs = sms / 2;
-  if (pairs > max_clusters[dev & 63]) pairs = max_clusters[dev & 63];
-  if (pairs > num_tiles) pairs = num_tiles;
-  if (pairs < 1) pairs = 1;
+  int avail = sms / 2;                       // CTA pairs that run at a time
+  if (avail > max_clusters[dev & 63]) avail = max_clusters[dev & 63];
+  if (avail < 1) avail = 1;
+  // A last round with work for at most half of the pairs: its tiles are cut into two items of 128 columns each, which
+  // costs 0.8 - 0.9 of a whole round (at N = 128 an MMA reads A from shared memory for half the math), with the same sums:
+  // 8192 x 2048 x 2048 49.4 -> 46.8 us, 8192 x 2048 x 8192 189.5 -> 185.3, 8192 x 2048 x 50304 1189 -> 1124,
+  // 4096 x 4096 x 4096 with a residual 102.1 -> 98.3. Above half a round two of the items would meet on one pair again.
+  const int rest = num_tiles % avail;
+  const bool halve = cm == nullptr && rest > 0 && 2 * rest <= avail;
   // Split K when the tiles alone cannot fill the GPU (weight gradients of narrow layers: few tiles, long K).
   // Splits add their partial products into `out` with TMA reduction stores.
   int k_splits = 1;
   // Between a decode step's rows and 512 a product keeps its single fp32 sum: the partial products meet in bf16.
   if (plain && tma_epi && (a->M <= 256 || a->M >= 512)) {
     const int kb_all = (a->K + BK - 1) / BK;
-    int avail = sms / 2;
-    if (avail > max_clusters[dev & 63]) avail = max_clusters[dev & 63];
-    double best = (double)((num_tiles + avail - 1) / avail);
+    double best = (double)((num_tiles + avail - 1) / avail) - (halve ? 0.2 : 0.0);
     for (int ks = 2; ks <= 8; ++ks) {
       if (kb_all / ks < 8) break;
       const double cost = (double)((num_tiles * ks + avail - 1) / avail) / ks;
@@ -686,6 +704,8 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
       if (cost < best * 0.8) { best = cost; k_splits = ks; }
     }
   }
+  const int n_whole = halve && k_splits == 1 ? num_tiles - rest : num_tiles;
+  const int num_items = n_whole * k_splits + 2 * (num_tiles - n_whole);
   // Two epilogue warps per quarter where the work of one does not fit behind the next tile's products: gated and
   // derivative epilogues (8192 x 14336 x 4096 with dSwiGLU 960 -> 691 us, 4096 x 28672 x 4096 with SwiGLU 686 -> 612 us,
   // 8192 x 8192 x 2048 with dGELU 225 -> 211 us), a residual (its tile has to arrive first), and any short K (2331 x 4096
@@ -696,16 +716,13 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   const int reduce_out = (k_splits > 1 || (a->flags & MLF_EPI_ACCUM)) ? 1 : 0;
   if (k_splits > 1 && !(a->flags & MLF_EPI_ACCUM))
     MLF_CHECK_CUDA(cudaMemset2DAsync(a->out, (size_t)a->ldo * 2, 0, (size_t)a->N * 2, (size_t)a->M, st));
-  pairs = sms / 2;
-  if (pairs > max_clusters[dev & 63]) pairs = max_clusters[dev & 63];
-  if (pairs > num_tiles * k_splits) pairs = num_tiles * k_splits;
-  if (pairs < 1) pairs = 1;
+  const int pairs = avail < num_items ? avail : num_items;
   if (cm == nullptr) {
     MLF_CHECK_CUDA(launch_pdl(gemm_tcgen05_2cta_kernel, dim3(2 * pairs), dim3(T2_THREADS), T2_SMEM, st, tmA, tmB, tmOut, tmPre, tmAux,
-                              peer_maps, p, tma_epi, tma_aux, k_splits, reduce_out, epi_halves));
+                              peer_maps, p, tma_epi, tma_aux, k_splits, reduce_out, epi_halves, n_whole));
   } else {                                       // copy CTAs and routed rows touch peers' memory: after everything ahead
     gemm_tcgen05_2cta_kernel<<<n_copy + 2 * pairs, T2_THREADS, T2_SMEM, st>>>(tmA, tmB, tmOut, tmPre, tmAux, peer_maps, p, tma_epi, tma_aux,
-                                                                                k_splits, reduce_out, epi_halves);
+                                                                                k_splits, reduce_out, epi_halves, n_whole);
     MLF_CHECK_CUDA(cudaGetLastError());
   }
   count_launch();
