@@ -323,7 +323,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       // two elements per fused multiply-add and addition: the pipes beside the exponentials' one issue half as often
       const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2), nm2 = pack_f32x2(-m_used, -m_used);
-      uint64_t rs0 = 0ull, rs1 = 0ull;
+      uint64_t rs = 0ull;                      // sums of the even and of the odd keys (four sums are no faster)
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         uint32_t pk[32];
@@ -334,7 +334,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           unpack_f32x2(e, e0, e1);
           e0 = exp2f(e0);
           e1 = exp2f(e1);
-          if (i & 1) rs1 = add_f32x2(rs1, pack_f32x2(e0, e1)); else rs0 = add_f32x2(rs0, pack_f32x2(e0, e1));
+          rs = add_f32x2(rs, pack_f32x2(e0, e1));
           pk[i] = pack_bf16x2(e0, e1);
         }
         tmem_st_32x32b_x32(tS(t) + 32 * hh + lane_off, pk);
@@ -342,10 +342,9 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_fence_before_sync();
         mbar_arrive(hh == 0 ? p_half(t) : p_full(t));
       }
-      float ra, rb, rc, rd;
-      unpack_f32x2(rs0, ra, rb);
-      unpack_f32x2(rs1, rc, rd);
-      l += (ra + rb) + (rc + rd);
+      float rs0, rs1;
+      unpack_f32x2(rs, rs0, rs1);
+      l += rs0 + rs1;
     }
     if (ok && n_mine > 0) ok = mbar_wait_warp(pv_done(t), (n_mine - 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN);
     if (ok && n_mine > 0) {

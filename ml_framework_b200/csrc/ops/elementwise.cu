@@ -419,8 +419,9 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* dst, const
       Vec<__nv_bfloat16>::load(reinterpret_cast<const __nv_bfloat16*>(s + 8), b);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        x[j] = a[j] * cs[j] - b[j] * sn[j];
-        y[j] = b[j] * cs[j] + a[j] * sn[j];
+        // the roundings of rope_kernel as it is compiled, spelled out: the same bits
+        x[j] = __fmaf_rn(a[j], cs[j], -__fmul_rn(b[j], sn[j]));
+        y[j] = __fmaf_rn(a[j], sn[j], __fmul_rn(b[j], cs[j]));
       }
       Vec<__nv_bfloat16>::store(reinterpret_cast<__nv_bfloat16*>(o), x);
       Vec<__nv_bfloat16>::store(reinterpret_cast<__nv_bfloat16*>(o + 8), y);

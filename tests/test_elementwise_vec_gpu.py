@@ -52,7 +52,7 @@ def test_rope_qkv(T, Hq, Hkv, inverse):
     native.rope_(want[:, Hq * 128:(Hq + Hkv) * 128].view(T, Hkv, 128), pos, 500000.0, inverse)
     before = wide.clone()
     got = native.rope_qkv(src, pos, Hq, Hkv, 500000.0, inverse)
-    # the same formula, but the compiler may contract a * c - b * s the other way round: an fp32 rounding (2^-24 of values
+    # the same formula; the in-place kernel leaves it to the compiler how a * c - b * s is contracted: an fp32 rounding (2^-24 of values
     # below 8) apart before both are rounded to bf16, so neighbours (2^-7 of the value) at most and almost always equal
     assert ((got.float() - want.float()).abs() <= 2 ** -7 * want.float().abs() + 2 ** -20).all()
     assert (got != want).float().mean() < 1e-3
