@@ -260,6 +260,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       uint32_t ph = 0;
       int it = 0;
       bool ok = true;
+      // The first A tile is requested behind the producer's wait for the kernels ahead: waiting for it from before that
+      // would count their remaining run time against this kernel's wait budget.
+      pdl_wait();
       for (int t = pair; t < num_items && ok; t += n_pairs) {
         const uint32_t idesc = t < whole_items ? idesc_whole : idesc_half;
         const int kb0 = (t % k_splits) * kb_per, kb1 = min(num_kb_all, kb0 + kb_per);

@@ -51,3 +51,32 @@ def test_norm_clears_a_buffer(rows, D, zero_elems):
     assert torch.equal(y0, y1)
     assert not guard[:zero_elems].any() and bool((guard[zero_elems:] == 1).all())
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("M,flags", [(256, 0), (256, _lib.EPI_B_STATIC), (512, 0)])
+def test_wait_budget_starts_behind_the_kernels_ahead(M, flags):
+    """A pair product becomes resident beside a long decode kernel of one CTA (some 0.9 ms for 64 Ki tokens): the time until
+    that kernel's end is not part of the product's own wait budget (400,000 cycles, 0.2 ms; its waits are microseconds)."""
+    from ml_framework_b200.dist.symm import set_wait_budget_cycles
+    torch.manual_seed(M)
+    n, bs = 65536, 16
+    cache = torch.randn(n // bs, 2, bs, 1, 128, device="cuda").to(torch.bfloat16)
+    table = torch.arange(n // bs, dtype=torch.int32, device="cuda")[None]
+    lens = torch.tensor([n], dtype=torch.int32, device="cuda")
+    q = torch.randn(1, 1, 128, device="cuda").to(torch.bfloat16)
+    a = torch.randn(M, 2048, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(4096, 2048, device="cuda") * 2048 ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(4096, device="cuda").to(torch.bfloat16)
+    want = (a.double() @ w.double().t() + bias.double()).float()
+    out = torch.zeros(M, 4096, device="cuda", dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    set_wait_budget_cycles(400_000)
+    try:
+        native.paged_decode(q, cache, table, lens, n, split_tokens=n)
+        gemm(a, w, out=out, bias=bias, flags=flags)
+        status = _lib.read_status()
+    finally:
+        set_wait_budget_cycles(0)
+    assert status == 0
+    # one rounding to bf16 and the fp32 sum of 2048 products of order 2^-5
+    assert bool(((out.float() - want).abs() <= 2 ** -8 * want.abs() + 5e-4).all())
