@@ -538,6 +538,44 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 
 using namespace mlf;
 
+// A last round with work for at most half of the pairs: its tiles are cut into two items of 128 columns each, which
+// costs 0.8 - 0.9 of a whole round (at N = 128 an MMA reads A from shared memory for half the math), with the same sums:
+// 8192 x 2048 x 2048 49.4 -> 46.8 us, 8192 x 2048 x 8192 189.5 -> 185.3, 8192 x 2048 x 50304 1189 -> 1124,
+// 4096 x 4096 x 4096 with a residual 102.1 -> 98.3. Above half a round two of the items would meet on one pair again.
+static bool halves_last_round(int num_tiles, int pairs) {
+  const int rest = num_tiles % pairs;
+  return rest > 0 && 2 * rest <= pairs;
+}
+
+// Parts of K for `num_tiles` tiles on `pairs` CTA pairs when the tiles alone cannot fill the GPU (weight gradients of
+// narrow layers: few tiles, long K). Splits add their partial products into `out` with TMA reduction stores.
+// Candidates are the counts that save a tenth of the rounds each, coarse ones first. One is taken when it saves a fifth
+// of the time that the product takes in one piece (its last round halved where that applies): a split clears the output,
+// adds every tile once more in L2 and rounds the partial sums to bf16. Cost in rounds, then us and the error against 64
+// bits in units of 1e-3, in one piece and split:
+//   75 tiles 1.20 of 1.80 (1280 x 3840 x 8192 in six)  74.8 / 1.66 and 65.1 / 3.62     taken
+//   96 tiles 1.33 of 1.80 (2048 x 3072 x 8192 in three) 78.0 / 1.66 and 73.5 / 2.85    taken
+//  100 tiles 1.50 of 1.80 (2560 x 2560 in two, K = 8192) 80.8 / 1.66 and 77.8 / 2.45, (K = 4096) 42.8 and 44.7   not
+//  108 tiles 1.50 of 1.80 (2304 x 3072 in two, K = 8192) 85.1 and 81.4, (K = 4096) 43.2 and 45.4                 not
+//  112 tiles 1.67 of 2.00 (2048 x 3584 in three, K = 8192) 88.1 and 87.0, (K = 4096) 48.4 and 50.1               not
+//   56 tiles 0.80 of 1.00 (2048 x 1792 in five, K = 8192) 49.4 and 48.1, (K = 4096) 28.8 and 33.0                not
+//  128 tiles 1.75 of 2.00 (2048 x 4096 x 14336 in four) 161 and 170                                              not
+// A finer count never stands in for a coarse one that does not pay: 100 tiles in five (1.40) take 79.5 us at K = 8192 and
+// 49.4 at 4096, with twice the error of one piece.
+MLF_API int mlf_gemm_k_splits(int num_tiles, int K, int pairs) {
+  const int kb_all = (K + BK - 1) / BK;
+  double best = (double)((num_tiles + pairs - 1) / pairs);
+  const double whole = best - (halves_last_round(num_tiles, pairs) ? 0.2 : 0.0);
+  int k_splits = 1;
+  for (int ks = 2; ks <= 8 && kb_all / ks >= 8; ++ks) {
+    const double cost = (double)((num_tiles * ks + pairs - 1) / pairs) / ks;
+    if (cost >= best * 0.9) continue;
+    best = cost;
+    if (cost < whole * 0.8) k_splits = ks;
+  }
+  return k_splits;
+}
+
 // GEMM on CTA pairs, with the same in-kernel communication options as the single-CTA kernel (copy
 // CTAs that gather an operand or prefetch extra segments; an epilogue that routes rows to their
 // owners). Same arguments as mlf_gemm_bf16; returns -4 without launching when the problem is not a
@@ -685,32 +723,10 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   int avail = sms / 2;                       // CTA pairs that run at a time
   if (avail > max_clusters[dev & 63]) avail = max_clusters[dev & 63];
   if (avail < 1) avail = 1;
-  // A last round with work for at most half of the pairs: its tiles are cut into two items of 128 columns each, which
-  // costs 0.8 - 0.9 of a whole round (at N = 128 an MMA reads A from shared memory for half the math), with the same sums:
-  // 8192 x 2048 x 2048 49.4 -> 46.8 us, 8192 x 2048 x 8192 189.5 -> 185.3, 8192 x 2048 x 50304 1189 -> 1124,
-  // 4096 x 4096 x 4096 with a residual 102.1 -> 98.3. Above half a round two of the items would meet on one pair again.
-  const int rest = num_tiles % avail;
-  const bool halve = cm == nullptr && rest > 0 && 2 * rest <= avail;
-  // Split K when the tiles alone cannot fill the GPU (weight gradients of narrow layers: few tiles, long K).
-  // Splits add their partial products into `out` with TMA reduction stores.
-  int k_splits = 1;
+  const bool halve = cm == nullptr && halves_last_round(num_tiles, avail);
   // Between a decode step's rows and 512 a product keeps its single fp32 sum: the partial products meet in bf16.
-  if (plain && tma_epi && (a->M <= 256 || a->M >= 512)) {
-    const int kb_all = (a->K + BK - 1) / BK;
-    const double whole = (double)((num_tiles + avail - 1) / avail) - (halve ? 0.2 : 0.0);
-    double best = whole;
-    for (int ks = 2; ks <= 8; ++ks) {
-      if (kb_all / ks < 8) break;
-      const double cost = (double)((num_tiles * ks + avail - 1) / avail) / ks;
-      // a split has to save a fifth of the rounds: it clears the output, adds every tile once more in L2 and rounds the
-      // partial sums (8192 x 2048 x 8192, 3.5 rounds in two splits against 4: 194 us against 193 us unsplit;
-      // 2048 x 4096 x 14336, 1.75 against 2: 180 us against 167 us). A finer split than one that does pays from a tenth on;
-      // that line is about the sums, not the time: 2331 x 1024 x 50304 takes 212 us in five splits and 203 in three, and a
-      // training step keeps the rounding of its logits' gradient.
-      if (cost < whole * 0.8 && cost < best * 0.9) { best = cost; k_splits = ks; }
-    }
-  }
-  const int n_whole = halve && k_splits == 1 ? num_tiles - rest : num_tiles;
+  const int k_splits = plain && tma_epi && (a->M <= 256 || a->M >= 512) ? mlf_gemm_k_splits(num_tiles, a->K, avail) : 1;
+  const int n_whole = halve && k_splits == 1 ? num_tiles - num_tiles % avail : num_tiles;
   const int num_items = n_whole * k_splits + 2 * (num_tiles - n_whole);
   // Two epilogue warps per quarter where the work of one does not fit behind the next tile's products: gated and
   // derivative epilogues (8192 x 14336 x 4096 with dSwiGLU 960 -> 691 us, 4096 x 28672 x 4096 with SwiGLU 686 -> 612 us,

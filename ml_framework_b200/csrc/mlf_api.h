@@ -75,6 +75,8 @@ int mlf_read_status(int clear);
 int mlf_sm_count(void);
 
 int mlf_gemm_bf16(const MlfGemmArgs* args, uint64_t stream);
+// Host only: into how many parts a CTA-pair product of `num_tiles` tiles splits K when `pairs` pairs run at a time.
+int mlf_gemm_k_splits(int num_tiles, int K, int pairs);
 
 #ifdef __cplusplus
 }
