@@ -329,14 +329,14 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
 
 using namespace mlf;
 
-MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream);
+MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, int split_few_rows, uint64_t stream);
 
 static int g_use_2cta = 1;
 // Selects the CTA-pair kernel for large plain GEMMs (tile_n == 0). tile_n == 512 always selects it.
 MLF_API void mlf_set_gemm_2cta(int on) { g_use_2cta = on; }
 MLF_API int mlf_get_gemm_2cta() { return g_use_2cta; }
 static int g_small_m_split = 1;
-// Routes plain GEMMs with M <= 256 and a large weight to the split-K CTA-pair kernel.
+// Lets plain GEMMs with M <= 256 and a large weight split K on the CTA-pair kernel; off, they keep one fp32 sum.
 MLF_API void mlf_set_gemm_small_m_split(int on) { g_small_m_split = on; }
 
 namespace mlf {
@@ -361,13 +361,15 @@ MLF_API int mlf_gemm_bf16(const MlfGemmArgs* a, uint64_t stream) {
   // Few rows against a large weight (a decode step: M <= 256) is a weight-streaming problem: one row of
   // tiles cannot occupy the GPU, so the pair kernel splits K and every SM streams a slice of the weight.
   const bool plain_out = (a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) == 0 && a->comm == nullptr;
+  // At K = 961 to 1023 a split would still be possible, but does not pay: 200 x 4096 x 1000 takes 10.9 us in one piece,
+  // 14.3 us in two, 16.9 us on single CTAs.
   const bool small_m = g_small_m_split && a->tile_n == 0 && plain_out && a->M <= 256 && a->N >= 1024 && a->K >= 1024;
   // An accumulation on pairs is a bf16 addition to the rounded product; below 512 rows it keeps the single-CTA kernel's
   // fp32 one (a decode step's rows, small_m, aside).
   const int row_line = a->comm != nullptr || (a->flags & MLF_EPI_ACCUM) ? 511 : 128;
   if (a->tile_n == 512 || small_m ||
       (g_use_2cta && a->tile_n == 0 && a->M > row_line && a->N >= 512 && (long long)((a->M + 255) / 256) * ((a->N + 255) / 256) >= 16)) {
-    const int rc2 = mlf_gemm_bf16_2cta(a, stream);
+    const int rc2 = mlf_gemm_bf16_2cta(a, small_m || a->tile_n == 512, stream);
     if (rc2 != -4) return rc2;
   }
   MLF_REQUIRE(a->M > 0 && a->N > 0 && a->K > 0, "bad GEMM shape %d %d %d", a->M, a->N, a->K);

@@ -579,8 +579,9 @@ MLF_API int mlf_gemm_k_splits(int num_tiles, int K, int pairs) {
 // GEMM on CTA pairs, with the same in-kernel communication options as the single-CTA kernel (copy
 // CTAs that gather an operand or prefetch extra segments; an epilogue that routes rows to their
 // owners). Same arguments as mlf_gemm_bf16; returns -4 without launching when the problem is not a
-// fit (the caller then uses the single-CTA kernel).
-MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
+// fit (the caller then uses the single-CTA kernel). split_few_rows: a plain product of up to 256 rows may split K, which
+// the caller decides by its small_m rule; the partial products meet in bf16.
+MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, int split_few_rows, uint64_t stream) {
   MLF_REQUIRE(a != nullptr, "null args");
   const MlfGemmComm* cm = a->comm;
   // one row of tiles that is mostly padding only as a plain product (optionally accumulated), where K is split over the pairs
@@ -724,8 +725,8 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, uint64_t stream) {
   if (avail > max_clusters[dev & 63]) avail = max_clusters[dev & 63];
   if (avail < 1) avail = 1;
   const bool halve = cm == nullptr && halves_last_round(num_tiles, avail);
-  // Between a decode step's rows and 512 a product keeps its single fp32 sum: the partial products meet in bf16.
-  const int k_splits = plain && tma_epi && (a->M <= 256 || a->M >= 512) ? mlf_gemm_k_splits(num_tiles, a->K, avail) : 1;
+  // Below 512 rows a product keeps its single fp32 sum, a decode step's rows aside.
+  const int k_splits = plain && tma_epi && ((split_few_rows && a->M <= 256) || a->M >= 512) ? mlf_gemm_k_splits(num_tiles, a->K, avail) : 1;
   const int n_whole = halve && k_splits == 1 ? num_tiles - num_tiles % avail : num_tiles;
   const int num_items = n_whole * k_splits + 2 * (num_tiles - n_whole);
   // Two epilogue warps per quarter where the work of one does not fit behind the next tile's products: gated and

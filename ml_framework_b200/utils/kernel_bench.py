@@ -195,8 +195,11 @@ def bench_gemm_decode(args) -> list[dict]:
             lib.mlf_set_gemm_fewrow(0)
             lib.mlf_set_gemm_small_m_split(1)
             ms = time_cuda(lambda: gemm(a, b, out=out), iters=20)
+            pairs = lib.mlf_get_gemm_2cta()
             lib.mlf_set_gemm_small_m_split(0)
+            lib.mlf_set_gemm_2cta(0)
             ms_1 = time_cuda(lambda: gemm(a, b, out=out), iters=20)
+            lib.mlf_set_gemm_2cta(pairs)
             lib.mlf_set_gemm_small_m_split(1)
             lib.mlf_set_gemm_fewrow(1)
             ms_ref = time_cuda(lambda: torch.matmul(a, b.t(), out=out), iters=20)
