@@ -342,6 +342,42 @@ MLF_API void mlf_set_gemm_small_m_split(int on) { g_small_m_split = on; }
 namespace mlf {
 int gemm_fewrow(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldw, long long ldo,
                 int accumulate, int max_ctas, int w_static, uint64_t stream);
+bool halves_last_round(int num_tiles, int pairs);
+
+// Tile columns of the single-CTA kernel: the widest tile that still gives every SM one.
+static int single_cta_bn(int M, int N, int sms) {
+  const long long tm = (M + BM - 1) / BM;
+  if (tm * ((N + 255) / 256) >= sms || N >= 4096) return 256;
+  return tm * ((N + 127) / 128) >= sms ? 128 : 64;
+}
+}  // namespace mlf
+
+// Which kernel takes a product that both could: 1 = CTA pairs (256 x 256 tiles on two SMs), 0 = single CTAs (128 rows).
+// From 512 rows on, and for an operand or rows that come from or go to peers, the line is 16 pair tiles. An accumulation on
+// pairs is a bf16 addition to the rounded product: below 512 rows it keeps the single-CTA kernel's fp32 one.
+// With 129 - 511 rows a pair tile may be half padding, and the SMs that each kernel occupies decide:
+//  - where all 128 x 64 tiles of single CTAs run at once, they do: 300 rows x 2048 x 2048 11.6 us against 13.5 on pairs,
+//    x 2048 x 8192 32.5 / 36.7, x 3072 x 3072 15.6 / 17.7, 200 x 4000 x 2048 13.1 / 15.4; one tile column further they
+//    need a second round: 400 x 2560 x 2560 22.0 / 15.7, 300 x 3584 x 4096 32.7 / 21.8.
+//  - otherwise rounds of 256 columns are compared (a halved last round counts 0.8). Pairs do one faster: they win with up
+//    to one and a half times as many (300 x 28672 x 4096, 3.8 against 3: 85.9 / 93.1 us; x 50304 x 2048, 5.8 against 4:
+//    72.2 / 74.6) and lose above (x 12288 x 4096, 1.8 against 1: 43.1 / 39.3), GELU and stored pre-activations aside, whose
+//    epilogue costs single CTAs more (x 12288 x 2048 with both 29.8 / 37.5). fp32 outputs leave through plain row stores,
+//    which are slower with two SMs at 256 columns each: from a fifth more rounds on single CTAs win (x 12288 x 2048 29.1 / 35.5 us,
+//    x 50304 x 2048 84 / 96; x 18944 x 2048, 2 against 2, 48.5 / 42.5), up to K = 1024 at equal rounds (x 6144 x 1024
+//    19.2 / 20.5 us).
+MLF_API int mlf_gemm_takes_pairs(int M, int N, int K, int flags, int has_comm, int sms) {
+  const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
+  const bool always = M >= 512 || has_comm;
+  if (N < 512 || tiles < 16 || M <= (has_comm || (flags & MLF_EPI_ACCUM) ? 511 : 128)) return 0;
+  if (always) return 1;
+  const long long tm = (M + BM - 1) / BM;
+  if (single_cta_bn(M, N, sms) == 64 && tm * ((N + 63) / 64) <= sms) return 0;
+  const int pairs = sms / 2 > 0 ? sms / 2 : 1;
+  const double on_pairs = (double)((tiles + pairs - 1) / pairs) - (halves_last_round((int)tiles, pairs) ? 0.2 : 0.0);
+  const double single = (double)((tm * ((N + 255) / 256) + sms - 1) / sms);
+  if (flags & MLF_EPI_OUT_FP32) return K <= 1024 ? on_pairs < single : on_pairs < 1.2 * single;
+  return on_pairs < 1.5 * single || (flags & (MLF_EPI_GELU | MLF_EPI_STORE_PRE)) != 0;
 }
 static int g_fewrow = 1;
 // Routes plain products with at most 128 rows against a K-major weight to the weight-as-M stream-K kernel.
@@ -355,20 +391,15 @@ MLF_API int mlf_gemm_bf16(const MlfGemmArgs* a, uint64_t stream) {
                                 a->max_ctas, (a->flags & MLF_EPI_B_STATIC) ? 1 : 0, stream);
     if (rcf != -4) return rcf;
   }
-  // CTA pairs for everything with more than 128 rows and at least 16 pair tiles (split-K fills the GPU when tiles alone
-  // cannot). The line lies at one single-CTA row tile: at 160 / 300 / 400 rows a residual product 4096 x 4096 takes 30 us
-  // on pairs and 38 us on single CTAs, 4096 x 14336 76 against 102 us, SwiGLU 28672 x 4096 54 / 91 / 93 against 66 / 94 / 118.
   // Few rows against a large weight (a decode step: M <= 256) is a weight-streaming problem: one row of
   // tiles cannot occupy the GPU, so the pair kernel splits K and every SM streams a slice of the weight.
   const bool plain_out = (a->flags & ~(MLF_EPI_ACCUM | MLF_EPI_B_STATIC)) == 0 && a->comm == nullptr;
   // At K = 961 to 1023 a split would still be possible, but does not pay: 200 x 4096 x 1000 takes 10.9 us in one piece,
   // 14.3 us in two, 16.9 us on single CTAs.
   const bool small_m = g_small_m_split && a->tile_n == 0 && plain_out && a->M <= 256 && a->N >= 1024 && a->K >= 1024;
-  // An accumulation on pairs is a bf16 addition to the rounded product; below 512 rows it keeps the single-CTA kernel's
-  // fp32 one (a decode step's rows, small_m, aside).
-  const int row_line = a->comm != nullptr || (a->flags & MLF_EPI_ACCUM) ? 511 : 128;
+  const int sms = a->max_ctas > 0 ? a->max_ctas : sm_count();
   if (a->tile_n == 512 || small_m ||
-      (g_use_2cta && a->tile_n == 0 && a->M > row_line && a->N >= 512 && (long long)((a->M + 255) / 256) * ((a->N + 255) / 256) >= 16)) {
+      (g_use_2cta && a->tile_n == 0 && mlf_gemm_takes_pairs(a->M, a->N, a->K, a->flags, a->comm != nullptr, sms))) {
     const int rc2 = mlf_gemm_bf16_2cta(a, small_m || a->tile_n == 512, stream);
     if (rc2 != -4) return rc2;
   }
@@ -379,14 +410,7 @@ MLF_API int mlf_gemm_bf16(const MlfGemmArgs* a, uint64_t stream) {
   const bool gatherB = cm && cm->gather_operand == 2;
 
   int BN = a->tile_n;
-  const int sms = a->max_ctas > 0 ? a->max_ctas : sm_count();
-  if (BN == 0) {
-    const long long tm = (a->M + BM - 1) / BM;
-    if (tm * ((a->N + 255) / 256) >= sms || a->N >= 4096) BN = 256;
-    else if (tm * ((a->N + 127) / 128) >= sms) BN = 128;
-    else BN = 64;
-    if ((a->flags & (MLF_EPI_SWIGLU)) && BN < 64) BN = 64;
-  }
+  if (BN == 0) BN = single_cta_bn(a->M, a->N, sms);
   if (BN == 512) BN = 256;
   MLF_REQUIRE(BN == 64 || BN == 128 || BN == 256, "tile_n must be 64, 128, 256 or 512 (CTA pair)");
 

@@ -542,10 +542,12 @@ using namespace mlf;
 // costs 0.8 - 0.9 of a whole round (at N = 128 an MMA reads A from shared memory for half the math), with the same sums:
 // 8192 x 2048 x 2048 49.4 -> 46.8 us, 8192 x 2048 x 8192 189.5 -> 185.3, 8192 x 2048 x 50304 1189 -> 1124,
 // 4096 x 4096 x 4096 with a residual 102.1 -> 98.3. Above half a round two of the items would meet on one pair again.
-static bool halves_last_round(int num_tiles, int pairs) {
+namespace mlf {
+bool halves_last_round(int num_tiles, int pairs) {
   const int rest = num_tiles % pairs;
   return rest > 0 && 2 * rest <= pairs;
 }
+}  // namespace mlf
 
 // Parts of K for `num_tiles` tiles on `pairs` CTA pairs when the tiles alone cannot fill the GPU (weight gradients of
 // narrow layers: few tiles, long K). Splits add their partial products into `out` with TMA reduction stores.

@@ -77,6 +77,8 @@ int mlf_sm_count(void);
 int mlf_gemm_bf16(const MlfGemmArgs* args, uint64_t stream);
 // Host only: into how many parts a CTA-pair product of `num_tiles` tiles splits K when `pairs` pairs run at a time.
 int mlf_gemm_k_splits(int num_tiles, int K, int pairs);
+// Host only: 1 when a product of this shape, whose few-row forms are settled, runs on CTA pairs of `sms` SMs.
+int mlf_gemm_takes_pairs(int M, int N, int K, int flags, int has_comm, int sms);
 
 #ifdef __cplusplus
 }

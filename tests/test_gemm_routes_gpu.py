@@ -1,5 +1,5 @@
-"""Products with 129 - 511 rows, which run on CTA pairs: against the fp32 statement, around the row counts where the route
-or the split of K changes."""
+"""Products with 129 - 511 rows, on CTA pairs or single CTAs: against the fp32 statement, around the row and column counts
+where the route or the split of K changes."""
 import pytest
 import torch
 
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M", [128, 129, 255, 256, 257, 300, 511, 512])
-@pytest.mark.parametrize("N,K", [(4096, 1024), (4112, 2056)])
+@pytest.mark.parametrize("N,K", [(4096, 1024), (4112, 2056), (3136, 520), (3152, 1024), (12288, 512)])
 @pytest.mark.parametrize("flags,b_mn", [(0, False), (0, True), (L.EPI_RESIDUAL, False), (L.EPI_SWIGLU, False), (L.EPI_ACCUM, False)])
 def test_middle_rows(M, N, K, flags, b_mn):
     torch.manual_seed(M)
