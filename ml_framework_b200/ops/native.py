@@ -359,13 +359,25 @@ def flash_bwd(q, k, v, o, dout, lse, B: int, S: int, *, causal: bool = True, sca
 
 
 # ------------------------------------------------------------------ paged attention / KV cache
-def _decode_split(pairs: int, max_seq_len: int) -> int:
-    """Tokens per split of the decode kernel for ``pairs`` (sequence, KV head) pairs: as many splits as keep all CTAs
-    resident at once (three per SM, 444), none when the pairs alone fill the GPU -- CTAs of a second round start when the
-    short sequences of the first end, and a split costs its start and the merge launch. At least 128 tokens per split.
-    13 sequences of up to 2500 tokens x 8 KV heads: 4 splits 26 us (8: 29 us); 64 of up to 576: none 28.6 us (2: 31 us);
-    128 of up to 1024: none 74 us (2: 79 us); 8 of up to 4000: 6 splits 27.5 us (11: 33 us)."""
-    splits = min(max(1, 444 // pairs), max(1, -(-max_seq_len // 128)))
+def _decode_split(pairs: int, max_seq_len: int, sms: int) -> int:
+    """Tokens per split of the decode kernel for ``pairs`` (sequence, KV head) pairs on ``sms`` SMs, three CTAs of it on
+    each. As many splits as keep all CTAs resident at once, none when the pairs alone fill the GPU: CTAs of a second round
+    start when the short sequences of the first end, and a split costs its start and the merge launch. At least 128 tokens
+    per split. us at the longest of 8 KV heads' sequences, lengths from half of it on: 13 x 2500 4 splits 26 (8: 29);
+    48 x 1024 none 35 (3: 45); 8 x 4000 6 splits 28 (11: 34).
+
+    A split of more than 1024 tokens takes long enough for its CTA to be alone at the end, above all when one sequence is
+    much longer than the others: then what fits two rounds, or three, of resident CTAs (just above a whole number of rounds
+    the last one is nearly empty: 16 x 4096 in 3 / 4 / 6 / 7 splits 47 / 58 / 49 / 53). Up to 2048 tokens, pairs that fill two
+    thirds of the first round stay whole (40 x 2048 1 / 2 / 3 splits 53 / 57 / 56; 36 x 1500 1 / 3 39 / 38). Counts on both
+    sides: 28 x 2048 1 / 3 / 4 splits 46 / 41 / 40, 32 x 4096 1 / 3 / 4 / 5 96 / 82 / 86 / 82, 40 x 4096 1 / 3 / 4
+    101 / 103 / 95, 48 x 4096 1 / 3 109 / 112, 64 x 4096 1 / 2 163 / 148; one sequence of 4000 beside others of 300: 20 in
+    2 / 5 / 6 splits 39 / 25 / 23, 32 in 1 / 3 / 5 66 / 34 / 28, 48 in 1 / 3 67 / 39, 64 in 1 / 2 73 / 52."""
+    splits = most = max(1, -(-max_seq_len // 128))
+    for rounds in (1, 2, 3):
+        splits = min(max(1, 3 * sms * rounds // pairs), most)
+        if max_seq_len <= 1024 * splits or (2 * sms <= pairs <= 3 * sms and max_seq_len <= 2048):
+            break
     return -(-max_seq_len // splits)
 
 
@@ -388,7 +400,7 @@ def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Ten
     L = _L()
     L.mlf_paged_decode_ws_elems.restype = C.c_longlong
     if split_tokens <= 0:
-        split_tokens = _decode_split(B * Hkv, max_seq_len)
+        split_tokens = _decode_split(B * Hkv, max_seq_len, L.mlf_sm_count())
     st = (max(split_tokens, 128) + 127) // 128 * 128
     splits = max(1, (max_seq_len + st - 1) // st)
     ws = scratch("paged_decode", L.mlf_paged_decode_ws_elems(B, Hq, splits) * 4, q.device) if splits > 1 else None
@@ -423,7 +435,7 @@ def paged_decode_rope(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: to
     L = _L()
     L.mlf_paged_decode_ws_elems.restype = C.c_longlong
     if split_tokens <= 0:
-        split_tokens = _decode_split(B * Hkv, max_seq_len)
+        split_tokens = _decode_split(B * Hkv, max_seq_len, L.mlf_sm_count())
     st = (max(split_tokens, 128) + 127) // 128 * 128
     splits = max(1, (max_seq_len + st - 1) // st)
     ws = torch.empty(int(L.mlf_paged_decode_ws_elems(B, Hq, splits)), dtype=torch.float32, device=qkv.device) if splits > 1 else None
