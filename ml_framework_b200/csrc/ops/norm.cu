@@ -1,7 +1,8 @@
 // LayerNorm and RMSNorm, forward and backward, bf16 activations with fp32 statistics.
 //
 // One warp owns one row at a time and keeps it in registers as packed bf16 (NV 16-byte
-// vectors per lane), so x is read from HBM exactly once per pass; from D = 2048 on a CTA owns whole rows. The backward pass adds the
+// vectors per lane), so x is read from HBM exactly once per pass; from D = 2048 on a CTA owns whole rows, unless rows are
+// many and D is no 2048 or 4096. The backward pass adds the
 // per-row contributions to gamma/beta gradients into a per-CTA shared-memory accumulator with
 // shared atomics and writes one partial per CTA; a second tiny kernel sums the partials. The wide
 // model dimensions (2048 and 4096) use a backward kernel with whole-CTA rows instead.
@@ -209,9 +210,11 @@ norm_fwd_cta_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ ga
   }
 }
 
-// Forward for the wide D that are no multiple of 2048 (3072, 5120, 6144) and for 8192: one thread per 16-byte vector of a
-// row, D / 8 threads per CTA, R rows loaded together. One warp per row keeps D / 256 vectors per lane and walks them
-// three times, which no other warp of the SM covers when there are few rows: 24 x 5120 took 12.5 us that way, 2.9 us here.
+// Forward of not too many rows for the wide D that are no multiple of 2048 (3072, 5120, 6144) and for 8192: one thread per
+// 16-byte vector of a row, D / 8 threads per CTA, R rows loaded together. One warp per row keeps D / 256 vectors per lane
+// and walks them three times, which no other warp of the SM covers when there are few rows: 24 x 5120 took 8.5 us (RMS)
+// that way, 2.2 us here. With many rows the other warps do, and the two CTAs per SM that fit here meet twice per row:
+// 8192 x 5120 37 us that way, 55 us here; norm_row_line() says up to where this kernel is used.
 template <int R>
 __global__ void __launch_bounds__(1024)
 norm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
@@ -532,6 +535,16 @@ norm_bwd_finalize_kernel(const float* __restrict__ partials, int nparts, int D, 
   }
 }
 
+// Rows from which one warp per row is as fast as one thread per vector, in us there / here. RMS norm: 1536 x 3072 6.0 / 6.5,
+// 2304 x 5120 14.3 / 14.6, 2560 x 5120 16.5 / 16.2, 2816 x 6144 21.0 / 20.1, 3072 x 6144 21.9 / 22.3, 3072 x 8192 30.8 / 28.1,
+// 4096 x 8192 37.3 / 37.1, 4608 x 8192 39.9 / 42.1. Layer norm (another meeting here, another walk there): 2560 x 3072
+// 13.6 / 11.1, 4096 x 3072 14.9 / 14.9, 4096 x 5120 31.4 / 31.2, 4608 x 5120 33.3 / 36.3, 4608 x 6144 42.8 / 41.4,
+// 5120 x 6144 45.2 / 45.5, 6144 x 8192 65.8 / 64.8, 7168 x 8192 72.5 / 76.0.
+static int norm_row_line(int D, int rms) {
+  if (rms) return D / 2;
+  return max(4096, D / 16 * 13);
+}
+
 template <int NV>
 static int launch_fwd(const void* x, const void* g, const void* b, void* y, float* mean, float* rstd, int rows,
                       float eps, int rms, uint4* zero, long long n_zero, int zero_ctas, cudaStream_t st) {
@@ -601,7 +614,7 @@ MLF_API int mlf_norm_fwd_zero(const void* x, const void* gamma, const void* beta
     count_launch();
     return 0;
   }
-  if (D == 3072 || D == 5120 || D == 6144 || D == 8192) {
+  if ((D == 3072 || D == 5120 || D == 6144 || D == 8192) && rows < norm_row_line(D, rms)) {
     // two rows per CTA once every SM has two CTAs with work
     const int cap = 2 * sm_count();
     const int r = rows >= 2 * cap ? 2 : 1;
@@ -616,6 +629,7 @@ MLF_API int mlf_norm_fwd_zero(const void* x, const void* gamma, const void* beta
 #define CALL(NV) launch_fwd<NV>(x, gamma, beta, y, mean, rstd, rows, eps, rms, zp, nz, zc, st)
   switch (D / 256) {
     case 1: return CALL(1); case 2: return CALL(2); case 3: return CALL(3); case 4: return CALL(4); case 6: return CALL(6);
+    case 12: return CALL(12); case 20: return CALL(20); case 24: return CALL(24); case 32: return CALL(32);
     default: break;
   }
 #undef CALL

@@ -1,5 +1,6 @@
-"""Normalisation forward at the widths that take one thread per vector of a row: row counts around the change of the
-rows per CTA (twice two CTAs per SM) and around the end of the grid."""
+"""Normalisation forward at the widths that take one thread per vector of a row, or one warp per row when rows are many:
+row counts around the change of the rows per CTA (twice two CTAs per SM), around the end of the grid and on both sides of
+the change of the kernel."""
 import pytest
 import torch
 
@@ -14,6 +15,17 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("rows", [1, 24, 297, 591, 593, 1185])
 @pytest.mark.parametrize("rms", [False, True])
 def test_norm_fwd_one_vector_per_thread(rows, D, rms):
+    _check(rows, D, rms)
+
+
+@pytest.mark.parametrize("D,rms,line", [(3072, True, 1536), (5120, True, 2560), (6144, True, 3072), (8192, True, 4096),
+                                        (3072, False, 4096), (5120, False, 4160), (6144, False, 4992), (8192, False, 6656)])
+@pytest.mark.parametrize("past", [-1, 0, 4800])
+def test_norm_fwd_one_warp_per_row(D, rms, line, past):
+    _check(line + past, D, rms)
+
+
+def _check(rows, D, rms):
     torch.manual_seed(rows)
     x = (torch.randn(rows, D, device="cuda") * 1.5 + 0.3).to(torch.bfloat16)
     g = (1 + 0.1 * torch.randn(D, device="cuda")).to(torch.bfloat16)
