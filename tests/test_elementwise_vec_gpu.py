@@ -8,7 +8,7 @@ from ml_framework_b200.ops import native
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 4099, 1 << 20])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 4099, 1 << 20, 303104 * 4 + 5])
 @pytest.mark.parametrize("shift", [0, 1, 4])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_cast(n, shift, accumulate):
