@@ -208,7 +208,13 @@ clip_scale_kernel(G* grad, long long n, const float* sumsq, float max_norm, floa
 // loss_rows[t] = logsumexp - logit[target]; logits <- (softmax - onehot) * gscale (pad cols 0).
 // target < 0 (ignore) gives loss 0 and a zero gradient row.
 // ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(512)
+// LD loads in flight per thread in the first pass: the running maximum chains the iterations, and one load at a time leaves
+// the few CTAs that fit beside their cached rows waiting on memory (8192 x 32000 305 -> 269 us, 8192 x 50304 526 -> 456 us
+// with four). Below two vectors per thread there is nothing to overlap, and the registers cost a resident CTA: 8192 x 1000
+// 62 us with one, 66 us with four; 8192 x 8192 114 and 115 us, 512 x 8192 14.1 and 12.6 us.
+constexpr int CE_THREADS = 512;
+template <int LD>
+__global__ void __launch_bounds__(CE_THREADS)
 cross_entropy_kernel(__nv_bfloat16* logits, const long long* targets, float* loss_rows, float* loss_sum, int T, int V,
                      long long ld, float gscale, const float* gscale_ptr, float loss_weight, int cache_row, int* err) {
   extern __shared__ uint4 row_cache[];  // ld bf16 values when cache_row != 0
@@ -220,9 +226,6 @@ cross_entropy_kernel(__nv_bfloat16* logits, const long long* targets, float* los
   const float gs = gscale * (gscale_ptr ? *gscale_ptr : 1.f);
   // pass 1: online max / sum-exp
   float mx = -FLT_MAX, se = 0.f;
-  // four loads in flight per thread: the running maximum chains the iterations, and one load at a time left the few CTAs
-  // that fit beside their cached rows waiting on memory (8192 x 32000: 430 -> 397 us, 8192 x 50304: 652 -> 565 us)
-  constexpr int LD = 4;
   for (int i0 = threadIdx.x; i0 < nvec; i0 += LD * blockDim.x) {
     uint4 uu[LD];
 #pragma unroll
@@ -230,19 +233,19 @@ cross_entropy_kernel(__nv_bfloat16* logits, const long long* targets, float* los
       if (i0 + k * (int)blockDim.x < nvec) uu[k] = reinterpret_cast<const uint4*>(row)[i0 + k * blockDim.x];
 #pragma unroll
     for (int k = 0; k < LD; ++k) {
-    const int i = i0 + k * blockDim.x;
-    if (i >= nvec) break;
-    const uint4 u = uu[k];
-    if (cache_row) row_cache[i] = u;
-    float f[8];
-    float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
-    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-    float lm = f[0];
+      const int i = i0 + k * blockDim.x;
+      if (i >= nvec) break;
+      const uint4 u = uu[k];
+      if (cache_row) row_cache[i] = u;
+      float f[8];
+      float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
+      f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+      float lm = f[0];
 #pragma unroll
-    for (int j = 1; j < 8; ++j) lm = fmaxf(lm, f[j]);
-    if (lm > mx) { se *= __expf(mx - lm); mx = lm; }
+      for (int j = 1; j < 8; ++j) lm = fmaxf(lm, f[j]);
+      if (lm > mx) { se *= __expf(mx - lm); mx = lm; }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) se += __expf(f[j] - mx);
+      for (int j = 0; j < 8; ++j) se += __expf(f[j] - mx);
     }
   }
   for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) {
@@ -387,12 +390,14 @@ MLF_API int mlf_cross_entropy(void* logits, const long long* targets, float* los
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev & 63]) {
-    MLF_CHECK_CUDA(cudaFuncSetAttribute(cross_entropy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    MLF_CHECK_CUDA(cudaFuncSetAttribute(cross_entropy_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    MLF_CHECK_CUDA(cudaFuncSetAttribute(cross_entropy_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr_set[dev & 63] = true;
   }
-  cross_entropy_kernel<<<T, 512, cache ? smem : 0, st>>>((__nv_bfloat16*)logits, targets, loss_rows, loss_sum, T, V, ld, gscale,
-                                                         gscale_ptr, loss_weight, cache, device_status_word());
-                                                         count_launch();
+  const auto kernel = V / 8 < 2 * CE_THREADS ? cross_entropy_kernel<1> : cross_entropy_kernel<4>;
+  kernel<<<T, CE_THREADS, cache ? smem : 0, st>>>((__nv_bfloat16*)logits, targets, loss_rows, loss_sum, T, V, ld, gscale, gscale_ptr,
+                                                  loss_weight, cache, device_status_word());
+  count_launch();
   MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

@@ -60,3 +60,24 @@ def test_rope_qkv(T, Hq, Hkv, inverse):
     native.rope_qkv(src, pos, Hq, Hkv, 500000.0, inverse, out=src)
     assert torch.equal(src, got) and torch.equal(wide[:, :8], before[:, :8]) and torch.equal(wide[:, 8 + W:], before[:, 8 + W:])
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("V", [7, 4095, 8184, 8191, 8192, 8199, 16400])
+def test_cross_entropy_around_two_vectors_per_thread(V):
+    torch.manual_seed(V)
+    ld = (V + 7) // 8 * 8
+    logits = (torch.randn(9, ld, device="cuda") * 3).to(torch.bfloat16)
+    logits[2, : V // 2] = -torch.inf
+    tg = torch.randint(V // 2, V, (9,), device="cuda")
+    tg[4] = -100
+    z = logits[:, :V].double()
+    lse = z.logsumexp(-1)
+    keep = tg >= 0
+    want = torch.where(keep, lse - z.gather(1, tg.clamp(min=0)[:, None])[:, 0], 0.0)
+    grad = (z.softmax(-1) - torch.nn.functional.one_hot(tg.clamp(min=0), V)) * keep[:, None] * 0.25
+    loss, _ = native.cross_entropy_(logits, tg, V, grad_scale=0.25)
+    # fp32 sums of V terms with exponentials of 2^-21 each; one rounding of the gradient to bf16
+    assert ((loss.double() - want).abs() <= 1e-5 * (1 + want.abs())).all()
+    assert ((logits[:, :V].double() - grad).abs() <= 2 ** -8 * grad.abs() + 1e-6).all()
+    assert not logits[:, V:].any()
+    assert _lib.read_status() == 0
