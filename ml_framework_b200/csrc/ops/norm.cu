@@ -40,11 +40,12 @@ __device__ __forceinline__ void zero_role(uint4* z, long long n, int norm_ctas) 
   for (long long i = (long long)(blockIdx.x - norm_ctas) * blockDim.x + threadIdx.x; i < n; i += stride) z[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// D = NV * 256. rms != 0 selects RMSNorm (no mean subtraction, no beta).
+// D = NV * 256. rms != 0 selects RMSNorm (no mean subtraction, no beta). gamma and beta are loaded GV vectors at a time
+// ahead of the stores that use them: behind a store, which may alias as far as the compiler knows, every vector waited for its own load
+// (8192 rows of 8192: 67 us, 55 us with GV = 4; with GV = NV the registers cost warps: 8192 x 1024 7.8 us, 6.8 us with 2).
 template <int NV>
-__global__ void __launch_bounds__(256)
-norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
-                const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* y,
+__global__ void __launch_bounds__(256, NV <= 3 ? 4 : NV <= 6 ? 3 : NV <= 12 ? 2 : 1)   // NV = 12 unasked: 130 registers, half the warps
+norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma, const __nv_bfloat16* beta, __nv_bfloat16* y,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, int rms, int norm_ctas,
                 uint4* zero, long long n_zero) {
   constexpr int D = NV * 256;
@@ -58,9 +59,21 @@ norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
   const int warps_per_cta = blockDim.x >> 5;
   for (int row = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); row < rows; row += norm_ctas * warps_per_cta) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * D);
-    uint4 xv[NV];
+    const uint4* gr = reinterpret_cast<const uint4*>(gamma);
+    const uint4* br = reinterpret_cast<const uint4*>(beta);
+    constexpr int GV = NV <= 3 ? NV : NV <= 12 ? 2 : 4;
+    uint4 xv[NV], gv[GV], bv[GV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) xv[i] = xr[i * 32 + lane];
+    auto load_affine = [&](int i0) {
+#pragma unroll
+      for (int i = 0; i < GV; ++i) gv[i] = gr[(i0 + i) * 32 + lane];
+      if (beta) {
+#pragma unroll
+        for (int i = 0; i < GV; ++i) bv[i] = br[(i0 + i) * 32 + lane];
+      }
+    };
+    load_affine(0);
     float s = 0.f;
     if (!rms) {
 #pragma unroll
@@ -90,17 +103,19 @@ norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
       if (rstd_out) rstd_out[row] = rstd;
     }
     uint4* yr = reinterpret_cast<uint4*>(y + (long long)row * D);
-    const uint4* gr = reinterpret_cast<const uint4*>(gamma);
-    const uint4* br = reinterpret_cast<const uint4*>(beta);
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      float f[8], g[8], b[8];
-      unpack8(xv[i], f);
-      unpack8(gr[i * 32 + lane], g);
-      if (beta) unpack8(br[i * 32 + lane], b);
+    for (int i0 = 0; i0 < NV; i0 += GV) {
+      if (i0 > 0) load_affine(i0);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = (f[j] - mean) * rstd * g[j] + (beta ? b[j] : 0.f);
-      yr[i * 32 + lane] = pack8(f);
+      for (int i = 0; i < GV; ++i) {
+        float f[8], g[8], b[8];
+        unpack8(xv[i0 + i], f);
+        unpack8(gv[i], g);
+        if (beta) unpack8(bv[i], b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = (f[j] - mean) * rstd * g[j] + (beta ? b[j] : 0.f);
+        yr[(i0 + i) * 32 + lane] = pack8(f);
+      }
     }
   }
 }
@@ -110,8 +125,8 @@ norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
 // Few rows (a decode step: 64 x 4096) then still occupy one CTA per row group instead of one warp per row.
 template <int NVT, int R>
 __global__ void __launch_bounds__(256, 3)
-norm_fwd_cta_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
-                    const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* y,
+norm_fwd_cta_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma,
+                    const __nv_bfloat16* beta, __nv_bfloat16* y,
                     float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, int rms, int norm_ctas,
                     uint4* zero, long long n_zero) {
   constexpr int D = NVT * 2048;
@@ -214,10 +229,10 @@ norm_fwd_cta_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ ga
 // 16-byte vector of a row, D / 8 threads per CTA, R rows loaded together. One warp per row keeps D / 256 vectors per lane
 // and walks them three times, which no other warp of the SM covers when there are few rows: 24 x 5120 took 8.5 us (RMS)
 // that way, 2.2 us here. With many rows the other warps do, and the two CTAs per SM that fit here meet twice per row:
-// 8192 x 5120 37 us that way, 55 us here; norm_row_line() says up to where this kernel is used.
+// 8192 x 5120 34 us that way, 55 us here; norm_row_line() says up to where this kernel is used.
 template <int R>
 __global__ void __launch_bounds__(1024)
-norm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
+norm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma, const __nv_bfloat16* beta,
                     __nv_bfloat16* y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int D, float eps, int rms,
                     int norm_ctas, uint4* zero, long long n_zero) {
   pdl_trigger();
@@ -535,15 +550,11 @@ norm_bwd_finalize_kernel(const float* __restrict__ partials, int nparts, int D, 
   }
 }
 
-// Rows from which one warp per row is as fast as one thread per vector, in us there / here. RMS norm: 1536 x 3072 6.0 / 6.5,
-// 2304 x 5120 14.3 / 14.6, 2560 x 5120 16.5 / 16.2, 2816 x 6144 21.0 / 20.1, 3072 x 6144 21.9 / 22.3, 3072 x 8192 30.8 / 28.1,
-// 4096 x 8192 37.3 / 37.1, 4608 x 8192 39.9 / 42.1. Layer norm (another meeting here, another walk there): 2560 x 3072
-// 13.6 / 11.1, 4096 x 3072 14.9 / 14.9, 4096 x 5120 31.4 / 31.2, 4608 x 5120 33.3 / 36.3, 4608 x 6144 42.8 / 41.4,
-// 5120 x 6144 45.2 / 45.5, 6144 x 8192 65.8 / 64.8, 7168 x 8192 72.5 / 76.0.
-static int norm_row_line(int D, int rms) {
-  if (rms) return D / 2;
-  return max(4096, D / 16 * 13);
-}
+// Rows from which one warp per row is as fast as one thread per vector, in us there / here (RMS norm; layer norm, which meets
+// once more here and walks once more there, crosses at the same rows): 1024 x 3072 4.8 / 4.6, 1536 x 3072 5.6 / 6.4,
+// 600 x 5120 6.2 / 5.6, 1024 x 5120 6.2 / 8.4, 600 x 6144 7.3 / 6.6, 1024 x 6144 7.3 / 9.0, 1536 x 8192 16.1 / 14.3,
+// 2048 x 8192 17.8 / 17.2, 2304 x 8192 19.1 / 19.5, 8192 x 8192 55 / 71.
+static int norm_row_line(int D) { return D == 8192 ? 2304 : D == 3072 ? 1184 : 800; }
 
 template <int NV>
 static int launch_fwd(const void* x, const void* g, const void* b, void* y, float* mean, float* rstd, int rows,
@@ -614,7 +625,7 @@ MLF_API int mlf_norm_fwd_zero(const void* x, const void* gamma, const void* beta
     count_launch();
     return 0;
   }
-  if ((D == 3072 || D == 5120 || D == 6144 || D == 8192) && rows < norm_row_line(D, rms)) {
+  if ((D == 3072 || D == 5120 || D == 6144 || D == 8192) && rows < norm_row_line(D)) {
     // two rows per CTA once every SM has two CTAs with work
     const int cap = 2 * sm_count();
     const int r = rows >= 2 * cap ? 2 : 1;

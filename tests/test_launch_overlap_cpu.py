@@ -1,0 +1,42 @@
+"""Kernels that may start before the ones ahead of them have ended: nothing that those may write is read through the
+non-coherent path, which const __restrict__ parameters and __ldg ask for."""
+import re
+from pathlib import Path
+
+import ml_framework_b200
+
+CSRC = Path(ml_framework_b200.__file__).parent / "csrc"
+
+
+def _kernels():
+    """(name, parameters, body) of every __global__ function."""
+    for path in sorted(CSRC.rglob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"__global__", text):
+            depth, i = 0, text.index("{", m.end())
+            head, j = text[m.end():i], i
+            while True:
+                depth += {"{": 1, "}": -1}.get(text[j], 0)
+                if depth == 0:
+                    break
+                j += 1
+            name, params = re.search(r"(\w+)\s*\(((?:[^()]|\([^()]*\))*)\)\s*$", head).groups()
+            yield name, params, text[i:j]
+
+
+def test_no_non_coherent_reads_under_overlap():
+    seen = 0
+    for name, params, body in _kernels():
+        if "pdl_wait()" not in body:
+            continue
+        seen += 1
+        assert not re.search(r"const[^,]*__restrict__", params), name
+        assert "__ldg" not in body, name
+    assert seen >= 12
+
+
+def test_every_overlapped_launch_waits():
+    text = "\n".join(re.sub(r"//[^\n]*", "", p.read_text()) for p in CSRC.rglob("*.cu"))
+    launched = set(re.findall(r"launch_pdl\(\s*(\w+)", text)) - {"kernel"}
+    waits = {name for name, _, body in _kernels() if "pdl_wait()" in body}
+    assert launched and launched <= waits

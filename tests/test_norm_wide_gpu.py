@@ -18,10 +18,10 @@ def test_norm_fwd_one_vector_per_thread(rows, D, rms):
     _check(rows, D, rms)
 
 
-@pytest.mark.parametrize("D,rms,line", [(3072, True, 1536), (5120, True, 2560), (6144, True, 3072), (8192, True, 4096),
-                                        (3072, False, 4096), (5120, False, 4160), (6144, False, 4992), (8192, False, 6656)])
-@pytest.mark.parametrize("past", [-1, 0, 4800])
-def test_norm_fwd_one_warp_per_row(D, rms, line, past):
+@pytest.mark.parametrize("D,line", [(3072, 1184), (5120, 800), (6144, 800), (8192, 2304)])
+@pytest.mark.parametrize("past", [-1, 0, 9500])
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_fwd_one_warp_per_row(D, line, past, rms):
     _check(line + past, D, rms)
 
 
