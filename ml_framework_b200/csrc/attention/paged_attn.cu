@@ -21,6 +21,7 @@
 
 #include "../common/host.h"
 #include "../common/ptx.cuh"
+#include "../common/rope.cuh"
 #include "../mlf_api.h"
 
 namespace mlf {
@@ -54,13 +55,6 @@ struct PagedDecodeParams {
   float theta;
   int early;
 };
-
-// Rotary embedding of a pair (d, d + 64); cs = (cosine, sine) of its angle.
-__device__ __forceinline__ void rope_pair(float& a, float& b, float2 cs) {
-  const float x = a, y = b;
-  a = x * cs.x - y * cs.y;
-  b = y * cs.x + x * cs.y;
-}
 
 // 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros (rows past the sequence end)
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int src_bytes) {
@@ -209,12 +203,7 @@ paged_decode_kernel(const PagedDecodeParams p) {
   // elements they took longer than the first chunk's loads
   __shared__ float2 s_cs[ROPE ? PD / 2 : 1];
   if (ROPE) {
-    if (tid < PD / 2) {
-      const float inv_freq = __expf(-__logf(p.theta) * (2.f * tid / PD));
-      float sn, cs;
-      sincosf((float)(len - 1) * inv_freq, &sn, &cs);
-      s_cs[tid] = make_float2(cs, sn);
-    }
+    if (tid < PD / 2) s_cs[tid] = rope_cos_sin((float)(len - 1), __logf(p.theta), tid, PD);
     __syncthreads();
   }
   if (early) pdl_wait();
@@ -233,8 +222,8 @@ paged_decode_kernel(const PagedDecodeParams p) {
     for (int j = 0; j < 4; ++j) {
       const float2 a = unpack_bf16x2(dl < 8 ? ow[j] : tw[j]), c = unpack_bf16x2(dl < 8 ? tw[j] : ow[j]);
       float2 lo = a, hi = c;
-      rope_pair(lo.x, hi.x, s_cs[(dl & 7) * 8 + 2 * j]);
-      rope_pair(lo.y, hi.y, s_cs[(dl & 7) * 8 + 2 * j + 1]);
+      rope_rotate(lo.x, hi.x, s_cs[(dl & 7) * 8 + 2 * j]);
+      rope_rotate(lo.y, hi.y, s_cs[(dl & 7) * 8 + 2 * j + 1]);
       rw[j] = dl < 8 ? pack_bf16x2(lo.x, lo.y) : pack_bf16x2(hi.x, hi.y);
     }
     nk = make_uint4(rw[0], rw[1], rw[2], rw[3]);
@@ -269,8 +258,8 @@ paged_decode_kernel(const PagedDecodeParams p) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         float2 lo = unpack_bf16x2(qa[ks][h]), hi = unpack_bf16x2(qa[ks + PD / 32][h]);
-        rope_pair(lo.x, hi.x, s_cs[ks * 16 + h * 8 + qcol]);
-        rope_pair(lo.y, hi.y, s_cs[ks * 16 + h * 8 + qcol + 1]);
+        rope_rotate(lo.x, hi.x, s_cs[ks * 16 + h * 8 + qcol]);
+        rope_rotate(lo.y, hi.y, s_cs[ks * 16 + h * 8 + qcol + 1]);
         qa[ks][h] = pack_bf16x2(lo.x, lo.y);
         qa[ks + PD / 32][h] = pack_bf16x2(hi.x, hi.y);
       }
@@ -450,14 +439,7 @@ rope_kv_write_kernel(__nv_bfloat16* qkv, long long ld, const long long* pos, con
       const float2 a0 = unpack_bf16x2(lo.x), a1 = unpack_bf16x2(lo.y), b0 = unpack_bf16x2(hi.x), b1 = unpack_bf16x2(hi.y);
       float a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float inv_freq = __expf(-log_theta * (2.f * (d + j) / PD));
-        float sn, cs;
-        sincosf(p * inv_freq, &sn, &cs);
-        const float x = a[j], y = b[j];
-        a[j] = x * cs - y * sn;
-        b[j] = y * cs + x * sn;
-      }
+      for (int j = 0; j < 4; ++j) rope_rotate(a[j], b[j], rope_cos_sin(p, log_theta, d + j, PD));
       lo.x = pack_bf16x2(a[0], a[1]); lo.y = pack_bf16x2(a[2], a[3]);
       hi.x = pack_bf16x2(b[0], b[1]); hi.y = pack_bf16x2(b[2], b[3]);
       *reinterpret_cast<uint2*>(row + d) = lo;

@@ -10,6 +10,7 @@
 
 #include "../common/host.h"
 #include "../common/ptx.cuh"
+#include "../common/rope.cuh"
 #include "../mlf_api.h"
 
 namespace mlf {
@@ -391,18 +392,17 @@ __global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* x, const long 
     const long long th = i / half;
     const int h = (int)(th % H);
     const long long t = th / H;
-    const float inv_freq = __expf(-log_theta * (2.f * d / Dh));
-    float s, c;
-    sincosf((float)pos[t] * inv_freq, &s, &c);
-    if (inverse) s = -s;
+    float2 cs = rope_cos_sin((float)pos[t], log_theta, d, Dh);
+    if (inverse) cs.y = -cs.y;
     __nv_bfloat16* p = x + t * row_stride + (long long)h * Dh;
-    const float a = __bfloat162float(p[d]), b = __bfloat162float(p[d + half]);
-    p[d] = __float2bfloat16(a * c - b * s);
-    p[d + half] = __float2bfloat16(b * c + a * s);
+    float a = __bfloat162float(p[d]), b = __bfloat162float(p[d + half]);
+    rope_rotate(a, b, cs);
+    p[d] = __float2bfloat16(a);
+    p[d + half] = __float2bfloat16(b);
   }
 }
 
-// Packed QKV rows [T, (Hq + 2 Hkv) * 128]: dst = src with the query and key heads rotated (the arithmetic of rope_kernel) and
+// Packed QKV rows [T, (Hq + 2 Hkv) * 128]: dst = src with the query and key heads rotated (as rope_kernel does) and
 // the value heads copied; dst == src rotates in place. One warp per token: a lane keeps the sines and cosines of its eight
 // pairs (d .. d + 7, d + 64 ..) for all heads, and every access is 16 bytes. Bound by HBM; 8192 tokens, 32 + 2 x 8 heads:
 // a copy and two rotary launches 34 + 140 us, one sine per element and head -> 37 us.
@@ -413,12 +413,12 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* dst, const
   const float log_theta = __logf(theta);
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < T; t += warps) {
-    float cs[8], sn[8];
+    float2 cs[8];
     const float p = (float)pos[t];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      sincosf(p * __expf(-log_theta * (2.f * (d + j) / RQ_D)), &sn[j], &cs[j]);
-      if (inverse) sn[j] = -sn[j];
+      cs[j] = rope_cos_sin(p, log_theta, d + j, RQ_D);
+      if (inverse) cs[j].y = -cs[j].y;
     }
     for (int h = h0; h < heads; h += 4) {
       const uint4* s = reinterpret_cast<const uint4*>(src + t * ld_src + (long long)h * RQ_D + d);
@@ -427,17 +427,13 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* dst, const
         if (dst != src) { o[0] = s[0]; o[8] = s[8]; }
         continue;
       }
-      float a[8], b[8], x[8], y[8];
+      float a[8], b[8];
       Vec<__nv_bfloat16>::load(reinterpret_cast<const __nv_bfloat16*>(s), a);
       Vec<__nv_bfloat16>::load(reinterpret_cast<const __nv_bfloat16*>(s + 8), b);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        // the roundings of rope_kernel as it is compiled, spelled out: the same bits
-        x[j] = __fmaf_rn(a[j], cs[j], -__fmul_rn(b[j], sn[j]));
-        y[j] = __fmaf_rn(a[j], sn[j], __fmul_rn(b[j], cs[j]));
-      }
-      Vec<__nv_bfloat16>::store(reinterpret_cast<__nv_bfloat16*>(o), x);
-      Vec<__nv_bfloat16>::store(reinterpret_cast<__nv_bfloat16*>(o + 8), y);
+      for (int j = 0; j < 8; ++j) rope_rotate(a[j], b[j], cs[j]);
+      Vec<__nv_bfloat16>::store(reinterpret_cast<__nv_bfloat16*>(o), a);
+      Vec<__nv_bfloat16>::store(reinterpret_cast<__nv_bfloat16*>(o + 8), b);
     }
   }
 }
