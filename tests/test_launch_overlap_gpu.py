@@ -12,30 +12,39 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("M", [1, 32, 33, 64, 128, 129, 256])
 @pytest.mark.parametrize("N,K", [(1024, 512), (1096, 2048), (4096, 5120)])
-def test_chain_with_static_weights(M, N, K):
+@pytest.mark.parametrize("shared", [False, True])
+def test_chain_with_static_weights(M, N, K, shared):
+    """norm -> product -> product -> norm ... with no ordinary launch in between. Every round has rows of its own, so that a
+    read ahead of its time sees another round's values; with ``shared`` the rounds clear and fill one and the same buffer,
+    so that a clear ahead of its time takes the round before's values from its second product."""
     torch.manual_seed(M + N)
-    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    rounds = 6
+    xs = [torch.randn(M, K, device="cuda").to(torch.bfloat16) for r in range(rounds)]
     g = torch.rand(K, device="cuda").to(torch.bfloat16)
     w1 = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
     w2 = (torch.randn(K, N, device="cuda") * N ** -0.5).to(torch.bfloat16)
     flags = _lib.EPI_ACCUM | _lib.EPI_B_STATIC
-    mid = torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16)
-    res = x.clone()
-    for _ in range(3):                       # each round overlaps the end of the one before it
+    mids = [torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(1 if shared else rounds)] * (rounds if shared else 1)
+    ress = [x.clone() for x in xs]
+    torch.cuda.synchronize()
+    torch.cuda._sleep(2_000_000)             # the host gets ahead: the launches stand back to back
+    for x, mid, res in zip(xs, mids, ress):
         h, _, _ = native.norm_fwd(x, g, None, 1e-5, True, want_stats=False, zero=mid)
         gemm(h, w1, out=mid, flags=flags)
-        res.copy_(x)
         gemm(mid, w2, out=res, flags=flags)
     torch.cuda.synchronize()
-    xf = x.float()
-    hf = (xf * torch.rsqrt((xf * xf).mean(-1, keepdim=True) + 1e-5) * g.float()).to(torch.bfloat16).float()
-    mf = hf @ w1.float().t()
-    # every partial tile is added in bf16: at most one rounding (2^-9 of the running value) per SM that shares the tile,
-    # and a value at a rounding boundary of h may round the other way; 4 sigma of that in the root mean square
     rms = lambda t: t.pow(2).mean().sqrt().item()
-    assert rms(mid.float() - mf) <= 2 ** -7 * rms(mf)
-    rf = x.float() + mid.float() @ w2.float().t()
-    assert rms(res.float() - rf) <= 2 ** -7 * rms(rf)
+    for r, (x, mid, res) in enumerate(zip(xs, mids, ress)):
+        xf = x.float()
+        hf = (xf * torch.rsqrt((xf * xf).mean(-1, keepdim=True) + 1e-5) * g.float()).to(torch.bfloat16).float()
+        mf = hf @ w1.float().t()
+        # every partial tile is added in bf16: at most one rounding (2^-9 of the running value) per SM that shares the tile,
+        # and a value at a rounding boundary of h may round the other way; 4 sigma of that in the root mean square
+        if not shared or r == rounds - 1:
+            assert rms(mid.float() - mf) <= 2 ** -7 * rms(mf), r
+        # the same for the second product, whose rows (unit norm) carry the first one's error on
+        rf = xf + mf @ w2.float().t()
+        assert rms(res.float() - rf) <= 2 ** -7 * (rms(rf) + rms(mf)), r
     assert _lib.read_status() == 0
 
 

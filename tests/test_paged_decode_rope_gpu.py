@@ -5,6 +5,7 @@ import torch
 
 from ml_framework_b200 import _lib
 from ml_framework_b200.ops import native
+from ml_framework_b200.ops.gemm import gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -44,4 +45,47 @@ def test_same_as_separate_launches(Hq, Hkv, split, bs, static):
                                    inputs_static=static)
     assert torch.equal(got, want)
     assert torch.equal(a_cache, b_cache)
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("B,Hq,Hkv", [(1, 32, 8), (13, 16, 4), (40, 8, 8)])
+def test_behind_a_running_product(B, Hq, Hkv):
+    """norm -> QKV product -> decode with early reads, back to back and with rows of its own in every round: lengths, tables
+    and cached rows are read while the product runs, what the product writes is not. Each round is a token further."""
+    torch.manual_seed(B)
+    K, D, bs, rounds, pages = 4096, 128, 16, 5, 40
+    width = (Hq + 2 * Hkv) * D
+    cache = torch.randn(B * pages, 2, bs, Hkv, D, device="cuda").to(torch.bfloat16)
+    table = torch.randperm(B * pages, device="cuda").to(torch.int32).view(B, pages)
+    start = torch.randint(1, pages * bs - rounds, (B,), device="cuda")
+    lens = [(start + r).to(torch.int32) for r in range(rounds)]
+    slots = [table.gather(1, ((n.long() - 1) // bs)[:, None])[:, 0].long() * bs + (n.long() - 1) % bs for n in lens]
+    xs = [torch.randn(B, K, device="cuda").to(torch.bfloat16) for r in range(rounds)]
+    g = torch.rand(K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(width, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    qkv = torch.full((B, width), 7.0, device="cuda", dtype=torch.bfloat16)
+    rows = [torch.empty_like(qkv) for _ in range(rounds)]
+    a_cache, b_cache = cache.clone(), cache.clone()
+    flags = _lib.EPI_ACCUM | _lib.EPI_B_STATIC
+    got = []
+    torch.cuda.synchronize()
+    torch.cuda._sleep(2_000_000)
+    for r in range(rounds):
+        h, _, _ = native.norm_fwd(xs[r], g, None, 1e-5, True, want_stats=False, zero=qkv)
+        gemm(h, w, out=qkv, flags=flags)
+        got.append(native.paged_decode_rope(qkv, a_cache, table, lens[r], slots[r], Hq, Hkv, pages * bs, 500000.0, inputs_static=True))
+        rows[r].copy_(qkv)                   # an ordinary launch: the early reads of the next round start behind it
+    torch.cuda.synchronize()
+    for r in range(rounds):
+        rot = rows[r].clone()
+        native.rope_kv_write_(rot, lens[r].long() - 1, slots[r], b_cache, Hq, Hkv, 500000.0)
+        want = native.paged_decode(rot[:, :Hq * D].view(B, Hq, D), b_cache, table, lens[r], pages * bs, split_tokens=0)
+        assert torch.equal(got[r], want), r
+    assert torch.equal(a_cache, b_cache)
+    # and the rows themselves are this round's product, as close as one sum of bf16 partial tiles is
+    for r in range(rounds):
+        xf = xs[r].float()
+        hf = (xf * torch.rsqrt((xf * xf).mean(-1, keepdim=True) + 1e-5) * g.float()).to(torch.bfloat16).float()
+        wantq = hf @ w.float().t()
+        assert (rows[r].float() - wantq).pow(2).mean().sqrt() <= 2 ** -7 * wantq.pow(2).mean().sqrt()
     assert _lib.read_status() == 0
