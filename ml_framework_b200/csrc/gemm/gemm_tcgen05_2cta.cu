@@ -302,7 +302,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     const int q = warp & 3;
     const int ew = warp - 2;
     const int half = ew >> 2;                  // which half of the tile's columns (0 when there is one warp per quarter)
-    const bool two_bufs = epi_halves == 1;     // the staging tiles of the absent warps are the second ones
+    const bool two_bufs = epi_halves == 1;     // the staging tiles of the absent warps are the second ones; never with an aux tile
     const bool out_fp32 = (p.flags & MLF_EPI_OUT_FP32) != 0;
     const bool swiglu = (p.flags & MLF_EPI_SWIGLU) != 0;
     const bool dswiglu = (p.flags & MLF_EPI_DSWIGLU) != 0;
@@ -311,9 +311,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     const uint32_t stg0 = stg_base + (uint32_t)ew * T2_STG_BYTES;
     uint32_t emits = 0;                        // staging tiles handed out by this warp
     uint32_t aux_units = 0;                    // aux tiles consumed by this warp
-    // aux_in (residual, dGELU or dSwiGLU input) comes in through the staging tile, one unit ahead
+    // aux_in (residual, dGELU or dSwiGLU input) comes in through the warp's one staging tile: the next unit's is requested
+    // when the store of this unit has read the tile, the first one of a tile while its products are still running
     int ax_t = pair, ax_u = -1;                // unit whose aux tile was requested last
-    uint32_t ax_n = 0;                         // aux tiles requested
     auto request_aux = [&]() {                 // lane 0; the staging tile it goes to is free
       while (true) {
         ++ax_u;
@@ -325,8 +325,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         const int nb = col0 + half * my_cols + ax_u * unit_cols;
         if (nb >= p.N) continue;
         mbar_expect_tx(aux_bar(ew), T2_STG_BYTES);
-        tma_load_2d(stg0 + (two_bufs ? (ax_n & 1u) * 4u * T2_STG_BYTES : 0u), &tmAux, dswiglu ? 2 * nb : nb, tm * 256 + (int)rank * BM + q * 32, aux_bar(ew));
-        ++ax_n;
+        tma_load_2d(stg0, &tmAux, dswiglu ? 2 * nb : nb, tm * 256 + (int)rank * BM + q * 32, aux_bar(ew));
         return;
       }
     };
@@ -392,13 +391,12 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         // this warp's aux row of the current unit, 64 bf16 in the staging tile
         auto aux_row = [&](float (&a)[64]) -> bool {
           if (!mbar_wait_warp(aux_bar(ew), aux_units & 1u, abort_flag, p.err, ERR_WAIT_TMEM_FULL)) return false;
-          const uint32_t src = stg0 + (two_bufs ? (aux_units & 1u) * 4u * T2_STG_BYTES : 0u);
           ++aux_units;
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             uint4 w;
             asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
-                         : "r"(src + lane * 128 + (((uint32_t)c ^ (uint32_t)(lane & 7)) << 4)));
+                         : "r"(stg0 + lane * 128 + (((uint32_t)c ^ (uint32_t)(lane & 7)) << 4)));
             const float2 f0 = unpack_bf16x2(w.x), f1 = unpack_bf16x2(w.y), f2 = unpack_bf16x2(w.z), f3 = unpack_bf16x2(w.w);
             a[8 * c + 0] = f0.x; a[8 * c + 1] = f0.y; a[8 * c + 2] = f1.x; a[8 * c + 3] = f1.y;
             a[8 * c + 4] = f2.x; a[8 * c + 5] = f2.y; a[8 * c + 6] = f3.x; a[8 * c + 7] = f3.y;
@@ -483,8 +481,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             emit(v, &tmOut, nb, false);
           }
           if (tma_aux && lane == 0) {          // the next unit's aux tile, once the store that read its buffer is through
-            if (two_bufs) tma_store_wait_read<1>();
-            else tma_store_wait_read<0>();
+            tma_store_wait_read<0>();
             request_aux();
           }
         }
@@ -736,6 +733,7 @@ MLF_API int mlf_gemm_bf16_2cta(const MlfGemmArgs* a, int split_few_rows, uint64_
   // 8192 x 8192 x 2048 with dGELU 225 -> 211 us), a residual (its tile has to arrive first), and any short K (2331 x 4096
   // x 1024 with GELU 33.5 -> 28.1 us). Elsewhere the second warp only takes power from the products: 8192 x 8192 x 2048
   // plain 182 us with one, 186 us with two.
+  // Every product with an aux tile is one of these: its loads use the one staging tile that a warp has then.
   const bool heavy = (a->flags & (MLF_EPI_DGELU_MUL | MLF_EPI_SWIGLU | MLF_EPI_DSWIGLU | MLF_EPI_RESIDUAL)) != 0;
   const int epi_halves = heavy || a->K <= 1024 * k_splits ? 2 : 1;
   const int reduce_out = (k_splits > 1 || (a->flags & MLF_EPI_ACCUM)) ? 1 : 0;
