@@ -52,7 +52,8 @@ struct FlashBwdParams {
   int* err;
 };
 
-// delta[b, h, s] = sum_d dO[t, h, d] * O[t, h, d] (and lse2, the logsumexp in the log2 domain), rows of pitch Sp; one warp per (token, head), two such rows per warp in flight.
+// delta[b, h, s] = sum_d dO[t, h, d] * O[t, h, d] (and lse2, the logsumexp in the log2 domain), rows of pitch Sp; one warp
+// per (token, head), two such rows per warp in flight.
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout, float* delta, const float* lse, float* lse2, int B, int S, int Sp,
                   int H, long long ldo, long long lddo) {

@@ -73,7 +73,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t sK = sQ + 2 * W_TILE_BYTES;                  // W_STAGES tiles
   const uint32_t sV = sK + W_STAGES * W_TILE_BYTES;           // W_STAGES tiles
   const uint32_t bars = sV + W_STAGES * W_TILE_BYTES;
-  // barriers: q_full[2] k_full[2] v_full[2] k_empty[2] v_empty[2] s_full[2] p_full[2] pv_done[2]
+  // barriers: q_full[2] k_full[2] v_full[2] k_empty[2] v_empty[2] s_full[2] p_full[2] pv_done[2] p_half[2]
   auto q_full = [&](int t) { return bars + 8u * t; };
   auto k_full = [&](int s) { return bars + 8u * (2 + s); };
   auto v_full = [&](int s) { return bars + 8u * (4 + s); };

@@ -610,9 +610,9 @@ MLF_API int mlf_paged_decode_ld(const void* q, long long ldq, const void* cache,
 // Decode attention straight from the QKV product: qkv [B, (Hq + 2 Hkv) * 128] (pitch ld, 16-byte aligned rows), not yet
 // rotated. The new token of sequence b is the last of its seq_lens[b] tokens; its rotated key and its value are written
 // to cache slot slots[b] (< 0: not written) and attended to like the cached ones. Same results as mlf_rope_kv_write with
-// positions seq_lens - 1 followed by mlf_paged_decode_ld. inputs_static: no kernel queued on the stream since the last
-// launch without programmatic overlap writes block_table, seq_lens or the cached rows of earlier tokens; they may then be
-// read before the kernels ahead have finished.
+// positions seq_lens - 1 followed by mlf_paged_decode_ld. inputs_static: neither the last launch on the stream without
+// programmatic overlap nor any launch after it writes block_table, seq_lens or the cached rows of earlier tokens; they may
+// then be read before the kernels ahead have finished.
 MLF_API int mlf_paged_decode_rope(const void* qkv, long long ld, void* cache, const int* block_table, const int* seq_lens,
                                   const long long* slots, void* out, float* ws, int B, int Hq, int Hkv, int block_size, int max_blocks,
                                   int num_blocks, int max_seq_len, int split_tokens, float scale, float theta, int inputs_static,

@@ -21,8 +21,9 @@ enum {
   MLF_EPI_ACCUM = 32,      // out += previous contents of out
   MLF_EPI_OUT_FP32 = 64,   // out is fp32 instead of bf16
   MLF_EPI_SWIGLU = 128,    // columns come in (gate, up) pairs: out[m, n/2] = silu(gate) * up
-  MLF_EPI_B_STATIC = 512,  // b is a weight that no kernel queued on the stream since the last launch without
-                           // programmatic overlap writes: it may be read before the kernels ahead have finished
+  MLF_EPI_B_STATIC = 512,  // b may be read before the kernels ahead on the stream have finished: neither the last
+                           // launch without programmatic overlap nor any launch after it writes b (what that last
+                           // one writes need not be visible yet when the kernels behind it become resident)
   MLF_EPI_DSWIGLU = 256,   // aux_in holds (gate, up) pairs [M, 2N]; out[m, 2n..2n+1] = grads
 };
 

@@ -422,9 +422,9 @@ def paged_decode_rope(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: to
                       Hq: int, Hkv: int, max_seq_len: int, theta: float, *, scale: Optional[float] = None, split_tokens: int = 0, inputs_static: bool = False) -> torch.Tensor:
     """:func:`rope_kv_write_` at positions ``seq_lens - 1`` followed by :func:`paged_decode` in one launch: ``qkv``
     [B, (Hq + 2 Hkv) * 128] holds the unrotated projection of each sequence's newest token, which ``seq_lens`` counts;
-    its key and value go to cache slot ``slots`` (int64, < 0 skips the write). ``qkv`` is left as it is. ``inputs_static``: no kernel
-    queued since the last launch without programmatic overlap writes ``block_table``, ``seq_lens`` or the cached rows of
-    earlier tokens, which may then be read ahead of the kernels before this one."""
+    its key and value go to cache slot ``slots`` (int64, < 0 skips the write). ``qkv`` is left as it is. ``inputs_static``:
+    neither the last launch without programmatic overlap nor any launch after it writes ``block_table``, ``seq_lens`` or the
+    cached rows of earlier tokens, which may then be read ahead of the kernels before this one."""
     B = qkv.shape[0]
     nb, two, bs, Hc, D = kv_cache.shape
     assert D == 128 and two == 2 and Hc == Hkv and kv_cache.is_contiguous() and qkv.shape[1] == (Hq + 2 * Hkv) * D

@@ -103,7 +103,8 @@ class PagedLlamaExecutor:
 
     def _norm_product(self, x: torch.Tensor, gamma: torch.Tensor, w: torch.Tensor, few_rows: bool):
         """(rms_norm(x), rms_norm(x) @ w^T). The first kernel of a step is the embedding lookup, which starts after all
-        earlier work of the stream; nothing in the step writes a weight, so the products may read theirs early."""
+        earlier work of the stream has ended; neither it nor anything behind it writes a weight, so the products may read
+        theirs early."""
         if not few_rows:
             h, _, _ = native.norm_fwd(x, gamma, None, self.mc.norm_eps, True, want_stats=False)
             return h, gemm(h, w, flags=_lib.EPI_B_STATIC)
