@@ -313,10 +313,10 @@ class _AttentionFn(torch.autograd.Function):
         v = qkv2[:, (Hq + Hkv) * D:].view(T, Hkv, D)
         if rope_theta is not None:
             # rotate into a private copy; the GEMM output stays untouched for autograd
-            if positions.dtype == torch.int64 and qkv2.stride(1) == 1 and qkv2.stride(0) % 8 == 0 and qkv2.data_ptr() % 16 == 0:
-                qkv2 = native.rope_qkv(qkv2, positions.reshape(-1), Hq, Hkv, rope_theta)
-            else:
-                qkv2 = native.rope_qkv(qkv2.contiguous().clone(), positions.reshape(-1).long(), Hq, Hkv, rope_theta)
+            if qkv2.stride(1) != 1 or qkv2.stride(0) % 8 != 0 or qkv2.data_ptr() % 16 != 0:
+                qkv2 = qkv2.clone(memory_format=torch.contiguous_format)
+            positions = positions.reshape(-1)[:T].long()          # a longer buffer serves every batch
+            qkv2 = native.rope_qkv(qkv2, positions, Hq, Hkv, rope_theta)
             q = qkv2[:, :Hq * D].view(T, Hq, D)
             k = qkv2[:, Hq * D:(Hq + Hkv) * D].view(T, Hkv, D)
             v = qkv2[:, (Hq + Hkv) * D:].view(T, Hkv, D)
@@ -341,7 +341,7 @@ class _AttentionFn(torch.autograd.Function):
         do = dout.reshape(T, Hq, D)
         native.flash_bwd(q, k, v, out, do, lse, B, S, causal=causal, dq=dq, dk=dk, dv=dv)
         if rope_theta is not None:
-            native.rope_qkv(dqkv, positions.reshape(-1).long(), Hq, Hkv, rope_theta, inverse=True, out=dqkv)
+            native.rope_qkv(dqkv, positions, Hq, Hkv, rope_theta, inverse=True, out=dqkv)
         return dqkv.view(ctx.in_shape), None, None, None, None, None, None, None
 
 

@@ -78,3 +78,24 @@ def test_cross_entropy_around_two_vectors_per_thread(V):
     assert ((logits[:, :V].double() - grad).abs() <= 2 ** -8 * grad.abs() + 1e-6).all()
     assert not logits[:, V:].any()
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("extra", [0, 5])
+def test_packed_attention_takes_a_longer_position_buffer(dtype, extra):
+    from ml_framework_b200.ops import functional as Fm
+    torch.manual_seed(0)
+    B, S, Hq, Hkv = 2, 48, 4, 2
+    base = torch.randn(B * S, (Hq + 2 * Hkv) * 128, device="cuda").to(torch.bfloat16)
+    pos = torch.cat([torch.arange(S).repeat(B), torch.full((extra,), 7)]).to("cuda", dtype)
+    outs = []
+    for p in (None, pos):
+        qkv = base.clone().requires_grad_()
+        o = Fm.attention_packed(qkv, B, S, Hq, Hkv, 128, True, 10000.0, p)
+        o.backward(torch.ones_like(o))
+        outs.append((o.detach(), qkv.grad))
+    # forward bit for bit; dQ is summed over key tiles in any order before it is rounded to bf16
+    assert torch.equal(outs[0][0], outs[1][0])
+    assert ((outs[0][1].float() - outs[1][1].float()).abs() <= 2 ** -7 * outs[0][1].float().abs() + 2 ** -12).all()
+    with pytest.raises(AssertionError):
+        Fm.attention_packed(base, B, S, Hq, Hkv, 128, True, 10000.0, pos[:B * S - 1])
