@@ -105,7 +105,7 @@ class PagedLlamaExecutor:
         """(rms_norm(x), rms_norm(x) @ w^T). The first kernel of a step is the embedding lookup, which starts after all
         earlier work of the stream has ended; neither it nor anything behind it writes a weight, so the products may read
         theirs early."""
-        if not few_rows:
+        if not few_rows or w.shape[0] % 8:           # a head of any width: rows that TMA cannot add into
             h, _, _ = native.norm_fwd(x, gamma, None, self.mc.norm_eps, True, want_stats=False)
             return h, gemm(h, w, flags=_lib.EPI_B_STATIC)
         out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
