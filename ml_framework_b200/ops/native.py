@@ -366,7 +366,7 @@ def _decode_split(pairs: int, max_seq_len: int, sms: int) -> int:
     per split. us at the longest of 8 KV heads' sequences, lengths from half of it on: 13 x 2500 4 splits 26 (8: 29);
     48 x 1024 none 35 (3: 45); 8 x 4000 6 splits 28 (11: 34).
 
-    A split of more than 1024 tokens takes long enough for its CTA to be alone at the end, above all when one sequence is
+    A split of more than 1400 tokens takes long enough for its CTA to be alone at the end, above all when one sequence is
     much longer than the others: then what fits two rounds, or three, of resident CTAs (just above a whole number of rounds
     the last one is nearly empty: 16 x 4096 in 3 / 4 / 6 / 7 splits 47 / 58 / 49 / 53). Up to 2048 tokens, pairs that fill two
     thirds of the first round stay whole (40 x 2048 1 / 2 / 3 splits 53 / 57 / 56; 36 x 1500 1 / 3 39 / 38). Counts on both
@@ -376,7 +376,7 @@ def _decode_split(pairs: int, max_seq_len: int, sms: int) -> int:
     splits = most = max(1, -(-max_seq_len // 128))
     for rounds in (1, 2, 3):
         splits = min(max(1, 3 * sms * rounds // pairs), most)
-        if max_seq_len <= 1024 * splits or (2 * sms <= pairs <= 3 * sms and max_seq_len <= 2048):
+        if max_seq_len <= 1400 * splits or (2 * sms <= pairs <= 3 * sms and max_seq_len <= 2048):
             break
     return -(-max_seq_len // splits)
 
