@@ -203,7 +203,7 @@ paged_decode_kernel(const PagedDecodeParams p) {
   // elements they took longer than the first chunk's loads
   __shared__ float2 s_cs[ROPE ? PD / 2 : 1];
   if (ROPE) {
-    if (tid < PD / 2) s_cs[tid] = rope_cos_sin((float)(len - 1), __logf(p.theta), tid, PD);
+    if (tid < PD / 2) s_cs[tid] = rope_cos_sin((float)(len - 1), __logf(p.theta), rope_exponent<PD>(tid));
     __syncthreads();
   }
   if (early) pdl_wait();
@@ -439,7 +439,7 @@ rope_kv_write_kernel(__nv_bfloat16* qkv, long long ld, const long long* pos, con
       const float2 a0 = unpack_bf16x2(lo.x), a1 = unpack_bf16x2(lo.y), b0 = unpack_bf16x2(hi.x), b1 = unpack_bf16x2(hi.y);
       float a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) rope_rotate(a[j], b[j], rope_cos_sin(p, log_theta, d + j, PD));
+      for (int j = 0; j < 4; ++j) rope_rotate(a[j], b[j], rope_cos_sin(p, log_theta, rope_exponent<PD>(d + j)));
       lo.x = pack_bf16x2(a[0], a[1]); lo.y = pack_bf16x2(a[2], a[3]);
       hi.x = pack_bf16x2(b[0], b[1]); hi.y = pack_bf16x2(b[2], b[3]);
       *reinterpret_cast<uint2*>(row + d) = lo;

@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* x, const long 
     const long long th = i / half;
     const int h = (int)(th % H);
     const long long t = th / H;
-    float2 cs = rope_cos_sin((float)pos[t], log_theta, d, Dh);
+    float2 cs = rope_cos_sin((float)pos[t], log_theta, rope_exponent(d, Dh));
     if (inverse) cs.y = -cs.y;
     __nv_bfloat16* p = x + t * row_stride + (long long)h * Dh;
     float a = __bfloat162float(p[d]), b = __bfloat162float(p[d + half]);
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(256) rope_qkv_kernel(__nv_bfloat16* dst, const
     const float p = (float)pos[t];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      cs[j] = rope_cos_sin(p, log_theta, d + j, RQ_D);
+      cs[j] = rope_cos_sin(p, log_theta, rope_exponent<RQ_D>(d + j));
       if (inverse) cs[j].y = -cs[j].y;
     }
     for (int h = h0; h < heads; h += 4) {
