@@ -358,7 +358,10 @@ static int single_cta_bn(int M, int N, int sms) {
 // With 129 - 511 rows a pair tile may be half padding, and the SMs that each kernel occupies decide:
 //  - where all 128 x 64 tiles of single CTAs run at once, they do: 300 rows x 2048 x 2048 11.6 us against 13.5 on pairs,
 //    x 2048 x 8192 32.5 / 36.7, x 3072 x 3072 15.6 / 17.7, 200 x 4000 x 2048 13.1 / 15.4; one tile column further they
-//    need a second round: 400 x 2560 x 2560 22.0 / 15.7, 300 x 3584 x 4096 32.7 / 21.8.
+//    need a second round: 400 x 2560 x 2560 22.0 / 15.7, 300 x 3584 x 4096 32.7 / 21.8. Up to K = 4096 the two epilogues
+//    that move most per element stay on pairs, which stage their rows: GELU with its input stored (300 x 2328 x 1024
+//    14.6 / 11.5, x 3072 x 1024 12.0 / 11.3, x 2048 x 4096 22.3 / 23.3) and dSwiGLU (x 3072 x 1024 13.3 / 12.5, x 4096
+//    24.3 / 24.1, x 8192 38.8 / 40.8).
 //  - otherwise rounds of 256 columns are compared (a halved last round counts 0.8). Pairs do one faster: they win with up
 //    to one and a half times as many (300 x 28672 x 4096, 3.8 against 3: 85.9 / 93.1 us; x 50304 x 2048, 5.8 against 4:
 //    72.2 / 74.6) and lose above (x 12288 x 4096, 1.8 against 1: 43.1 / 39.3), GELU and stored pre-activations aside, whose
@@ -372,7 +375,9 @@ MLF_API int mlf_gemm_takes_pairs(int M, int N, int K, int flags, int has_comm, i
   if (N < 512 || tiles < 16 || M <= (has_comm || (flags & MLF_EPI_ACCUM) ? 511 : 128)) return 0;
   if (always) return 1;
   const long long tm = (M + BM - 1) / BM;
-  if (single_cta_bn(M, N, sms) == 64 && tm * ((N + 63) / 64) <= sms) return 0;
+  const int gelu_pre = MLF_EPI_GELU | MLF_EPI_STORE_PRE;
+  const bool wide_epilogue = K <= 4096 && ((flags & gelu_pre) == gelu_pre || (flags & MLF_EPI_DSWIGLU));
+  if (single_cta_bn(M, N, sms) == 64 && tm * ((N + 63) / 64) <= sms && !wide_epilogue) return 0;
   const int pairs = sms / 2 > 0 ? sms / 2 : 1;
   const double on_pairs = (double)((tiles + pairs - 1) / pairs) - (halves_last_round((int)tiles, pairs) ? 0.2 : 0.0);
   const double single = (double)((tm * ((N + 255) / 256) + sms - 1) / sms);

@@ -11,6 +11,8 @@ ACC, F32, RES, STATIC = _lib.EPI_ACCUM, _lib.EPI_OUT_FP32, _lib.EPI_RESIDUAL, _l
     # 129 - 511 rows: single CTAs while their 128 x 64 tiles run at once, pairs from the next tile column on
     (129, 4032, 512, RES, 0, 0), (256, 4095, 512, RES, 0, 0), (256, 4096, 512, RES, 0, 1),
     (300, 2048, 8192, 0, 0, 0), (300, 3136, 3072, STATIC, 0, 0), (300, 3137, 3072, 0, 0, 1), (400, 2368, 2304, 0, 0, 0), (400, 2369, 2304, 0, 0, 1),
+    (300, 2048, 4096, _lib.EPI_DSWIGLU, 0, 1), (300, 2048, 4104, _lib.EPI_DSWIGLU, 0, 0),
+    (300, 3072, 1024, _lib.EPI_GELU | _lib.EPI_STORE_PRE, 0, 1), (300, 3072, 1024, _lib.EPI_GELU, 0, 0),
     (257, 4096, 1024, 0, 0, 1), (511, 28672, 4096, 0, 0, 1),
     # rounds: 1.8 against 1, then 2 against 2; 5.8 against 4
     (300, 12288, 4096, 0, 0, 0), (300, 12288, 4096, _lib.EPI_GELU, 0, 1), (385, 12288, 4096, 0, 0, 1), (300, 50304, 2048, 0, 0, 1),
