@@ -315,7 +315,8 @@ class _AttentionFn(torch.autograd.Function):
             # rotate into a private copy; the GEMM output stays untouched for autograd
             if qkv2.stride(1) != 1 or qkv2.stride(0) % 8 != 0 or qkv2.data_ptr() % 16 != 0:
                 qkv2 = qkv2.clone(memory_format=torch.contiguous_format)
-            positions = positions.reshape(-1)[:T].long()          # a longer buffer serves every batch
+            if positions.dim() != 1 or positions.shape[0] != T or positions.dtype != torch.int64:
+                positions = positions.reshape(-1)[:T].long()      # a longer buffer serves every batch
             qkv2 = native.rope_qkv(qkv2, positions, Hq, Hkv, rope_theta)
             q = qkv2[:, :Hq * D].view(T, Hq, D)
             k = qkv2[:, Hq * D:(Hq + Hkv) * D].view(T, Hkv, D)

@@ -8,6 +8,7 @@ The PyTorch statements of the same math, used on CPU tensors and as test oracles
 from __future__ import annotations
 
 import ctypes as C
+from functools import lru_cache
 from typing import Optional
 
 import torch
@@ -359,6 +360,12 @@ def flash_bwd(q, k, v, o, dout, lse, B: int, S: int, *, causal: bool = True, sca
 
 
 # ------------------------------------------------------------------ paged attention / KV cache
+@lru_cache(maxsize=None)
+def _sm_count(device_index: int) -> int:
+    """SMs of the current device, whose index the caller passes."""
+    return int(_L().mlf_sm_count())
+
+
 def _decode_split(pairs: int, max_seq_len: int, sms: int) -> int:
     """Tokens per split of the decode kernel for ``pairs`` (sequence, KV head) pairs on ``sms`` SMs, three CTAs of it on
     each. As many splits as keep all CTAs resident at once, none when the pairs alone fill the GPU: CTAs of a second round
@@ -400,7 +407,7 @@ def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Ten
     L = _L()
     L.mlf_paged_decode_ws_elems.restype = C.c_longlong
     if split_tokens <= 0:
-        split_tokens = _decode_split(B * Hkv, max_seq_len, L.mlf_sm_count())
+        split_tokens = _decode_split(B * Hkv, max_seq_len, _sm_count(torch._C._cuda_getDevice()))
     st = (max(split_tokens, 128) + 127) // 128 * 128
     splits = max(1, (max_seq_len + st - 1) // st)
     ws = scratch("paged_decode", L.mlf_paged_decode_ws_elems(B, Hq, splits) * 4, q.device) if splits > 1 else None
@@ -435,7 +442,7 @@ def paged_decode_rope(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: to
     L = _L()
     L.mlf_paged_decode_ws_elems.restype = C.c_longlong
     if split_tokens <= 0:
-        split_tokens = _decode_split(B * Hkv, max_seq_len, L.mlf_sm_count())
+        split_tokens = _decode_split(B * Hkv, max_seq_len, _sm_count(torch._C._cuda_getDevice()))
     st = (max(split_tokens, 128) + 127) // 128 * 128
     splits = max(1, (max_seq_len + st - 1) // st)
     ws = torch.empty(int(L.mlf_paged_decode_ws_elems(B, Hq, splits)), dtype=torch.float32, device=qkv.device) if splits > 1 else None
