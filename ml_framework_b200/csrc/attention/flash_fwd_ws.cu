@@ -1,13 +1,15 @@
-// Self-attention forward, head_dim 128: two 128-row query tiles per CTA, ping-ponged.
+// Self-attention forward, head_dim 128: two 128-row query tiles per item, ping-ponged; one persistent CTA per SM.
 //
-// One CTA = 256 query rows of one (batch, head) as two tiles of 128. 384 threads in three warpgroups;
-// the control warpgroup hands most of its registers to the softmax warpgroups (setmaxnreg):
-//   warp 0        TMA producer: both Q tiles once, then K and V tiles of 128 keys through 2-stage rings
+// An item is 256 query rows of one (batch, head) as two tiles of 128. 384 threads in three warpgroups;
+// the control warpgroup hands most of its registers to the softmax warpgroups (setmaxnreg 72 / 216 / 216 of 3 x 168:
+// with 88 / 208 the softmax spills, and every spill sits on the chain below; 4 x 2048, 16 heads: 84 -> 80 us):
+//   warp 0        TMA producer: an item's Q tiles, its K and V tiles of 128 keys through 2-stage rings
 //   warp 1        MMA issuer (one thread). Per key tile j and query tile t:
 //                   S_t = Q_t K_j^T   (M128 N128 K128, operands in shared memory)  -> TMEM S_t
 //                   O_t += P_t V_j    (M128 N128 K128, P read from TENSOR MEMORY, V from shared memory)
 //                 issued in the order PV_0(j), S_0(j+1), PV_1(j), S_1(j+1) so that the tensor pipe
-//                 works on one tile while the other tile's softmax runs
+//                 works on one tile while the other tile's softmax runs (an issuing thread per tile lets the tiles fall
+//                 into step: 2 x 4096, 32 / 8 heads 254 -> 263 us)
 //   warps 4..7    softmax of tile 0: one query row per thread; reads S_0 from TMEM into registers,
 //                 running max / sum in the log2 domain, writes P_0 as packed bf16 back over S_0
 //   warps 8..11   softmax of tile 1
@@ -16,10 +18,17 @@
 // only after PV_t(j) has read it. O is rescaled lazily: only when a row's maximum has grown by
 // more than 2^8 since the value P and O are expressed against (then O_t is read, scaled and
 // written back by its softmax warps, after PV_t(j-1) has completed).
-// The chain S -> P -> PV -> next S of a tile bounds the kernel (softmax alone 84 us, products alone 67 us of 104 us at
-// 4 x 2048, 16 heads): P is published in halves so that PV starts on the first 64 keys while the exponentials of the
-// others run, and the arithmetic around the exponentials is done two elements at a time. 4 x 2048, 16 heads: 104 -> 97 us;
-// 2 x 4096, 32 / 8 heads: 310 -> 278 us (297 us without the paired arithmetic).
+// The chain S -> P -> PV -> next S of a tile bounds the kernel (about 3300 clocks for 2048 of tensor work): P is published
+// in halves so that PV starts on the first 64 keys while the exponentials of the others run, the arithmetic around the
+// exponentials is done two elements at a time, and every eighth pair of exponentials runs on the FMA pipe (2 x 4096, 32 / 8
+// heads: 254 -> 244 us; every sixth 245, every fourth 256).
+// A CTA walks over its items instead of ending with each: set-up, the first loads and the write-out took a third of the
+// clocks of an item of eight key tiles and two thirds of one of two. The next item's Q, K and V arrive and its first S is
+// issued behind the last products of this one, while the softmax warps write its rows out, each through its own staging
+// tile and the copy engine (32 rows of 16 bytes per store instruction took 2500 clocks). Only the 32-column blocks of a
+// diagonal tile that a warp does not see whole are masked (2000 clocks a tile before).
+// One launch, before -> now: 8 x 512, 32 / 8 heads 57 -> 44 us; 4 x 2048, 16 heads 100 -> 80 us; 2 x 4096, 32 / 8 heads
+// 283 -> 244 us; 1404 queries of 5500 keys, 32 / 8 heads 152 -> 143 us.
 // Per SM and key tile: 4 x 128x128x128 of tensor work against 2 x 16384 exponentials.
 //
 // Math reference: StandardPagedAttentionKernel.ComputePagedAttention
@@ -42,8 +51,10 @@ constexpr int W_D = 128;
 constexpr int W_THREADS = 384;   // warps 0..3 control (TMA, MMA, two idle), 4..7 softmax of tile 0, 8..11 softmax of tile 1
 constexpr int W_TILE_BYTES = 128 * 128 * 2;     // 32 KB: two 64-column blocks of 16 KB
 constexpr int W_STAGES = 2;
-constexpr int W_SMEM = 2 * W_TILE_BYTES + 2 * W_STAGES * W_TILE_BYTES + 256;
+constexpr int W_STG_BYTES = 32 * 128;           // output staging tile of a softmax warp: 32 rows x 64 bf16 columns, 128B-swizzled
+constexpr int W_SMEM = 2 * W_TILE_BYTES + 2 * W_STAGES * W_TILE_BYTES + 8 * W_STG_BYTES + 256;
 constexpr int W_TMEM_COLS = 512;
+constexpr int W_EXP_EVERY = 8;                  // every eighth pair of exponentials runs on the FMA pipe
 
 struct FlashWsParams {
   __nv_bfloat16* out;
@@ -64,16 +75,49 @@ struct FlashWsParams {
 constexpr int W_PAGE = 16;                      // tokens per KV-cache block on the paged path
 constexpr int W_PAGE_BYTES = W_PAGE * 128;      // one page of one 64-column half: 16 rows of 128 bytes
 
+// One unit of work: 256 query rows of one (batch, head).
+struct FlashWsItem {
+  int q0, h, hkv, b;
+  int n_t[2];                  // key tiles that each query tile needs (0: the tile lies past the sequence)
+  int n_kv;
+};
+
+// Item k of a CTA. Items are numbered by work, the longest query pairs first; the CTAs take them in rounds, every other
+// round in reverse, so that the CTA with the longest item of one round gets the shortest of the next.
+__device__ __forceinline__ bool flash_ws_item(const FlashWsParams& p, int n_items, int k, FlashWsItem& it) {
+  const int g = (int)gridDim.x;
+  const long long at = (long long)k * g + ((k & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  if (at >= n_items) return false;
+  const int i = (int)at;
+  const int n_pairs = (p.S + 2 * W_BQ - 1) / (2 * W_BQ);
+  const int hb = p.Hq * p.B;
+  const int pair = p.causal ? n_pairs - 1 - i / hb : i / hb;
+  it.h = (i % hb) % p.Hq;
+  it.b = (i % hb) / p.Hq;
+  it.hkv = it.h / (p.Hq / p.Hkv);
+  it.q0 = pair * 2 * W_BQ;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int qs = it.q0 + t * W_BQ;
+    int n = (p.Skv + W_BKV - 1) / W_BKV;
+    if (p.causal) n = min(n, (qs + p.qoff + W_BQ + W_BKV - 1) / W_BKV);
+    it.n_t[t] = qs < p.S ? n : 0;
+  }
+  it.n_kv = max(it.n_t[0], it.n_t[1]);
+  return true;
+}
+
 __global__ void __launch_bounds__(W_THREADS, 1)
 flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                    const __grid_constant__ CUtensorMap tmV, const FlashWsParams p) {
+                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FlashWsParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const uint32_t sQ = sbase;                                  // 2 tiles
   const uint32_t sK = sQ + 2 * W_TILE_BYTES;                  // W_STAGES tiles
   const uint32_t sV = sK + W_STAGES * W_TILE_BYTES;           // W_STAGES tiles
-  const uint32_t bars = sV + W_STAGES * W_TILE_BYTES;
-  // barriers: q_full[2] k_full[2] v_full[2] k_empty[2] v_empty[2] s_full[2] p_full[2] pv_done[2] p_half[2]
+  const uint32_t sStg = sV + W_STAGES * W_TILE_BYTES;         // one staging tile per softmax warp
+  const uint32_t bars = sStg + 8 * W_STG_BYTES;
+  // barriers: q_full[2] k_full[2] v_full[2] k_empty[2] v_empty[2] s_full[2] p_full[2] pv_done[2] p_half[2] q_empty[2]
   auto q_full = [&](int t) { return bars + 8u * t; };
   auto k_full = [&](int s) { return bars + 8u * (2 + s); };
   auto v_full = [&](int s) { return bars + 8u * (4 + s); };
@@ -83,31 +127,13 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   auto p_full = [&](int t) { return bars + 8u * (12 + t); };
   auto pv_done = [&](int t) { return bars + 8u * (14 + t); };
   auto p_half = [&](int t) { return bars + 8u * (16 + t); };
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + (bars - sbase) + 8 * 18);
+  auto q_empty = [&](int t) { return bars + 8u * (18 + t); };
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + (bars - sbase) + 8 * 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int n_pairs = (p.S + 2 * W_BQ - 1) / (2 * W_BQ);
-  // 1-D grid ordered by work: all (batch, head) of the longest query pair first, the shortest last
-  const int hb = p.Hq * p.B;
-  const int pair = p.causal ? n_pairs - 1 - (int)blockIdx.x / hb : (int)blockIdx.x / hb;
-  const int h = ((int)blockIdx.x % hb) % p.Hq;
-  const int b = ((int)blockIdx.x % hb) / p.Hq;
-  const int hkv = h / (p.Hq / p.Hkv);
-  const int q0 = pair * 2 * W_BQ;
-  const long long row_base = (long long)b * p.S;
-  const long long kv_row_base = (long long)b * p.Skv;
-  // key tiles each query tile needs
-  int n_t[2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int qs = q0 + t * W_BQ;
-    int n = (p.Skv + W_BKV - 1) / W_BKV;
-    if (p.causal) n = min(n, (qs + p.qoff + W_BQ + W_BKV - 1) / W_BKV);
-    n_t[t] = qs < p.S ? n : 0;
-  }
-  const int n_kv = max(n_t[0], n_t[1]);
+  const int n_items = ((p.S + 2 * W_BQ - 1) / (2 * W_BQ)) * p.Hq * p.B;
 
   if ((sbase & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(p.err, 0, ERR_BAD_INDEX);
@@ -124,6 +150,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(p_full(i), 128);
       mbar_init(p_half(i), 128);
       mbar_init(pv_done(i), 1);
+      mbar_init(q_empty(i), 1);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -140,62 +167,77 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   pdl_wait();
   auto tS = [&](int t) { return tmem_base + 128u * t; };
   auto tO = [&](int t) { return tmem_base + 256u + 128u * t; };
+  FlashWsItem w;
 
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0) {
     // ===================== TMA producer =====================
     if (elect_one()) {
-      for (int t = 0; t < 2; ++t) {
-        mbar_expect_tx(q_full(t), W_TILE_BYTES);
-        const int qrow = (int)(row_base + q0 + t * W_BQ);
-        tma_load_2d(sQ + t * W_TILE_BYTES, &tmQ, h * W_D, qrow, q_full(t));
-        tma_load_2d(sQ + t * W_TILE_BYTES + W_TILE_BYTES / 2, &tmQ, h * W_D + 64, qrow, q_full(t));
-      }
-      const int* bt = p.block_table ? p.block_table + (long long)b * p.max_blocks : nullptr;
+      int kt = 0;                               // key tiles fetched so far: ring position and phase
+      int n_q[2] = {0, 0};                      // query tiles fetched so far
+      bool ok = true;
       const int seq_pages = (p.Skv + W_PAGE - 1) / W_PAGE;
-      for (int j = 0; j < n_kv; ++j) {
-        const int s = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        const int krow = (int)(kv_row_base + j * W_BKV);
-        int blk[W_BKV / W_PAGE];
-        if (bt) {
-          // the eight table entries of this tile first (independent loads); pages past the end of the sequence
-          // repeat its first page: their keys are masked, they only have to be readable
+      for (int k = 0; ok && flash_ws_item(p, n_items, k, w); ++k) {
+        const long long row_base = (long long)w.b * p.S;
+        const long long kv_row_base = (long long)w.b * p.Skv;
+        const int* bt = p.block_table ? p.block_table + (long long)w.b * p.max_blocks : nullptr;
+        for (int j = 0; j < w.n_kv && ok; ++j, ++kt) {
+          const int s = kt & 1;
+          const uint32_t ph = (kt >> 1) & 1;
+          const int krow = (int)(kv_row_base + j * W_BKV);
+          int blk[W_BKV / W_PAGE];
+          if (bt) {
+            // the eight table entries of this tile first (independent loads); pages past the end of the sequence
+            // repeat its first page: their keys are masked, they only have to be readable
 #pragma unroll
-          for (int g = 0; g < W_BKV / W_PAGE; ++g) {
-            const int pg = j * (W_BKV / W_PAGE) + g;
-            blk[g] = bt[pg < seq_pages && pg < p.max_blocks ? pg : 0];
+            for (int g = 0; g < W_BKV / W_PAGE; ++g) {
+              const int pg = j * (W_BKV / W_PAGE) + g;
+              blk[g] = bt[pg < seq_pages && pg < p.max_blocks ? pg : 0];
+            }
+#pragma unroll
+            for (int g = 0; g < W_BKV / W_PAGE; ++g)
+              if (blk[g] < 0 || blk[g] >= p.num_blocks) { atomicCAS(p.err, 0, ERR_BAD_INDEX); blk[g] = 0; }
           }
+          if (!mbar_wait(k_empty(s), ph ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+          mbar_expect_tx(k_full(s), W_TILE_BYTES);
+          if (bt) {
 #pragma unroll
-          for (int g = 0; g < W_BKV / W_PAGE; ++g)
-            if (blk[g] < 0 || blk[g] >= p.num_blocks) { atomicCAS(p.err, 0, ERR_BAD_INDEX); blk[g] = 0; }
-        }
-        if (!mbar_wait(k_empty(s), ph ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) break;
-        mbar_expect_tx(k_full(s), W_TILE_BYTES);
-        if (bt) {
-#pragma unroll
-          for (int g = 0; g < W_BKV / W_PAGE; ++g) {
-            const uint32_t dst = sK + s * W_TILE_BYTES + g * W_PAGE_BYTES;
-            tma_load_2d(dst, &tmK, hkv * W_D, blk[g] * 2 * W_PAGE, k_full(s));
-            tma_load_2d(dst + W_TILE_BYTES / 2, &tmK, hkv * W_D + 64, blk[g] * 2 * W_PAGE, k_full(s));
+            for (int g = 0; g < W_BKV / W_PAGE; ++g) {
+              const uint32_t dst = sK + s * W_TILE_BYTES + g * W_PAGE_BYTES;
+              tma_load_2d(dst, &tmK, w.hkv * W_D, blk[g] * 2 * W_PAGE, k_full(s));
+              tma_load_2d(dst + W_TILE_BYTES / 2, &tmK, w.hkv * W_D + 64, blk[g] * 2 * W_PAGE, k_full(s));
+            }
+          } else {
+            tma_load_2d(sK + s * W_TILE_BYTES, &tmK, w.hkv * W_D, krow, k_full(s));
+            tma_load_2d(sK + s * W_TILE_BYTES + W_TILE_BYTES / 2, &tmK, w.hkv * W_D + 64, krow, k_full(s));
           }
-        } else {
-          tma_load_2d(sK + s * W_TILE_BYTES, &tmK, hkv * W_D, krow, k_full(s));
-          tma_load_2d(sK + s * W_TILE_BYTES + W_TILE_BYTES / 2, &tmK, hkv * W_D + 64, krow, k_full(s));
-        }
-        if (!mbar_wait(v_empty(s), ph ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) break;
-        mbar_expect_tx(v_full(s), W_TILE_BYTES);
-        if (bt) {
-#pragma unroll
-          for (int g = 0; g < W_BKV / W_PAGE; ++g) {
-            const uint32_t dst = sV + s * W_TILE_BYTES + g * W_PAGE_BYTES;
-            tma_load_2d(dst, &tmV, hkv * W_D, (blk[g] * 2 + 1) * W_PAGE, v_full(s));
-            tma_load_2d(dst + W_TILE_BYTES / 2, &tmV, hkv * W_D + 64, (blk[g] * 2 + 1) * W_PAGE, v_full(s));
+          if (j == 0) {
+            // this item's queries, each as soon as the previous item's last S of that tile has read its buffer
+            for (int t = 0; t < 2; ++t) {
+              if (w.n_t[t] == 0) continue;
+              if (!mbar_wait(q_empty(t), (n_q[t] & 1) ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+              ++n_q[t];
+              mbar_expect_tx(q_full(t), W_TILE_BYTES);
+              const int qrow = (int)(row_base + w.q0 + t * W_BQ);
+              tma_load_2d(sQ + t * W_TILE_BYTES, &tmQ, w.h * W_D, qrow, q_full(t));
+              tma_load_2d(sQ + t * W_TILE_BYTES + W_TILE_BYTES / 2, &tmQ, w.h * W_D + 64, qrow, q_full(t));
+            }
+            if (!ok) break;
           }
-        } else {
-          tma_load_2d(sV + s * W_TILE_BYTES, &tmV, hkv * W_D, krow, v_full(s));
-          tma_load_2d(sV + s * W_TILE_BYTES + W_TILE_BYTES / 2, &tmV, hkv * W_D + 64, krow, v_full(s));
+          if (!mbar_wait(v_empty(s), ph ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+          mbar_expect_tx(v_full(s), W_TILE_BYTES);
+          if (bt) {
+#pragma unroll
+            for (int g = 0; g < W_BKV / W_PAGE; ++g) {
+              const uint32_t dst = sV + s * W_TILE_BYTES + g * W_PAGE_BYTES;
+              tma_load_2d(dst, &tmV, w.hkv * W_D, (blk[g] * 2 + 1) * W_PAGE, v_full(s));
+              tma_load_2d(dst + W_TILE_BYTES / 2, &tmV, w.hkv * W_D + 64, (blk[g] * 2 + 1) * W_PAGE, v_full(s));
+            }
+          } else {
+            tma_load_2d(sV + s * W_TILE_BYTES, &tmV, w.hkv * W_D, krow, v_full(s));
+            tma_load_2d(sV + s * W_TILE_BYTES + W_TILE_BYTES / 2, &tmV, w.hkv * W_D + 64, krow, v_full(s));
+          }
         }
       }
     }
@@ -204,91 +246,120 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(128, W_BKV, 0, 0);
       const uint32_t idesc_pv = make_idesc_bf16(128, W_D, 0, 1);
-      auto issue_s = [&](int t, int j) {
-        const uint32_t q = sQ + t * W_TILE_BYTES, k = sK + (j & 1) * W_TILE_BYTES;
-#pragma unroll
+      auto issue_s = [&](int t, int stage) {
+        const uint32_t q = sQ + t * W_TILE_BYTES, kk_base = sK + stage * W_TILE_BYTES;
+#pragma unroll 4
         for (int kk = 0; kk < W_D / 16; ++kk) {
           const uint32_t off = (kk >> 2) * (W_TILE_BYTES / 2) + (kk & 3) * 32;
-          umma_bf16_ss(tS(t), make_smem_desc_sw128(q + off, 16, 1024), make_smem_desc_sw128(k + off, 16, 1024), idesc_s, kk != 0);
+          umma_bf16_ss(tS(t), make_smem_desc_sw128(q + off, 16, 1024), make_smem_desc_sw128(kk_base + off, 16, 1024), idesc_s, kk != 0);
         }
         umma_commit(s_full(t));
       };
-      auto issue_pv = [&](int t, int j, int half) {      // 64 keys: P's half, as soon as the softmax has published it
-        const uint32_t v = sV + (j & 1) * W_TILE_BYTES;
+      auto issue_pv = [&](int t, int stage, int half, bool first) {   // 64 keys: P's half, as soon as the softmax has published it
+        const uint32_t v = sV + stage * W_TILE_BYTES;
 #pragma unroll
         for (int i = 0; i < W_BKV / 32; ++i) {
           const int kk = half * (W_BKV / 32) + i;
-          umma_bf16_ts(tO(t), tS(t) + 8u * kk, make_smem_desc_sw128(v + kk * 2048, W_TILE_BYTES / 2, 1024), idesc_pv, (j | kk) != 0);
+          umma_bf16_ts(tO(t), tS(t) + 8u * kk, make_smem_desc_sw128(v + kk * 2048, W_TILE_BYTES / 2, 1024), idesc_pv, !first || kk != 0);
         }
       };
+      int kt = 0;                               // ring position of this item's first key tile
+      int n_p[2] = {0, 0};                      // key tiles multiplied so far, per query tile
+      int n_q[2] = {0, 0};
       bool ok = true;
-      // prologue: S_0(0), S_1(0)
-      if (n_kv > 0) {
-        ok = mbar_wait(k_full(0), 0, abort_flag, p.err, ERR_WAIT_ATTN);
-        for (int t = 0; t < 2 && ok; ++t) {
-          if (n_t[t] == 0) continue;
-          ok = mbar_wait(q_full(t), 0, abort_flag, p.err, ERR_WAIT_ATTN);
-          if (!ok) break;
-          tc_fence_after_sync();
-          issue_s(t, 0);
-        }
+      bool have = flash_ws_item(p, n_items, 0, w);
+      // S_t(0) of an item, its K and Q waited for; the last S of a tile gives its Q buffer back
+      auto first_s = [&](const FlashWsItem& x, int ring, int t) -> bool {
+        if (x.n_t[t] == 0) return true;
+        if (!mbar_wait(k_full(ring & 1), (ring >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) return false;
+        if (!mbar_wait(q_full(t), n_q[t] & 1, abort_flag, p.err, ERR_WAIT_ATTN)) return false;
+        ++n_q[t];
+        tc_fence_after_sync();
+        issue_s(t, ring & 1);
+        if (x.n_t[t] == 1) umma_commit(q_empty(t));
+        return true;
+      };
+      if (have) {
+        ok = first_s(w, 0, 0) && first_s(w, 0, 1);
         if (ok) umma_commit(k_empty(0));          // K_0 consumed by both tiles' S
       }
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int s = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        bool k_next_ready = false;
-        for (int t = 0; t < 2 && ok; ++t) {
-          if (j < n_t[t]) {
-            if (!mbar_wait(v_full(s), ph, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
-            if (!mbar_wait(p_half(t), j & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
-            tc_fence_after_sync();
-            issue_pv(t, j, 0);
-            if (!mbar_wait(p_full(t), j & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
-            tc_fence_after_sync();
-            issue_pv(t, j, 1);
-            umma_commit(pv_done(t));
-          }
-          if (j + 1 < n_t[t]) {
-            if (!k_next_ready) {
-              if (!mbar_wait(k_full((j + 1) & 1), ((j + 1) >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
-              k_next_ready = true;
+      for (int k = 0; ok && have; ++k) {
+        FlashWsItem nx;
+        const bool more = flash_ws_item(p, n_items, k + 1, nx);
+        for (int j = 0; j < w.n_kv && ok; ++j) {
+          const int r = kt + j, s = r & 1;
+          const uint32_t ph = (r >> 1) & 1;
+          const bool last = j + 1 == w.n_kv;
+          bool k_next_ready = false;
+          for (int t = 0; t < 2 && ok; ++t) {
+            if (j < w.n_t[t]) {
+              if (!mbar_wait(v_full(s), ph, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+              if (!mbar_wait(p_half(t), n_p[t] & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
               tc_fence_after_sync();
+              issue_pv(t, s, 0, j == 0);
+              if (!mbar_wait(p_full(t), n_p[t] & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+              tc_fence_after_sync();
+              issue_pv(t, s, 1, j == 0);
+              umma_commit(pv_done(t));
+              ++n_p[t];
             }
-            issue_s(t, j + 1);
+            if (j + 1 < w.n_t[t]) {
+              if (!k_next_ready) {
+                if (!mbar_wait(k_full((r + 1) & 1), ((r + 1) >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+                k_next_ready = true;
+                tc_fence_after_sync();
+              }
+              issue_s(t, (r + 1) & 1);
+              if (j + 2 == w.n_t[t]) umma_commit(q_empty(t));
+            } else if (last && more) {
+              // the next item's first S goes in behind this item's last products: its softmax warps find it ready when
+              // they have written their rows
+              if (!first_s(nx, r + 1, t)) { ok = false; break; }
+            }
           }
+          if (!ok) break;
+          umma_commit(v_empty(s));                               // V_j consumed by both tiles' PV
+          if (!last || more) umma_commit(k_empty((r + 1) & 1));  // K_{j+1}, or the next item's K_0, consumed by both tiles' S
         }
-        if (!ok) break;
-        umma_commit(v_empty(s));                               // V_j consumed by both tiles' PV
-        if (j + 1 < n_kv) umma_commit(k_empty((j + 1) & 1));   // K_{j+1} consumed by both tiles' S
+        kt += w.n_kv;
+        w = nx;
+        have = more;
       }
     }
   }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     // ===================== softmax warpgroups =====================
     const int t = (warp - 4) >> 2;            // query tile of this warpgroup
     const int q = warp & 3;                   // TMEM lane quarter this warp may access
     const int r = q * 32 + lane;
-    const int qi = q0 + t * W_BQ + r;
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-    const int n_mine = n_t[t];
-    float m_used = 0.f, l = 0.f;
+    int n = 0;                                // key tiles seen so far (phase of every barrier of this tile)
     bool ok = true;
-    for (int j = 0; j < n_mine; ++j) {
-      if (!mbar_wait_warp(s_full(t), j & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+    for (int k = 0; ok && flash_ws_item(p, n_items, k, w); ++k) {
+    const int qi = w.q0 + t * W_BQ + r;
+    const int n_mine = w.n_t[t];
+    float m_used = 0.f, l = 0.f;
+    for (int j = 0; j < n_mine; ++j, ++n) {
+      if (!mbar_wait_warp(s_full(t), n & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
       tc_fence_after_sync();
       const int k0 = j * W_BKV;
-      const bool need_mask = (p.causal && k0 + W_BKV - 1 > q0 + t * W_BQ + p.qoff) || (k0 + W_BKV > p.Skv);
       uint32_t sv[128];
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(tS(t) + 32 * c + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&sv[32 * c]));
       tmem_wait_ld();
-      if (need_mask) {
+      // last visible column of this row, and of the warp's first row: blocks of 32 columns that the whole warp sees are
+      // left alone, so that a diagonal tile costs as little as it can
+      const int lim = (p.causal ? min(p.Skv - 1, qi + p.qoff) : p.Skv - 1) - k0;
+      const int lim_warp = (p.causal ? min(p.Skv - 1, w.q0 + t * W_BQ + q * 32 + p.qoff) : p.Skv - 1) - k0;
+      if (lim_warp < W_BKV - 1) {
 #pragma unroll
-        for (int i = 0; i < 128; ++i) {
-          const int kj = k0 + i;
-          if (kj >= p.Skv || (p.causal && kj > qi + p.qoff)) sv[i] = __float_as_uint(-INFINITY);
+        for (int c = 0; c < 4; ++c) {
+          if (32 * c + 31 > lim_warp) {
+#pragma unroll
+            for (int i = 32 * c; i < 32 * c + 32; ++i)
+              if (i > lim) sv[i] = __float_as_uint(-INFINITY);
+          }
         }
       }
       // The tile's maximum first (three-input maxima), so that P can be published in halves: the tensor pipe multiplies
@@ -306,7 +377,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (j == 0) m_used = mx == -INFINITY ? 0.f : mx;
       const bool grow = j > 0 && mx > m_used + 8.f;
       if (__any_sync(0xffffffffu, grow)) {
-        if (!mbar_wait_warp(pv_done(t), (j - 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+        if (!mbar_wait_warp(pv_done(t), (n - 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
         tc_fence_after_sync();
         const float f = grow ? exp2f(m_used - mx) : 1.f;
 #pragma unroll
@@ -331,9 +402,13 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int i = 0; i < 32; ++i) {
           const uint64_t e = fma_f32x2(pack_f32x2(__uint_as_float(sv[64 * hh + 2 * i]), __uint_as_float(sv[64 * hh + 2 * i + 1])), c2, nm2);
           float e0, e1;
-          unpack_f32x2(e, e0, e1);
-          e0 = exp2f(e0);
-          e1 = exp2f(e1);
+          if (i % W_EXP_EVERY == W_EXP_EVERY - 1) {
+            exp2_fma_f32x2(e, e0, e1);
+          } else {
+            unpack_f32x2(e, e0, e1);
+            e0 = exp2f(e0);
+            e1 = exp2f(e1);
+          }
           rs = add_f32x2(rs, pack_f32x2(e0, e1));
           pk[i] = pack_bf16x2(e0, e1);
         }
@@ -346,12 +421,45 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       unpack_f32x2(rs, rs0, rs1);
       l += rs0 + rs1;
     }
-    if (ok && n_mine > 0) ok = mbar_wait_warp(pv_done(t), (n_mine - 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN);
-    if (ok && n_mine > 0) {
-      tc_fence_after_sync();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      const bool row_ok = qi < p.S;
-      __nv_bfloat16* orow = p.out + (row_base + qi) * p.ldo + (long long)h * W_D;
+    if (!ok || n_mine == 0) continue;
+    if (!mbar_wait_warp(pv_done(t), (n - 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+    // O_t is free for the next item's first product once this warpgroup publishes that item's first P, which every
+    // thread does after its reads here
+    tc_fence_after_sync();
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    const bool row_ok = qi < p.S;
+    const long long row = (long long)w.b * p.S + qi;
+    if (w.q0 + t * W_BQ + q * 32 + 32 <= p.S) {
+      // the warp's 32 rows go through its own swizzled staging tile, 64 columns at a time
+      const uint32_t stg = sStg + (uint32_t)(warp - 4) * W_STG_BYTES;
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        uint32_t o[64];
+        tmem_ld_32x32b_x32(tO(t) + hh * 64 + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&o[0]));
+        tmem_ld_32x32b_x32(tO(t) + hh * 64 + 32 + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&o[32]));
+        tmem_wait_ld();
+        if (lane == 0) tma_store_wait_read<0>();   // the store before has left the staging tile
+        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          const uint32_t addr = stg + lane * 128 + (((uint32_t)v ^ (uint32_t)(lane & 7)) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
+                       "r"(pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv)),
+                       "r"(pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv)),
+                       "r"(pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv)),
+                       "r"(pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv))
+                       : "memory");
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&tmO, stg, w.h * W_D + hh * 64, (int)((long long)w.b * p.S + w.q0 + t * W_BQ + q * 32));
+          tma_store_commit();
+        }
+      }
+    } else {
+      // the sequence's last rows: the ones behind them belong to the next sequence
+      __nv_bfloat16* orow = p.out + row * p.ldo + (long long)w.h * W_D;
 #pragma unroll
       for (int c = 0; c < W_D / 32; ++c) {
         uint32_t o[32];
@@ -360,17 +468,19 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (row_ok) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
-            w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
-            w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
-            w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
-            reinterpret_cast<uint4*>(orow + 32 * c)[v] = w;
+            uint4 x;
+            x.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
+            x.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
+            x.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
+            x.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
+            reinterpret_cast<uint4*>(orow + 32 * c)[v] = x;
           }
         }
       }
-      if (row_ok && p.lse) p.lse[((long long)b * p.Hq + h) * p.S + qi] = (m_used + log2f(l)) * 0.6931471805599453f;
     }
+    if (row_ok && p.lse) p.lse[((long long)w.b * p.Hq + w.h) * p.S + qi] = (m_used + log2f(l)) * 0.6931471805599453f;
+    }
+    if (lane == 0) tma_store_wait_all<0>();
     tc_fence_before_sync();
   }
 
@@ -385,6 +495,24 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, W_TMEM_COLS);
   }
+}
+
+static int launch_flash_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FlashWsParams& p, cudaStream_t st) {
+  CUtensorMap to;
+  if (int rc = cached_tmap_bf16(&to, p.out, (uint64_t)p.Hq * W_D, (uint64_t)p.B * p.S, (uint64_t)p.ldo, 64, 32)) return rc;
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_set[dev & 63]) {
+    MLF_CHECK_CUDA(cudaFuncSetAttribute(flash_fwd_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM));
+    attr_set[dev & 63] = true;
+  }
+  // one CTA per SM (shared memory and tensor memory hold no second one): each walks over items / SMs of them
+  const long long items = (long long)((p.S + 2 * W_BQ - 1) / (2 * W_BQ)) * p.Hq * p.B;
+  const int sms = sm_count();
+  MLF_CHECK_CUDA(launch_pdl(flash_fwd_ws_kernel, dim3((unsigned)(items < sms ? items : sms)), dim3(W_THREADS), W_SMEM, st, tq, tk, tv, to, p));
+  count_launch();
+  return 0;
 }
 
 }  // namespace mlf
@@ -420,17 +548,7 @@ MLF_API int mlf_flash_fwd_prefix(const void* q, const void* k, const void* v, vo
   p.block_table = nullptr;
   p.max_blocks = p.num_blocks = 0;
   MLF_REQUIRE(p.err != nullptr, "no device status word");
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set[dev & 63]) {
-    MLF_CHECK_CUDA(cudaFuncSetAttribute(flash_fwd_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM));
-    attr_set[dev & 63] = true;
-  }
-  dim3 grid(((S + 2 * W_BQ - 1) / (2 * W_BQ)) * Hq * B);
-  MLF_CHECK_CUDA(launch_pdl(flash_fwd_ws_kernel, grid, dim3(W_THREADS), W_SMEM, st, tq, tk, tv, p));
-  count_launch();
-  return 0;
+  return launch_flash_ws(tq, tk, tv, p, st);
 }
 
 // Prefill attention whose keys and values are read straight out of the paged KV cache: queries [B * Sq rows] are the
@@ -466,17 +584,7 @@ MLF_API int mlf_flash_fwd_paged(const void* q, const void* cache, const int* blo
   p.max_blocks = max_blocks;
   p.num_blocks = num_blocks;
   MLF_REQUIRE(p.err != nullptr, "no device status word");
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set[dev & 63]) {
-    MLF_CHECK_CUDA(cudaFuncSetAttribute(flash_fwd_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM));
-    attr_set[dev & 63] = true;
-  }
-  dim3 grid(((Sq + 2 * W_BQ - 1) / (2 * W_BQ)) * Hq * B);
-  MLF_CHECK_CUDA(launch_pdl(flash_fwd_ws_kernel, grid, dim3(W_THREADS), W_SMEM, st, tq, tkv, tkv, p));
-  count_launch();
-  return 0;
+  return launch_flash_ws(tq, tkv, tkv, p, st);
 }
 
 // Same arguments as mlf_flash_fwd.
