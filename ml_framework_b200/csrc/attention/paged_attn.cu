@@ -694,8 +694,8 @@ MLF_API int mlf_rope_kv_write(void* qkv, long long ld, const long long* pos, con
   if (parts > groups) parts = groups;
   const int heads_per_warp = (int)((groups + parts - 1) / parts) * 4;
   const dim3 grid((unsigned)((T + 7) / 8), (unsigned)((Hq + 2 * Hkv + heads_per_warp - 1) / heads_per_warp));
-  MLF_CHECK_CUDA(launch_pdl(v16 ? rope_kv_write_kernel<true> : rope_kv_write_kernel<false>, grid, dim3(256), 0,
-                            reinterpret_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), ld, pos, slots,
+  const auto kernel = v16 ? rope_kv_write_kernel<true> : rope_kv_write_kernel<false>;
+  MLF_CHECK_CUDA(launch_pdl(kernel, grid, dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), ld, pos, slots,
                             static_cast<__nv_bfloat16*>(cache), T, Hq, Hkv, block_size, num_blocks, heads_per_warp, theta, device_status_word()));
   count_launch();
   return 0;
