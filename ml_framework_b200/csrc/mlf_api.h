@@ -71,6 +71,36 @@ typedef struct MlfGemmArgs {
   const MlfGemmComm* comm;  // host pointer or null
 } MlfGemmArgs;
 
+// ---- one transformer block (csrc/ops/block.cu) ----
+// Bits of MlfBlockArgs.accumulate: the parameter's gradient is added to its buffer instead of written.
+enum {
+  MLF_BLOCK_G1, MLF_BLOCK_B1, MLF_BLOCK_WQKV, MLF_BLOCK_BQKV, MLF_BLOCK_WO, MLF_BLOCK_BO, MLF_BLOCK_G2, MLF_BLOCK_B2, MLF_BLOCK_W1,
+  MLF_BLOCK_BB1, MLF_BLOCK_W2, MLF_BLOCK_BB2
+};
+
+typedef struct MlfBlockArgs {
+  int B, S, d, Hq, Hkv, ff;   // T = B * S rows of d; heads of 128; MLP width
+  int gated;                  // 0: layer norm, biases, GELU; 1: RMS norm, no biases (null), rotary embedding, SwiGLU
+  int causal, accumulate;
+  float eps1, eps2, rope_theta, scale;
+  const void *g1, *b1, *wqkv, *bqkv, *wo, *bo, *g2, *b2, *w1, *bb1, *w2, *bb2;   // bf16 parameters
+  const long long* pos;       // rotary positions [T], or null
+  // rows of the forward (bf16, packed) and statistics (fp32; means null when gated)
+  const void* x;
+  void *h1, *qkv, *a, *x1, *h2, *pre, *act;
+  float *mean1, *rstd1, *mean2, *rstd2, *lse;
+  void* y;
+  // backward: dy in, dx out; wide [T, max(MLP's first product, QKV)], row [T, d], da [T, Hq * 128], dx1 [T, d] are work
+  const void* dy;
+  void *wide, *row, *da, *dx1, *dx;
+  void *dg1, *db1, *dwqkv, *dbqkv, *dwo, *dbo, *dg2, *db2, *dw1, *dbb1, *dw2, *dbb2;   // bf16, shaped like the parameters
+  float* norm_scratch;
+  void *colsum_scratch, *flash_scratch;   // these three as mlf_norm_bwd, mlf_colsum (for every width here), mlf_flash_bwd need them
+} MlfBlockArgs;
+
+int mlf_block_forward(const MlfBlockArgs* args, uint64_t stream);
+int mlf_block_backward(const MlfBlockArgs* args, uint64_t stream);
+
 const char* mlf_last_error(void);
 int mlf_read_status(int clear);
 int mlf_sm_count(void);

@@ -13,8 +13,9 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from ..nn.layers import Embedding, GeluMLP, LayerNorm, SelfAttention
+from ..nn.layers import Embedding, GeluMLP, LayerNorm, Linear, SelfAttention
 from ..ops import functional as Fm
+from ..ops.block import block as whole_block
 
 
 @dataclass
@@ -69,6 +70,12 @@ class GPTBlock(nn.Module):
                            out_init_std=out_std)
 
     def forward(self, x):
+        mlp = self.mlp
+        if type(self.ln1) is LayerNorm and type(self.ln2) is LayerNorm and type(self.attn) is SelfAttention and type(mlp) is GeluMLP \
+                and type(self.attn.qkv) is Linear and type(self.attn.proj) is Linear:
+            y = whole_block(self.ln1, self.attn, self.ln2, mlp, mlp.fc1, mlp.fc2, x, None, gated=False)
+            if y is not None:
+                return y
         h, skip = self.ln1.with_skip(x)
         x = self.attn(h, residual=skip)
         h, skip = self.ln2.with_skip(x)

@@ -13,8 +13,9 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from ..nn.layers import Embedding, RMSNorm, SelfAttention, SwiGLUMLP
+from ..nn.layers import Embedding, Linear, RMSNorm, SelfAttention, SwiGLUMLP
 from ..ops import functional as Fm
+from ..ops.block import block as whole_block
 
 
 @dataclass
@@ -77,6 +78,12 @@ class LlamaBlock(nn.Module):
         self.mlp = SwiGLUMLP(cfg.d_model, cfg.d_ff, dtype, device, cfg.init_std, out_std)
 
     def forward(self, x, positions=None):
+        mlp = self.mlp
+        if type(self.norm1) is RMSNorm and type(self.norm2) is RMSNorm and type(self.attn) is SelfAttention and type(mlp) is SwiGLUMLP \
+                and type(self.attn.qkv) is Linear and type(self.attn.proj) is Linear:
+            y = whole_block(self.norm1, self.attn, self.norm2, mlp, mlp.gate_up, mlp.down, x, positions, gated=True)
+            if y is not None:
+                return y
         h, skip = self.norm1.with_skip(x)
         x = self.attn(h, residual=skip, positions=positions)
         h, skip = self.norm2.with_skip(x)

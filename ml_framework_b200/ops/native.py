@@ -161,19 +161,26 @@ def swiglu_bwd(dout: torch.Tensor, gu: torch.Tensor, interleaved: bool = False) 
     return dgu.view(gu.shape)
 
 
+def colsum_scratch(M: int, widths, device) -> torch.Tensor:
+    """Scratch for the column sums of matrices of M rows and each of ``widths`` columns."""
+    L = _L()
+    L.mlf_colsum_scratch_bytes.restype = C.c_longlong
+    need = max(int(L.mlf_colsum_scratch_bytes(M, n)) for n in widths)
+    key = ("colsum0", device.index)
+    sc = _scratch.get(key)
+    if sc is None or sc.numel() < need:                  # zero-filled once: the kernel keeps its counters at zero
+        sc = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
+        _scratch[key] = sc
+    return sc
+
+
 def colsum(dy: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False) -> torch.Tensor:
     """bf16 column sums of a 2-D bf16 matrix (bias gradient)."""
     assert dy.dim() == 2 and dy.stride(1) == 1
     M, N = dy.shape
     out = torch.empty(N, dtype=torch.bfloat16, device=dy.device) if out is None else out
     L = _L()
-    L.mlf_colsum_scratch_bytes.restype = C.c_longlong
-    need = int(L.mlf_colsum_scratch_bytes(M, N))
-    key = ("colsum0", dy.device.index)
-    sc = _scratch.get(key)
-    if sc is None or sc.numel() < need:                  # zero-filled once: the kernel keeps its counters at zero
-        sc = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dy.device)
-        _scratch[key] = sc
+    sc = colsum_scratch(M, (N,), dy.device)
     _lib.check(L.mlf_colsum(_p(out), _p(dy), M, N, C.c_longlong(dy.stride(0)), _p(sc), int(accumulate), _st()), "mlf_colsum")
     return out
 
