@@ -1,11 +1,9 @@
 // LayerNorm and RMSNorm, forward and backward, bf16 activations with fp32 statistics.
 //
-// One warp owns one row at a time and keeps it in registers as packed bf16 (NV 16-byte
+// Forward: one warp owns one row at a time and keeps it in registers as packed bf16 (NV 16-byte
 // vectors per lane), so x is read from HBM exactly once per pass; from D = 2048 on a CTA owns whole rows, unless rows are
-// many and D is no 2048 or 4096. The backward pass adds the
-// per-row contributions to gamma/beta gradients into a per-CTA shared-memory accumulator with
-// shared atomics and writes one partial per CTA; a second tiny kernel sums the partials. The wide
-// model dimensions (2048 and 4096) use a backward kernel with whole-CTA rows instead.
+// many and D is no 2048 or 4096. Backward: every thread owns fixed columns of the rows that pass by and keeps its share of the
+// gamma / beta gradients in registers, one partial per CTA; a second tiny kernel sums the partials.
 //
 // The reference has no norm kernels (its AMP rules only name layernorm as an fp32 op,
 // src/MLFramework/Amp/DefaultAmpRules.cs:48-110); these are required by the GPT and Llama
@@ -306,152 +304,74 @@ norm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma, const __
   }
 }
 
-// Backward. Each warp walks rows with a grid stride. Gamma / beta gradient contributions are kept
-// per lane in registers when they fit (MODE 0: D <= 2048, row cached in registers too; MODE 1:
-// RMSNorm up to D = 5120, row re-read from L1/L2 for the second pass) and only folded into a
-// per-CTA shared-memory accumulator once per kernel. MODE 2 (everything else) adds every row's
-// contribution to shared memory directly.
-template <int NV, int MODE>
-__global__ void __launch_bounds__(256)
-norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                float* __restrict__ partials /* [grid, 2, D] */, int rows, int rms,
-                const __nv_bfloat16* __restrict__ dx_add /* optional: added to dx (gradient of a skip connection) */) {
-  constexpr int D = NV * 256;
-  constexpr int NK = MODE == 0 ? NV : 1;          // cached row vectors
-  constexpr int NG = MODE <= 1 ? NV : 1;          // register dgamma partials
-  constexpr int NB = MODE == 0 ? NV : 1;          // register dbeta partials
-  extern __shared__ float acc[];  // [2][D]
-  for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) acc[i] = 0.f;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int warps_per_cta = blockDim.x >> 5;
-  const uint4* gr = reinterpret_cast<const uint4*>(gamma);
-  float dg[NG][8], db[NB][8];
-#pragma unroll
-  for (int i = 0; i < NG; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dg[i][j] = 0.f;
-#pragma unroll
-  for (int i = 0; i < NB; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) db[i][j] = 0.f;
-  for (int row = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps_per_cta) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * D);
-    const uint4* dr = reinterpret_cast<const uint4*>(dy + (long long)row * D);
-    uint4 xv[NK], dv[NK];
-    if (MODE == 0) {
-#pragma unroll
-      for (int i = 0; i < NK; ++i) {
-        xv[i] = xr[i * 32 + lane];
-        dv[i] = dr[i * 32 + lane];
-      }
-    }
-    const float mean = rms ? 0.f : mean_in[row];
-    const float rstd = rstd_in[row];
-    float c1 = 0.f, c2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      float f[8], d[8], g[8];
-      unpack8(MODE == 0 ? xv[MODE == 0 ? i : 0] : xr[i * 32 + lane], f);
-      unpack8(MODE == 0 ? dv[MODE == 0 ? i : 0] : dr[i * 32 + lane], d);
-      unpack8(gr[i * 32 + lane], g);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xh = (f[j] - mean) * rstd;
-        const float dxh = d[j] * g[j];
-        c1 += dxh;
-        c2 += dxh * xh;
-        if (MODE <= 1) dg[MODE <= 1 ? i : 0][j] += d[j] * xh;
-        if (MODE == 0) db[MODE == 0 ? i : 0][j] += d[j];
-      }
-    }
-    c1 = rms ? 0.f : warp_sum(c1) * (1.f / D);
-    c2 = warp_sum(c2) * (1.f / D);
-    uint4* dxr = reinterpret_cast<uint4*>(dx + (long long)row * D);
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      float f[8], d[8], g[8], o[8];
-      unpack8(MODE == 0 ? xv[MODE == 0 ? i : 0] : xr[i * 32 + lane], f);
-      unpack8(MODE == 0 ? dv[MODE == 0 ? i : 0] : dr[i * 32 + lane], d);
-      unpack8(gr[i * 32 + lane], g);
-      const int col = (i * 32 + lane) * 8;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xh = (f[j] - mean) * rstd;
-        o[j] = rstd * (d[j] * g[j] - c1 - xh * c2);
-        if (MODE == 2) {
-          atomicAdd(&acc[col + j], d[j] * xh);
-          if (!rms) atomicAdd(&acc[D + col + j], d[j]);
-        }
-        if (MODE == 1 && !rms) atomicAdd(&acc[D + col + j], d[j]);
-      }
-      if (dx_add) {
-        float e[8];
-        unpack8(reinterpret_cast<const uint4*>(dx_add + (long long)row * D)[i * 32 + lane], e);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += e[j];
-      }
-      dxr[i * 32 + lane] = pack8(o);
-    }
-  }
-  if (MODE <= 1) {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int col = (i * 32 + lane) * 8;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        atomicAdd(&acc[col + j], dg[MODE <= 1 ? i : 0][j]);
-        if (MODE == 0 && !rms) atomicAdd(&acc[D + col + j], db[MODE == 0 ? i : 0][j]);
-      }
-    }
-  }
-  __syncthreads();
-  float* po = partials + (long long)blockIdx.x * 2 * D;
-  for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) po[i] = acc[i];
-}
-
-// Backward for D = NVT * 2048 (the model widths 2048 and 4096): a CTA of 256 threads owns
-// R rows at a time and every thread a fixed set of 8 * NVT columns, so gamma sits in registers as
-// fp32, the gamma / beta gradient partials need only 16 * NVT registers, and R rows of x and dy
-// (R * 12 KB per CTA at D = 2048) are in flight per CTA while several CTAs share an SM. The two row
-// sums meet across the eight warps through a double-buffered shared array: one barrier per R rows.
-template <int NVT, int R>
-__global__ void __launch_bounds__(256, 2)
+// Backward for D = 256, 512, 1024, 2048 and 4096: 2048 columns' worth of rows side by side (GROUPS rows of D = 2048 / GROUPS,
+// or a row of D = NVT * 2048), a CTA of 256 threads, every thread with a fixed set of 8 * NVT columns, so that gamma and the
+// gamma / beta gradient partials sit in registers. R rows of x, dy and the skip gradient are summed and written while the next
+// R are in flight. The two row sums meet across the warps of a row through a double-buffered shared array: one barrier per R
+// rows. NORM_BWD_FIGURES
+template <int NVT, int R, int GROUPS, bool RMS, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
 norm_bwd_cta_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                     const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                     const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                    float* __restrict__ partials /* [grid, 2, D] */, int rows, int rms,
+                    float* __restrict__ partials /* [grid, 2, D] */, int rows,
                     const __nv_bfloat16* __restrict__ dx_add /* optional: added to dx */) {
-  constexpr int D = NVT * 2048;
-  __shared__ float red[2][8][2 * R];
+  static_assert(NVT == 1 || GROUPS == 1, "a row is either shared by the CTA or a group's own");
+  // threads and warps of a row: THREADS != 256 stands for any number of up to THREADS threads, all of them on one row
+  const int TPR = THREADS == 256 ? 256 / GROUPS : (int)blockDim.x, WPR = TPR / 32, D = NVT * 8 * TPR;
+  __shared__ float red[2][THREADS / 32][2 * R];
+  __shared__ float fold[GROUPS > 1 ? 2 * 2048 / GROUPS : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float g[NVT][8], dg[NVT][8], db[NVT][8];
+  const int grp = tid / TPR, col = tid % TPR, warp0 = grp * WPR;
+  uint4 gv[NVT];
+  float dg[NVT][8], db[RMS ? 1 : NVT][8];
 #pragma unroll
   for (int v = 0; v < NVT; ++v) {
-    unpack8(reinterpret_cast<const uint4*>(gamma)[v * 256 + tid], g[v]);
+    gv[v] = reinterpret_cast<const uint4*>(gamma)[v * TPR + col];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dg[v][j] = db[v][j] = 0.f;
+    for (int j = 0; j < 8; ++j) {
+      dg[v][j] = 0.f;
+      if (!RMS) db[RMS ? 0 : v][j] = 0.f;
+    }
   }
-  const float inv_d = 1.f / D;
-  int buf = 0;
-  for (int row0 = blockIdx.x * R; row0 < rows; row0 += gridDim.x * R, buf ^= 1) {
+  const float inv_d = 1.f / (float)D;
+  uint4 nx[R][NVT], nd[R][NVT], ne[R][NVT];
+  float nmean[R], nrstd[R];
+  const int step = gridDim.x * GROUPS * R;
+  auto load = [&](int row0) {                  // rows past the end: the last row, with a gradient of zero
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool ok = row0 + r < rows;
+      const int row = ok ? row0 + r : rows - 1;
+      const long long base = (long long)row * (D / 8);
+#pragma unroll
+      for (int v = 0; v < NVT; ++v) {
+        nx[r][v] = reinterpret_cast<const uint4*>(x)[base + v * TPR + col];
+        nd[r][v] = ok ? reinterpret_cast<const uint4*>(dy)[base + v * TPR + col] : make_uint4(0, 0, 0, 0);
+        ne[r][v] = dx_add ? reinterpret_cast<const uint4*>(dx_add)[base + v * TPR + col] : make_uint4(0, 0, 0, 0);
+      }
+      nmean[r] = RMS ? 0.f : mean_in[row];
+      nrstd[r] = rstd_in[row];
+    }
+  };
+  int row0 = (blockIdx.x * GROUPS + grp) * R, buf = 0;
+  load(row0);
+  // every group makes the CTA's number of rounds: they meet at its barrier
+  for (int first = blockIdx.x * GROUPS * R; first < rows; first += step, row0 += step, buf ^= 1) {
     uint4 xv[R][NVT], dv[R][NVT], ev[R][NVT];
     float mean[R], rstd[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const bool ok = row0 + r < rows;
-      const long long base = (long long)(ok ? row0 + r : row0) * (D / 8);
 #pragma unroll
       for (int v = 0; v < NVT; ++v) {
-        xv[r][v] = reinterpret_cast<const uint4*>(x)[base + v * 256 + tid];
-        dv[r][v] = ok ? reinterpret_cast<const uint4*>(dy)[base + v * 256 + tid] : make_uint4(0, 0, 0, 0);
-        ev[r][v] = dx_add ? reinterpret_cast<const uint4*>(dx_add)[base + v * 256 + tid] : make_uint4(0, 0, 0, 0);
+        xv[r][v] = nx[r][v];
+        dv[r][v] = nd[r][v];
+        ev[r][v] = ne[r][v];
       }
-      mean[r] = rms ? 0.f : mean_in[ok ? row0 + r : row0];
-      rstd[r] = rstd_in[ok ? row0 + r : row0];
+      mean[r] = nmean[r];
+      rstd[r] = nrstd[r];
     }
+    if (first + step < rows) load(row0 + step);
     float c[2 * R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -459,20 +379,21 @@ norm_bwd_cta_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
       const float nm = -mean[r] * rstd[r];
 #pragma unroll
       for (int v = 0; v < NVT; ++v) {
-        float f[8], d[8];
+        float f[8], d[8], g[8];
         unpack8(xv[r][v], f);
         unpack8(dv[r][v], d);
+        unpack8(gv[v], g);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float xh = fmaf(f[j], rstd[r], nm);
-          const float dxh = d[j] * g[v][j];
+          const float dxh = d[j] * g[j];
           c1 += dxh;
           c2 = fmaf(dxh, xh, c2);
           dg[v][j] = fmaf(d[j], xh, dg[v][j]);
-          db[v][j] += d[j];
+          if (!RMS) db[RMS ? 0 : v][j] += d[j];
         }
       }
-      c[2 * r] = warp_sum(c1);
+      c[2 * r] = RMS ? 0.f : warp_sum(c1);
       c[2 * r + 1] = warp_sum(c2);
     }
     if (lane < 2 * R) {
@@ -485,39 +406,69 @@ norm_bwd_cta_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
 #pragma unroll
     for (int k = 0; k < 2 * R; ++k) {
       float t = 0.f;
+      if (THREADS == 256) {
 #pragma unroll
-      for (int w = 0; w < 8; ++w) t += red[buf][w][k];
+        for (int w = 0; w < 8 / GROUPS; ++w) t += red[buf][warp0 + w][k];
+      } else {
+        t = warp_sum(lane < WPR ? red[buf][lane][k] : 0.f);
+      }
       c[k] = t * inv_d;
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (row0 + r >= rows) break;
-      const float c1 = rms ? 0.f : c[2 * r], c2 = c[2 * r + 1];
+      const float c1 = RMS ? 0.f : c[2 * r], c2 = c[2 * r + 1];
       const float nm = -mean[r] * rstd[r];
 #pragma unroll
       for (int v = 0; v < NVT; ++v) {
-        float f[8], d[8], e[8], o[8];
+        float f[8], d[8], e[8], g[8], o[8];
         unpack8(xv[r][v], f);
         unpack8(dv[r][v], d);
         unpack8(ev[r][v], e);
+        unpack8(gv[v], g);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float xh = fmaf(f[j], rstd[r], nm);
-          o[j] = fmaf(rstd[r], fmaf(d[j], g[v][j], -c1) - xh * c2, e[j]);
+          o[j] = fmaf(rstd[r], fmaf(d[j], g[j], -c1) - xh * c2, e[j]);
         }
-        reinterpret_cast<uint4*>(dx)[(long long)(row0 + r) * (D / 8) + v * 256 + tid] = pack8(o);
+        reinterpret_cast<uint4*>(dx)[(long long)(row0 + r) * (D / 8) + v * TPR + col] = pack8(o);
       }
     }
+  }
+  // the groups' partial sums of a column, one group after the other
+  if (GROUPS > 1) {
+#pragma unroll 1
+    for (int k = 1; k < GROUPS; ++k) {
+      __syncthreads();
+      if (grp == k) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          fold[j * TPR + col] = dg[0][j];
+          if (!RMS) fold[D + j * TPR + col] = db[0][j];
+        }
+      }
+      __syncthreads();
+      if (grp == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          dg[0][j] += fold[j * TPR + col];
+          if (!RMS) db[0][j] += fold[D + j * TPR + col];
+        }
+      }
+    }
+    if (grp != 0) return;
   }
   float* po = partials + (long long)blockIdx.x * 2 * D;
 #pragma unroll
   for (int v = 0; v < NVT; ++v) {
-    float4* pg = reinterpret_cast<float4*>(po + (v * 256 + tid) * 8);
-    float4* pb = reinterpret_cast<float4*>(po + D + (v * 256 + tid) * 8);
+    float4* pg = reinterpret_cast<float4*>(po + (v * TPR + col) * 8);
     pg[0] = make_float4(dg[v][0], dg[v][1], dg[v][2], dg[v][3]);
     pg[1] = make_float4(dg[v][4], dg[v][5], dg[v][6], dg[v][7]);
-    pb[0] = make_float4(db[v][0], db[v][1], db[v][2], db[v][3]);
-    pb[1] = make_float4(db[v][4], db[v][5], db[v][6], db[v][7]);
+    if (!RMS) {
+      float4* pb = reinterpret_cast<float4*>(po + D + (v * TPR + col) * 8);
+      pb[0] = make_float4(db[RMS ? 0 : v][0], db[RMS ? 0 : v][1], db[RMS ? 0 : v][2], db[RMS ? 0 : v][3]);
+      pb[1] = make_float4(db[RMS ? 0 : v][4], db[RMS ? 0 : v][5], db[RMS ? 0 : v][6], db[RMS ? 0 : v][7]);
+    }
   }
 }
 
@@ -575,28 +526,6 @@ static int launch_fwd(const void* x, const void* g, const void* b, void* y, floa
                             static_cast<const __nv_bfloat16*>(g), static_cast<const __nv_bfloat16*>(b), static_cast<__nv_bfloat16*>(y), mean,
                             rstd, rows, eps, rms, grid, zero, n_zero));
   count_launch();
-  return 0;
-}
-
-template <int NV>
-static int launch_bwd(const void* x, const void* dy, const void* g, const float* mean, const float* rstd, void* dx,
-                      float* partials, int grid, int rows, int rms, const void* dx_add, cudaStream_t st) {
-  constexpr int smem = 2 * NV * 256 * 4;
-  constexpr int MODE = NV <= 8 ? 0 : (NV <= 20 ? 1 : 2);
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (smem > 48 * 1024 && !attr_set[dev & 63]) {
-    MLF_CHECK_CUDA(cudaFuncSetAttribute(norm_bwd_kernel<NV, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr_set[dev & 63] = true;
-  }
-  norm_bwd_kernel<NV, MODE><<<grid, 256, smem, st>>>(static_cast<const __nv_bfloat16*>(x),
-                                               static_cast<const __nv_bfloat16*>(dy),
-                                               static_cast<const __nv_bfloat16*>(g), mean, rstd,
-                                               static_cast<__nv_bfloat16*>(dx), partials, rows, rms,
-                                               static_cast<const __nv_bfloat16*>(dx_add));
-                                               count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -664,20 +593,16 @@ MLF_API int mlf_norm_fwd(const void* x, const void* gamma, const void* beta, voi
   return mlf_norm_fwd_zero(x, gamma, beta, y, mean, rstd, rows, D, eps, rms, nullptr, 0, stream);
 }
 
-// CTAs of the backward kernel: whole-CTA rows for the wide model dimensions, warp rows otherwise.
-static int norm_bwd_grid(int rows, int D, bool* cta_rows) {
-  const bool wide = D == 2048 || D == 4096;
-  if (cta_rows) *cta_rows = wide;
-  if (wide) {
-    const int r = D == 2048 ? 4 : 2;
-    return min((rows + r - 1) / r, 2 * sm_count());
-  }
-  return min((rows + 7) / 8, sm_count());
+// Rows that a CTA of the backward takes at a time, and how many CTAs there are: as many as an SM holds.
+static int norm_bwd_rows(int D) { return D == 4096 || D > 4096 ? 1 : D == 256 || D == 512 || D == 1024 ? 2 * (2048 / D) : 2; }
+static int norm_bwd_grid(int rows, int D) {
+  const int r = norm_bwd_rows(D), per_sm = D == 768 ? 5 : D == 1536 ? 2 : D == 3072 || D > 4096 ? 1 : 2;
+  return min((rows + r - 1) / r, per_sm * sm_count());
 }
 
 // Number of fp32 elements the caller must provide as `partials` scratch for mlf_norm_bwd.
 MLF_API long long mlf_norm_bwd_scratch_elems(int rows, int D) {
-  return (long long)norm_bwd_grid(rows, D, nullptr) * 2 * D;
+  return (long long)norm_bwd_grid(rows, D) * 2 * D;
 }
 
 // dx_add (optional, bf16 [rows, D]) is added to dx: the gradient arriving over a skip connection that
@@ -687,32 +612,29 @@ MLF_API int mlf_norm_bwd_add(const void* x, const void* dy, const void* gamma, c
                              int grads_fp32, int accumulate, const void* dx_add, uint64_t stream) {
   MLF_REQUIRE(D % 256 == 0, "norm: D=%d must be a multiple of 256", D);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  bool cta_rows = false;
-  const int grid = norm_bwd_grid(rows, D, &cta_rows);
-  int rc = -2;
-  bool matched = true;
-  if (cta_rows) {
-    const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
-    const __nv_bfloat16* dyp = static_cast<const __nv_bfloat16*>(dy);
-    const __nv_bfloat16* gp = static_cast<const __nv_bfloat16*>(gamma);
-    __nv_bfloat16* dxp = static_cast<__nv_bfloat16*>(dx);
-    const __nv_bfloat16* addp = static_cast<const __nv_bfloat16*>(dx_add);
-    switch (D / 2048) {
-      case 1: norm_bwd_cta_kernel<1, 4><<<grid, 256, 0, st>>>(xp, dyp, gp, mean, rstd, dxp, partials, rows, rms, addp); break;
-      default: norm_bwd_cta_kernel<2, 2><<<grid, 256, 0, st>>>(xp, dyp, gp, mean, rstd, dxp, partials, rows, rms, addp); break;
-    }
-    count_launch();
-    MLF_CHECK_CUDA(cudaGetLastError());
-    rc = 0;
-  } else
-  switch (D / 256) {
-#define CASE(NV) case NV: rc = launch_bwd<NV>(x, dy, gamma, mean, rstd, dx, partials, grid, rows, rms, dx_add, st); break;
-    CASE(1) CASE(2) CASE(3) CASE(4) CASE(6) CASE(8) CASE(12) CASE(16) CASE(20) CASE(24) CASE(32)
-#undef CASE
-    default: matched = false;
+  const int grid = norm_bwd_grid(rows, D);
+  const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
+  const __nv_bfloat16* dyp = static_cast<const __nv_bfloat16*>(dy);
+  const __nv_bfloat16* gp = static_cast<const __nv_bfloat16*>(gamma);
+  __nv_bfloat16* dxp = static_cast<__nv_bfloat16*>(dx);
+  const __nv_bfloat16* addp = static_cast<const __nv_bfloat16*>(dx_add);
+#define LAUNCH(NVT, R, GROUPS, THREADS, BLOCK)                                                                             \
+  if (rms) norm_bwd_cta_kernel<NVT, R, GROUPS, true, THREADS><<<grid, BLOCK, 0, st>>>(xp, dyp, gp, mean, rstd, dxp, partials, rows, addp); \
+  else norm_bwd_cta_kernel<NVT, R, GROUPS, false, THREADS><<<grid, BLOCK, 0, st>>>(xp, dyp, gp, mean, rstd, dxp, partials, rows, addp);    \
+  break;
+  switch (D) {
+    case 256: LAUNCH(1, 2, 8, 256, 256)
+    case 512: LAUNCH(1, 2, 4, 256, 256)
+    case 1024: LAUNCH(1, 2, 2, 256, 256)
+    case 2048: LAUNCH(1, 2, 1, 256, 256)
+    case 4096: LAUNCH(2, 1, 1, 256, 256)
+    case 768: case 1536: case 3072: LAUNCH(1, 2, 1, 384, D / 8)
+    case 5120: case 6144: case 8192: LAUNCH(1, 1, 1, 1024, D / 8)
+    default: MLF_REQUIRE(false, "norm: unsupported D=%d", D);
   }
-  MLF_REQUIRE(matched, "norm: unsupported D=%d", D);
-  if (rc) return rc;
+#undef LAUNCH
+  count_launch();
+  MLF_CHECK_CUDA(cudaGetLastError());
   norm_bwd_finalize_kernel<<<(D + 31) / 32, NF_WARPS * 32, 0, st>>>(partials, grid, D, dgamma, rms ? nullptr : dbeta,
                                                             grads_fp32, accumulate);
                                                             count_launch();
