@@ -52,11 +52,16 @@ struct FlashBwdParams {
   int* err;
 };
 
-// delta[b, h, s] = sum_d dO[t, h, d] * O[t, h, d] (and lse2, the logsumexp in the log2 domain), rows of pitch Sp; one warp
-// per (token, head), two such rows per warp in flight.
+// delta[b, h, s] = sum_d dO[t, h, d] * O[t, h, d] (and lse2, the logsumexp in the log2 domain), rows of pitch Sp, and the fp32
+// dQ accumulator's row cleared in the same pass. Half a warp per (token, head), 16 bytes a lane, four rows in flight: one warp
+// a row, 8 bytes a lane and two rows, behind a memset of its own, took 50 us where 134 MB (4 x 2048 tokens, 16 heads) take 20
+// at the copy rate.
+constexpr int DELTA_ROWS = 4;
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout, float* delta, const float* lse, float* lse2, int B, int S, int Sp,
-                  int H, long long ldo, long long lddo) {
+attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout, float* delta, const float* lse, float* lse2, float* dq_accum, int B,
+                  int S, int Sp, int H, long long ldo, long long lddo) {
+  pdl_trigger();
+  pdl_wait();
   const int pad = Sp - S;                      // statistics past the end of a sequence are zero
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)B * H * pad; i += (long long)gridDim.x * blockDim.x) {
     const long long at = i / pad * Sp + S + i % pad;
@@ -64,32 +69,43 @@ attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout, float* delt
     if (lse2) lse2[at] = 0.f;
   }
   const long long total = (long long)B * S * H;
-  const int lane = threadIdx.x & 31;
+  const int half = (threadIdx.x >> 4) & 1, lane = threadIdx.x & 15;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long w0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w0 < total; w0 += 2 * nwarps) {
-    const long long w1 = w0 + nwarps;
-    const bool two = w1 < total;
-    const long long t0 = w0 / H, t1 = two ? w1 / H : t0;
-    const int h0 = (int)(w0 % H), h1 = two ? (int)(w1 % H) : h0;
-    const uint2 a0v = *reinterpret_cast<const uint2*>(o + t0 * ldo + h0 * FB_D + lane * 4);
-    const uint2 g0v = *reinterpret_cast<const uint2*>(dout + t0 * lddo + h0 * FB_D + lane * 4);
-    const uint2 a1v = *reinterpret_cast<const uint2*>(o + t1 * ldo + h1 * FB_D + lane * 4);
-    const uint2 g1v = *reinterpret_cast<const uint2*>(dout + t1 * lddo + h1 * FB_D + lane * 4);
-    float2 p0 = unpack_bf16x2(a0v.x), p1 = unpack_bf16x2(a0v.y), q0 = unpack_bf16x2(g0v.x), q1 = unpack_bf16x2(g0v.y);
-    float s0 = p0.x * q0.x + p0.y * q0.y + p1.x * q1.x + p1.y * q1.y;
-    p0 = unpack_bf16x2(a1v.x); p1 = unpack_bf16x2(a1v.y); q0 = unpack_bf16x2(g1v.x); q1 = unpack_bf16x2(g1v.y);
-    float s1 = p0.x * q0.x + p0.y * q0.y + p1.x * q1.x + p1.y * q1.y;
+  // rows 2 w and 2 w + 1 belong to a warp: neighbouring heads of a token, the same number of rounds for both halves
+  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); 2 * w < total; w += DELTA_ROWS * nwarps) {
+    uint4 a[DELTA_ROWS], g[DELTA_ROWS];
+    long long t[DELTA_ROWS];
+    int h[DELTA_ROWS];
+    bool ok[DELTA_ROWS];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      s0 += __shfl_xor_sync(0xffffffffu, s0, off);
-      s1 += __shfl_xor_sync(0xffffffffu, s1, off);
+    for (int k = 0; k < DELTA_ROWS; ++k) {
+      const long long row = 2 * (w + k * nwarps) + half;
+      ok[k] = row < total;
+      t[k] = ok[k] ? row / H : 0;
+      h[k] = ok[k] ? (int)(row - t[k] * H) : 0;
+      a[k] = *reinterpret_cast<const uint4*>(o + t[k] * ldo + h[k] * FB_D + lane * 8);
+      g[k] = *reinterpret_cast<const uint4*>(dout + t[k] * lddo + h[k] * FB_D + lane * 8);
     }
-    if (lane < 2 && (lane == 0 || two)) {
-      const long long t = lane ? t1 : t0;
-      const int h = lane ? h1 : h0;
-      const long long b = t / S, sidx = t % S;
-      delta[(b * H + h) * Sp + sidx] = lane ? s1 : s0;
-      if (lse2) lse2[(b * H + h) * Sp + sidx] = lse[(b * H + h) * S + sidx] * 1.4426950408889634f;
+#pragma unroll
+    for (int k = 0; k < DELTA_ROWS; ++k) {
+      const uint32_t* x = reinterpret_cast<const uint32_t*>(&a[k]);
+      const uint32_t* y = reinterpret_cast<const uint32_t*>(&g[k]);
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 p = unpack_bf16x2(x[j]), q = unpack_bf16x2(y[j]);
+        sum += p.x * q.x + p.y * q.y;
+      }
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+      if (!ok[k]) continue;
+      float4* z = reinterpret_cast<float4*>(dq_accum + (t[k] * H + h[k]) * FB_D);
+      z[lane] = z[lane + 16] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (lane == 0) {
+        const long long b = t[k] / S, at = (b * H + h[k]) * Sp + t[k] - b * S;
+        delta[at] = sum;
+        if (lse2) lse2[at] = lse[(b * H + h[k]) * S + t[k] - b * S] * 1.4426950408889634f;
+      }
     }
   }
 }
@@ -99,6 +115,8 @@ __global__ void __launch_bounds__(256)
 cast_rows_f32_bf16_kernel(__nv_bfloat16* out, const float* in, long long rows, int cols, long long ldo, long long ldi) {
   const int vpr = cols / 4;
   const long long total = rows * vpr;
+  pdl_trigger();
+  pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / vpr;
     const int c = (int)(i % vpr) * 4;
@@ -418,18 +436,18 @@ MLF_API int mlf_flash_bwd(const void* q, const void* k, const void* v, const voi
   const int Sp = stat_pitch(S);
   float* lse2 = delta + (long long)B * Hq * Sp;
   const bool use_ws = g_flash_bwd_ws && S >= 128 && ((reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(lse2)) & 15) == 0;
-  MLF_CHECK_CUDA(cudaMemsetAsync(dq_accum, 0, sizeof(float) * rows * Hq * FB_D, st));
+  MLF_REQUIRE((reinterpret_cast<uintptr_t>(dq_accum) & 15) == 0, "flash_bwd: scratch must be 16-byte aligned");
   {
     MLF_REQUIRE(((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15) == 0 && ldo % 8 == 0 && lddo % 8 == 0,
                 "flash_bwd: O and dO must be 16-byte aligned with pitches that are multiples of 8");
-    const long long warps = rows * Hq;
-    long long grid = (warps + 7) / 8;
-    const long long cap = (long long)sm_count() * 8;
+    const long long warps = (rows * Hq + 1) / 2;
+    long long grid = (warps + 8 * DELTA_ROWS - 1) / (8 * DELTA_ROWS);
+    const long long cap = (long long)sm_count() * 4;
     if (grid > cap) grid = cap;
-    attn_delta_kernel<<<(int)grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout),
-                                                 delta, lse, use_ws ? lse2 : nullptr, B, S, use_ws ? Sp : S, Hq, ldo, lddo);
-                                                 count_launch();
-    MLF_CHECK_CUDA(cudaGetLastError());
+    MLF_CHECK_CUDA(launch_pdl(attn_delta_kernel, dim3((unsigned)grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(o),
+                              static_cast<const __nv_bfloat16*>(dout), delta, lse, use_ws ? lse2 : (float*)nullptr, dq_accum, B, S,
+                              use_ws ? Sp : S, Hq, ldo, lddo));
+    count_launch();
   }
   CUtensorMap tq, tk, tv, tdo;
   int rc;
@@ -473,10 +491,9 @@ MLF_API int mlf_flash_bwd(const void* q, const void* k, const void* v, const voi
     long long g = (total + 255) / 256;
     const long long cap = (long long)sm_count() * 8;
     if (g > cap) g = cap;
-    cast_rows_f32_bf16_kernel<<<(int)g, 256, 0, st>>>(static_cast<__nv_bfloat16*>(dq), dq_accum, rows, Hq * FB_D, lddq,
-                                                      (long long)Hq * FB_D);
-                                                      count_launch();
-    MLF_CHECK_CUDA(cudaGetLastError());
+    MLF_CHECK_CUDA(launch_pdl(cast_rows_f32_bf16_kernel, dim3((unsigned)g), dim3(256), 0, st, static_cast<__nv_bfloat16*>(dq),
+                              (const float*)dq_accum, rows, Hq * FB_D, lddq, (long long)Hq * FB_D));
+    count_launch();
   }
   return 0;
 }

@@ -21,6 +21,10 @@
 // Bound by the chain dS -> dK, dQ -> dQ read-out -> dP^T -> dS of a tile: without any of the compute
 // warpgroups' arithmetic 4 x 2048, 16 heads takes 268 us. A second compute warpgroup and paired fp32
 // arithmetic shorten their link: 315 -> 300 us; 2 x 4096, 32 / 8 heads 891 -> 862 us.
+// Around the chain: a CTA's first S^T waits for K and Q only, dK and dV leave through the copy engine, only the blocks that
+// the mask cuts for a warp are masked, and the launch overlaps the end of the one before. With the statistics' pass
+// (attn_delta_kernel), all launches of a backward: 4 x 2048, 16 heads 302 -> 274 us; 2 x 4096, 32 / 8 heads 855 -> 840 us;
+// 3 x 777, 8 heads 56 -> 42 us; 8 x 512, 16 heads 107 -> 86 us (dQ ahead of dK: 275, 868, 43, 85 us).
 // Issue order on the tensor pipe: dV(i), S^T(i+1), dK(i), dQ(i), dP^T(i+1): the next tile's
 // exponentials run while this tile's gradients are multiplied. The issuing thread polls its barriers:
 // it is on the chain, and a suspended wait wakes late (2 x 4096, 32 / 8 heads: 854 -> 811 us; 4 x 2048,
@@ -36,6 +40,9 @@
 #include "../mlf_api.h"
 
 namespace mlf {
+
+int cached_tmap_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
+                     uint32_t bi, uint32_t bo, bool swizzle = true);
 
 constexpr int G_T = 128;                       // tile edge (keys and queries)
 constexpr int G_D = 128;
@@ -69,7 +76,8 @@ __device__ __forceinline__ void bulk_g2s(uint32_t smem_dst, const void* src, uin
 __global__ void __launch_bounds__(G_THREADS, 1)
 flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                    const __grid_constant__ CUtensorMap tmDQ, const FlashBwdWsParams p) {
+                    const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ CUtensorMap tmDK,
+                    const __grid_constant__ CUtensorMap tmDV, const FlashBwdWsParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const uint32_t sK = sbase;
@@ -80,13 +88,13 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t sStg = sV + 5u * G_TILE;                  // two dQ staging tiles of 4 KB for each of four warps
   const uint32_t sStats = sStg + G_TILE;                    // stage s at + s * G_STATS
   const uint32_t bars = sStats + 2 * G_STATS;
-  // barriers: kv_full, q_full[2], q_empty[2], s_full, dp_full, p_full, ds_full, dq_full, dq_empty, do_full, do_empty
-  const uint32_t kv_full = bars;
+  // barriers: k_full, q_full[2], q_empty[2], s_full, dp_full, p_full, ds_full, dq_full, dq_empty, do_full, do_empty, v_full
+  const uint32_t k_full = bars, v_full = bars + 8u * 13;
   auto q_full = [&](int s) { return bars + 8u * (1 + s); };
   auto q_empty = [&](int s) { return bars + 8u * (3 + s); };
   const uint32_t s_full = bars + 8u * 5, dp_full = bars + 8u * 6, p_full = bars + 8u * 7, ds_full = bars + 8u * 8,
                  dq_full = bars + 8u * 9, dq_empty = bars + 8u * 10, do_full = bars + 8u * 11, do_empty = bars + 8u * 12;
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + (bars - sbase) + 8 * 13);
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + (bars - sbase) + 8 * 14);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -109,7 +117,8 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     return;
   }
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
+    mbar_init(k_full, 1);
+    mbar_init(v_full, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(q_full(s), 1);
       mbar_init(q_empty(s), 1);
@@ -133,6 +142,8 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_trigger();
+  pdl_wait();
   const uint32_t t_dK = tmem_base, t_dV = tmem_base + 128, t_S = tmem_base + 256, t_dP = tmem_base + 384;
 
   if (warp < 4) {
@@ -141,11 +152,9 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // ===================== TMA producer =====================
       if (elect_one()) {
         const int krow = (int)(row_base + k0);
-        mbar_expect_tx(kv_full, 2 * G_TILE);
-        tma_load_2d(sK, &tmK, hkv * G_D, krow, kv_full);
-        tma_load_2d(sK + G_HALF, &tmK, hkv * G_D + 64, krow, kv_full);
-        tma_load_2d(sV, &tmV, hkv * G_D, krow, kv_full);
-        tma_load_2d(sV + G_HALF, &tmV, hkv * G_D + 64, krow, kv_full);
+        mbar_expect_tx(k_full, G_TILE);
+        tma_load_2d(sK, &tmK, hkv * G_D, krow, k_full);
+        tma_load_2d(sK + G_HALF, &tmK, hkv * G_D + 64, krow, k_full);
         for (int it = 0; it < n_it; ++it) {
           const int s = it & 1;
           if (!mbar_wait(q_empty(s), ((it >> 1) & 1) ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) break;
@@ -158,6 +167,11 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tma_load_2d(sQ(s) + G_HALF, &tmQ, h * G_D + 64, qrow, q_full(s));
           bulk_g2s(sStats + s * G_STATS, p.lse2 + sidx, G_T * 4, q_full(s));
           bulk_g2s(sStats + s * G_STATS + G_T * 4, p.delta + sidx, G_T * 4, q_full(s));
+          if (it == 0) {                         // V behind the operands of the first S^T
+            mbar_expect_tx(v_full, G_TILE);
+            tma_load_2d(sV, &tmV, hkv * G_D, krow, v_full);
+            tma_load_2d(sV + G_HALF, &tmV, hkv * G_D + 64, krow, v_full);
+          }
           if (!mbar_wait(do_empty, (it & 1) ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) break;
           mbar_expect_tx(do_full, G_TILE);
           tma_load_2d(sdO, &tmdO, h * G_D, qrow, do_full);
@@ -177,13 +191,13 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             umma_bf16_ss(d_tmem, make_smem_desc_sw128(a + off, 16, 1024), make_smem_desc_sw128(bm + off, 16, 1024), idesc_kk, k != 0);
           }
         };
-        bool ok = mbar_wait_poll(kv_full, 0, abort_flag, p.err, ERR_WAIT_ATTN);
+        bool ok = mbar_wait_poll(k_full, 0, abort_flag, p.err, ERR_WAIT_ATTN);
         if (ok && n_it > 0) ok = mbar_wait_poll(q_full(0), 0, abort_flag, p.err, ERR_WAIT_ATTN);
         if (ok && n_it > 0) {
           tc_fence_after_sync();
           issue_kk(t_S, sK, sQ(0));
           umma_commit(s_full);
-          ok = mbar_wait_poll(do_full, 0, abort_flag, p.err, ERR_WAIT_ATTN);
+          ok = mbar_wait_poll(v_full, 0, abort_flag, p.err, ERR_WAIT_ATTN) && mbar_wait_poll(do_full, 0, abort_flag, p.err, ERR_WAIT_ATTN);
           if (ok) {
             tc_fence_after_sync();
             issue_kk(t_dP, sV, sdO);
@@ -237,7 +251,7 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int qd = warp & 3;
     const int g = (warp - 4) >> 2;             // which 64 query columns
     const int r = qd * 32 + lane;
-    const int kv_i = k0 + r;
+    const int kv_i = k0 + r, kv_w = k0 + qd * 32;     // this thread's key, its warp's first
     const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
     const uint32_t t_Sg = t_S + 64u * g, t_dPg = t_dP + 64u * g;      // P^T of these columns replaces their own S^T
     const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2), scale2 = pack_f32x2(p.scale, p.scale);
@@ -263,12 +277,13 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int c4 = 0; c4 < 8; ++c4)
           asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(ls[2 * c4]), "=l"(ls[2 * c4 + 1]) : "r"(st_addr + (32 * hh + 4 * c4) * 4));
         tmem_wait_ld();
-        if (need_mask) {                       // diagonal / ragged tiles only: masked scores become -inf, exp2 gives 0
+        const int qb = q0 + 64 * g + 32 * hh;
+        if (need_mask && (qb + 32 > p.S || kv_w + 32 > p.S || (p.causal && qb < kv_w + 31))) {
+          // blocks of a diagonal or ragged tile that the mask cuts for this warp: masked scores become -inf, exp2 gives 0
+          const int lo = kv_i >= p.S ? 32 : p.causal ? kv_i - qb : 0, hi = p.S - qb;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int qi = q0 + 64 * g + 32 * hh + i;
-            if (qi >= p.S || kv_i >= p.S || (p.causal && qi < kv_i)) sv[i] = __float_as_uint(-INFINITY);
-          }
+          for (int i = 0; i < 32; ++i)
+            if (i < lo || i >= hi) sv[i] = __float_as_uint(-INFINITY);
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -316,33 +331,63 @@ flash_bwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       tc_fence_before_sync();
       mbar_arrive(ds_full);
     }
-    // the last dq_full also covers the final dV / dK accumulations
-    if (ok && n_it > 0) ok = mbar_wait_warp(dq_full, (n_it - 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN);
+    // with the last Q buffer given back every product has been added up, and nothing reads the Q buffers any more
+    if (ok && n_it > 0) ok = mbar_wait_warp(q_empty((n_it - 1) & 1), ((n_it - 1) >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN);
     if (ok && n_it > 0) {
       tc_fence_after_sync();
-      const bool row_ok = kv_i < p.S;
-      __nv_bfloat16* dk_row = p.dk + (row_base + kv_i) * p.lddk + (long long)hkv * G_D;
-      __nv_bfloat16* dv_row = p.dv + (row_base + kv_i) * p.lddv + (long long)hkv * G_D;
+      if (kv_w + 32 <= p.S) {
+        // The warp's 32 rows of dK and of dV, 64 columns each, leave through the Q buffers and the copy engine: row stores
+        // of 16 bytes a thread were most of the 6000 clocks that a CTA's end took.
 #pragma unroll
-      for (int c = 2 * g; c < 2 * g + 2; ++c) {
-        uint32_t a[32], e[32];
-        tmem_ld_32x32b_x32(t_dK + 32 * c + lane_off, a);
-        tmem_ld_32x32b_x32(t_dV + 32 * c + lane_off, e);
-        tmem_wait_ld();
-        if (row_ok) {
+        for (int o = 0; o < 2; ++o) {
+          uint32_t a[64];
+          tmem_ld_32x32b_x32((o ? t_dV : t_dK) + 64 * g + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&a[0]));
+          tmem_ld_32x32b_x32((o ? t_dV : t_dK) + 64 * g + 32 + lane_off, *reinterpret_cast<uint32_t(*)[32]>(&a[32]));
+          tmem_wait_ld();
+          const uint32_t stg = sQ(o) + g * G_HALF + (uint32_t)qd * 4096u;
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint4 w, x;
-            w.x = pack_bf16x2(__uint_as_float(a[8 * v + 0]), __uint_as_float(a[8 * v + 1]));
-            w.y = pack_bf16x2(__uint_as_float(a[8 * v + 2]), __uint_as_float(a[8 * v + 3]));
-            w.z = pack_bf16x2(__uint_as_float(a[8 * v + 4]), __uint_as_float(a[8 * v + 5]));
-            w.w = pack_bf16x2(__uint_as_float(a[8 * v + 6]), __uint_as_float(a[8 * v + 7]));
-            x.x = pack_bf16x2(__uint_as_float(e[8 * v + 0]), __uint_as_float(e[8 * v + 1]));
-            x.y = pack_bf16x2(__uint_as_float(e[8 * v + 2]), __uint_as_float(e[8 * v + 3]));
-            x.z = pack_bf16x2(__uint_as_float(e[8 * v + 4]), __uint_as_float(e[8 * v + 5]));
-            x.w = pack_bf16x2(__uint_as_float(e[8 * v + 6]), __uint_as_float(e[8 * v + 7]));
-            reinterpret_cast<uint4*>(dk_row + 32 * c)[v] = w;
-            reinterpret_cast<uint4*>(dv_row + 32 * c)[v] = x;
+          for (int v = 0; v < 8; ++v) {
+            const uint32_t addr = stg + lane * 128 + (((uint32_t)v ^ (uint32_t)(lane & 7)) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
+                         "r"(pack_bf16x2(__uint_as_float(a[8 * v + 0]), __uint_as_float(a[8 * v + 1]))),
+                         "r"(pack_bf16x2(__uint_as_float(a[8 * v + 2]), __uint_as_float(a[8 * v + 3]))),
+                         "r"(pack_bf16x2(__uint_as_float(a[8 * v + 4]), __uint_as_float(a[8 * v + 5]))),
+                         "r"(pack_bf16x2(__uint_as_float(a[8 * v + 6]), __uint_as_float(a[8 * v + 7])))
+                         : "memory");
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(o ? &tmDV : &tmDK, stg, hkv * G_D + 64 * g, (int)(row_base + kv_w));
+            tma_store_commit();
+          }
+        }
+        if (lane == 0) tma_store_wait_all<0>();
+      } else {
+        const bool row_ok = kv_i < p.S;
+        __nv_bfloat16* dk_row = p.dk + (row_base + kv_i) * p.lddk + (long long)hkv * G_D;
+        __nv_bfloat16* dv_row = p.dv + (row_base + kv_i) * p.lddv + (long long)hkv * G_D;
+#pragma unroll
+        for (int c = 2 * g; c < 2 * g + 2; ++c) {
+          uint32_t a[32], e[32];
+          tmem_ld_32x32b_x32(t_dK + 32 * c + lane_off, a);
+          tmem_ld_32x32b_x32(t_dV + 32 * c + lane_off, e);
+          tmem_wait_ld();
+          if (row_ok) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              uint4 w, x;
+              w.x = pack_bf16x2(__uint_as_float(a[8 * v + 0]), __uint_as_float(a[8 * v + 1]));
+              w.y = pack_bf16x2(__uint_as_float(a[8 * v + 2]), __uint_as_float(a[8 * v + 3]));
+              w.z = pack_bf16x2(__uint_as_float(a[8 * v + 4]), __uint_as_float(a[8 * v + 5]));
+              w.w = pack_bf16x2(__uint_as_float(a[8 * v + 6]), __uint_as_float(a[8 * v + 7]));
+              x.x = pack_bf16x2(__uint_as_float(e[8 * v + 0]), __uint_as_float(e[8 * v + 1]));
+              x.y = pack_bf16x2(__uint_as_float(e[8 * v + 2]), __uint_as_float(e[8 * v + 3]));
+              x.z = pack_bf16x2(__uint_as_float(e[8 * v + 4]), __uint_as_float(e[8 * v + 5]));
+              x.w = pack_bf16x2(__uint_as_float(e[8 * v + 6]), __uint_as_float(e[8 * v + 7]));
+              reinterpret_cast<uint4*>(dk_row + 32 * c)[v] = w;
+              reinterpret_cast<uint4*>(dv_row + 32 * c)[v] = x;
+            }
           }
         }
       }
@@ -441,10 +486,13 @@ int launch_flash_bwd_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
     const int rc = make_tmap_2d(&tdq, dq_accum, 4, (uint64_t)Hq * G_D, (uint64_t)B * S, (uint64_t)Hq * G_D, 32, 32, true);
     if (rc) return rc;
   }
+  CUtensorMap tdk, tdv;
+  int rc;
+  if ((rc = cached_tmap_bf16(&tdk, dk, (uint64_t)Hkv * G_D, (uint64_t)B * S, (uint64_t)lddk, 64, 32))) return rc;
+  if ((rc = cached_tmap_bf16(&tdv, dv, (uint64_t)Hkv * G_D, (uint64_t)B * S, (uint64_t)lddv, 64, 32))) return rc;
   dim3 grid(((S + G_T - 1) / G_T) * Hkv * B);
-  flash_bwd_ws_kernel<<<grid, G_THREADS, G_SMEM, st>>>(tq, tk, tv, tdo, tdq, p);
+  MLF_CHECK_CUDA(launch_pdl(flash_bwd_ws_kernel, grid, dim3(G_THREADS), G_SMEM, st, tq, tk, tv, tdo, tdq, tdk, tdv, p));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
