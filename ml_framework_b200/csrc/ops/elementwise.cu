@@ -244,9 +244,11 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(__nv_bfloat16* dgu, con
 // fixed, so the result is the same from run to run.
 // ------------------------------------------------------------------------------------------
 constexpr int CS_COLS = 256;     // columns per CTA: a warp reads 512 contiguous bytes of a row
-__global__ void __launch_bounds__(256) colsum_kernel(__nv_bfloat16* __restrict__ db, const __nv_bfloat16* __restrict__ dy,
-                                                     float* __restrict__ part, unsigned int* __restrict__ counters, int M, int N,
+__global__ void __launch_bounds__(256) colsum_kernel(__nv_bfloat16* db, const __nv_bfloat16* dy,
+                                                     float* part, unsigned int* counters, int M, int N,
                                                      long long ld, int rows_per_cta, int accumulate) {
+  pdl_trigger();
+  pdl_wait();
   const int col0 = blockIdx.x * CS_COLS;
   const int r0 = blockIdx.y * rows_per_cta;
   const int r1 = min(M, r0 + rows_per_cta);
@@ -536,10 +538,9 @@ MLF_API int mlf_colsum(void* db, const void* dy, int M, int N, long long ld, voi
   colsum_shape(M, N, col_ctas, row_ctas, rows_per_cta);
   unsigned int* counters = static_cast<unsigned int*>(scratch);
   float* part = reinterpret_cast<float*>(static_cast<char*>(scratch) + (((long long)col_ctas * 4 + 255) / 256) * 256);
-  colsum_kernel<<<dim3(col_ctas, row_ctas), 256, 0, st>>>((__nv_bfloat16*)db, (const __nv_bfloat16*)dy, part, counters, M, N, ld,
-                                                          rows_per_cta, accumulate);
+  MLF_CHECK_CUDA(launch_pdl(colsum_kernel, dim3(col_ctas, row_ctas), dim3(256), 0, st, (__nv_bfloat16*)db, (const __nv_bfloat16*)dy, part,
+                            counters, M, N, ld, rows_per_cta, accumulate));
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 MLF_API int mlf_embedding_fwd(void* out, const long long* ids, const long long* pos, const void* wte, const void* wpe,

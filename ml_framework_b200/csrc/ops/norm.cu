@@ -313,11 +313,11 @@ norm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma, const __
 // 21.5 -> 15.4, 2331 x 3072 73 -> 21.5, 8192 x 5120 RMS 386 -> 79, 8192 x 8192 layer / RMS norm 1232 / 1082 -> 206 / 99 (82).
 template <int NVT, int R, int GROUPS, bool RMS, int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
-norm_bwd_cta_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                    const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                    const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                    float* __restrict__ partials /* [grid, 2, D] */, int rows,
-                    const __nv_bfloat16* __restrict__ dx_add /* optional: added to dx */) {
+norm_bwd_cta_kernel(const __nv_bfloat16* x, const __nv_bfloat16* dy,
+                    const __nv_bfloat16* gamma, const float* mean_in,
+                    const float* rstd_in, __nv_bfloat16* dx,
+                    float* partials /* [grid, 2, D] */, int rows,
+                    const __nv_bfloat16* dx_add /* optional: added to dx */) {
   static_assert(NVT == 1 || GROUPS == 1, "a row is either shared by the CTA or a group's own");
   // threads and warps of a row: THREADS != 256 stands for any number of up to THREADS threads, all of them on one row
   const int TPR = THREADS == 256 ? 256 / GROUPS : (int)blockDim.x, WPR = TPR / 32, D = NVT * 8 * TPR;
@@ -325,6 +325,8 @@ norm_bwd_cta_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
   __shared__ float fold[GROUPS > 1 ? 2 * 2048 / GROUPS : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int grp = tid / TPR, col = tid % TPR, warp0 = grp * WPR;
+  pdl_trigger();
+  pdl_wait();
   uint4 gv[NVT];
   float dg[NVT][8], db[RMS ? 1 : NVT][8];
 #pragma unroll
@@ -478,9 +480,11 @@ norm_bwd_cta_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
 // partial rows: the kernel is pure load latency, so the rows are spread over 32 warps).
 constexpr int NF_WARPS = 32;
 __global__ void __launch_bounds__(NF_WARPS * 32)
-norm_bwd_finalize_kernel(const float* __restrict__ partials, int nparts, int D, void* dgamma, void* dbeta,
+norm_bwd_finalize_kernel(const float* partials, int nparts, int D, void* dgamma, void* dbeta,
                          int out_fp32, int accumulate) {
   __shared__ float sg[NF_WARPS][33], sb[NF_WARPS][33];
+  pdl_trigger();
+  pdl_wait();
   const int cl = threadIdx.x & 31, pl = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cl;
   float g = 0.f, b = 0.f;
@@ -621,9 +625,10 @@ MLF_API int mlf_norm_bwd_add(const void* x, const void* dy, const void* gamma, c
   __nv_bfloat16* dxp = static_cast<__nv_bfloat16*>(dx);
   const __nv_bfloat16* addp = static_cast<const __nv_bfloat16*>(dx_add);
 #define LAUNCH(NVT, R, GROUPS, THREADS, BLOCK)                                                                             \
-  if (rms) norm_bwd_cta_kernel<NVT, R, GROUPS, true, THREADS><<<grid, BLOCK, 0, st>>>(xp, dyp, gp, mean, rstd, dxp, partials, rows, addp); \
-  else norm_bwd_cta_kernel<NVT, R, GROUPS, false, THREADS><<<grid, BLOCK, 0, st>>>(xp, dyp, gp, mean, rstd, dxp, partials, rows, addp);    \
-  break;
+  {                                                                                                                        \
+    const auto kernel = rms ? norm_bwd_cta_kernel<NVT, R, GROUPS, true, THREADS> : norm_bwd_cta_kernel<NVT, R, GROUPS, false, THREADS>; \
+    MLF_CHECK_CUDA(launch_pdl(kernel, dim3(grid), dim3(BLOCK), 0, st, xp, dyp, gp, mean, rstd, dxp, partials, rows, addp));   \
+  } break;
   switch (D) {
     case 256: LAUNCH(1, 2, 8, 256, 256)
     case 512: LAUNCH(1, 2, 4, 256, 256)
@@ -636,11 +641,9 @@ MLF_API int mlf_norm_bwd_add(const void* x, const void* dy, const void* gamma, c
   }
 #undef LAUNCH
   count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
-  norm_bwd_finalize_kernel<<<(D + 31) / 32, NF_WARPS * 32, 0, st>>>(partials, grid, D, dgamma, rms ? nullptr : dbeta,
-                                                            grads_fp32, accumulate);
-                                                            count_launch();
-  MLF_CHECK_CUDA(cudaGetLastError());
+  MLF_CHECK_CUDA(launch_pdl(norm_bwd_finalize_kernel, dim3((D + 31) / 32), dim3(NF_WARPS * 32), 0, st, (const float*)partials, grid, D, dgamma,
+                            rms ? (void*)nullptr : dbeta, grads_fp32, accumulate));
+  count_launch();
   return 0;
 }
 
