@@ -522,11 +522,13 @@ static void colsum_shape(int M, int N, int& col_ctas, int& row_ctas, int& rows_p
   row_ctas = (M + rows_per_cta - 1) / rows_per_cta;
 }
 // Scratch layout of mlf_colsum: ceil(N / 256) counters (uint32, zero before the first use; the kernel
-// leaves them zero), padded to 256 bytes, then row_ctas x N floats of partial sums.
+// leaves them zero), then row_ctas x N floats of partial sums. Matrices of different widths share a buffer, so the counters'
+// part has one size for all of them (up to 512 K columns): a narrower one's partial sums must not land on a wider one's counters.
+static long long colsum_counter_bytes(int col_ctas) { return col_ctas <= 2048 ? 8192 : ((long long)col_ctas * 4 + 255) / 256 * 256; }
 MLF_API long long mlf_colsum_scratch_bytes(int M, int N) {
   int c, r, rp;
   colsum_shape(M, N, c, r, rp);
-  return (((long long)c * 4 + 255) / 256) * 256 + (long long)r * N * 4;
+  return colsum_counter_bytes(c) + (long long)r * N * 4;
 }
 // db (bf16 [N]) = column sums of dy (+ db when accumulate). One launch; calls that share a scratch
 // buffer must be ordered on one stream.
@@ -537,7 +539,7 @@ MLF_API int mlf_colsum(void* db, const void* dy, int M, int N, long long ld, voi
   int col_ctas, row_ctas, rows_per_cta;
   colsum_shape(M, N, col_ctas, row_ctas, rows_per_cta);
   unsigned int* counters = static_cast<unsigned int*>(scratch);
-  float* part = reinterpret_cast<float*>(static_cast<char*>(scratch) + (((long long)col_ctas * 4 + 255) / 256) * 256);
+  float* part = reinterpret_cast<float*>(static_cast<char*>(scratch) + colsum_counter_bytes(col_ctas));
   MLF_CHECK_CUDA(launch_pdl(colsum_kernel, dim3(col_ctas, row_ctas), dim3(256), 0, st, (__nv_bfloat16*)db, (const __nv_bfloat16*)dy, part,
                             counters, M, N, ld, rows_per_cta, accumulate));
   count_launch();
