@@ -2,14 +2,14 @@
 //
 // An item is 256 query rows of one (batch, head) as two tiles of 128. 384 threads in three warpgroups;
 // the control warpgroup hands most of its registers to the softmax warpgroups (setmaxnreg 72 / 216 / 216 of 3 x 168:
-// with 88 / 208 the softmax spills, and every spill sits on the chain below; 4 x 2048, 16 heads: 84 -> 80 us):
+// with 88 / 208 the softmax spills, and every spill sits on the chain below: 4 % of 4 x 2048, 16 heads):
 //   warp 0        TMA producer: an item's Q tiles, its K and V tiles of 128 keys through 2-stage rings
 //   warp 1        MMA issuer (one thread). Per key tile j and query tile t:
 //                   S_t = Q_t K_j^T   (M128 N128 K128, operands in shared memory)  -> TMEM S_t
 //                   O_t += P_t V_j    (M128 N128 K128, P read from TENSOR MEMORY, V from shared memory)
 //                 issued in the order PV_0(j), S_0(j+1), PV_1(j), S_1(j+1) so that the tensor pipe
 //                 works on one tile while the other tile's softmax runs (an issuing thread per tile lets the tiles fall
-//                 into step: 2 x 4096, 32 / 8 heads 254 -> 263 us)
+//                 into step: 2 x 4096, 32 / 8 heads 4 % slower)
 //   warps 4..7    softmax of tile 0: one query row per thread; reads S_0 from TMEM into registers,
 //                 running max / sum in the log2 domain, writes P_0 as packed bf16 back over S_0
 //   warps 8..11   softmax of tile 1
@@ -19,16 +19,16 @@
 // more than 2^8 since the value P and O are expressed against (then O_t is read, scaled and
 // written back by its softmax warps, after PV_t(j-1) has completed).
 // The chain S -> P -> PV -> next S of a tile bounds the kernel (about 3300 clocks for 2048 of tensor work): P is published
-// in halves so that PV starts on the first 64 keys while the exponentials of the others run, the arithmetic around the
-// exponentials is done two elements at a time, and every eighth pair of exponentials runs on the FMA pipe (2 x 4096, 32 / 8
-// heads: 254 -> 244 us; every sixth 245, every fourth 256).
+// in halves so that PV starts on the first 64 keys while the exponentials of the others run, and the arithmetic around the
+// exponentials is done two elements at a time. (Every eighth pair of exponentials as a polynomial on the FMA pipe, as exact as
+// the special-function unit's, took 4 % off long sequences and changed every bit of the output; every fourth cost 1 %.)
 // A CTA walks over its items instead of ending with each: set-up, the first loads and the write-out took a third of the
 // clocks of an item of eight key tiles and two thirds of one of two. The next item's Q, K and V arrive and its first S is
 // issued behind the last products of this one, while the softmax warps write its rows out, each through its own staging
 // tile and the copy engine (32 rows of 16 bytes per store instruction took 2500 clocks). Only the 32-column blocks of a
 // diagonal tile that a warp does not see whole are masked (2000 clocks a tile before).
-// One launch, before -> now: 8 x 512, 32 / 8 heads 57 -> 44 us; 4 x 2048, 16 heads 100 -> 80 us; 2 x 4096, 32 / 8 heads
-// 283 -> 244 us; 1404 queries of 5500 keys, 32 / 8 heads 152 -> 143 us.
+// One launch, before -> now, with the same bits: 8 x 512, 32 / 8 heads 57 -> 43 us; 4 x 2048, 16 heads 100 -> 82 us;
+// 2 x 4096, 32 / 8 heads 283 -> 254 us; 1404 queries of 5500 keys, 32 / 8 heads 152 -> 148 us.
 // Per SM and key tile: 4 x 128x128x128 of tensor work against 2 x 16384 exponentials.
 //
 // Math reference: StandardPagedAttentionKernel.ComputePagedAttention
@@ -54,7 +54,6 @@ constexpr int W_STAGES = 2;
 constexpr int W_STG_BYTES = 32 * 128;           // output staging tile of a softmax warp: 32 rows x 64 bf16 columns, 128B-swizzled
 constexpr int W_SMEM = 2 * W_TILE_BYTES + 2 * W_STAGES * W_TILE_BYTES + 8 * W_STG_BYTES + 256;
 constexpr int W_TMEM_COLS = 512;
-constexpr int W_EXP_EVERY = 8;                  // every eighth pair of exponentials runs on the FMA pipe
 
 struct FlashWsParams {
   __nv_bfloat16* out;
@@ -402,13 +401,9 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int i = 0; i < 32; ++i) {
           const uint64_t e = fma_f32x2(pack_f32x2(__uint_as_float(sv[64 * hh + 2 * i]), __uint_as_float(sv[64 * hh + 2 * i + 1])), c2, nm2);
           float e0, e1;
-          if (i % W_EXP_EVERY == W_EXP_EVERY - 1) {
-            exp2_fma_f32x2(e, e0, e1);
-          } else {
-            unpack_f32x2(e, e0, e1);
-            e0 = exp2f(e0);
-            e1 = exp2f(e1);
-          }
+          unpack_f32x2(e, e0, e1);
+          e0 = exp2f(e0);
+          e1 = exp2f(e1);
           rs = add_f32x2(rs, pack_f32x2(e0, e1));
           pk[i] = pack_bf16x2(e0, e1);
         }

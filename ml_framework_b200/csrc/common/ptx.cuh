@@ -380,36 +380,6 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   return r;
 }
 
-// Maximum that keeps a NaN of either operand.
-__device__ __forceinline__ float fmax_nan(float a, float b) {
-  float d;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
-  return d;
-}
-
-// 2^x of two values on the FMA and integer pipes, for kernels whose exponentials keep the special-function unit busy
-// (16 lanes a clock and SM). x = n + f with n = round(x), |f| <= 1/2; 2^f = 1 + f q(f), q fitted by iteratively weighted
-// least squares to the smallest relative error (1.7e-7 over the interval in fp32 Horner form; ex2.approx: 2.4e-7); 2^n is
-// put together in the exponent field. Everything up to -127 gives 0, a NaN stays one. x must stay below 128.
-__device__ __forceinline__ void exp2_fma_f32x2(uint64_t x, float& e0, float& e1) {
-  const float kRound = 12582912.f;             // 1.5 * 2^23: adding it leaves round(x) in the low mantissa bits
-  const uint64_t round2 = pack_f32x2(kRound, kRound);
-  float x0, x1;
-  unpack_f32x2(x, x0, x1);
-  x = pack_f32x2(fmax_nan(x0, -127.f), fmax_nan(x1, -127.f));
-  const uint64_t t = add_f32x2(x, round2);
-  const uint64_t f = add_f32x2(x, neg_f32x2(add_f32x2(t, neg_f32x2(round2))));
-  uint64_t p = fma_f32x2(f, pack_f32x2(0.001326472731307149f, 0.001326472731307149f), pack_f32x2(0.009671512991189957f, 0.009671512991189957f));
-  p = fma_f32x2(f, p, pack_f32x2(0.05550733581185341f, 0.05550733581185341f));
-  p = fma_f32x2(f, p, pack_f32x2(0.24022242426872253f, 0.24022242426872253f));
-  p = fma_f32x2(f, p, pack_f32x2(0.6931470036506653f, 0.6931470036506653f));
-  p = fma_f32x2(f, p, pack_f32x2(1.f, 1.f));
-  float t0, t1;
-  unpack_f32x2(t, t0, t1);
-  const float s0 = __int_as_float((__float_as_int(t0) << 23) + 0x3f800000), s1 = __int_as_float((__float_as_int(t1) << 23) + 0x3f800000);
-  unpack_f32x2(mul_f32x2(p, pack_f32x2(s0, s1)), e0, e1);
-}
-
 // Three-input maximum (one instruction on sm_100).
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;

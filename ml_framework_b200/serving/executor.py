@@ -56,11 +56,13 @@ class PagedLlamaExecutor:
         self.max_blocks = (self.cfg.max_seq_len + kv.block_size - 1) // kv.block_size
         self.tokens_generated = 0
         self._graphs = None
-        self._prompt_graphs = set()          # names of the graphs that prompts run through
+        self._prompt_graphs = None           # whole prompts: a graph per batch size and bucket of rows
+        self._prompts_seen: Dict[str, int] = {}
         self._ar_calls = 0
         if self.native and self.cfg.use_cuda_graphs and (tp is None or tp.world == 1 or tp.fused):
             from ..hal.cuda_graphs import CaptureOptions, CUDAGraphManager
             self._graphs = CUDAGraphManager(CaptureOptions(warmup_iterations=self.cfg.graph_warmup_steps))
+            self._prompt_graphs = CUDAGraphManager(CaptureOptions(warmup_iterations=0))
 
     # ---- tensor-parallel reduction of partial projections
     def _ar_staging(self, T: int):
@@ -356,11 +358,12 @@ class PagedLlamaExecutor:
         if B * Tp > 512:
             return None
         name = f"prefill_B{B}_T{Tp}"
-        if name not in self._prompt_graphs:
-            if len(self._prompt_graphs) >= 32:
+        if name not in self._prompts_seen:
+            if len(self._prompts_seen) >= 32:
                 return None
-            self._prompt_graphs.add(name)
-        return name
+            self._prompts_seen[name] = 0
+        self._prompts_seen[name] += 1
+        return name if self._prompts_seen[name] > self.cfg.graph_warmup_steps else None      # launch by launch until then
 
     @torch.no_grad()
     def _prefill_graph(self, name: str, reqs: List[Request], n: int) -> Dict[int, int]:
@@ -388,7 +391,7 @@ class PagedLlamaExecutor:
             for li, blk in enumerate(self.m.blocks):
                 x = self._block(li, blk, x, buf[T:2 * T], buf[2 * T:3 * T], attend)
             return self._logits_argmax(x[buf[3 * T:]])
-        toks = self._graphs.run_from_host(name, step, host, self.device).tolist()
+        toks = self._prompt_graphs.run_from_host(name, step, host, self.device).tolist()
         for r in reqs:
             r.prefilled = n
         return {r.id: int(t) for r, t in zip(reqs, toks)}

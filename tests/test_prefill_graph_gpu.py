@@ -41,7 +41,7 @@ def _run(ex, kv, prompts, first_id):
 def test_same_as_launch_by_launch(B, n):
     (ex, kv), (plain, kv2) = _setup(True), _setup(False)
     g = torch.Generator().manual_seed(n)
-    for step in range(5):                     # two warm-up passes, the capture, replays; new prompts each time
+    for step in range(5):                     # two passes launch by launch, the capture, replays; new prompts each time
         prompts = torch.randint(1, 500, (B, n), generator=g).tolist()
         tok, rows = _run(ex, kv, prompts, 10 * step)
         want, want_rows = _run(plain, kv2, prompts, 10 * step)
@@ -51,7 +51,7 @@ def test_same_as_launch_by_launch(B, n):
                 # the second layer's rows follow products that may split K differently for the padded row count: a few
                 # roundings to bf16 of partial sums
                 assert (x - y).norm() <= 2e-2 * y.norm()
-    assert ex._graphs.stats()["replays"] == 3 and ex._graphs.stats()["fallbacks"] == 0
+    assert ex._prompt_graphs.stats() == {"graphs": 1, "replays": 3, "fallbacks": 0}
     assert _lib.read_status() == 0
 
 
@@ -74,7 +74,7 @@ def test_padding_writes_nothing():
 
 def test_graphs_are_bounded_and_long_or_chunked_prompts_are_not_captured():
     ex, kv = _setup(True)
-    ex._prompt_graphs = {f"prefill_B1_T{i}" for i in range(1000, 1032)}
+    ex._prompts_seen = {f"prefill_B1_T{i}": 9 for i in range(1000, 1032)}
     for step in range(4):
         _run(ex, kv, [[1, 2, 3]], step)
     for n in (513, 1025, 1500):
@@ -83,7 +83,7 @@ def test_graphs_are_bounded_and_long_or_chunked_prompts_are_not_captured():
             while r.prefilled < n:
                 ex.execute_batch(Batch([r], prefill=[r]))
             kv.free_sequence_blocks(step)
-    assert len(ex._prompt_graphs) == 32 and ex._graphs.stats()["graphs"] == 0
+    assert len(ex._prompts_seen) == 32 and ex._prompt_graphs.stats()["graphs"] == 0
     small, kv2 = _setup(True, blocks=2)
     with pytest.raises(MemoryError):
         _run(small, kv2, [[1] * 40], 0)
