@@ -8,8 +8,8 @@
 //             each, added)
 // gated = 0: layer norm, biases, tanh-GELU; gated = 1: RMS norm, rotary embedding, SwiGLU over interleaved gate / up rows.
 //
-// A step of two layers of 256 on 2 x 256 tokens, whose kernels take 0.4 ms: 1.88 ms operator by operator, 0.92 ms like this
-// (0.24 ms of it because the engine no longer hands the backward to autograd's device thread).
+// A step of two layers of 256 on 2 x 256 tokens, whose kernels take 0.4 ms: 1.88 ms operator by operator, 0.88 ms like this
+// (0.24 ms of the gain because the engine no longer hands the backward to autograd's device thread).
 #include "../common/host.h"
 #include "../mlf_api.h"
 

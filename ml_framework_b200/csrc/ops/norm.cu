@@ -304,9 +304,9 @@ norm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma, const __
   }
 }
 
-// Backward for D = 256, 512, 1024, 2048 and 4096: 2048 columns' worth of rows side by side (GROUPS rows of D = 2048 / GROUPS,
-// or a row of D = NVT * 2048), a CTA of 256 threads, every thread with a fixed set of 8 * NVT columns, so that gamma and the
-// gamma / beta gradient partials sit in registers. R rows of x, dy and the skip gradient are summed and written while the next
+// Backward. D = 256, 512, 1024, 2048 and 4096: 2048 columns' worth of rows side by side (GROUPS rows of D = 2048 / GROUPS, or a
+// row of D = NVT * 2048), a CTA of 256 threads; other widths: a row to a CTA of as many threads as it has vectors (or every
+// NVT-th). Every thread has a fixed set of 8 * NVT columns, so that gamma and the gamma / beta gradient partials sit in registers. R rows of x, dy and the skip gradient are summed and written while the next
 // R are in flight. The two row sums meet across the warps of a row through a double-buffered shared array: one barrier per R
 // rows.
 // us, before (one warp per row; for 2048 and 4096 no rows in flight ahead) -> now: 8192 x 4096 RMS 69 -> 56 (floor 41), 2331 x 1024
