@@ -392,16 +392,22 @@ class _EmbeddingFn(torch.autograd.Function):
         def one(w, idx):
             if w is None or not w.requires_grad:
                 return None
-            acc = native.embedding_bwd(dout, idx, w.shape[0])
             tgt, accum = _sink(w)
-            if tgt is not None:
-                if tgt.dtype == torch.bfloat16:
-                    native.cast_f32_to_bf16(acc, tgt.view(w.shape), accumulate=accum)
+            out = torch.empty(w.shape, dtype=w.dtype, device=dout.device) if tgt is None else tgt.view(w.shape)
+            # Fewer tokens than rows: a sum per token, in less memory than a table of them. Beyond that the fp32 table is the smaller:
+            # 2331 ids of 2048 x 1024 19.4 us in a table, 17.4 per token, 8192 of 2048 x 2048 40 and 48 us.
+            if out.dtype == dout.dtype == torch.bfloat16 and idx.numel() < w.shape[0] and out.data_ptr() % 16 == 0:
+                native.embedding_grad(dout, idx, out, accum)
+            else:
+                acc = native.embedding_bwd(dout, idx, w.shape[0])
+                if out.dtype == torch.bfloat16:
+                    native.cast_f32_to_bf16(acc, out, accumulate=accum)
                 else:
-                    tgt.view(w.shape).copy_(tgt.view(w.shape) + acc if accum else acc)
-                _done(w)
-                return None
-            return acc.to(w.dtype)
+                    out.copy_(out + acc if accum else acc)
+            if tgt is None:
+                return out
+            _done(w)
+            return None
         dwte = one(wte, ids)
         dwpe = one(wpe, pos) if wpe is not None else None
         return None, dwte, None, dwpe

@@ -207,6 +207,20 @@ def embedding_bwd(dout: torch.Tensor, ids: torch.Tensor, vocab: int, dw_fp32: Op
     return dw_fp32
 
 
+def embedding_grad(dout: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
+    """out[v] (+)= sum of dout's rows with id v, summed in fp32 and rounded once. ``out``: contiguous bf16 [vocab, D],
+    16-byte aligned."""
+    vocab, D = out.shape
+    T = ids.numel()
+    L = _L()
+    L.mlf_embedding_grad_scratch_bytes.restype = C.c_longlong
+    scratch = torch.empty(L.mlf_embedding_grad_scratch_bytes(C.c_longlong(T), D, vocab), dtype=torch.uint8, device=dout.device)
+    rc = L.mlf_embedding_grad(_p(out), _p(dout.reshape(T, D).contiguous()), _p(ids.reshape(-1).contiguous()), _p(scratch),
+                              C.c_longlong(T), D, vocab, int(accumulate), _st())
+    _lib.check(rc, "mlf_embedding_grad")
+    return out
+
+
 def cast_f32_to_bf16(src: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
     _lib.check(_L().mlf_cast_f32_to_bf16(_p(out), _p(src), C.c_longlong(src.numel()), int(accumulate), _st()), "mlf_cast")
     return out
