@@ -27,7 +27,8 @@ int mlf_flash_fwd(const void* q, const void* k, const void* v, void* out, float*
 int mlf_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse, void* dq, void* dk, void* dv,
                   void* scratch, int B, int S, int Hq, int Hkv, long long ldq, long long ldk, long long ldv, long long ldo, long long lddo,
                   long long lddq, long long lddk, long long lddv, float scale, int causal, uint64_t stream);
-int mlf_colsum(void* out, const void* dy, int M, int N, long long ld, void* scratch, int accumulate, uint64_t stream);
+int mlf_colsum2(void* db0, const void* dy0, int N0, long long ld0, int accumulate0, void* db1, const void* dy1, int N1, long long ld1,
+                int accumulate1, int M, void* scratch, uint64_t stream);
 }
 
 namespace {
@@ -82,24 +83,25 @@ MLF_API int mlf_block_backward(const MlfBlockArgs* p, uint64_t st) {
   auto wgrad = [&](const void* dy, const void* x, void* dw, int out, int in, int bit) {
     return product(dy, x, dw, out, in, T, out, in, in, 1, 1, add(bit) ? MLF_EPI_ACCUM : 0, nullptr, nullptr, 0, nullptr, 0, st);
   };
-  auto bgrad = [&](const void* dy, void* db, int n, int bit) { return db == nullptr ? 0 : mlf_colsum(db, dy, T, n, n, p->colsum_scratch, add(bit), st); };
+  // Bias gradients of two products, the column sums of their dY. Layer-norm blocks have all of them, gated ones none.
+  auto bgrads = [&](const void* dy0, void* db0, int bit0, const void* dy1, void* db1, int width1, int bit1) {
+    return db0 == nullptr ? 0 : mlf_colsum2(db0, dy0, d, d, add(bit0), db1, dy1, width1, width1, add(bit1), T, p->colsum_scratch, st);
+  };
   // MLP: dpre, then dh2
   RUN(product(p->dy, p->w2, p->wide, T, p->ff, d, d, p->ff, n1, 0, 1, p->gated ? MLF_EPI_DSWIGLU : MLF_EPI_DGELU_MUL, nullptr, p->pre, n1, nullptr, 0, st));
   RUN(wgrad(p->dy, p->act, p->dw2, d, p->ff, MLF_BLOCK_W2));
-  RUN(bgrad(p->dy, p->dbb2, d, MLF_BLOCK_BB2));
   RUN(wgrad(p->wide, p->h2, p->dw1, n1, d, MLF_BLOCK_W1));
-  RUN(bgrad(p->wide, p->dbb1, n1, MLF_BLOCK_BB1));
+  RUN(bgrads(p->dy, p->dbb2, MLF_BLOCK_BB2, p->wide, p->dbb1, n1, MLF_BLOCK_BB1));
   RUN(product(p->wide, p->w1, p->row, T, d, n1, n1, d, d, 0, 1, 0, nullptr, nullptr, 0, nullptr, 0, st));
   RUN(mlf_norm_bwd_add(p->x1, p->row, p->g2, p->mean2, p->rstd2, p->dx1, p->dg2, p->db2, p->norm_scratch, T, d, p->gated, 0, add(MLF_BLOCK_G2), p->dy, st));
   // attention: da, dqkv (in the MLP's place), then dh1
   RUN(product(p->dx1, p->wo, p->da, T, q, d, d, q, q, 0, 1, 0, nullptr, nullptr, 0, nullptr, 0, st));
   RUN(wgrad(p->dx1, p->a, p->dwo, d, q, MLF_BLOCK_WO));
-  RUN(bgrad(p->dx1, p->dbo, d, MLF_BLOCK_BO));
   RUN(mlf_flash_bwd(p->qkv, at(p->qkv, q), at(p->qkv, q + kv), p->a, p->da, p->lse, p->wide, at(p->wide, q), at(p->wide, q + kv), p->flash_scratch,
                     p->B, p->S, p->Hq, p->Hkv, w, w, w, q, q, w, w, w, p->scale, p->causal, st));
   if (p->pos != nullptr) RUN(mlf_rope_qkv(p->wide, p->wide, p->pos, T, p->Hq, p->Hkv, w, w, p->rope_theta, 1, st));
   RUN(product(p->wide, p->wqkv, p->row, T, d, w, w, d, d, 0, 1, 0, nullptr, nullptr, 0, nullptr, 0, st));
   RUN(wgrad(p->wide, p->h1, p->dwqkv, w, d, MLF_BLOCK_WQKV));
-  RUN(bgrad(p->wide, p->dbqkv, w, MLF_BLOCK_BQKV));
+  RUN(bgrads(p->dx1, p->dbo, MLF_BLOCK_BO, p->wide, p->dbqkv, w, MLF_BLOCK_BQKV));
   return mlf_norm_bwd_add(p->x, p->row, p->g1, p->mean1, p->rstd1, p->dx, p->dg1, p->db1, p->norm_scratch, T, d, p->gated, 0, add(MLF_BLOCK_G1), p->dx1, st);
 }

@@ -237,19 +237,33 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(__nv_bfloat16* dgu, con
 }
 
 // ------------------------------------------------------------------------------------------
-// column sum (bias gradient): db[n] = sum_m dy[m, n]; dy bf16 [M, N] with pitch ld.
+// column sum (bias gradient): db[n] = sum_m dy[m, n]; dy bf16 [M, N] with pitch ld; one matrix, or two of as many rows whose
+// column blocks share the launch (its ramp and its last CTAs' sums weigh as much as
+// the reading of a narrow one; us, cold, two launches -> one: 2331 x (1024 + 4096) 21.5 -> 14.4, 8192 x (2048 + 8192) 50 -> 43).
 // One launch, no atomics on the data: each CTA owns 256 columns x a slab of rows and writes its fp32
-// partial sums to part[slab][N]; the CTA that finishes last for a column block (a counter per block,
+// partial sums to part[slab]; the CTA that finishes last for a column block (a counter per block,
 // reset by that CTA) adds the slabs in slab order and writes bf16. The order of the additions is
 // fixed, so the result is the same from run to run.
 // ------------------------------------------------------------------------------------------
 constexpr int CS_COLS = 256;     // columns per CTA: a warp reads 512 contiguous bytes of a row
-__global__ void __launch_bounds__(256) colsum_kernel(__nv_bfloat16* db, const __nv_bfloat16* dy,
-                                                     float* part, unsigned int* counters, int M, int N,
-                                                     long long ld, int rows_per_cta, int accumulate) {
+struct ColsumMatrix {
+  __nv_bfloat16* db;
+  const __nv_bfloat16* dy;
+  long long ld;
+  int N, accumulate;
+};
+__global__ void __launch_bounds__(256) colsum_kernel(const ColsumMatrix first, const ColsumMatrix second, int first_blocks,
+                                                     float* part, unsigned int* counters, int M, int rows_per_cta) {
   pdl_trigger();
   pdl_wait();
-  const int col0 = blockIdx.x * CS_COLS;
+  const bool in_first = (int)blockIdx.x < first_blocks;
+  __nv_bfloat16* const db = in_first ? first.db : second.db;
+  const __nv_bfloat16* const dy = in_first ? first.dy : second.dy;
+  const long long ld = in_first ? first.ld : second.ld;
+  const int N = in_first ? first.N : second.N;
+  const int accumulate = in_first ? first.accumulate : second.accumulate;
+  part += (long long)blockIdx.x * gridDim.y * CS_COLS;   // this column block's partial sums: [gridDim.y][256]
+  const int col0 = ((int)blockIdx.x - (in_first ? 0 : first_blocks)) * CS_COLS;
   const int r0 = blockIdx.y * rows_per_cta;
   const int r1 = min(M, r0 + rows_per_cta);
   const int cl = (threadIdx.x & 31) * 8;  // 32 threads x 8 columns = 256 columns
@@ -281,7 +295,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(__nv_bfloat16* db, const __
     float t = 0.f;
 #pragma unroll
     for (int r = 0; r < 8; ++r) t += sm[r][threadIdx.x];
-    if (col0 + threadIdx.x < N) part[(long long)blockIdx.y * N + col0 + threadIdx.x] = t;
+    part[blockIdx.y * CS_COLS + threadIdx.x] = t;
   }
   __threadfence();
   __syncthreads();
@@ -291,7 +305,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(__nv_bfloat16* db, const __
   __threadfence();
   if (col0 + threadIdx.x < N) {
     float t = 0.f;
-    for (int y = 0; y < (int)gridDim.y; ++y) t += __ldcg(part + (long long)y * N + col0 + threadIdx.x);
+    for (int y = 0; y < (int)gridDim.y; ++y) t += __ldcg(part + y * CS_COLS + threadIdx.x);
     __nv_bfloat16* o = db + col0 + threadIdx.x;
     *o = __float2bfloat16(t + (accumulate ? __bfloat162float(*o) : 0.f));
   }
@@ -587,37 +601,51 @@ MLF_API int mlf_swiglu_bwd(void* dgu, const void* dout, const void* gu, long lon
   MLF_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
-static void colsum_shape(int M, int N, int& col_ctas, int& row_ctas, int& rows_per_cta) {
-  col_ctas = (N + CS_COLS - 1) / CS_COLS;
+static void colsum_shape(int M, int col_ctas, int& row_ctas, int& rows_per_cta) {
   row_ctas = (sm_count() * 6 + col_ctas - 1) / col_ctas;      // six CTAs fit per SM (40 registers): one full wave
   if (row_ctas > (M + 31) / 32) row_ctas = (M + 31) / 32;
   if (row_ctas < 1) row_ctas = 1;
   rows_per_cta = ((M + row_ctas - 1) / row_ctas + 31) / 32 * 32;
   row_ctas = (M + rows_per_cta - 1) / rows_per_cta;
 }
-// Scratch layout of mlf_colsum: ceil(N / 256) counters (uint32, zero before the first use; the kernel
-// leaves them zero), then row_ctas x N floats of partial sums. Matrices of different widths share a buffer, so the counters'
-// part has one size for all of them (up to 512 K columns): a narrower one's partial sums must not land on a wider one's counters.
+// Scratch layout of mlf_colsum: a counter per 256 columns (uint32, zero before the first use; the kernel
+// leaves them zero), then row_ctas x 256 floats of partial sums for each. Matrices of different widths share a buffer, so the
+// counters' part has one size for all of them (up to 512 K columns): a narrower one's partial sums must not land on a wider
+// one's counters.
+static int colsum_blocks(int N) { return (N + CS_COLS - 1) / CS_COLS; }
 static long long colsum_counter_bytes(int col_ctas) { return col_ctas <= 2048 ? 8192 : ((long long)col_ctas * 4 + 255) / 256 * 256; }
-MLF_API long long mlf_colsum_scratch_bytes(int M, int N) {
-  int c, r, rp;
-  colsum_shape(M, N, c, r, rp);
-  return colsum_counter_bytes(c) + (long long)r * N * 4;
+// N1 > 0: of a launch for two matrices
+MLF_API long long mlf_colsum2_scratch_bytes(int M, int N0, int N1) {
+  const int c = colsum_blocks(N0) + colsum_blocks(N1);
+  int r, rp;
+  colsum_shape(M, c, r, rp);
+  return colsum_counter_bytes(c) + (long long)r * c * CS_COLS * 4;
+}
+MLF_API long long mlf_colsum_scratch_bytes(int M, int N) { return mlf_colsum2_scratch_bytes(M, N, 0); }
+static int colsum_launch(const ColsumMatrix& first, const ColsumMatrix& second, int M, void* scratch, cudaStream_t st) {
+  MLF_REQUIRE(first.ld % 8 == 0 && second.ld % 8 == 0, "colsum: pitch must be a multiple of 8 elements");
+  MLF_REQUIRE(scratch != nullptr && M > 0 && first.N > 0, "colsum: bad arguments");
+  const int first_blocks = colsum_blocks(first.N), col_ctas = first_blocks + colsum_blocks(second.N);
+  int row_ctas, rows_per_cta;
+  colsum_shape(M, col_ctas, row_ctas, rows_per_cta);
+  unsigned int* counters = static_cast<unsigned int*>(scratch);
+  float* part = reinterpret_cast<float*>(static_cast<char*>(scratch) + colsum_counter_bytes(col_ctas));
+  MLF_CHECK_CUDA(launch_pdl(colsum_kernel, dim3(col_ctas, row_ctas), dim3(256), 0, st, first, second, first_blocks, part, counters, M, rows_per_cta));
+  count_launch();
+  return 0;
 }
 // db (bf16 [N]) = column sums of dy (+ db when accumulate). One launch; calls that share a scratch
 // buffer must be ordered on one stream.
 MLF_API int mlf_colsum(void* db, const void* dy, int M, int N, long long ld, void* scratch, int accumulate, uint64_t stream) {
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  MLF_REQUIRE(ld % 8 == 0, "colsum: pitch must be a multiple of 8 elements");
-  MLF_REQUIRE(scratch != nullptr && M > 0 && N > 0, "colsum: bad arguments");
-  int col_ctas, row_ctas, rows_per_cta;
-  colsum_shape(M, N, col_ctas, row_ctas, rows_per_cta);
-  unsigned int* counters = static_cast<unsigned int*>(scratch);
-  float* part = reinterpret_cast<float*>(static_cast<char*>(scratch) + colsum_counter_bytes(col_ctas));
-  MLF_CHECK_CUDA(launch_pdl(colsum_kernel, dim3(col_ctas, row_ctas), dim3(256), 0, st, (__nv_bfloat16*)db, (const __nv_bfloat16*)dy, part,
-                            counters, M, N, ld, rows_per_cta, accumulate));
-  count_launch();
-  return 0;
+  return colsum_launch({(__nv_bfloat16*)db, (const __nv_bfloat16*)dy, ld, N, accumulate}, {nullptr, nullptr, 0, 0, 0}, M, scratch,
+                       reinterpret_cast<cudaStream_t>(stream));
+}
+// Two matrices of M rows in one launch.
+MLF_API int mlf_colsum2(void* db0, const void* dy0, int N0, long long ld0, int accumulate0, void* db1, const void* dy1, int N1, long long ld1,
+                        int accumulate1, int M, void* scratch, uint64_t stream) {
+  MLF_REQUIRE(N1 > 0, "colsum: bad arguments");
+  return colsum_launch({(__nv_bfloat16*)db0, (const __nv_bfloat16*)dy0, ld0, N0, accumulate0},
+                       {(__nv_bfloat16*)db1, (const __nv_bfloat16*)dy1, ld1, N1, accumulate1}, M, scratch, reinterpret_cast<cudaStream_t>(stream));
 }
 MLF_API int mlf_embedding_fwd(void* out, const long long* ids, const long long* pos, const void* wte, const void* wpe,
                               long long T, int D, int vocab, int max_pos, uint64_t stream) {

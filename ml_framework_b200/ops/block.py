@@ -115,7 +115,7 @@ class _BlockFn(torch.autograd.Function):
         L.mlf_norm_bwd_scratch_elems.restype = L.mlf_flash_bwd_scratch_bytes.restype = C.c_longlong
         norm = native.scratch("norm_bwd", L.mlf_norm_bwd_scratch_elems(T, d) * 4, dev)
         flash = native.scratch("flash_bwd", L.mlf_flash_bwd_scratch_bytes(B, S, Hq), dev)
-        col = None if gated else native.colsum_scratch(T, (d, w, n1), dev)
+        col = None if gated else native.colsum_scratch(T, ((d, w), (d, n1)), dev)
         args = _Args(B, S, d, Hq, Hkv, ff, gated, causal, accumulate, eps1, eps2, theta, 128 ** -0.5, *[_ptr(p) for p in params], _ptr(positions),
                      x.data_ptr(), *_BlockFn._saved(rows, stats, T, d, w, q, n1, gated), None, dy.data_ptr(), wp, row,
                      row + 4 * T * d, row + 2 * T * d, dx.data_ptr(), *targets, norm.data_ptr(), _ptr(col), flash.data_ptr())

@@ -162,10 +162,10 @@ def swiglu_bwd(dout: torch.Tensor, gu: torch.Tensor, interleaved: bool = False) 
 
 
 def colsum_scratch(M: int, widths, device) -> torch.Tensor:
-    """Scratch for the column sums of matrices of M rows and each of ``widths`` columns."""
+    """Scratch for column sums of matrices of M rows: launches over ``widths`` columns, of one matrix or (a pair) of two."""
     L = _L()
-    L.mlf_colsum_scratch_bytes.restype = C.c_longlong
-    need = max(int(L.mlf_colsum_scratch_bytes(M, n)) for n in widths)
+    L.mlf_colsum2_scratch_bytes.restype = C.c_longlong
+    need = max(int(L.mlf_colsum2_scratch_bytes(M, *(n if isinstance(n, tuple) else (n, 0)))) for n in widths)
     key = ("colsum0", device.index)
     sc = _scratch.get(key)
     if sc is None or sc.numel() < need:                  # zero-filled once: the kernel keeps its counters at zero
