@@ -602,7 +602,7 @@ MLF_API int mlf_swiglu_bwd(void* dgu, const void* dout, const void* gu, long lon
   return 0;
 }
 static void colsum_shape(int M, int col_ctas, int& row_ctas, int& rows_per_cta) {
-  row_ctas = (sm_count() * 6 + col_ctas - 1) / col_ctas;      // six CTAs fit per SM (40 registers): one full wave
+  row_ctas = (sm_count() * 6 + col_ctas - 1) / col_ctas;      // six CTAs per SM of the eight that fit: one wave
   if (row_ctas > (M + 31) / 32) row_ctas = (M + 31) / 32;
   if (row_ctas < 1) row_ctas = 1;
   rows_per_cta = ((M + row_ctas - 1) / row_ctas + 31) / 32 * 32;
