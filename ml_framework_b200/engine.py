@@ -120,11 +120,12 @@ class TrainEngine:
         flat.zero_grad()
         scale_t = self.scaler.scale_t if self.scaler is not None else None
         # on its own, nothing works on single operators of a block: blocks may be one launch sequence each way, and the
-        # backward runs in this thread (handing every node to the device's autograd thread and back cost 0.24 ms of a step)
+        # backward runs in this thread (handing every node to the device's autograd thread and back cost 0.24 ms of a step).
+        # Blocks that it recomputes take the forward's path: torch's checkpoint wants the same tensors saved both times.
         alone = self.world == 1 and self.reducer is None
         with nvtx_range("forward"), whole_blocks(alone):
             loss = self.model(ids, targets, loss_scale=scale_t)
-        with nvtx_range("backward"), torch.autograd.set_multithreading_enabled(False) if alone else nullcontext():
+        with nvtx_range("backward"), whole_blocks(alone), torch.autograd.set_multithreading_enabled(False) if alone else nullcontext():
             loss.backward()
         flat.gather_missing_grads()
         grad_scale = 1.0

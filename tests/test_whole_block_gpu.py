@@ -5,8 +5,10 @@ import copy
 
 import pytest
 import torch
+import torch.utils.checkpoint
 
 from ml_framework_b200 import _lib
+from ml_framework_b200.engine import EngineConfig, TrainEngine
 from ml_framework_b200.models.gpt import GPT, GPTConfig
 from ml_framework_b200.models.llama import Llama, LlamaConfig
 from ml_framework_b200.ops import block as block_mod
@@ -142,3 +144,35 @@ def test_saved_tensor_hooks_and_in_place_checks(calls):
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         y.backward(dy)
     assert len(calls) == 3
+
+
+class _Recomputed(torch.nn.Module):
+    def __init__(self, inner, reentrant):
+        super().__init__()
+        self.inner, self.reentrant = inner, reentrant
+
+    def forward(self, x):
+        return torch.utils.checkpoint.checkpoint(self.inner, x, use_reentrant=self.reentrant)
+
+
+@pytest.mark.parametrize("kind", ["gpt", "llama"])
+@pytest.mark.parametrize("how", ["torch", "torch reentrant", "package"])
+def test_recomputed_blocks_under_the_engine(kind, how, calls):
+    """What is recomputed in the backward takes the forward's path: torch's checkpoint compares the tensors that both save."""
+    grads, losses = [], []
+    ids, targets = (torch.randint(0, 500, (2, 128), device="cuda", generator=torch.Generator("cuda").manual_seed(n)) for n in (1, 2))
+    for wrap in (False, True):
+        m = _model(kind, layers=2)
+        if wrap and how == "package":
+            m.cfg.activation_checkpointing = True
+        elif wrap:
+            m.blocks = torch.nn.ModuleList(_Recomputed(b, how != "torch") for b in m.blocks)
+        eng = TrainEngine(m, EngineConfig(strategy="none"))
+        calls.clear()
+        losses.append(eng.step(ids, targets).item())
+        grads.append(eng.flat.grad.clone())
+    # the loss is an fp32 sum over 256 rows in any order
+    assert abs(losses[0] - losses[1]) <= 256 * 2.0 ** -24 * losses[0] and _close(grads[1], grads[0])
+    # two blocks, in the forward where it records gradients (torch's own form) and where they are recomputed
+    assert len(calls) == (4 if how == "torch" else 2)
+    assert _lib.read_status() == 0
