@@ -157,6 +157,8 @@ def block(norm1, attn, norm2, mlp, first, second, x, positions, gated: bool):
         return None
     params = (norm1.weight, None if gated else norm1.bias, qkv.weight, qkv.bias, proj.weight, proj.bias, norm2.weight,
               None if gated else norm2.bias, first.weight, first.bias, second.weight, second.bias)
+    if len({id(p) for p in params if p is not None}) < (6 if gated else 12):
+        return None                # one used twice: its second gradient has to find the first in the buffer
     n1 = 2 * ff if gated else ff
     shapes = ((d,), (d,), (w, d), (w,), (d, Hq * 128), (d,), (d,), (d,), (n1, d), (n1,), (d, ff), (d,))
     for i, (p, shape) in enumerate(zip(params, shapes)):

@@ -176,3 +176,20 @@ def test_recomputed_blocks_under_the_engine(kind, how, calls):
     # two blocks, in the forward where it records gradients (torch's own form) and where they are recomputed
     assert len(calls) == (4 if how == "torch" else 2)
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["gpt", "llama"])
+def test_a_parameter_used_twice(kind, calls):
+    """Its second gradient is added to the first."""
+    blk = _model(kind).blocks[0]
+    if kind == "gpt":
+        blk.ln2.weight = blk.ln1.weight
+    else:
+        blk.norm2.weight = blk.norm1.weight
+    other = copy.deepcopy(blk)
+    x, dy = (torch.randn(2, 64, _width(blk), device="cuda").to(torch.bfloat16) for _ in range(2))
+    for b, on in ((blk, True), (other, False)):
+        FlatParams(list(b.parameters()))
+        _pass(b, x, dy, on)
+    for (name, p), p2 in zip(blk.named_parameters(), other.parameters()):
+        assert _close(p.main_grad, p2.main_grad), name
