@@ -19,7 +19,8 @@ extern "C" {
 int mlf_norm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, int rows, int D, float eps, int rms,
                  uint64_t stream);
 int mlf_norm_bwd_add(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx, void* dgamma, void* dbeta,
-                     float* partials, int rows, int D, int rms, int grads_fp32, int accumulate, const void* dx_add, uint64_t stream);
+                     float* partials, int rows, int D, int rms, int grads_fp32, int accumulate_gamma, int accumulate_beta, const void* dx_add,
+                     uint64_t stream);
 int mlf_rope_qkv(void* out, const void* in, const long long* pos, long long T, int Hq, int Hkv, long long ldo, long long ldi, float theta,
                  int inverse, uint64_t stream);
 int mlf_flash_fwd(const void* q, const void* k, const void* v, void* out, float* lse, int B, int S, int Hq, int Hkv, long long ldq, long long ldk,
@@ -93,7 +94,8 @@ MLF_API int mlf_block_backward(const MlfBlockArgs* p, uint64_t st) {
   RUN(wgrad(p->wide, p->h2, p->dw1, n1, d, MLF_BLOCK_W1));
   RUN(bgrads(p->dy, p->dbb2, MLF_BLOCK_BB2, p->wide, p->dbb1, n1, MLF_BLOCK_BB1));
   RUN(product(p->wide, p->w1, p->row, T, d, n1, n1, d, d, 0, 1, 0, nullptr, nullptr, 0, nullptr, 0, st));
-  RUN(mlf_norm_bwd_add(p->x1, p->row, p->g2, p->mean2, p->rstd2, p->dx1, p->dg2, p->db2, p->norm_scratch, T, d, p->gated, 0, add(MLF_BLOCK_G2), p->dy, st));
+  RUN(mlf_norm_bwd_add(p->x1, p->row, p->g2, p->mean2, p->rstd2, p->dx1, p->dg2, p->db2, p->norm_scratch, T, d, p->gated, 0, add(MLF_BLOCK_G2),
+                       add(MLF_BLOCK_B2), p->dy, st));
   // attention: da, dqkv (in the MLP's place), then dh1
   RUN(product(p->dx1, p->wo, p->da, T, q, d, d, q, q, 0, 1, 0, nullptr, nullptr, 0, nullptr, 0, st));
   RUN(wgrad(p->dx1, p->a, p->dwo, d, q, MLF_BLOCK_WO));
@@ -103,5 +105,6 @@ MLF_API int mlf_block_backward(const MlfBlockArgs* p, uint64_t st) {
   RUN(product(p->wide, p->wqkv, p->row, T, d, w, w, d, d, 0, 1, 0, nullptr, nullptr, 0, nullptr, 0, st));
   RUN(wgrad(p->wide, p->h1, p->dwqkv, w, d, MLF_BLOCK_WQKV));
   RUN(bgrads(p->dx1, p->dbo, MLF_BLOCK_BO, p->wide, p->dbqkv, w, MLF_BLOCK_BQKV));
-  return mlf_norm_bwd_add(p->x, p->row, p->g1, p->mean1, p->rstd1, p->dx, p->dg1, p->db1, p->norm_scratch, T, d, p->gated, 0, add(MLF_BLOCK_G1), p->dx1, st);
+  return mlf_norm_bwd_add(p->x, p->row, p->g1, p->mean1, p->rstd1, p->dx, p->dg1, p->db1, p->norm_scratch, T, d, p->gated, 0, add(MLF_BLOCK_G1),
+                          add(MLF_BLOCK_B1), p->dx1, st);
 }

@@ -481,7 +481,7 @@ norm_bwd_cta_kernel(const __nv_bfloat16* x, const __nv_bfloat16* dy,
 constexpr int NF_WARPS = 32;
 __global__ void __launch_bounds__(NF_WARPS * 32)
 norm_bwd_finalize_kernel(const float* partials, int nparts, int D, void* dgamma, void* dbeta,
-                         int out_fp32, int accumulate) {
+                         int out_fp32, int accumulate_gamma, int accumulate_beta) {
   __shared__ float sg[NF_WARPS][33], sb[NF_WARPS][33];
   pdl_trigger();
   pdl_wait();
@@ -503,17 +503,17 @@ norm_bwd_finalize_kernel(const float* partials, int nparts, int D, void* dgamma,
   for (int k = 1; k < NF_WARPS; ++k) { g += sg[k][cl]; b += sb[k][cl]; }
   if (out_fp32) {
     float* dgp = static_cast<float*>(dgamma);
-    dgp[c] = g + (accumulate ? dgp[c] : 0.f);
+    dgp[c] = g + (accumulate_gamma ? dgp[c] : 0.f);
     if (dbeta) {
       float* dbp = static_cast<float*>(dbeta);
-      dbp[c] = b + (accumulate ? dbp[c] : 0.f);
+      dbp[c] = b + (accumulate_beta ? dbp[c] : 0.f);
     }
   } else {
     __nv_bfloat16* dgp = static_cast<__nv_bfloat16*>(dgamma);
-    dgp[c] = __float2bfloat16(g + (accumulate ? __bfloat162float(dgp[c]) : 0.f));
+    dgp[c] = __float2bfloat16(g + (accumulate_gamma ? __bfloat162float(dgp[c]) : 0.f));
     if (dbeta) {
       __nv_bfloat16* dbp = static_cast<__nv_bfloat16*>(dbeta);
-      dbp[c] = __float2bfloat16(b + (accumulate ? __bfloat162float(dbp[c]) : 0.f));
+      dbp[c] = __float2bfloat16(b + (accumulate_beta ? __bfloat162float(dbp[c]) : 0.f));
     }
   }
 }
@@ -612,10 +612,11 @@ MLF_API long long mlf_norm_bwd_scratch_elems(int rows, int D) {
 }
 
 // dx_add (optional, bf16 [rows, D]) is added to dx: the gradient arriving over a skip connection that
-// branched off the normalised tensor's input, so that the sum needs no pass of its own.
+// branched off the normalised tensor's input, so that the sum needs no pass of its own. dgamma and dbeta are of one type (fp32 if
+// grads_fp32, else bf16); each is written or added to by a switch of its own.
 MLF_API int mlf_norm_bwd_add(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
                              void* dx, void* dgamma, void* dbeta, float* partials, int rows, int D, int rms,
-                             int grads_fp32, int accumulate, const void* dx_add, uint64_t stream) {
+                             int grads_fp32, int accumulate_gamma, int accumulate_beta, const void* dx_add, uint64_t stream) {
   MLF_REQUIRE(D % 256 == 0, "norm: D=%d must be a multiple of 256", D);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int grid = norm_bwd_grid(rows, D);
@@ -642,7 +643,7 @@ MLF_API int mlf_norm_bwd_add(const void* x, const void* dy, const void* gamma, c
 #undef LAUNCH
   count_launch();
   MLF_CHECK_CUDA(launch_pdl(norm_bwd_finalize_kernel, dim3((D + 31) / 32), dim3(NF_WARPS * 32), 0, st, (const float*)partials, grid, D, dgamma,
-                            rms ? (void*)nullptr : dbeta, grads_fp32, accumulate));
+                            rms ? (void*)nullptr : dbeta, grads_fp32, accumulate_gamma, accumulate_beta));
   count_launch();
   return 0;
 }
@@ -650,5 +651,6 @@ MLF_API int mlf_norm_bwd_add(const void* x, const void* dy, const void* gamma, c
 MLF_API int mlf_norm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
                          void* dx, void* dgamma, void* dbeta, float* partials, int rows, int D, int rms,
                          int grads_fp32, int accumulate, uint64_t stream) {
-  return mlf_norm_bwd_add(x, dy, gamma, mean, rstd, dx, dgamma, dbeta, partials, rows, D, rms, grads_fp32, accumulate, nullptr, stream);
+  return mlf_norm_bwd_add(x, dy, gamma, mean, rstd, dx, dgamma, dbeta, partials, rows, D, rms, grads_fp32, accumulate, accumulate, nullptr,
+                          stream);
 }

@@ -210,6 +210,28 @@ def mlp_swiglu(x, w_gu, w_down, residual=None):
 # ------------------------------------------------------------------------------------------
 # norms
 # ------------------------------------------------------------------------------------------
+def _norm_grads(ctx, x, dy, gamma, mean, rstd, dx_add=None):
+    """dx, and the gradients of gamma and beta that go to autograd (None for one that went into its buffer). The kernel writes
+    both in one type: a buffer of another gets its gradient from a tensor in between."""
+    refs = (ctx.gamma_ref, None if ctx.rms else ctx.beta_ref)
+    sinks = [_sink(p) for p in refs]
+    dtype = torch.float32 if any(t is not None and t.dtype != gamma.dtype for t, _ in sinks) else gamma.dtype
+    out = [t if t is not None and t.dtype == dtype else None if p is None else torch.empty(p.shape, dtype=dtype, device=x.device)
+           for p, (t, _) in zip(refs, sinks)]
+    direct = [o is t for o, (t, _) in zip(out, sinks)]
+    dx, *grads = native.norm_bwd(x, dy, gamma, None if ctx.rms else mean, rstd, ctx.rms, dgamma_out=out[0], dbeta_out=out[1],
+                                 accumulate=direct[0] and sinks[0][1], accumulate_beta=direct[1] and sinks[1][1], dx_add=dx_add)
+    for i, (p, (t, acc)) in enumerate(zip(refs, sinks)):
+        if t is not None:
+            if not direct[i]:
+                t.copy_(t + grads[i] if acc else grads[i])
+            _done(p)
+            grads[i] = None
+        else:
+            grads[i] = None if p is None else grads[i].to(p.dtype)
+    return dx, *grads
+
+
 class _NormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gamma, beta, eps, rms):
@@ -223,17 +245,8 @@ class _NormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, gamma, mean, rstd = ctx.saved_tensors
-        gt, gacc = _sink(ctx.gamma_ref)
-        bt, _ = _sink(ctx.beta_ref)
-        dx, dg, db = native.norm_bwd(x, dy.contiguous(), gamma, None if ctx.rms else mean, rstd, ctx.rms,
-                                     dgamma_out=gt, dbeta_out=bt if not ctx.rms else None, accumulate=gacc)
-        if gt is not None:
-            _done(ctx.gamma_ref)
-            dg = None
-        if bt is not None and not ctx.rms:
-            _done(ctx.beta_ref)
-            db = None
-        return dx, dg, (db if not ctx.rms else None), None, None
+        dx, dg, db = _norm_grads(ctx, x, dy.contiguous(), gamma, mean, rstd)
+        return dx, dg, db, None, None
 
 
 class _NormSkipFn(torch.autograd.Function):
@@ -253,8 +266,6 @@ class _NormSkipFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dskip):
         x, gamma, mean, rstd = ctx.saved_tensors
-        gt, gacc = _sink(ctx.gamma_ref)
-        bt, _ = _sink(ctx.beta_ref)
         if dy is None:
             return dskip, None, None, None, None
         add = None
@@ -262,15 +273,8 @@ class _NormSkipFn(torch.autograd.Function):
             add = dskip.contiguous()
             if add.dtype != x.dtype:
                 add = add.to(x.dtype)
-        dx, dg, db = native.norm_bwd(x, dy.contiguous(), gamma, None if ctx.rms else mean, rstd, ctx.rms,
-                                     dgamma_out=gt, dbeta_out=bt if not ctx.rms else None, accumulate=gacc, dx_add=add)
-        if gt is not None:
-            _done(ctx.gamma_ref)
-            dg = None
-        if bt is not None and not ctx.rms:
-            _done(ctx.beta_ref)
-            db = None
-        return dx, dg, (db if not ctx.rms else None), None, None
+        dx, dg, db = _norm_grads(ctx, x, dy.contiguous(), gamma, mean, rstd, add)
+        return dx, dg, db, None, None
 
 
 def layer_norm_skip(x, gamma, beta, eps: float = 1e-5):
