@@ -29,6 +29,8 @@ def _st():
 
 
 def _p(t: Optional[torch.Tensor]):
+    """Address of ``t``, which the caller has to hold until the launch is queued: a copy that nothing else holds is freed at
+    once, and the next one may be put in its place."""
     return C.c_void_p(t.data_ptr()) if t is not None else None
 
 
@@ -144,7 +146,8 @@ def norm_bwd(x: torch.Tensor, dy: torch.Tensor, gamma: torch.Tensor, mean, rstd,
 # ------------------------------------------------------------------ activations
 def gelu_bwd(dy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     dx = torch.empty_like(x)
-    _lib.check(_L().mlf_gelu_bwd(_p(dx), _p(dy.contiguous()), _p(x.contiguous()), C.c_longlong(x.numel()), _st()), "mlf_gelu_bwd")
+    dy, x = dy.contiguous(), x.contiguous()
+    _lib.check(_L().mlf_gelu_bwd(_p(dx), _p(dy), _p(x), C.c_longlong(x.numel()), _st()), "mlf_gelu_bwd")
     return dx
 
 
@@ -160,7 +163,8 @@ def swiglu_bwd(dout: torch.Tensor, gu: torch.Tensor, interleaved: bool = False) 
     F = gu.shape[-1] // 2
     g2 = gu.reshape(-1, 2 * F)
     dgu = torch.empty_like(g2)
-    _lib.check(_L().mlf_swiglu_bwd(_p(dgu), _p(dout.reshape(-1, F).contiguous()), _p(g2), C.c_longlong(g2.shape[0]), F,
+    dout = dout.reshape(-1, F).contiguous()
+    _lib.check(_L().mlf_swiglu_bwd(_p(dgu), _p(dout), _p(g2), C.c_longlong(g2.shape[0]), F,
                                    int(interleaved), _st()), "mlf_swiglu_bwd")
     return dgu.view(gu.shape)
 
@@ -194,8 +198,9 @@ def embedding_fwd(ids: torch.Tensor, wte: torch.Tensor, pos: Optional[torch.Tens
     T = ids.numel()
     D = wte.shape[1]
     out = torch.empty(T, D, dtype=wte.dtype, device=wte.device)
-    rc = _L().mlf_embedding_fwd(_p(out), _p(ids.reshape(-1).contiguous()), _p(pos.reshape(-1).contiguous()) if pos is not None else None,
-                                _p(wte), _p(wpe), C.c_longlong(T), D, wte.shape[0], wpe.shape[0] if wpe is not None else 0, _st())
+    flat = ids.reshape(-1).contiguous()
+    pos = pos.reshape(-1).contiguous() if pos is not None else None
+    rc = _L().mlf_embedding_fwd(_p(out), _p(flat), _p(pos), _p(wte), _p(wpe), C.c_longlong(T), D, wte.shape[0], wpe.shape[0] if wpe is not None else 0, _st())
     _lib.check(rc, "mlf_embedding_fwd")
     return out.view(*ids.shape, D)
 
@@ -205,8 +210,8 @@ def embedding_bwd(dout: torch.Tensor, ids: torch.Tensor, vocab: int, dw_fp32: Op
     T = ids.numel()
     if dw_fp32 is None:
         dw_fp32 = torch.zeros(vocab, D, dtype=torch.float32, device=dout.device)
-    rc = _L().mlf_embedding_bwd(_p(dw_fp32), _p(dout.reshape(T, D).contiguous()), _p(ids.reshape(-1).contiguous()),
-                                C.c_longlong(T), D, vocab, _st())
+    dout, ids = dout.reshape(T, D).contiguous(), ids.reshape(-1).contiguous()
+    rc = _L().mlf_embedding_bwd(_p(dw_fp32), _p(dout), _p(ids), C.c_longlong(T), D, vocab, _st())
     _lib.check(rc, "mlf_embedding_bwd")
     return dw_fp32
 
@@ -219,8 +224,8 @@ def embedding_grad(dout: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, acc
     L = _L()
     L.mlf_embedding_grad_scratch_bytes.restype = C.c_longlong
     scratch = torch.empty(L.mlf_embedding_grad_scratch_bytes(C.c_longlong(T), D, vocab), dtype=torch.uint8, device=dout.device)
-    rc = L.mlf_embedding_grad(_p(out), _p(dout.reshape(T, D).contiguous()), _p(ids.reshape(-1).contiguous()), _p(scratch),
-                              C.c_longlong(T), D, vocab, int(accumulate), _st())
+    dout, ids = dout.reshape(T, D).contiguous(), ids.reshape(-1).contiguous()
+    rc = L.mlf_embedding_grad(_p(out), _p(dout), _p(ids), _p(scratch), C.c_longlong(T), D, vocab, int(accumulate), _st())
     _lib.check(rc, "mlf_embedding_grad")
     return out
 
@@ -234,7 +239,8 @@ def rope_(x: torch.Tensor, pos: torch.Tensor, theta: float, inverse: bool = Fals
     """In-place rotary embedding on ``x`` [T, H, Dh] (may be a strided view over a packed row)."""
     T, H, Dh = x.shape
     assert x.stride(2) == 1 and x.stride(1) == Dh
-    rc = _L().mlf_rope(_p(x), _p(pos.contiguous()), C.c_longlong(T), H, Dh, C.c_longlong(x.stride(0)), C.c_float(theta),
+    pos = pos.contiguous()
+    rc = _L().mlf_rope(_p(x), _p(pos), C.c_longlong(T), H, Dh, C.c_longlong(x.stride(0)), C.c_float(theta),
                        int(inverse), _st())
     _lib.check(rc, "mlf_rope")
     return x
@@ -249,7 +255,8 @@ def rope_qkv(qkv: torch.Tensor, pos: torch.Tensor, Hq: int, Hkv: int, theta: flo
     if out is None:
         out = torch.empty(qkv.shape, dtype=qkv.dtype, device=qkv.device)
     assert out.shape == qkv.shape and out.dtype == qkv.dtype and out.stride(1) == 1
-    rc = _L().mlf_rope_qkv(_p(out), _p(qkv), _p(pos.contiguous()), C.c_longlong(qkv.shape[0]), Hq, Hkv, C.c_longlong(out.stride(0)),
+    pos = pos.contiguous()
+    rc = _L().mlf_rope_qkv(_p(out), _p(qkv), _p(pos), C.c_longlong(qkv.shape[0]), Hq, Hkv, C.c_longlong(out.stride(0)),
                            C.c_longlong(qkv.stride(0)), C.c_float(theta), int(inverse), _st())
     _lib.check(rc, "mlf_rope_qkv")
     return out
@@ -297,7 +304,8 @@ def cross_entropy_(logits: torch.Tensor, targets: torch.Tensor, vocab: int, *, g
     T = logits.shape[0]
     loss_rows = torch.empty(T, dtype=torch.float32, device=logits.device)
     loss_sum = torch.zeros((), dtype=torch.float32, device=logits.device)
-    rc = _L().mlf_cross_entropy(_p(logits), _p(targets.contiguous()), _p(loss_rows), _p(loss_sum), T, vocab,
+    targets = targets.contiguous()
+    rc = _L().mlf_cross_entropy(_p(logits), _p(targets), _p(loss_rows), _p(loss_sum), T, vocab,
                                 C.c_longlong(logits.stride(0)), C.c_float(grad_scale), _p(grad_scale_dev),
                                 C.c_float(loss_weight), _st())
     _lib.check(rc, "mlf_cross_entropy")
@@ -471,9 +479,9 @@ def paged_decode_rope(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: to
     st = (max(split_tokens, 128) + 127) // 128 * 128
     splits = max(1, (max_seq_len + st - 1) // st)
     ws = torch.empty(int(L.mlf_paged_decode_ws_elems(B, Hq, splits)), dtype=torch.float32, device=qkv.device) if splits > 1 else None
-    rc = L.mlf_paged_decode_rope(_p(qkv), C.c_longlong(qkv.stride(0)), _p(kv_cache), _p(block_table), _p(seq_lens.contiguous()),
-                                 _p(slots.contiguous()), _p(out), _p(ws), B, Hq, Hkv, bs, block_table.shape[1], nb, int(max_seq_len), st,
-                                 C.c_float(scale if scale is not None else D ** -0.5), C.c_float(theta), int(inputs_static), _st())
+    seq_lens, slots = seq_lens.contiguous(), slots.contiguous()
+    rc = L.mlf_paged_decode_rope(_p(qkv), C.c_longlong(qkv.stride(0)), _p(kv_cache), _p(block_table), _p(seq_lens), _p(slots), _p(out), _p(ws), B, Hq, Hkv, bs,
+                                 block_table.shape[1], nb, int(max_seq_len), st, C.c_float(scale if scale is not None else D ** -0.5), C.c_float(theta), int(inputs_static), _st())
     _lib.check(rc, "mlf_paged_decode_rope")
     return out
 
@@ -483,7 +491,8 @@ def kv_cache_write(kv_cache: torch.Tensor, k: torch.Tensor, v: torch.Tensor, slo
     nb, _, bs, Hkv, D = kv_cache.shape
     T = k.shape[0]
     assert k.stride(2) == 1 and k.stride(1) == D and v.stride(2) == 1 and v.stride(1) == D
-    rc = _L().mlf_kv_cache_write(_p(kv_cache), _p(k), _p(v), _p(slots.contiguous()), C.c_longlong(T), Hkv, bs, nb,
+    slots = slots.contiguous()
+    rc = _L().mlf_kv_cache_write(_p(kv_cache), _p(k), _p(v), _p(slots), C.c_longlong(T), Hkv, bs, nb,
                                  C.c_longlong(k.stride(0)), C.c_longlong(v.stride(0)), _st())
     _lib.check(rc, "mlf_kv_cache_write")
 
@@ -494,7 +503,8 @@ def rope_kv_write_(qkv: torch.Tensor, pos: torch.Tensor, slots: torch.Tensor, kv
     nb, _, bs, Hc, D = kv_cache.shape
     assert D == 128 and Hc == Hkv and qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.shape[1] == (Hq + 2 * Hkv) * 128
     assert qkv.dtype == torch.bfloat16 and pos.dtype == torch.int64 and slots.dtype == torch.int64
-    rc = _L().mlf_rope_kv_write(_p(qkv), C.c_longlong(qkv.stride(0)), _p(pos.contiguous()), _p(slots.contiguous()), _p(kv_cache),
+    pos, slots = pos.contiguous(), slots.contiguous()
+    rc = _L().mlf_rope_kv_write(_p(qkv), C.c_longlong(qkv.stride(0)), _p(pos), _p(slots), _p(kv_cache),
                                 C.c_longlong(qkv.shape[0]), Hq, Hkv, bs, nb, C.c_float(theta), _st())
     _lib.check(rc, "mlf_rope_kv_write")
     return qkv
