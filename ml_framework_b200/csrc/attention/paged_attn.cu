@@ -444,7 +444,7 @@ template <bool V16>
 __global__ void __launch_bounds__(256)
 rope_kv_write_kernel(__nv_bfloat16* qkv, long long ld, const long long* pos, const long long* slots, __nv_bfloat16* cache, long long T,
                      int Hq, int Hkv, int block_size, int num_blocks, int heads_per_warp, float theta, int* err) {
-  __shared__ float2 s_cs[8][PD / 2];
+  __shared__ __align__(16) float2 s_cs[8][PD / 2];   // read two at a time
   pdl_trigger();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

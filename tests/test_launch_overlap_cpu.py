@@ -40,3 +40,15 @@ def test_every_overlapped_launch_waits():
     launched = set(re.findall(r"launch_pdl\(\s*(\w+)", text)) - {"kernel"}
     waits = {name for name, _, body in _kernels() if "pdl_wait()" in body}
     assert launched and launched <= waits
+
+
+def test_shared_arrays_are_aligned_for_their_widest_access():
+    """An array that is also read or written 16 bytes at a time says so where it is declared."""
+    seen = 0
+    for name, _, body in _kernels():
+        for array in re.findall(r"reinterpret_cast<(?:const )?(?:uint4|int4|float4)\s*\*>\(&?(\w+)\b", body):
+            declared = re.search(r"__shared__([^;]*?)\b" + array + r"\s*\[", body)
+            if declared:
+                seen += 1
+                assert re.search(r"__align__\(\d*(16|32|64|128|1024)\)|\b(uint4|int4|float4)\b", declared.group(1)), (name, array)
+    assert seen >= 1
