@@ -29,3 +29,19 @@ def test_against_64_bits(D, rows, rms, skip):
     assert (dg.double() - gd.grad).norm() <= 2.5e-3 * gd.grad.norm()
     assert rms or (db.double() - bd.grad).norm() <= 2.5e-3 * bd.grad.norm()
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("D", [256, 512, 768, 1024, 1536, 2048, 3072, 4096, 5120, 6144, 8192])
+def test_rows_far_from_zero(D):
+    """x - mean is formed before it is scaled: rows of 1000 +- 4 keep the digits that x * rstd - mean * rstd would round away."""
+    torch.manual_seed(D)
+    x = 1000 + 4 * (torch.randint(0, 2, (2, D), device="cuda") * 2 - 1).to(torch.bfloat16)
+    dy = torch.randn(2, D, device="cuda").to(torch.bfloat16)
+    g = torch.ones(D, device="cuda").to(torch.bfloat16)
+    mean = torch.full((2,), 1000.0, device="cuda")
+    rstd = torch.tensor([0.24999992, 0.2371823], device="cuda")
+    dg, db = (torch.empty(D, device="cuda") for _ in range(2))
+    native.norm_bwd(x, dy, g, mean, rstd, False, dgamma_out=dg, dbeta_out=db)
+    terms = dy.double() * (x.double() - 1000) * rstd.double()[:, None]
+    # two products and a sum per row, and the sum of both rows, in fp32
+    assert ((dg.double() - terms.sum(0)).abs() <= 8 * 2.0 ** -24 * terms.abs().sum(0)).all()
