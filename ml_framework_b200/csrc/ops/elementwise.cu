@@ -610,18 +610,28 @@ static void colsum_shape(int M, int col_ctas, int& row_ctas, int& rows_per_cta) 
 }
 // Scratch layout of mlf_colsum: a counter per 256 columns (uint32, zero before the first use; the kernel
 // leaves them zero), then row_ctas x 256 floats of partial sums for each. Matrices of different widths share a buffer, so the
-// counters' part has one size for all of them (up to 512 K columns): a narrower one's partial sums must not land on a wider
-// one's counters.
+// counters' part has one size for all launches, none of which has more column blocks than it has counters: a narrower one's
+// partial sums must not land on a wider one's counters. Wider matrices (more than 512 K columns) take several launches.
+constexpr int CS_MAX_BLOCKS = 2048;
+constexpr long long CS_COUNTER_BYTES = CS_MAX_BLOCKS * 4;
 static int colsum_blocks(int N) { return (N + CS_COLS - 1) / CS_COLS; }
-static long long colsum_counter_bytes(int col_ctas) { return col_ctas <= 2048 ? 8192 : ((long long)col_ctas * 4 + 255) / 256 * 256; }
+static long long colsum_launch_bytes(int M, int col_ctas) {
+  int r, rp;
+  colsum_shape(M, col_ctas, r, rp);
+  return CS_COUNTER_BYTES + (long long)r * col_ctas * CS_COLS * 4;
+}
+MLF_API long long mlf_colsum_scratch_bytes(int M, int N) {
+  const int c = colsum_blocks(N), rest = c % CS_MAX_BLOCKS;
+  const long long a = c >= CS_MAX_BLOCKS ? colsum_launch_bytes(M, CS_MAX_BLOCKS) : 0, b = rest ? colsum_launch_bytes(M, rest) : 0;
+  return a > b ? a : b;
+}
 // N1 > 0: of a launch for two matrices
 MLF_API long long mlf_colsum2_scratch_bytes(int M, int N0, int N1) {
   const int c = colsum_blocks(N0) + colsum_blocks(N1);
-  int r, rp;
-  colsum_shape(M, c, r, rp);
-  return colsum_counter_bytes(c) + (long long)r * c * CS_COLS * 4;
+  if (c <= CS_MAX_BLOCKS) return colsum_launch_bytes(M, c);
+  const long long a = mlf_colsum_scratch_bytes(M, N0), b = N1 > 0 ? mlf_colsum_scratch_bytes(M, N1) : 0;
+  return a > b ? a : b;
 }
-MLF_API long long mlf_colsum_scratch_bytes(int M, int N) { return mlf_colsum2_scratch_bytes(M, N, 0); }
 static int colsum_launch(const ColsumMatrix& first, const ColsumMatrix& second, int M, void* scratch, cudaStream_t st) {
   MLF_REQUIRE(first.ld % 8 == 0 && second.ld % 8 == 0, "colsum: pitch must be a multiple of 8 elements");
   MLF_REQUIRE(scratch != nullptr && M > 0 && first.N > 0, "colsum: bad arguments");
@@ -629,21 +639,31 @@ static int colsum_launch(const ColsumMatrix& first, const ColsumMatrix& second, 
   int row_ctas, rows_per_cta;
   colsum_shape(M, col_ctas, row_ctas, rows_per_cta);
   unsigned int* counters = static_cast<unsigned int*>(scratch);
-  float* part = reinterpret_cast<float*>(static_cast<char*>(scratch) + colsum_counter_bytes(col_ctas));
+  float* part = reinterpret_cast<float*>(static_cast<char*>(scratch) + CS_COUNTER_BYTES);
   MLF_CHECK_CUDA(launch_pdl(colsum_kernel, dim3(col_ctas, row_ctas), dim3(256), 0, st, first, second, first_blocks, part, counters, M, rows_per_cta));
   count_launch();
   return 0;
 }
-// db (bf16 [N]) = column sums of dy (+ db when accumulate). One launch; calls that share a scratch
+// db (bf16 [N]) = column sums of dy (+ db when accumulate). One launch per 512 K columns; calls that share a scratch
 // buffer must be ordered on one stream.
 MLF_API int mlf_colsum(void* db, const void* dy, int M, int N, long long ld, void* scratch, int accumulate, uint64_t stream) {
-  return colsum_launch({(__nv_bfloat16*)db, (const __nv_bfloat16*)dy, ld, N, accumulate}, {nullptr, nullptr, 0, 0, 0}, M, scratch,
-                       reinterpret_cast<cudaStream_t>(stream));
+  MLF_REQUIRE(N > 0, "colsum: bad arguments");
+  constexpr int step = CS_MAX_BLOCKS * CS_COLS;
+  for (int n0 = 0;; n0 += step) {
+    const int n = N - n0 < step ? N - n0 : step;
+    const int rc = colsum_launch({(__nv_bfloat16*)db + n0, (const __nv_bfloat16*)dy + n0, ld, n, accumulate}, {nullptr, nullptr, 0, 0, 0}, M, scratch,
+                                 reinterpret_cast<cudaStream_t>(stream));
+    if (rc || n == N - n0) return rc;
+  }
 }
 // Two matrices of M rows in one launch.
 MLF_API int mlf_colsum2(void* db0, const void* dy0, int N0, long long ld0, int accumulate0, void* db1, const void* dy1, int N1, long long ld1,
                         int accumulate1, int M, void* scratch, uint64_t stream) {
-  MLF_REQUIRE(N1 > 0, "colsum: bad arguments");
+  MLF_REQUIRE(N0 > 0 && N1 > 0, "colsum: bad arguments");
+  if (colsum_blocks(N0) + colsum_blocks(N1) > CS_MAX_BLOCKS) {
+    const int rc = mlf_colsum(db0, dy0, M, N0, ld0, scratch, accumulate0, stream);
+    return rc ? rc : mlf_colsum(db1, dy1, M, N1, ld1, scratch, accumulate1, stream);
+  }
   return colsum_launch({(__nv_bfloat16*)db0, (const __nv_bfloat16*)dy0, ld0, N0, accumulate0},
                        {(__nv_bfloat16*)db1, (const __nv_bfloat16*)dy1, ld1, N1, accumulate1}, M, scratch, reinterpret_cast<cudaStream_t>(stream));
 }

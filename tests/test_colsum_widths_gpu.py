@@ -20,3 +20,15 @@ def test_wide_after_narrow(wide):
         want = x.double().sum(0)
         # sums in fp32, one rounding to bf16
         assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
+
+
+@pytest.mark.parametrize("wide", [(1 << 19) + 264, (1 << 20) + 8])
+def test_more_columns_than_counters(wide):
+    torch.manual_seed(wide)
+    x = torch.randn(40, wide, device="cuda").to(torch.bfloat16)
+    want = x.double().sum(0)
+    for _ in range(2):
+        native.colsum(x[:, :256])
+        got = native.colsum(x, out=torch.full_like(x[0], float("nan")))
+        # sums in fp32, one rounding to bf16
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
