@@ -1,4 +1,4 @@
-// Self-attention forward, head_dim 128: two 128-row query tiles per item, ping-ponged; one persistent CTA per SM.
+// Self-attention forward, head_dim 128: two 128-row query tiles per item, ping-ponged; a CTA goes from item to item.
 //
 // An item is 256 query rows of one (batch, head) as two tiles of 128. 384 threads in three warpgroups;
 // the control warpgroup hands most of its registers to the softmax warpgroups (setmaxnreg 72 / 216 / 216 of 3 x 168:
@@ -22,13 +22,16 @@
 // in halves so that PV starts on the first 64 keys while the exponentials of the others run, and the arithmetic around the
 // exponentials is done two elements at a time. (Every eighth pair of exponentials as a polynomial on the FMA pipe, as exact as
 // the special-function unit's, took 4 % off long sequences and changed every bit of the output; every fourth cost 1 %.)
-// A CTA walks over its items instead of ending with each: set-up, the first loads and the write-out took a third of the
+// A CTA takes over items instead of ending with its first: set-up, the first loads and the write-out took a third of the
 // clocks of an item of eight key tiles and two thirds of one of two. The next item's Q, K and V arrive and its first S is
 // issued behind the last products of this one, while the softmax warps write its rows out, each through its own staging
 // tile and the copy engine (32 rows of 16 bytes per store instruction took 2500 clocks). Only the 32-column blocks of a
 // diagonal tile that a warp does not see whole are masked (2000 clocks a tile before).
-// One launch, before -> now, with the same bits: 8 x 512, 32 / 8 heads 57 -> 43 us; 4 x 2048, 16 heads 100 -> 82 us;
-// 2 x 4096, 32 / 8 heads 283 -> 254 us; 1404 queries of 5500 keys, 32 / 8 heads 152 -> 148 us.
+// The grid has a CTA per item, the longest first; a CTA that nears its end has the launch control cancel one that has not
+// started and does that one's item. Rounds of fixed shares (a CTA per SM) left the shares of CTAs that found no place beside
+// another stream's kernel until the others had ended. us back to back, a CTA that ends with its item / fixed shares / now: 4 x 2048,
+// 16 heads 97 / 82 / 79, with 1 SM held by another kernel 99 / 141 / 82, with 8 101 / 142 / 85; 8 x 512, 32 / 8 heads
+// 54 / 41 / 39, 55 / 60 / 40, 57 / 61 / 41; 2 x 4096, 32 / 8 heads 278 / 258 / 246, 288 / 464 / 258, 303 / 466 / 269.
 // Per SM and key tile: 4 x 128x128x128 of tensor work against 2 x 16384 exponentials.
 //
 // Math reference: StandardPagedAttentionKernel.ComputePagedAttention
@@ -81,13 +84,9 @@ struct FlashWsItem {
   int n_kv;
 };
 
-// Item k of a CTA. Items are numbered by work, the longest query pairs first; the CTAs take them in rounds, every other
-// round in reverse, so that the CTA with the longest item of one round gets the shortest of the next.
-__device__ __forceinline__ bool flash_ws_item(const FlashWsParams& p, int n_items, int k, FlashWsItem& it) {
-  const int g = (int)gridDim.x;
-  const long long at = (long long)k * g + ((k & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
-  if (at >= n_items) return false;
-  const int i = (int)at;
+// Item i. Items are numbered by work, the longest query pairs first; false for i < 0.
+__device__ __forceinline__ bool flash_ws_item(const FlashWsParams& p, int i, FlashWsItem& it) {
+  if (i < 0) return false;
   const int n_pairs = (p.S + 2 * W_BQ - 1) / (2 * W_BQ);
   const int hb = p.Hq * p.B;
   const int pair = p.causal ? n_pairs - 1 - i / hb : i / hb;
@@ -127,12 +126,15 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   auto pv_done = [&](int t) { return bars + 8u * (14 + t); };
   auto p_half = [&](int t) { return bars + 8u * (16 + t); };
   auto q_empty = [&](int t) { return bars + 8u * (18 + t); };
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + (bars - sbase) + 8 * 20);
+  // the next item: answers of the launch control, two of them in turn
+  auto next_full = [&](int s) { return bars + 8u * (20 + s); };
+  auto next_empty = [&](int s) { return bars + 8u * (22 + s); };
+  auto answer = [&](int s) { return bars + 8u * 26 + 16u * s; };
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + (bars - sbase) + 8 * 24);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int n_items = ((p.S + 2 * W_BQ - 1) / (2 * W_BQ)) * p.Hq * p.B;
 
   if ((sbase & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(p.err, 0, ERR_BAD_INDEX);
@@ -150,6 +152,8 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(p_half(i), 128);
       mbar_init(pv_done(i), 1);
       mbar_init(q_empty(i), 1);
+      mbar_init(next_full(i), 1);
+      mbar_init(next_empty(i), 9);              // the MMA issuer and eight softmax warps have read the answer
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -177,7 +181,8 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       int n_q[2] = {0, 0};                      // query tiles fetched so far
       bool ok = true;
       const int seq_pages = (p.Skv + W_PAGE - 1) / W_PAGE;
-      for (int k = 0; ok && flash_ws_item(p, n_items, k, w); ++k) {
+      int item = blockIdx.x;
+      for (int k = 0; ok && flash_ws_item(p, item, w); ++k) {
         const long long row_base = (long long)w.b * p.S;
         const long long kv_row_base = (long long)w.b * p.Skv;
         const int* bt = p.block_table ? p.block_table + (long long)w.b * p.max_blocks : nullptr;
@@ -224,6 +229,12 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
             if (!ok) break;
           }
+          if (j == max(0, w.n_kv - 2)) {
+            // the next item, asked for as late as its answer (a microsecond) allows: an item that a CTA has taken waits for it
+            if (!mbar_wait(next_empty(k & 1), ((k >> 1) & 1) ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+            mbar_expect_tx(next_full(k & 1), 16);
+            clc_try_cancel(answer(k & 1), next_full(k & 1));
+          }
           if (!mbar_wait(v_empty(s), ph ^ 1u, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
           mbar_expect_tx(v_full(s), W_TILE_BYTES);
           if (bt) {
@@ -238,6 +249,8 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             tma_load_2d(sV + s * W_TILE_BYTES + W_TILE_BYTES / 2, &tmV, w.hkv * W_D + 64, krow, v_full(s));
           }
         }
+        if (!ok || !mbar_wait(next_full(k & 1), (k >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) break;
+        item = clc_answer(answer(k & 1));
       }
     }
   } else if (warp == 1) {
@@ -266,7 +279,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       int n_p[2] = {0, 0};                      // key tiles multiplied so far, per query tile
       int n_q[2] = {0, 0};
       bool ok = true;
-      bool have = flash_ws_item(p, n_items, 0, w);
+      bool have = flash_ws_item(p, blockIdx.x, w);
       // S_t(0) of an item, its K and Q waited for; the last S of a tile gives its Q buffer back
       auto first_s = [&](const FlashWsItem& x, int ring, int t) -> bool {
         if (x.n_t[t] == 0) return true;
@@ -284,7 +297,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       for (int k = 0; ok && have; ++k) {
         FlashWsItem nx;
-        const bool more = flash_ws_item(p, n_items, k + 1, nx);
+        bool more = false;
         for (int j = 0; j < w.n_kv && ok; ++j) {
           const int r = kt + j, s = r & 1;
           const uint32_t ph = (r >> 1) & 1;
@@ -310,10 +323,15 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               }
               issue_s(t, (r + 1) & 1);
               if (j + 2 == w.n_t[t]) umma_commit(q_empty(t));
-            } else if (last && more) {
+            } else if (last) {
               // the next item's first S goes in behind this item's last products: its softmax warps find it ready when
               // they have written their rows
-              if (!first_s(nx, r + 1, t)) { ok = false; break; }
+              if (t == 0) {
+                if (!mbar_wait(next_full(k & 1), (k >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+                more = flash_ws_item(p, clc_answer(answer(k & 1)), nx);
+                mbar_arrive(next_empty(k & 1));
+              }
+              if (more && !first_s(nx, r + 1, t)) { ok = false; break; }
             }
           }
           if (!ok) break;
@@ -335,7 +353,15 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
     int n = 0;                                // key tiles seen so far (phase of every barrier of this tile)
     bool ok = true;
-    for (int k = 0; ok && flash_ws_item(p, n_items, k, w); ++k) {
+    int item = blockIdx.x;
+    auto next_item = [&](int k) {
+      if (!mbar_wait_warp(next_full(k & 1), (k >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) return false;
+      item = clc_answer(answer(k & 1));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(next_empty(k & 1));
+      return true;
+    };
+    for (int k = 0; ok && flash_ws_item(p, item, w); ok = ok && next_item(k), ++k) {
     const int qi = w.q0 + t * W_BQ + r;
     const int n_mine = w.n_t[t];
     float m_used = 0.f, l = 0.f;
@@ -502,10 +528,10 @@ static int launch_flash_ws(const CUtensorMap& tq, const CUtensorMap& tk, const C
     MLF_CHECK_CUDA(cudaFuncSetAttribute(flash_fwd_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM));
     attr_set[dev & 63] = true;
   }
-  // one CTA per SM (shared memory and tensor memory hold no second one): each walks over items / SMs of them
+  // a CTA per item, of which one per SM starts (shared memory and tensor memory hold no second one) and takes over the others
   const long long items = (long long)((p.S + 2 * W_BQ - 1) / (2 * W_BQ)) * p.Hq * p.B;
-  const int sms = sm_count();
-  MLF_CHECK_CUDA(launch_pdl(flash_fwd_ws_kernel, dim3((unsigned)(items < sms ? items : sms)), dim3(W_THREADS), W_SMEM, st, tq, tk, tv, to, p));
+  MLF_REQUIRE(items < (1LL << 31), "flash_fwd: too many rows");
+  MLF_CHECK_CUDA(launch_pdl(flash_fwd_ws_kernel, dim3((unsigned)items), dim3(W_THREADS), W_SMEM, st, tq, tk, tv, to, p));
   count_launch();
   return 0;
 }

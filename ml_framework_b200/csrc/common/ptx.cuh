@@ -216,6 +216,31 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------
+// cluster launch control: a running CTA takes the place of one of its grid that has not started
+// ---------------------------------------------------------------------------------
+// Asks for such a CTA. The answer (16 bytes, 16-byte aligned) arrives in shared memory and completes 16 bytes of `bar`. A CTA
+// asks again only after an answer with which it got one, and does not end before its last answer has arrived.
+__device__ __forceinline__ void clc_try_cancel(uint32_t answer, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar) : "memory");
+}
+// blockIdx.x of the CTA that will not start, or -1 where none was left. The read is ordered before the next answer.
+__device__ __forceinline__ int clc_answer(uint32_t answer) {
+  uint32_t got, x = 0;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\t"
+      "ld.shared.b128 a, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, a;\n\t}"
+      : "=r"(got), "=r"(x)
+      : "r"(answer)
+      : "memory");
+  fence_proxy_async_smem();
+  return got ? (int)x : -1;
+}
+
+// ---------------------------------------------------------------------------------
 // tcgen05: TMEM management
 // ---------------------------------------------------------------------------------
 // One full warp calls these. ncols is a power of two in [32, 512].

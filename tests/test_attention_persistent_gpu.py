@@ -5,6 +5,7 @@ import torch
 
 from ml_framework_b200 import _lib
 from ml_framework_b200.ops import native
+from ml_framework_b200.ops.gemm import gemm
 
 pytestmark = pytest.mark.gpu
 D = 128
@@ -70,3 +71,33 @@ def test_nan_key_reaches_every_row_that_sees_it():
         out, _ = native.flash_fwd(q, kk, v, B, S, causal=True)
         bad = ~torch.isfinite(out.float()).all(-1)
         assert bad[pos:, 0].all() and not bad[:pos].any() and not bad[:, 1].any(), pos
+
+
+def test_beside_a_kernel_that_holds_sms():
+    """The items of CTAs that find no place beside another stream's kernel go to those that run: as many rounds as before, and
+    not twice as many because some CTAs start when the others have ended."""
+    B, S, H = 4, 2048, 16
+    q, k, v = _inputs(B, S, S, H, H)
+    a, o = torch.randn(8192, 8192, device="cuda").to(torch.bfloat16), torch.empty(8192, 8192, dtype=torch.bfloat16, device="cuda")
+    side, reps, outs = torch.cuda.Stream(), 8, []
+
+    def run(beside):
+        torch.cuda.synchronize()
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
+        if beside:
+            with torch.cuda.stream(side):
+                gemm(a, a, out=o, tile_n=128, max_ctas=8)            # 15 ms on eight SMs
+                e[2].record()
+            torch.cuda._sleep(1_000_000)                             # until it holds them
+        e[0].record()
+        outs[:] = [native.flash_fwd(q, k, v, B, S)[0] for _ in range(reps)]
+        e[1].record()
+        torch.cuda.synchronize()
+        assert not beside or e[1].elapsed_time(e[2]) > 0             # it held them to the end
+        return e[0].elapsed_time(e[1]) / reps, outs[0]
+
+    run(False)
+    alone, want = min((run(False) for _ in range(3)), key=lambda r: r[0])
+    beside, got = min((run(True) for _ in range(3)), key=lambda r: r[0])
+    # 140 of 148 SMs: 1.06 times the time, and the last round's items; CTAs that wait for a place cost 1.7 times
+    assert torch.equal(got, want) and beside <= 1.35 * alone, (alone, beside)
