@@ -1,8 +1,10 @@
 // Self-attention forward, head_dim 128: two 128-row query tiles per item, ping-ponged; a CTA goes from item to item.
 //
 // An item is 256 query rows of one (batch, head) as two tiles of 128. 384 threads in three warpgroups;
-// the control warpgroup hands most of its registers to the softmax warpgroups (setmaxnreg 72 / 216 / 216 of 3 x 168:
-// with 88 / 208 the softmax spills, and every spill sits on the chain below: 4 % of 4 x 2048, 16 heads):
+// the control warpgroup hands most of its registers to the softmax warpgroups (setmaxnreg 56 / 224 / 224 of 3 x 168). With fewer
+// the softmax's instructions come in a slower order or spill, on the chain below: 128 queries of 4096 keys, one query tile
+// alone, 53.4 us, 56.6 with 72 / 216; 4 x 2048, 16 heads 74.2, 75.0, and 4 % more with 88 / 208. So the MMA issuer gets by with few: no
+// state of a tile is addressed by a variable (it would be in local memory), one descriptor per operand, stepped by constants:
 //   warp 0        TMA producer: an item's Q tiles, its K and V tiles of 128 keys through 2-stage rings
 //   warp 1        MMA issuer (one thread). Per key tile j and query tile t:
 //                   S_t = Q_t K_j^T   (M128 N128 K128, operands in shared memory)  -> TMEM S_t
@@ -173,7 +175,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   FlashWsItem w;
 
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
     // ===================== TMA producer =====================
     if (elect_one()) {
@@ -259,33 +261,35 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const uint32_t idesc_s = make_idesc_bf16(128, W_BKV, 0, 0);
       const uint32_t idesc_pv = make_idesc_bf16(128, W_D, 0, 1);
       auto issue_s = [&](int t, int stage) {
-        const uint32_t q = sQ + t * W_TILE_BYTES, kk_base = sK + stage * W_TILE_BYTES;
-#pragma unroll 4
+        uint64_t q = make_smem_desc_sw128(sQ + t * W_TILE_BYTES, 16, 1024), kd = make_smem_desc_sw128(sK + stage * W_TILE_BYTES, 16, 1024);
+        asm volatile("" : "+l"(q), "+l"(kd));      // sixteen descriptors kept in registers ahead of time would spill
+#pragma unroll
         for (int kk = 0; kk < W_D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * (W_TILE_BYTES / 2) + (kk & 3) * 32;
-          umma_bf16_ss(tS(t), make_smem_desc_sw128(q + off, 16, 1024), make_smem_desc_sw128(kk_base + off, 16, 1024), idesc_s, kk != 0);
+          const uint32_t off = ((kk >> 2) * (W_TILE_BYTES / 2) + (kk & 3) * 32) >> 4;     // a descriptor counts 16 bytes
+          umma_bf16_ss(tS(t), q + off, kd + off, idesc_s, kk != 0);
         }
         umma_commit(s_full(t));
       };
       auto issue_pv = [&](int t, int stage, int half, bool first) {   // 64 keys: P's half, as soon as the softmax has published it
-        const uint32_t v = sV + stage * W_TILE_BYTES;
+        uint64_t v = make_smem_desc_sw128(sV + stage * W_TILE_BYTES, W_TILE_BYTES / 2, 1024);
+        asm volatile("" : "+l"(v));
 #pragma unroll
         for (int i = 0; i < W_BKV / 32; ++i) {
           const int kk = half * (W_BKV / 32) + i;
-          umma_bf16_ts(tO(t), tS(t) + 8u * kk, make_smem_desc_sw128(v + kk * 2048, W_TILE_BYTES / 2, 1024), idesc_pv, !first || kk != 0);
+          umma_bf16_ts(tO(t), tS(t) + 8u * kk, v + (kk * 2048 >> 4), idesc_pv, !first || kk != 0);
         }
       };
       int kt = 0;                               // ring position of this item's first key tile
-      int n_p[2] = {0, 0};                      // key tiles multiplied so far, per query tile
-      int n_q[2] = {0, 0};
+      uint32_t p_phase[2] = {0, 0};             // per query tile: parity of its key tiles multiplied so far
+      uint32_t q_phase[2] = {0, 0};
       bool ok = true;
       bool have = flash_ws_item(p, blockIdx.x, w);
       // S_t(0) of an item, its K and Q waited for; the last S of a tile gives its Q buffer back
       auto first_s = [&](const FlashWsItem& x, int ring, int t) -> bool {
         if (x.n_t[t] == 0) return true;
         if (!mbar_wait(k_full(ring & 1), (ring >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) return false;
-        if (!mbar_wait(q_full(t), n_q[t] & 1, abort_flag, p.err, ERR_WAIT_ATTN)) return false;
-        ++n_q[t];
+        if (!mbar_wait(q_full(t), q_phase[t], abort_flag, p.err, ERR_WAIT_ATTN)) return false;
+        q_phase[t] ^= 1;
         tc_fence_after_sync();
         issue_s(t, ring & 1);
         if (x.n_t[t] == 1) umma_commit(q_empty(t));
@@ -303,21 +307,22 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const uint32_t ph = (r >> 1) & 1;
           const bool last = j + 1 == w.n_kv;
           bool k_next_ready = false;
-          for (int t = 0; t < 2 && ok; ++t) {
+          // called with each tile's number, so that no state of a tile is addressed by a variable
+          auto tile = [&](const int t) -> bool {
             if (j < w.n_t[t]) {
-              if (!mbar_wait(v_full(s), ph, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
-              if (!mbar_wait(p_half(t), n_p[t] & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+              if (!mbar_wait(v_full(s), ph, abort_flag, p.err, ERR_WAIT_ATTN)) return false;
+              if (!mbar_wait(p_half(t), p_phase[t], abort_flag, p.err, ERR_WAIT_ATTN)) return false;
               tc_fence_after_sync();
               issue_pv(t, s, 0, j == 0);
-              if (!mbar_wait(p_full(t), n_p[t] & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+              if (!mbar_wait(p_full(t), p_phase[t], abort_flag, p.err, ERR_WAIT_ATTN)) return false;
               tc_fence_after_sync();
               issue_pv(t, s, 1, j == 0);
               umma_commit(pv_done(t));
-              ++n_p[t];
+              p_phase[t] ^= 1;
             }
             if (j + 1 < w.n_t[t]) {
               if (!k_next_ready) {
-                if (!mbar_wait(k_full((r + 1) & 1), ((r + 1) >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+                if (!mbar_wait(k_full((r + 1) & 1), ((r + 1) >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) return false;
                 k_next_ready = true;
                 tc_fence_after_sync();
               }
@@ -327,13 +332,15 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               // the next item's first S goes in behind this item's last products: its softmax warps find it ready when
               // they have written their rows
               if (t == 0) {
-                if (!mbar_wait(next_full(k & 1), (k >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) { ok = false; break; }
+                if (!mbar_wait(next_full(k & 1), (k >> 1) & 1, abort_flag, p.err, ERR_WAIT_ATTN)) return false;
                 more = flash_ws_item(p, clc_answer(answer(k & 1)), nx);
                 mbar_arrive(next_empty(k & 1));
               }
-              if (more && !first_s(nx, r + 1, t)) { ok = false; break; }
+              if (more && !first_s(nx, r + 1, t)) return false;
             }
-          }
+            return true;
+          };
+          ok = tile(0) && tile(1);
           if (!ok) break;
           umma_commit(v_empty(s));                               // V_j consumed by both tiles' PV
           if (!last || more) umma_commit(k_empty((r + 1) & 1));  // K_{j+1}, or the next item's K_0, consumed by both tiles' S
@@ -345,7 +352,7 @@ flash_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
     // ===================== softmax warpgroups =====================
     const int t = (warp - 4) >> 2;            // query tile of this warpgroup
     const int q = warp & 3;                   // TMEM lane quarter this warp may access
