@@ -435,73 +435,74 @@ __device__ __forceinline__ void store16(__nv_bfloat16* p, uint4 v) {
 // pos[T]) in place on the query and key heads, and the rotated keys plus the values written to their cache
 // slots (slot < 0 skips the write). Replaces two rotary launches and the cache write of a serving step.
 //
-// A warp owns one token and a run of its heads (blockIdx.y); four heads at a time, eight lanes each, a lane holding
-// elements 8 v .. 8 v + 7 and their partners 64 further. The token's 64 angles are computed once, two per lane, instead of
-// by every thread of every head, which with 8-byte accesses bound the kernel: 4096 tokens of 32 + 2 x 8 heads
-// 26.6 -> 22.6 us, 2048 of 40 + 2 x 40 34.8 -> 26.6 us (events around a single launch; 16.7 and 22.4 us at the copy rate).
-constexpr int RK_UNROLL = 3;                    // groups of four heads whose loads are in flight together
+// A warp owns one token and up to three groups of four of its heads (blockIdx.y): eight lanes a head, a lane holding
+// elements 8 v .. 8 v + 7 and their partners 64 further, all of them loaded ahead of the angles. The token's 64 angles are
+// computed once per warp, two per lane, instead of by every thread of every head, which with 8-byte accesses bound the kernel.
+// us, one launch behind the other, a thread for four elements of a head / now: 1 token of 32 + 2 x 8 heads 1.92 / 1.84, 128 2.6 / 2.7,
+// 1000 6.5 / 6.5, 4096 21.2 / 16.4; of 40 + 2 x 40 heads 128 4.0 / 3.5, 1000 14.8 / 10.5, 4096 56.6 / 47.1.
+constexpr int RK_GROUPS = 3;                    // groups of four heads of a warp: 6 KB of it in flight
+constexpr int RK_WARPS = 4;                     // tokens per CTA (with 8, 64 tokens of 32 + 2 x 8 heads 2.4 us, 2.2 here)
 template <bool V16>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(RK_WARPS * 32)
 rope_kv_write_kernel(__nv_bfloat16* qkv, long long ld, const long long* pos, const long long* slots, __nv_bfloat16* cache, long long T,
                      int Hq, int Hkv, int block_size, int num_blocks, int heads_per_warp, float theta, int* err) {
-  __shared__ __align__(16) float2 s_cs[8][PD / 2];   // read two at a time
+  __shared__ __align__(16) float2 s_cs[RK_WARPS][PD / 2];   // read two at a time
   pdl_trigger();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long t = (long long)blockIdx.x * 8 + warp;
+  const long long t = (long long)blockIdx.x * RK_WARPS + warp;
   if (t >= T) return;
   const int heads = Hq + 2 * Hkv;
   const int h0 = blockIdx.y * heads_per_warp, h1 = min(heads, h0 + heads_per_warp);
+  const int v = lane & 7, first = h0 + (lane >> 3);
+  __nv_bfloat16* row = qkv + t * ld + v * 8;
+  uint4 lo[RK_GROUPS], hi[RK_GROUPS];
+#pragma unroll
+  for (int u = 0; u < RK_GROUPS; ++u) {
+    const int h = first + 4 * u;
+    if (h < h1) {
+      lo[u] = load16<V16>(row + h * PD);
+      hi[u] = load16<V16>(row + h * PD + 64);
+    }
+  }
+  const long long slot = slots[t];
   const float log_theta = __logf(theta), at = (float)pos[t];
   if (h0 < Hq + Hkv) {                          // not for a run of value heads
     s_cs[warp][lane] = rope_cos_sin(at, log_theta, rope_exponent<PD>(lane));
     s_cs[warp][lane + 32] = rope_cos_sin(at, log_theta, rope_exponent<PD>(lane + 32));
   }
   __syncwarp();
-  const int v = lane & 7;
-  const long long slot = slots[t];
   __nv_bfloat16* dst = nullptr;                 // this token's key rows in the cache; its values lie block_size rows on
   if (slot >= 0 && h1 > Hq) {
-    const long long blk = slot / block_size;
+    // a division of 64 bits takes as long as the rest of the kernel
+    const long long blk = slot <= 0x7fffffff ? (long long)((unsigned)slot / (unsigned)block_size) : slot / block_size;
     if (blk >= num_blocks) atomicCAS(err, 0, ERR_BAD_INDEX);
-    else dst = cache + (blk * 2LL * block_size + slot % block_size) * Hkv * PD + v * 8;
+    else dst = cache + (blk * block_size + slot) * Hkv * PD + v * 8;      // a block is block_size rows of keys, then of values
   }
   const long long v_off = (long long)block_size * Hkv * PD;
-  __nv_bfloat16* row = qkv + t * ld + v * 8;
-  for (int hb = h0 + (lane >> 3); hb < h1; hb += 4 * RK_UNROLL) {
-    uint4 lo[RK_UNROLL], hi[RK_UNROLL];
 #pragma unroll
-    for (int u = 0; u < RK_UNROLL; ++u) {
-      const int h = hb + 4 * u;
-      if (h < h1) {
-        lo[u] = load16<V16>(row + h * PD);
-        hi[u] = load16<V16>(row + h * PD + 64);
+  for (int u = 0; u < RK_GROUPS; ++u) {
+    const int h = first + 4 * u;
+    if (h >= h1) break;
+    if (h < Hq + Hkv) {
+      uint32_t* a = reinterpret_cast<uint32_t*>(&lo[u]);
+      uint32_t* b = reinterpret_cast<uint32_t*>(&hi[u]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 cs = *reinterpret_cast<const float4*>(&s_cs[warp][v * 8 + 2 * j]);
+        float2 x = unpack_bf16x2(a[j]), y = unpack_bf16x2(b[j]);
+        rope_rotate(x.x, y.x, make_float2(cs.x, cs.y));
+        rope_rotate(x.y, y.y, make_float2(cs.z, cs.w));
+        a[j] = pack_bf16x2(x.x, x.y);
+        b[j] = pack_bf16x2(y.x, y.y);
       }
+      store16<V16>(row + h * PD, lo[u]);
+      store16<V16>(row + h * PD + 64, hi[u]);
     }
-#pragma unroll
-    for (int u = 0; u < RK_UNROLL; ++u) {
-      const int h = hb + 4 * u;
-      if (h >= h1) break;
-      if (h < Hq + Hkv) {
-        uint32_t* a = reinterpret_cast<uint32_t*>(&lo[u]);
-        uint32_t* b = reinterpret_cast<uint32_t*>(&hi[u]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 cs = *reinterpret_cast<const float4*>(&s_cs[warp][v * 8 + 2 * j]);
-          float2 x = unpack_bf16x2(a[j]), y = unpack_bf16x2(b[j]);
-          rope_rotate(x.x, y.x, make_float2(cs.x, cs.y));
-          rope_rotate(x.y, y.y, make_float2(cs.z, cs.w));
-          a[j] = pack_bf16x2(x.x, x.y);
-          b[j] = pack_bf16x2(y.x, y.y);
-        }
-        store16<V16>(row + h * PD, lo[u]);
-        store16<V16>(row + h * PD + 64, hi[u]);
-      }
-      if (h >= Hq && dst != nullptr) {
-        __nv_bfloat16* d = h < Hq + Hkv ? dst + (h - Hq) * PD : dst + v_off + (h - Hq - Hkv) * PD;
-        store16<V16>(d, lo[u]);
-        store16<V16>(d + 64, hi[u]);
-      }
+    if (h >= Hq && dst != nullptr) {
+      __nv_bfloat16* d = h < Hq + Hkv ? dst + (h - Hq) * PD : dst + v_off + (h - Hq - Hkv) * PD;
+      store16<V16>(d, lo[u]);
+      store16<V16>(d + 64, hi[u]);
     }
   }
 }
@@ -688,14 +689,15 @@ MLF_API int mlf_rope_kv_write(void* qkv, long long ld, const long long* pos, con
   if (T <= 0) return 0;
   MLF_REQUIRE(ld % 4 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 7) == 0, "rope_kv_write: rows must be 8-byte aligned");
   const bool v16 = ld % 8 == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cache)) & 15) == 0;
-  // few tokens: their heads are split over more warps, down to four heads a warp, until every SM has 16 of them
-  const int groups = (Hq + 2 * Hkv + 3) / 4;
-  long long parts = (16LL * sm_count() + T - 1) / T;
-  if (parts > groups) parts = groups;
-  const int heads_per_warp = (int)((groups + parts - 1) / parts) * 4;
-  const dim3 grid((unsigned)((T + 7) / 8), (unsigned)((Hq + 2 * Hkv + heads_per_warp - 1) / heads_per_warp));
+  // As many groups of heads to a warp as leave every SM 27 warps. us with 1 / 2 / 3 groups of 32 + 2 x 8 heads (12 a token): 256 tokens
+  // 3.4 / 4.0 / 4.5, 512 4.8 / 4.8 / 5.6, 1000 6.6 / 6.3 / 6.2, 4096 20.8 / 17.4 / 16.9; of 40 + 2 x 40 (30): 128 3.6 / 4.6 / 4.7,
+  // 256 4.7 / 5.0 / 6.0, 512 7.8 / 6.6 / 6.8, 1000 13.2 / 11.1 / 10.6; of 16 + 2 x 4 (6): 1000 4.6 / 4.5 / 5.5, 1500 5.1 / 4.6 / 5.8,
+  // 2048 6.7 / 6.3 / 6.1. (More, which take several rounds, are at most 3 % faster, from 4096 tokens on.)
+  const long long groups = (Hq + 2 * Hkv + 3) / 4, fill = T * groups / (27LL * sm_count());
+  const int heads_per_warp = 4 * (int)(fill < 1 ? 1 : fill > RK_GROUPS ? RK_GROUPS : fill);
+  const dim3 grid((unsigned)((T + RK_WARPS - 1) / RK_WARPS), (unsigned)((Hq + 2 * Hkv + heads_per_warp - 1) / heads_per_warp));
   const auto kernel = v16 ? rope_kv_write_kernel<true> : rope_kv_write_kernel<false>;
-  MLF_CHECK_CUDA(launch_pdl(kernel, grid, dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), ld, pos, slots,
+  MLF_CHECK_CUDA(launch_pdl(kernel, grid, dim3(RK_WARPS * 32), 0, reinterpret_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), ld, pos, slots,
                             static_cast<__nv_bfloat16*>(cache), T, Hq, Hkv, block_size, num_blocks, heads_per_warp, theta, device_status_word()));
   count_launch();
   return 0;
