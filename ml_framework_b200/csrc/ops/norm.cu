@@ -307,7 +307,7 @@ norm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma, const __
 // f = (f - mean) * rstd. x * rstd - mean * rstd would be one operation an element but rounds mean * rstd: rows of 1000 +- 4 come
 // out up to 7.6e-6 off, 1.2e-7 here. Two elements an instruction, so that it costs the same (us, warm, that form / this one / this
 // one element by element: 8192 x 1536 24.1 / 23.9 / 24.8, 8192 x 2048 29.2 / 29.3 / 30.5, 8192 x 3072 41.7 / 41.5 / 42.9,
-// 8192 x 6144 155 / 159 / 166, 8192 x 8192 190 / 192 / 202).
+// and with a thread per vector 8192 x 6144 155 / 159 / 166, 8192 x 8192 190 / 192 / 202).
 template <bool RMS>
 __device__ __forceinline__ void normalise8(float (&f)[8], float mean, float rstd) {
   const uint64_t m2 = pack_f32x2(-mean, -mean), r2 = pack_f32x2(rstd, rstd);
@@ -319,12 +319,13 @@ __device__ __forceinline__ void normalise8(float (&f)[8], float mean, float rstd
 }
 
 // Backward. D = 256, 512, 1024, 2048 and 4096: 2048 columns' worth of rows side by side (GROUPS rows of D = 2048 / GROUPS, or a
-// row of D = NVT * 2048), a CTA of 256 threads; other widths: a row to a CTA of as many threads as it has vectors (or every
-// NVT-th). Every thread has a fixed set of 8 * NVT columns, so that gamma and the gamma / beta gradient partials sit in registers. R rows of x, dy and the skip gradient are summed and written while the next
-// R are in flight. The two row sums meet across the warps of a row through a double-buffered shared array: one barrier per R
-// rows.
+// row of D = NVT * 2048), a CTA of 256 threads; other widths: a row to a CTA of as many threads as it has vectors, or half as many
+// above 4096. Every thread has a fixed set of 8 * NVT columns, so that gamma and the gamma / beta gradient partials sit in registers.
+// R rows of x, dy and the skip gradient are summed and written while the next R are in flight. The two row sums meet across the
+// warps of a row through a double-buffered shared array: one barrier per R rows.
 // us, before (one warp per row; for 2048 and 4096 no rows in flight ahead) -> now: 8192 x 4096 RMS 69 -> 56 (floor 41), 2331 x 1024
-// 21.5 -> 15.4, 2331 x 3072 73 -> 21.5, 8192 x 5120 RMS 386 -> 79, 8192 x 8192 layer / RMS norm 1232 / 1082 -> 206 / 99 (82).
+// 21.5 -> 15.4, 2331 x 3072 73 -> 21.5; one launch behind the other 8192 x 5120 layer / RMS norm 497 / 344 -> 121 / 62, 8192 x 8192
+// 1136 / 992 -> 154 / 78 (a thread per vector, whose 64 registers spill: 190 / 83).
 template <int NVT, int R, int GROUPS, bool RMS, int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
 norm_bwd_cta_kernel(const __nv_bfloat16* x, const __nv_bfloat16* dy,
@@ -649,7 +650,7 @@ MLF_API int mlf_norm_bwd_add(const void* x, const void* dy, const void* gamma, c
     case 2048: LAUNCH(1, 2, 1, 256, 256)
     case 4096: LAUNCH(2, 1, 1, 256, 256)
     case 768: case 1536: case 3072: LAUNCH(1, 2, 1, 384, D / 8)
-    case 5120: case 6144: case 8192: LAUNCH(1, 1, 1, 1024, D / 8)
+    case 5120: case 6144: case 8192: LAUNCH(2, 1, 1, 512, D / 16)
     default: MLF_REQUIRE(false, "norm: unsupported D=%d", D);
   }
 #undef LAUNCH
