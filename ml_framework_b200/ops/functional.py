@@ -212,24 +212,26 @@ def mlp_swiglu(x, w_gu, w_down, residual=None):
 # ------------------------------------------------------------------------------------------
 def _norm_grads(ctx, x, dy, gamma, mean, rstd, dx_add=None):
     """dx, and the gradients of gamma and beta that go to autograd (None for one that went into its buffer). The kernel writes
-    both in one type: a buffer of another gets its gradient from a tensor in between."""
-    refs = (ctx.gamma_ref, None if ctx.rms else ctx.beta_ref)
-    sinks = [_sink(p) for p in refs]
-    dtype = torch.float32 if any(t is not None and t.dtype != gamma.dtype for t, _ in sinks) else gamma.dtype
-    out = [t if t is not None and t.dtype == dtype else None if p is None else torch.empty(p.shape, dtype=dtype, device=x.device)
-           for p, (t, _) in zip(refs, sinks)]
-    direct = [o is t for o, (t, _) in zip(out, sinks)]
-    dx, *grads = native.norm_bwd(x, dy, gamma, None if ctx.rms else mean, rstd, ctx.rms, dgamma_out=out[0], dbeta_out=out[1],
-                                 accumulate=direct[0] and sinks[0][1], accumulate_beta=direct[1] and sinks[1][1], dx_add=dx_add)
-    for i, (p, (t, acc)) in enumerate(zip(refs, sinks)):
-        if t is not None:
-            if not direct[i]:
-                t.copy_(t + grads[i] if acc else grads[i])
-            _done(p)
-            grads[i] = None
-        else:
-            grads[i] = None if p is None else grads[i].to(p.dtype)
-    return dx, *grads
+    both in one type: beta's buffer of another gets its gradient from a tensor in between."""
+    rms = ctx.rms
+    gt, gacc = _sink(ctx.gamma_ref)
+    bt, bacc = (None, False) if rms else _sink(ctx.beta_ref)
+    apart = gt is not None and bt is not None and gt.dtype != bt.dtype
+    dx, dg, db = native.norm_bwd(x, dy, gamma, None if rms else mean, rstd, rms, dgamma_out=gt, dbeta_out=None if apart else bt,
+                                 accumulate=gacc, dx_add=dx_add, accumulate_beta=bacc and not apart)
+    if gt is not None:
+        _done(ctx.gamma_ref)
+        dg = None
+    elif dg.dtype != gamma.dtype:
+        dg = dg.to(gamma.dtype)
+    if bt is not None:
+        if apart:
+            bt.copy_(bt + db if bacc else db)
+        _done(ctx.beta_ref)
+        db = None
+    elif not rms and db.dtype != gamma.dtype:
+        db = db.to(gamma.dtype)
+    return dx, dg, db
 
 
 class _NormFn(torch.autograd.Function):
