@@ -1,5 +1,6 @@
-"""Kernels that may start before the ones ahead of them have ended: nothing that those may write is read through the
-non-coherent path, which const __restrict__ parameters and __ldg ask for."""
+"""Read off the kernels' sources. Kernels that may start before the ones ahead of them have ended wait for those, and nothing that
+those may write is read through the non-coherent path, which const __restrict__ parameters and __ldg ask for; shared arrays
+are aligned for their accesses."""
 import re
 from pathlib import Path
 
@@ -35,11 +36,34 @@ def test_no_non_coherent_reads_under_overlap():
     assert seen >= 12
 
 
+def _given(text, name):
+    """What a variable, an array or an array of function pointers of that name is given: (where, what)."""
+    return [(m.start(), m.group(1)) for m in re.finditer(r"\b" + name + r"(?:\[[^\]]*\])*(?:\)\([^)]*\))?\s*=(?!=)([^;]*);", text)]
+
+
+def _launched(text, name, kernels):
+    """Kernels that `name` stands for at the end of this text."""
+    if name in kernels:
+        return {name}
+    given = _given(text, name)
+    if not given:
+        return set()
+    at, what = given[-1]
+    return set().union(*(_launched(text[:at], word, kernels) for word in set(re.findall(r"[A-Za-z_]\w*", what)) - {name}))
+
+
 def test_every_overlapped_launch_waits():
-    text = "\n".join(re.sub(r"//[^\n]*", "", p.read_text()) for p in CSRC.rglob("*.cu"))
-    launched = set(re.findall(r"launch_pdl\(\s*(\w+)", text)) - {"kernel"}
     waits = {name for name, _, body in _kernels() if "pdl_wait()" in body}
-    assert launched and launched <= waits
+    kernels = {name for name, _, _ in _kernels()}
+    launched = set()
+    for path in CSRC.rglob("*.cu"):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"launch_pdl\(\s*(\w+)", text):
+            found = _launched(text[:m.start()], m.group(1), kernels)
+            assert found, (path.name, m.group(1))
+            launched |= found
+    assert {"norm_bwd_cta_kernel", "norm_fwd_row_kernel", "rope_kv_write_kernel", "paged_decode_kernel", "flash_fwd_ws_kernel"} <= launched
+    assert launched <= waits
 
 
 def test_shared_arrays_are_aligned_for_their_widest_access():
