@@ -39,22 +39,3 @@ def test_matches_separate_steps(T, Hq, Hkv, pad, offset):
     rest[offset:offset + T * (W + pad)].view(T, W + pad)[:, :W] = False
     assert torch.equal(buf[rest], before[rest])
     assert _lib.read_status() == 0
-
-
-@pytest.mark.parametrize("D,rms", [(2048, False), (2048, True), (4096, False), (4096, True)])
-@pytest.mark.parametrize("rows", [1, 295, 296, 297, 591, 592, 593, 1183, 1185, 2371])
-def test_norm_rows_per_cta(D, rms, rows):
-    """Whole-CTA rows around one, two and several groups of rows per CTA (148 SMs: 296 CTAs), the buffer cleared beside."""
-    torch.manual_seed(rows)
-    x = torch.randn(rows, D, device="cuda").to(torch.bfloat16) + 0.5
-    g, b = (torch.randn(D, device="cuda").to(torch.bfloat16) for _ in range(2))
-    zero = torch.full((rows, 64), 5.0, dtype=torch.bfloat16, device="cuda")
-    y, mean, rstd = native.norm_fwd(x, g, None if rms else b, 1e-5, rms, zero=zero)
-    xd = x.double()
-    mu = torch.zeros(rows, 1, dtype=torch.float64, device="cuda") if rms else xd.mean(-1, keepdim=True)
-    r = ((xd - mu).square().mean(-1, keepdim=True) + 1e-5).rsqrt()
-    want = (xd - mu) * r * g.double() + (0 if rms else b.double())
-    assert ((rstd.double() - r[:, 0]) / r[:, 0]).abs().max() < 1e-5          # fp32 sums of 4096 squares
-    assert rms or (mean.double() - mu[:, 0]).abs().max() < 1e-5
-    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()      # one rounding to bf16
-    assert (zero == 0).all() and _lib.read_status() == 0
