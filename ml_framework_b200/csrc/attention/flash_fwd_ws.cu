@@ -32,8 +32,8 @@
 // The grid has a CTA per item, the longest first; a CTA that nears its end has the launch control cancel one that has not
 // started and does that one's item. Rounds of fixed shares (a CTA per SM) left the shares of CTAs that found no place beside
 // another stream's kernel until the others had ended. us back to back, a CTA that ends with its item / fixed shares / now: 4 x 2048,
-// 16 heads 97 / 82 / 79, with 1 SM held by another kernel 99 / 141 / 82, with 8 101 / 142 / 85; 8 x 512, 32 / 8 heads
-// 54 / 41 / 39, 55 / 60 / 40, 57 / 61 / 41; 2 x 4096, 32 / 8 heads 278 / 258 / 246, 288 / 464 / 258, 303 / 466 / 269.
+// 16 heads 98 / 85 / 78, with 1 SM held by another kernel 100 / 142 / 81, with 8 102 / 143 / 83; 8 x 512, 32 / 8 heads
+// 54 / 41 / 38, 55 / 60 / 39, 57 / 61 / 40; 2 x 4096, 32 / 8 heads 284 / 264 / 245, 292 / 471 / 255, 307 / 474 / 263.
 // Per SM and key tile: 4 x 128x128x128 of tensor work against 2 x 16384 exponentials.
 //
 // Math reference: StandardPagedAttentionKernel.ComputePagedAttention

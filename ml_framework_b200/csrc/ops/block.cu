@@ -1,6 +1,8 @@
 // One transformer block, forward and backward, as the sequence of launches that its operators make one by one: a training
 // step of a small model is bound by the host, which spends several times longer per operator on Python than on its launches.
-// Same kernels, same arguments and order as ml_framework_b200/ops/functional.py, so the results are the same.
+// The forward makes the launches of ml_framework_b200/ops/functional.py, in their order. The backward's are the same products,
+// attention and normalisation kernels with the same arguments; the bias gradients of two products share a launch, behind both
+// products' weight gradients, and have the row split of that launch.
 //
 //   forward   h1 = norm(x); qkv = h1 Wqkv^T (+ b); [rotary embedding in place]; a = attention(qkv); x1 = x + a Wo^T (+ b);
 //             h2 = norm(x1); act = f(h2 W1^T (+ b)), pre = its argument; y = x1 + act W2^T (+ b)

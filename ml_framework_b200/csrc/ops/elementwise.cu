@@ -399,8 +399,8 @@ __global__ void __launch_bounds__(256) embedding_bwd_kernel(float* dw, const __n
 // tokens stays, and its row of dout becomes row t of `rows` in fp32; (2) tokens that are not their id's owner add their rows to
 // the owner's; (3) owners' rows go to dw. Owners need no clearing: an entry counts only if it names a token with that very id.
 // Bound by the bytes of the tokens' rows (in L2 for most sizes) and of dw where it is written. us, cold, as a cleared fp32 table,
-// its sums and their rounding -> like this: 2331 ids of 50304 x 1024 added 113.5 -> 17.3, 8192 of 50304 x 2048 added 230 -> 52,
-// 8192 of 32000 x 4096 written 278 -> 130, 512 of 2048 x 256 written 15.3 -> 11.3.
+// its sums and their rounding -> like this: 2331 ids of 50304 x 1024 added 113 -> 17.4, 8192 of 50304 x 2048 added 230 -> 48,
+// 8192 of 32000 x 4096 written 278 -> 126, 512 of 2048 x 256 written 13.3 -> 11.3.
 __global__ void __launch_bounds__(256) embedding_grad_init_kernel(float* rows, int* owner, const __nv_bfloat16* dout, const long long* ids,
                                                                   long long T, int D, int vocab) {
   const int vec_per_row = D / 8;

@@ -1,11 +1,11 @@
 """A whole transformer block of the GPT or Llama kind as one autograd node whose forward and backward are one native call
-each (``csrc/ops/block.cu``): the same kernels in the same order as the operators of :mod:`.functional`, without their host
-work. A step of a small model is bound by that work.
+each (``csrc/ops/block.cu``): the launches of the operators of :mod:`.functional`, but for the bias gradients, two of which
+share a launch, without their host work. A step of a small model is bound by that work.
 
-It serves blocks that are exactly what the models build: bf16 on the GPU, plain layers, every parameter trained, no hooks on
-the layers inside. Whatever differs runs operator by operator as before. It is off unless the caller asks for it
-(:func:`whole_blocks`), which the training engine does where nothing works on single operators of a block, that is without
-data-parallel sharding or reduction.
+It serves blocks that are exactly what the models build: bf16 on the GPU, plain layers, every parameter trained and used once,
+no hooks on the layers inside. Whatever differs runs operator by operator. It is off unless the caller asks for it
+(:func:`whole_blocks`), which the training engine does for forward and backward (blocks may be recomputed there) where nothing
+works on single operators of a block, that is without data-parallel sharding or reduction.
 """
 from __future__ import annotations
 

@@ -400,8 +400,9 @@ class _EmbeddingFn(torch.autograd.Function):
                 return None
             tgt, accum = _sink(w)
             out = torch.empty(w.shape, dtype=w.dtype, device=dout.device) if tgt is None else tgt.view(w.shape)
-            # Fewer tokens than rows: a sum per token, in less memory than a table of them. Beyond that the fp32 table is the smaller:
-            # 2331 ids of 2048 x 1024 19.4 us in a table, 17.4 per token, 8192 of 2048 x 2048 40 and 48 us.
+            # Fewer tokens than rows: a sum per token; as many or more: an fp32 table of the rows, which is then the smaller of the
+            # two. The line is where their memory meets, not their times: 2331 ids of 2048 x 1024 take 19.4 us in a table and
+            # 17.4 per token, 8192 of 2048 x 2048 40 and 49 us.
             if out.dtype == dout.dtype == torch.bfloat16 and idx.numel() < w.shape[0] and out.data_ptr() % 16 == 0:
                 native.embedding_grad(dout, idx, out, accum)
             else:

@@ -403,7 +403,8 @@ def _decode_split(pairs: int, max_seq_len: int, sms: int) -> int:
     """Tokens per split of the decode kernel for ``pairs`` (sequence, KV head) pairs on ``sms`` SMs, three CTAs of it on
     each. As many splits as keep all CTAs resident at once, none when the pairs alone fill the GPU: CTAs of a second round
     start when the short sequences of the first end, and a split costs its start and the merge launch. At least 128 tokens
-    per split. us at the longest of 8 KV heads' sequences, lengths from half of it on: 13 x 2500 4 splits 26 (8: 29);
+    per split. (A captured decode step has one split for all lengths of its bucket, whose end is its ``max_seq_len``: 13 x 2500
+    run as 16 x 4096, in 3 splits.) us at the longest of 8 KV heads' sequences, lengths from half of it on: 13 x 2500 4 splits 26 (8: 29);
     48 x 1024 none 35 (3: 45); 8 x 4000 6 splits 28 (11: 34).
 
     A split of more than 1400 tokens takes long enough for its CTA to be alone at the end, above all when one sequence is

@@ -350,8 +350,10 @@ class PagedLlamaExecutor:
     def _prefill_key(self, B: int, n: int) -> Optional[str]:
         """Name of the graph that prefills ``B`` whole prompts of ``n`` tokens, or None where prompts run launch by launch:
         above 512 rows the GPU is busy for longer than the host takes to launch, and beyond 32 graphs further shapes are not
-        worth the memory of another one. Six layers of the Llama-8B shape, one prompt of 37 tokens: 941 us launch by launch,
-        715 us from the graph."""
+        worth the memory of another one. A bucket's first ``graph_warmup_steps`` passes run launch by launch; the pass after them
+        captures its graph and takes several times as long, so that the gain is one of traffic whose lengths come back. Six
+        layers of the Llama-8B shape, one prompt of 37 / 100 / 250 / 400 tokens: 0.95 / 0.95 / 1.13 / 1.68 ms launch by launch,
+        0.74 / 0.82 / 0.99 / 1.57 from the graph, 5 - 8 ms in the pass that captures it (33 in a process's first)."""
         if self._graphs is None or (self.tp is not None and self.tp.world > 1) or not 0 < n <= self.cfg.prefill_chunk:
             return None
         Tp = self._prompt_bucket(n)
@@ -368,7 +370,8 @@ class PagedLlamaExecutor:
     @torch.no_grad()
     def _prefill_graph(self, name: str, reqs: List[Request], n: int) -> Dict[int, int]:
         """Whole prompts of equal length, padded to a bucket of rows so that a handful of captured graphs covers them. The
-        rows behind a prompt are later positions, which no real row attends to, and their slot is -1: nothing is written."""
+        rows behind a prompt are later positions, which no real row attends to, and their slot is -1: nothing is written. The
+        padded row count may take another product kernel or split of K than the prompt's own: sums in another order."""
         B, Tp = len(reqs), self._prompt_bucket(n)
         T = B * Tp
         host = self._host_rows(1, 3 * T + B)[0]

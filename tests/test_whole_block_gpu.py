@@ -1,6 +1,6 @@
-"""A transformer block as one native call each way against the same block operator by operator: same kernels in the same
-order, so the outputs are equal bit for bit; gradients agree to within what the attention backward's order of fp32 additions
-leaves (a last bit of bf16 here and there)."""
+"""A transformer block as one native call each way against the same block operator by operator: the forward makes the same
+launches, so the outputs are equal bit for bit; gradients agree to within what the order of fp32 additions in the attention
+backward and in the bias gradients leaves (a last bit of bf16 here and there)."""
 import copy
 
 import pytest
